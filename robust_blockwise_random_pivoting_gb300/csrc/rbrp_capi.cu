@@ -369,6 +369,18 @@ rbrp_status cuda_check(rbrp_handle h, cudaError_t e, const char* what) {
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// cudaMalloc for what a run cannot do without: the slices, which it can, make room if needed.
+static rbrp_status device_alloc(rbrp_handle h, void** ptr, size_t bytes, const char* what) {
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && h->sl_ws) {
+    cudaGetLastError();
+    cudaStreamSynchronize(h->stream);
+    release_slices(h);
+    e = cudaMalloc(ptr, bytes);
+  }
+  return cuda_check(h, e, what);
+}
+
 rbrp_status ensure_workspace(rbrp_handle h, const Layout& L) {
   const size_t m = L.m, n = L.n, kmax = L.kmax, el = L.elem;
   const size_t M2 = (size_t)MAXB * MAXB;
@@ -421,7 +433,7 @@ rbrp_status ensure_workspace(rbrp_handle h, const Layout& L) {
     if (h->ws) cudaFree(h->ws);
     h->ws = nullptr;
     h->ws_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&h->ws, total), "workspace cudaMalloc");
+    rbrp_status s = device_alloc(h, &h->ws, total, "workspace cudaMalloc");
     if (s != RBRP_OK) return s;
     h->ws_bytes = total;
   }
@@ -468,13 +480,73 @@ rbrp_status make_tmap_f32(rbrp_handle h, void* map, const float* base, uint64_t 
   return RBRP_OK;
 }
 
+rbrp_status make_tmap_bf16(rbrp_handle h, void* map, const unsigned short* base, uint64_t inner, uint64_t outer,
+                           uint32_t box_outer) {
+  auto fn = tmap_encoder();
+  if (!fn) return set_error(h, RBRP_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
+  cuuint64_t dims[2] = {inner, outer};
+  cuuint64_t strides[1] = {inner * sizeof(unsigned short)};
+  cuuint32_t box[2] = {64, box_outer};
+  cuuint32_t es[2] = {1, 1};
+  CUresult r = fn(static_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                  const_cast<unsigned short*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(h, RBRP_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  return RBRP_OK;
+}
+
+void release_slices(rbrp_handle h) {
+  if (h->sl_ws) cudaFree(h->sl_ws);
+  h->sl_ws = nullptr;
+  h->sl_bytes = 0;
+}
+
+bool ensure_slices(rbrp_handle h, int m, int n) {
+  const size_t ldk = ((size_t)m + 63) / 64 * 64;
+  // row ranges of the projection: enough CTAs for four waves at the most, 16 ranges at the most
+  const int ctiles = (n + 127) / 128;
+  const int maxsplit = std::max(1, std::min(16, 608 / ctiles));
+  struct Item {
+    void** ptr;
+    size_t bytes;
+  } items[] = {
+      {(void**)&h->slA, 7 * ldk * (size_t)n * 2},
+      {(void**)&h->slQ, 7 * ldk * MAXB * 2},
+      {(void**)&h->sl_exA, (size_t)n * 4},
+      {(void**)&h->sl_exQ, MAXB * 4},
+      {(void**)&h->sl_Wpart, (size_t)maxsplit * MAXB * n * 8},
+  };
+  size_t total = 0;
+  for (auto& it : items) total += align_up(it.bytes);
+  if (total > h->sl_bytes) {
+    release_slices(h);
+    size_t avail = 0, all = 0;
+    if (cudaMemGetInfo(&avail, &all) != cudaSuccess || total > avail / 2 ||
+        cudaMalloc(&h->sl_ws, total) != cudaSuccess) {
+      cudaGetLastError();
+      h->sl_ws = nullptr;
+      return false;
+    }
+    h->sl_bytes = total;
+  }
+  char* base = static_cast<char*>(h->sl_ws);
+  size_t off = 0;
+  for (auto& it : items) {
+    *it.ptr = base + off;
+    off += align_up(it.bytes);
+  }
+  h->sl_maxsplit = maxsplit;
+  return true;
+}
+
 rbrp_status solve_T(rbrp_handle h, int k, int n) {
   const size_t bytes = (size_t)k * (size_t)(n - k) * sizeof(double);
   if (bytes > h->T_bytes) {
     if (h->T) cudaFree(h->T);
     h->T = nullptr;
     h->T_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc((void**)&h->T, bytes), "cudaMalloc(T)");
+    rbrp_status s = device_alloc(h, (void**)&h->T, bytes, "cudaMalloc(T)");
     if (s != RBRP_OK) return s;
     h->T_bytes = bytes;
   }
@@ -494,7 +566,7 @@ rbrp_status solve_T(rbrp_handle h, int k, int n) {
       if (h->df_buf) cudaFree(h->df_buf);
       h->df_buf = nullptr;
       h->df_bytes = 0;
-      s = cuda_check(h, cudaMalloc(&h->df_buf, need), "cudaMalloc(T solve operands)");
+      s = device_alloc(h, &h->df_buf, need, "cudaMalloc(T solve operands)");
       if (s != RBRP_OK) return s;
       h->df_bytes = need;
     }
@@ -777,6 +849,7 @@ rbrp_status rbrp_destroy(rbrp_handle h) {
     DeviceGuard g(h->device);
     if (h->ws) cudaFree(h->ws);
     if (h->T) cudaFree(h->T);
+    release_slices(h);
     if (h->df_buf) cudaFree(h->df_buf);
     if (h->hostA_dev) cudaFree(h->hostA_dev);
     if (h->given_order) cudaFree(h->given_order);

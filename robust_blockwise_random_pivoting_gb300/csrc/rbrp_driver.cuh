@@ -12,6 +12,7 @@
 #include "rbrp_internal.h"
 #include "rbrp_kernels.cuh"
 #include "rbrp_panel_df.cuh"
+#include "rbrp_slices.cuh"
 #include "rbrp_tc.cuh"
 #include "rbrp_update_tc.cuh"
 
@@ -72,6 +73,22 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
     cudaMemsetAsync(h->Qh, 0, (size_t)L.ld_res * MAXB * sizeof(float), st);
     cudaMemsetAsync(h->Ql, 0, (size_t)L.ld_res * MAXB * sizeof(float), st);
   }
+  // FP64 form: the projection as exact BF16 slices on the tensor cores, 9 to 25 times the
+  // FP64 pipe's rate for b of 30 to 64 (rbrp_slices.cuh).  Blocks of b <= 8 keep the column
+  // streams: they read 8 bytes per entry of A where the slices are 14, and use one in four or
+  // fewer of the MMA's columns.  So do variant 1 and matrices whose slices would not fit.
+  const bool use_sl = !RES && h->variant == 0 && p.b > 8 && ensure_slices(h, m, n);
+  const int64_t ldk = ((int64_t)m + tc::SL_BK - 1) / tc::SL_BK * tc::SL_BK;
+  CUtensorMap tmSA, tmSQ;
+  if (use_sl) {
+    s = make_tmap_bf16(h, &tmSA, h->slA, ldk, (uint64_t)tc::SL * n, tc::BM);
+    if (s == RBRP_OK) s = make_tmap_bf16(h, &tmSQ, h->slQ, ldk, tc::SL * MAXB, tc::SL * tc::SL_HALF);
+    if (s == RBRP_OK)
+      s = cuda_check(h, cudaFuncSetAttribute(tc::k_gemm_slices<tc::ProjEpi>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SL_SMEM),
+                     "cudaFuncSetAttribute(k_gemm_slices)");
+    if (s != RBRP_OK) return s;
+  }
   T* Q = static_cast<T*>(h->Q);
   T* Cpart = static_cast<T*>(h->Cpart);
   T* C = static_cast<T*>(h->C);
@@ -92,7 +109,11 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
                       n, cudaMemcpyDeviceToDevice, st);
   k_colnorm<T><<<(n + 7) / 8, 256, 0, st>>>(dA, lda, m, n, h->diags, h->perm, h->st);
   k_init<<<1, 1024, 0, st>>>(h->st, h->diags, n, kmax);
-  prof_end(h, RBRP_PHASE_NORMS, ev, (RES ? 3.0 : 1.0) * dm * n * es + 16.0 * n, 2.0 * dm * n, RES ? 3 : 2);
+  if constexpr (!RES)
+    if (use_sl)
+      tc::k_slice_cols<<<(n + 7) / 8, 256, 0, st>>>(dA, lda, m, n, n, ldk, h->slA, h->sl_exA);
+  prof_end(h, RBRP_PHASE_NORMS, ev, ((RES ? 3.0 : 1.0) * es + (use_sl ? 22.0 : 0.0)) * dm * n + 16.0 * n, 2.0 * dm * n,
+           RES || use_sl ? 3 : 2);
   cudaMemcpyAsync(h->hst, h->st, sizeof(State), cudaMemcpyDeviceToHost, st);
   s = cuda_check(h, cudaStreamSynchronize(st), "initial column norms");
   if (s != RBRP_OK) return s;
@@ -154,7 +175,14 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
     if (RES)
       k_swap_cols<<<dim3((m + 1023) / 1024, MAXB), 256, 0, st>>>(h->Ares, L.ld_res, h->st, m, h->K1, h->K2);
     if (!RES) k_panel2<T><<<ntiles, 256, panel_smem, st>>>(h->Q1, m, h->st, h->R2, Q, m, 1);
-    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 5 : 4) : (i > 0 ? 6 : 5));
+    if constexpr (!RES) {
+      if (use_sl) {
+        tc::k_slice_q<<<p.b > tc::SL_HALF ? MAXB : tc::SL_HALF, 256, 0, st>>>(Q, m, m, h->st, ldk, h->slQ,
+                                                                              h->sl_exQ);
+        tc::k_swap_slices<<<dim3(p.b, tc::SL), 256, 0, st>>>(h->slA, n, ldk, h->sl_exA, h->st, h->K1, h->K2);
+      }
+    }
+    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 5 : 4) : (i > 0 ? 6 : 5) + (use_sl ? 2 : 0));
     int nproj;
     ev = prof_begin(h);
     if (RES) {
@@ -238,6 +266,30 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       nproj = (n - i + 255) / 256;
       k_norm_reduce<<<nproj, 256, 0, st>>>(h->part_norm, nsplit, n, h->st, h->diags, h->part_res, h->part_nnz);
       prof_end(h, RBRP_PHASE_UPDATE, ev, 0.0, 0.0, use_tc ? 3 : 2);
+    } else if (use_sl) {
+      // row ranges by the wave rule, one CTA per SM; the fixed cost of a CTA (tensor memory,
+      // pipeline fill, the last drain) is about two stages
+      const int ctiles = (n - i + tc::BM - 1) / tc::BM;
+      const int nst = (int)(ldk / tc::SL_BK);
+      int sps = nst, nsplit = 1;
+      long best = -1;
+      for (int w = 1; w <= std::min(h->sl_maxsplit, nst); ++w) {
+        const int s_w = (nst + w - 1) / w, ws = (nst + s_w - 1) / s_w;
+        const long waves = ((long)ctiles * ws + h->sms - 1) / h->sms;
+        const long cost = waves * (s_w + 2);
+        if (best < 0 || cost < best) {
+          best = cost;
+          nsplit = ws;
+          sps = s_w;
+        }
+      }
+      tc::k_gemm_slices<<<dim3(ctiles, nsplit), tc::SL_THREADS, tc::SL_SMEM, st>>>(
+          tmSA, tmSQ, (int64_t)n, h->wait_budget > 0 ? h->wait_budget : kWaitBudgetDefault,
+          tc::ProjEpi{h->st, n, nst, sps, h->sl_exA, h->sl_exQ, h->sl_Wpart});
+      nproj = (n - i + 31) / 32;
+      tc::k_proj_finish<<<nproj, 256, 0, st>>>(h->st, h->sl_Wpart, nsplit, n, h->R, n, h->diags, h->part_res,
+                                               h->part_nnz);
+      prof_end(h, RBRP_PHASE_PROJECT, ev, 0.0, 0.0, 2);
     } else {
       // basis tile height: the smallest KB >= b (kept <= b); b <= 8 takes the column-streaming form
       auto project = [&](auto kb) {

@@ -68,6 +68,16 @@ struct rbrp_handle_st {
   float* Qrl = nullptr;
   float* Wth = nullptr;        // TF32 hi / lo parts of W^T (n x 64, position major) for the same
   float* Wtl = nullptr;
+  // FP64 form on the tensor cores (rbrp_slices.cuh): BF16 slices of A by position and of the
+  // block's basis, their exponents, and the row-split FP64 partials of the projection
+  void* sl_ws = nullptr;
+  size_t sl_bytes = 0;
+  unsigned short* slA = nullptr;
+  unsigned short* slQ = nullptr;
+  int* sl_exA = nullptr;
+  int* sl_exQ = nullptr;
+  double* sl_Wpart = nullptr;
+  int sl_maxsplit = 0;
   int variant = 0;             // 0: tensor-core projection and update, 1: CUDA-core ones
   bool tsolve_fp64 = false;    // T solve on the FP64 pipe instead of double-float
   long long wait_budget = 0;   // clock64 limit of bounded device waits (0: the default, ~2 s)
@@ -172,6 +182,15 @@ rbrp_status solve_T(rbrp_handle h, int k, int n);
 // 2-D FP32 TMA descriptor (inner dimension contiguous, 128-byte swizzle).
 rbrp_status make_tmap_f32(rbrp_handle h, void* map, const float* base, uint64_t inner, uint64_t outer,
                           uint64_t ld_elems, uint32_t box_inner, uint32_t box_outer);
+
+// The same for a BF16 array (boxes of 64 values).
+rbrp_status make_tmap_bf16(rbrp_handle h, void* map, const unsigned short* base, uint64_t inner, uint64_t outer,
+                           uint32_t box_outer);
+
+// Slice workspace of the FP64 form for an m x n matrix; false (and none held) where it would
+// take more than half of the free memory, which the CUDA-core projection then keeps.
+bool ensure_slices(rbrp_handle h, int m, int n);
+void release_slices(rbrp_handle h);
 
 template <typename T>
 rbrp_status id_error(rbrp_handle h, int m, int n, const T* dA, int64_t lda, double* err);

@@ -1,0 +1,490 @@
+// rbrp_slices.cuh - FP64-accurate products on the tcgen05 tensor cores (sm_103a), by
+// exact integer slices (the splitting of Ozaki, Ogita, Oishi and Rump, 2012).
+//
+// A row x of an operand (K values, |x| < 2^e) is held as X = rint(x 2^(54 - e)) in
+// balanced base-256 digits, X = sum_s d_s 256^(6 - s) with |d_0| <= 64 and
+// -128 <= d_s <= 127: seven slices of exact BF16 integers.  Then
+//   sum_k x(k) y(k) = 2^(ex + ey - 60) sum_c S_c 256^(6 - c),   S_c = sum_{i + j = c} sum_k d_i(k) e_j(k),
+// and every S_c is a sum of integer products that FP32 accumulates without rounding as
+// long as |S_c| <= 2^24.  Classes c <= 7 are taken (34 slice products).  Over a chunk of
+// 192 values of k, S_0 .. S_5 stay below 2^24 for any data; S_6 and S_7 can pass it only
+// by 1.13x, where a rounding of a unit or two is 2^-60 of max|x| max|y|.  After each
+// chunk the sums are folded into 64-bit integers, so the result carries no rounding
+// that grows with K: what is left is the operands' representation (2^-55 of each row's
+// largest entry per value) and the dropped classes (about 2^-62 per value), against
+// 2^-53 of every partial sum in an FP64 FMA chain.
+//
+// Why: GB300 retires about 1 FP64 FMA per clock and SM (0.3e12 /s over 152 SMs), the
+// BF16 tensor pipe 3,800; 34 slice products of the latter are 60 to 70 times faster.
+#pragma once
+#include "rbrp_tc.cuh"
+
+namespace rbrp {
+namespace tc {
+namespace {
+
+constexpr int SL = 7;                        // slices per operand
+constexpr int SL_BK = 64;                    // values of k per stage: one 128-byte swizzle row of BF16
+constexpr int SL_CHUNK = 3;                  // stages between drains (192 values of k)
+constexpr int SL_HALF = 32;                  // N per accumulator set
+constexpr int SL_CLASSES = 8;
+constexpr int SL_A_BYTES = BM * SL_BK * 2;              // one slice of the M operand: 16 KB
+constexpr int SL_B_BYTES = SL * SL_HALF * SL_BK * 2;    // seven slices of one half of the N operand: 28 KB
+constexpr int SL_DRAIN = 256;                           // 8 drain warps
+constexpr int SL_THREADS = 64 + SL_DRAIN;
+
+// Balanced base-256 digits of x 2^(-e) for |x| < 2^e, as BF16 bit patterns.
+// The integer comes from the bits of x: the FP64 pipe is 1/64 of the integer pipe's rate.
+__device__ __forceinline__ void slice_digits(double x, int e, unsigned short (&d)[SL]) {
+  const long long bits = __double_as_longlong(x);
+  const int ex = (int)((bits >> 52) & 0x7FF);
+  long long mant = bits & 0xFFFFFFFFFFFFFll;
+  if (ex) mant |= 1ll << 52;
+  // x = mant 2^(max(ex, 1) - 1075); X = mant 2^sh, sh <= 1 because |x| < 2^e
+  const int sh = (ex ? ex : 1) - 1075 + 54 - e;
+  long long X;
+  if (sh >= 0) {
+    X = mant << sh;
+  } else {
+    const int r = -sh;
+    X = r > 60 ? 0 : (mant + (1ll << (r - 1))) >> r;   // nearest, ties away from zero
+  }
+  if (bits < 0) X = -X;
+#pragma unroll
+  for (int s = SL - 1; s >= 0; --s) {
+    const int v = s ? (int)(signed char)(X & 0xFF) : (int)X;
+    X = (X - v) >> 8;
+    // float(v) by the 1.5 * 2^23 bias; at most 8 significant bits, so its upper half is the BF16
+    const float f = __int_as_float(0x4B400000 + v) - 12582912.0f;
+    d[s] = (unsigned short)(__float_as_uint(f) >> 16);
+  }
+}
+
+// Exponent e with |x| < 2^e from the largest |x| of a row, given as the upper 32 bits
+// of its FP64 pattern; zero and subnormal rows take the smallest normal one.
+__device__ __forceinline__ int slice_exponent(unsigned hi) {
+  const int ex = (int)((hi >> 20) & 0x7FF);
+  return (ex ? ex : 1) - 1022;
+}
+
+// Slices of the columns of an FP64 matrix: column c into rows s * srows + c of out
+// (ldk BF16 values each, zero past m), its exponent into ex[c].  One warp per column:
+// a pass for the largest entry, then a second one (L2) that writes 16 bytes per lane
+// and slice.  HBM bound: reads 8 and writes 14 bytes per entry (8192 x 8192: 0.36 ms,
+// 4.1 TB/s of those 22 bytes).
+__global__ void __launch_bounds__(256)
+k_slice_cols(const double* __restrict__ A, int64_t lda, int m, int n, int64_t srows, int64_t ldk,
+             unsigned short* __restrict__ out, int* __restrict__ exps) {
+  const int lane = threadIdx.x & 31;
+  const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (c >= n) return;
+  const double* col = A + (int64_t)c * lda;
+  unsigned mx = 0u;
+  for (int r = lane; r < m; r += 32) mx = max(mx, (unsigned)__double2hiint(col[r]) & 0x7FFFFFFFu);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  const int e = slice_exponent(mx);
+  if (lane == 0) exps[c] = e;
+  for (int r0 = 8 * lane; r0 < ldk; r0 += 256) {
+    unsigned short d[8][SL];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) slice_digits(r0 + u < m ? col[r0 + u] : 0.0, e, d[u]);
+#pragma unroll
+    for (int s = 0; s < SL; ++s) {
+      uint4 v;
+      v.x = d[0][s] | ((unsigned)d[1][s] << 16);
+      v.y = d[2][s] | ((unsigned)d[3][s] << 16);
+      v.z = d[4][s] | ((unsigned)d[5][s] << 16);
+      v.w = d[6][s] | ((unsigned)d[7][s] << 16);
+      *reinterpret_cast<uint4*>(out + ((int64_t)s * srows + c) * ldk + r0) = v;
+    }
+  }
+}
+
+// Slices of the block's basis columns Q(:, i .. i + kept) as the N operand: rows
+// (half, slice, column within the half), zero beyond the kept columns (up to 32, or 64
+// where more than 32 are kept).  One CTA per column.
+__global__ void __launch_bounds__(256)
+k_slice_q(const double* __restrict__ Q, int64_t ldq, int m, const State* __restrict__ st, int64_t ldk,
+          unsigned short* __restrict__ out, int* __restrict__ exps) {
+  __shared__ unsigned s_mx[8];
+  const int tid = threadIdx.x, a = blockIdx.x, i = st->i, kept = st->bs;
+  if (kept == 0 || a >= (kept > SL_HALF ? 2 * SL_HALF : SL_HALF)) return;
+  unsigned short* dst = out + ((int64_t)(a / SL_HALF) * SL * SL_HALF + a % SL_HALF) * ldk;
+  const double* col = Q + (int64_t)(i + (a < kept ? a : 0)) * ldq;
+  unsigned mx = 0u;
+  if (a < kept)
+    for (int r = tid; r < m; r += 256) mx = max(mx, (unsigned)__double2hiint(col[r]) & 0x7FFFFFFFu);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((tid & 31) == 0) s_mx[tid >> 5] = mx;
+  __syncthreads();
+  for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w]);
+  const int e = slice_exponent(mx);
+  if (tid == 0) exps[a] = e;
+  for (int r0 = 2 * tid; r0 < ldk; r0 += 512) {
+    unsigned short d0[SL], d1[SL];
+    slice_digits(a < kept && r0 < m ? col[r0] : 0.0, e, d0);
+    slice_digits(a < kept && r0 + 1 < m ? col[r0 + 1] : 0.0, e, d1);
+#pragma unroll
+    for (int s = 0; s < SL; ++s)
+      *reinterpret_cast<unsigned*>(dst + (int64_t)s * SL_HALF * ldk + r0) = d0[s] | ((unsigned)d1[s] << 16);
+  }
+}
+
+// Block swap of the sliced columns (they stay in position order, as perm):
+// columns K2 take the slices and exponents of K1.
+__global__ void __launch_bounds__(256)
+k_swap_slices(unsigned short* __restrict__ out, int64_t srows, int64_t ldk, int* __restrict__ exps,
+              const State* __restrict__ st, const int* __restrict__ K1g, const int* __restrict__ K2g) {
+  const int t = blockIdx.x;
+  if (t >= st->nK) return;
+  const int a = K1g[t], b = K2g[t];
+  const uint4* src = reinterpret_cast<const uint4*>(out + ((int64_t)blockIdx.y * srows + a) * ldk);
+  uint4* dst = reinterpret_cast<uint4*>(out + ((int64_t)blockIdx.y * srows + b) * ldk);
+  for (int64_t x = threadIdx.x; x < ldk / 8; x += 256) dst[x] = src[x];
+  if (blockIdx.y == 0 && threadIdx.x == 0) exps[b] = exps[a];
+}
+
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, int n, uint32_t accumulate) {
+  // D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1), K-major, N >> 3, M >> 4
+  const uint32_t idesc =
+      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
+}
+
+// (hi 2^24 + lo) 2^e rounded to the nearest FP64 value, on the integer pipe (the same
+// conversions and a scaling on the FP64 pipe cost ~25,000 clocks per 128 x 64 tile).
+__device__ __forceinline__ double slice_value(long long hi, long long lo, int e) {
+  hi += lo >> 24;
+  lo &= 0xFFFFFF;                       // now 0 <= lo < 2^24
+  const bool neg = hi < 0;
+  if (neg) {
+    hi = lo ? ~hi : -hi;
+    lo = lo ? 0x1000000 - lo : 0;
+  }
+  if (hi == 0) {                        // at most 24 significant bits
+    if (lo == 0) return 0.0;
+    hi = lo;
+    lo = 0;
+    e -= 24;
+  }
+  const int n = __clzll(hi);            // hi < 2^62: n >= 1
+  const unsigned long long lo40 = (unsigned long long)lo << 40;
+  unsigned long long t = ((unsigned long long)hi << n) | (lo40 >> (64 - n));
+  const bool rest = (lo40 << n) != 0;
+  unsigned long long m = t >> 11;
+  const unsigned r = (unsigned)t & 0x7FFu;
+  m += (r > 0x400u || (r == 0x400u && (rest || (m & 1)))) ? 1u : 0u;
+  const int be = 35 - n + e + 52 + 1023;   // value = m 2^(35 - n + e), 2^52 <= m <= 2^53
+  if (be >= 1 && be <= 2045) {
+    const long long bits = ((long long)be << 52) + (long long)(m - (1ull << 52));
+    return __longlong_as_double(neg ? bits | (long long)(1ull << 63) : bits);
+  }
+  const double v = ldexp((double)m, 35 - n + e);   // subnormal or out of range
+  return neg ? -v : v;
+}
+
+// Shared memory: the seven slices of the stage's M tile, each its own slot of a ring,
+// and two stages of the N operand's halves.
+struct __align__(1024) SliceSmem {
+  uint8_t as[SL][SL_A_BYTES];
+  uint8_t bs[2][2][SL_B_BYTES];             // [stage parity][half]
+  unsigned long long afull[SL], aempty[SL], bfull[2], bempty[2], accf[2], acce[2], mmadone;
+  uint32_t tmem_base;
+  int abort;
+};
+constexpr size_t SL_SMEM = sizeof(SliceSmem) + 1024;
+static_assert(SL_SMEM <= 232448, "227 KB of shared memory per CTA");
+
+// One 128 x 64 tile (128 x 32 when one half holds every column): D(p, a) over the
+// stages [s0, s0 + nst) of 64 values of k.
+//
+//   warp 0    TMA: per stage the N operand's halves, then the M operand's slices.
+//   warp 1    MMAs.  Slice i of M meets slices 0 .. min(6, 7 - i) of N at once: those sit
+//             in consecutive rows, so one MMA of N = 32 x (slices) adds classes i, i + 1, ...
+//             in consecutive accumulator columns.  An accumulator set (8 classes x 32
+//             columns) holds one half; tensor memory holds two sets, whose chunks are
+//             staggered by a stage, and the half that starts a chunk is issued last, so
+//             that its drain hides behind the other's MMAs.  With one half, chunks
+//             alternate between the sets.
+//   warps 2-9 drain a set each (four lane quarters): FP32 integers to int, folded into
+//             two 64-bit integers per column (weights 256^3 and 1, in units of class 6).
+//
+// What bounds it: the MMAs, 568 clocks per 16 values of k and half (N = 32 x 34 classes
+// at half a clock per column, or the shared-memory reads of the short ones), against
+// 1.75 KB of slices per value of k from HBM.  8192 x 8192, 64 columns: 0.37 ms a block
+// against 8.8 ms on the FP64 pipe; 1000 x 1000, 40 columns: 0.034 against 0.61 ms.
+//
+// epi.part(h, p, a0, hi, lo): the thread's 32 columns a0 .. a0 + 31 of row p, with
+// D = 2^(ex + ey - 60) (hi 2^24 + lo).
+template <typename Epi>
+__global__ void __launch_bounds__(SL_THREADS, 1)
+k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int64_t a_rows,
+              long long budget, Epi epi) {
+  extern __shared__ uint8_t sl_raw[];
+  SliceSmem& sm = *reinterpret_cast<SliceSmem*>((reinterpret_cast<uintptr_t>(sl_raw) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int p0, brow, s0, nst, nh;   // first M row, first N row, stage range, halves
+  if (!epi.tile(p0, brow, s0, nst, nh)) return;  // uniform over the CTA
+  volatile int* abort = &sm.abort;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < SL; ++s) {
+      mbar_init(&sm.afull[s], 1);
+      mbar_init(&sm.aempty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm.bfull[b], 1);
+      mbar_init(&sm.bempty[b], 1);
+      mbar_init(&sm.accf[b], 1);
+      mbar_init(&sm.acce[b], SL_DRAIN / 2);
+    }
+    mbar_init(&sm.mmadone, 1);
+    sm.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tbase = sm.tmem_base;
+  int aissued = 0, bissued = 0;  // producer: slices and N stages whose loads were issued
+
+  // chunk of half h at stage s: with two halves the second one's chunks start a stage early
+  auto chunk_of = [&](int h, int s) { return (s + (nh == 2 ? h : 0)) / SL_CHUNK; };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      for (int s = 0; s < nst && ok; ++s) {
+        const int b = s & 1, x = (s0 + s) * SL_BK;
+        if (s >= 2 && !mbar_wait(&sm.bempty[b], (uint32_t)((s >> 1) & 1) ^ 1, abort, budget)) break;
+        mbar_expect_tx(&sm.bfull[b], (uint32_t)(nh * SL_B_BYTES));
+        for (int h = 0; h < nh; ++h)
+          tma_load_2d(sm.bs[b][h], &tmB, &sm.bfull[b], x, brow + h * SL * SL_HALF);
+        bissued = s + 1;
+        for (int i = 0; i < SL; ++i) {
+          if (s >= 1 && !mbar_wait(&sm.aempty[i], (uint32_t)(s & 1) ^ 1, abort, budget)) { ok = false; break; }
+          mbar_expect_tx(&sm.afull[i], SL_A_BYTES);
+          tma_load_2d(sm.as[i], &tmA, &sm.afull[i], x, (int)(i * a_rows) + p0);
+          aissued = s * SL + i + 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int uses[2] = {0, 0};  // chunks started per accumulator set
+      bool ok = true;
+      for (int s = 0; s < nst && ok; ++s) {
+        const int b = s & 1;
+        if (!mbar_wait(&sm.bfull[b], (uint32_t)(s >> 1) & 1, abort, budget)) break;
+        const bool starts0 = s == 0 || chunk_of(0, s) != chunk_of(0, s - 1);
+        for (int q = 0; q < nh && ok; ++q) {
+          const int h = (nh == 2 && starts0) ? 1 - q : q;
+          const int ck = chunk_of(h, s);
+          const bool first = s == 0 || ck != chunk_of(h, s - 1);
+          const bool last = s == nst - 1 || ck != chunk_of(h, s + 1);
+          const int set = nh == 2 ? h : ck & 1;
+          if (first) {
+            if (uses[set] >= 1 && !mbar_wait(&sm.acce[set], (uint32_t)(uses[set] - 1) & 1, abort, budget)) {
+              ok = false;
+              break;
+            }
+            ++uses[set];
+          }
+          const uint32_t dset = tbase + (uint32_t)(set * SL_CLASSES * SL_HALF);
+          const uint64_t db = sw128_desc(smem_u32(sm.bs[b][h]));
+          for (int i = 0; i < SL; ++i) {
+            if (!mbar_wait(&sm.afull[i], (uint32_t)s & 1, abort, budget)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t da = sw128_desc(smem_u32(sm.as[i]));
+            const uint32_t d = dset + (uint32_t)(i * SL_HALF);
+            const int nsl = i == 0 ? SL : SL_CLASSES - i;   // N slices 0 .. nsl - 1: classes i .. i + nsl - 1
+            for (int k = 0; k < SL_BK / 16; ++k) {          // K = 16 BF16: 32 bytes
+              if (first && k == 0 && i == 1) {
+                // classes 1 .. 6 were started by slice 0; class 7 starts here
+                mma_bf16(d, da, db, (SL - 1) * SL_HALF, 1u);
+                mma_bf16(d + (uint32_t)((SL - 1) * SL_HALF), da,
+                         db + (uint64_t)(((SL - 1) * SL_HALF * SL_BK * 2) >> 4), SL_HALF, 0u);
+              } else {
+                mma_bf16(d, da + 2 * k, db + 2 * k, nsl * SL_HALF, (first && k == 0 && i == 0) ? 0u : 1u);
+              }
+            }
+            if (q == nh - 1) mma_commit(&sm.aempty[i]);
+          }
+          if (ok && last) mma_commit(&sm.accf[set]);
+        }
+        if (ok) mma_commit(&sm.bempty[b]);
+      }
+    }
+  } else {
+    const int q = warp & 3, set = (warp - 2) >> 2;
+    const uint32_t ta = tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(set * SL_CLASSES * SL_HALF);
+    long long hi[SL_HALF], lo[SL_HALF];
+#pragma unroll
+    for (int j = 0; j < SL_HALF; ++j) hi[j] = lo[j] = 0;
+    const int nchunk = nst > 0 ? chunk_of(set, nst - 1) + 1 : 0;
+    bool ok = true;
+    int use = 0;
+    for (int c = nh == 2 ? 0 : set; c < nchunk; c += nh == 2 ? 1 : 2, ++use) {
+      if (!mbar_wait(&sm.accf[set], (uint32_t)use & 1, abort, budget)) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll
+      for (int j0 = 0; j0 < SL_HALF; j0 += 4) {
+        float v[SL_CLASSES][4];
+#pragma unroll
+        for (int k = 0; k < SL_CLASSES; ++k) tmem_ld4(ta + (uint32_t)(k * SL_HALF + j0), v[k]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int s01 = __float2int_rn(v[0][j]) * 256 + __float2int_rn(v[1][j]);   // < 2^28
+          const int s23 = __float2int_rn(v[2][j]) * 256 + __float2int_rn(v[3][j]);   // < 2^31
+          hi[j0 + j] += (long long)s01 * 65536 + s23;
+          // class 7 joins class 6, rounded to its unit
+          lo[j0 + j] += (long long)__float2int_rn(v[4][j]) * 65536 + (long long)__float2int_rn(v[5][j]) * 256 +
+                        __float2int_rn(fmaf(v[7][j], 0.00390625f, v[6][j]));
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(&sm.acce[set]);
+    }
+    // one half: its chunks alternated between the sets, whose sums meet in shared memory
+    // (behind the barrier the last chunk of each set is drained: no load or MMA is left)
+    if (nh == 1) {
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      long long* sh = reinterpret_cast<long long*>(sm.as) + (32 * q + lane);
+      if (set == 1 && ok) {
+#pragma unroll
+        for (int j = 0; j < SL_HALF; ++j) {
+          sh[(2 * j) * BM] = hi[j];
+          sh[(2 * j + 1) * BM] = lo[j];
+        }
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (set == 0 && ok) {
+#pragma unroll
+        for (int j = 0; j < SL_HALF; ++j) {
+          hi[j] += sh[(2 * j) * BM];
+          lo[j] += sh[(2 * j + 1) * BM];
+        }
+      }
+    }
+    if (ok && !*abort && (nh == 2 || set == 0)) epi.part(p0 + 32 * q + lane, nh == 2 ? SL_HALF * set : 0, hi, lo);
+  }
+  __syncthreads();
+  if (*abort) {
+    // as k_proj_w_tc: the CTA's own TMA copies and issued MMAs finish before TMEM is freed
+    int dummy = 0;
+    volatile int* never = &dummy;
+    if (threadIdx.x == 0) epi.timeout();
+    if (warp == 0 && lane == 0) {
+      for (int x = aissued - SL > 0 ? aissued - SL : 0; x < aissued; ++x)
+        mbar_wait(&sm.afull[x % SL], (uint32_t)(x / SL) & 1, never);
+      for (int s = bissued - 2 > 0 ? bissued - 2 : 0; s < bissued; ++s)
+        mbar_wait(&sm.bfull[s & 1], (uint32_t)(s >> 1) & 1, never);
+    }
+    if (warp == 1 && lane == 0) {
+      mma_commit(&sm.mmadone);
+      mbar_wait(&sm.mmadone, 0u, never);
+    }
+    __syncthreads();
+  }
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------
+// a7 of the FP64 form: W = Q_blk^T A(:, perm[p]), M = positions (the slices of A stay
+// in position order), N = the block's basis columns, K = the m rows, split over
+// gridDim.y; FP64 partials per row range, summed by k_proj_finish.
+// ---------------------------------------------------------------------------
+struct ProjEpi {
+  State* st;
+  int n, nstages, sps;
+  const int* exA;
+  const int* exQ;
+  double* Wpart;
+  __device__ bool tile(int& p0, int& brow, int& s0, int& nst, int& nh) const {
+    const int kept = st->bs;
+    p0 = st->i + kept + blockIdx.x * BM;
+    brow = 0;
+    s0 = blockIdx.y * sps;
+    nst = min(sps, nstages - s0);
+    nh = kept > SL_HALF ? 2 : 1;
+    return kept > 0 && p0 < n && nst > 0;
+  }
+  __device__ void part(int p, int a0, const long long (&hi)[SL_HALF], const long long (&lo)[SL_HALF]) const {
+    if (p >= n) return;
+    const int kept = st->bs, e = exA[p] - 60;
+    double* w = Wpart + ((int64_t)blockIdx.y * MAXB + a0) * n + p;
+#pragma unroll
+    for (int j = 0; j < SL_HALF; ++j)
+      if (a0 + j < kept) w[(int64_t)j * n] = slice_value(hi[j], lo[j], e + exQ[a0 + j]);
+  }
+  __device__ void timeout() const { atomicExch(&st->status, ST_ERR_TIMEOUT); }
+};
+
+// R(I2, p) = W (the row ranges summed in order), diags(p) -= ||W(:, p)||^2 clipped at zero
+// (a8), and the partials of the residual and the positive count, 32 positions per CTA:
+// lane = position, warp w takes the basis columns w, w + 8, ...
+__global__ void __launch_bounds__(256)
+k_proj_finish(const State* __restrict__ st, const double* __restrict__ Wpart, int nsplit, int n,
+              double* __restrict__ R, int64_t ldr, double* __restrict__ diags, double* __restrict__ part_res,
+              int* __restrict__ part_nnz) {
+  __shared__ double s_sq[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = st->i, kept = st->bs;
+  const int p = i + kept + blockIdx.x * 32 + lane;
+  double s = 0.0;
+  if (kept > 0 && p < n) {
+    for (int a = w; a < kept; a += 8) {
+      double v = 0.0;
+      for (int z = 0; z < nsplit; ++z) v += Wpart[((int64_t)z * MAXB + a) * n + p];
+      R[(int64_t)(i + a) * ldr + p] = v;
+      s = fma(v, v, s);
+    }
+  }
+  s_sq[w][lane] = s;
+  __syncthreads();
+  if (w == 0) {
+    double d = 0.0;
+    if (kept > 0 && p < n) {
+      for (int x = 1; x < 8; ++x) s += s_sq[x][lane];
+      d = diags[p] - s;
+      d = d > 0.0 ? d : (d == d ? 0.0 : d);
+      diags[p] = d;
+    }
+    const int c = __popc(__ballot_sync(0xffffffffu, d > 0.0));
+    const double t = warp_sum(d);
+    if (lane == 0) {
+      part_res[blockIdx.x] = t;
+      part_nnz[blockIdx.x] = c;
+    }
+  }
+}
+
+}  // namespace
+}  // namespace tc
+}  // namespace rbrp

@@ -1,0 +1,67 @@
+"""The FP64 form's tensor-core products (exact BF16 slices) against the FP64 pipe."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+def colmajor(A):
+    return torch.from_numpy(np.asfortranarray(A)).cuda().t().contiguous().t()
+
+
+def first_block(A, b, variant):
+    """perm, L = A^T Q of a run of one block (both variants form the same Q on the FP64 pipe)."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    with Handle(0) as h:
+        h.set_variant(variant)
+        r = h.column_id(colmajor(A), b=b, tol=None, kmax=b, seed=3, compute_T=False)
+        assert len(r.ranks) >= 1
+        k1 = int(r.ranks[0])
+        return r.perm.cpu().numpy(), h.L().cpu().numpy()[:, :k1], k1
+
+
+def matrix(kind, m, n):
+    rng = np.random.Generator(np.random.Philox(key=m * 4099 + n))
+    A = rng.standard_normal((m, n))
+    if kind == "scaled":        # column scales over the whole exponent range, entries over 60 binades, zero columns
+        A *= 2.0 ** rng.integers(-60, 1, (m, n))
+        A *= 2.0 ** rng.integers(-400, 400, n)
+        A[:, 5] = 0.0
+    elif kind == "digits":      # every digit of every entry near its largest magnitude, one sign: the largest class sums
+        A = np.full((m, n), float(0x1F7F7F7F7F7F7F) * 2.0 ** -53) * (1.0 + 1e-3 * rng.standard_normal((1, n)))
+        A[rng.integers(0, m, n), np.arange(n)] += 1.0
+    return A
+
+
+@pytest.mark.parametrize("kind", ["normal", "scaled", "digits"])
+@pytest.mark.parametrize("m,n,b", [(40, 129, 9), (63, 300, 16), (64, 140, 32), (65, 200, 33), (192, 128, 31),
+                                   (193, 257, 64), (500, 1000, 48), (1100, 333, 64), (4000, 700, 40)])
+def test_projection_matches_the_fp64_pipe(kind, m, n, b):
+    A = matrix(kind, m, n)
+    perm0, L0, k0 = first_block(A, b, 0)
+    perm1, L1, k1 = first_block(A, b, 1)
+    assert k0 == k1 and np.array_equal(perm0[:k0], perm1[:k1])
+    # |fl(q^T a) - q^T a| <= gamma_m |q|^T |a| <= m eps ||a|| for the FMA chain and ||q|| = 1; the slices
+    # add the representation (2^-54 of each row's largest entry per value) and the dropped classes
+    norm = np.array([np.linalg.norm(c / s) * s if s > 0 else 0.0 for c, s in zip(A.T, np.abs(A).max(0))])
+    bound = (m + 1) * EPS * norm[:, None] + m * 2.0 ** -53 * np.abs(A).max(0)[:, None]
+    rest = perm0[k0:]
+    assert np.all(np.abs(L0 - L1)[rest] <= bound[rest])
+
+
+@pytest.mark.parametrize("m,n,b,kmax", [(300, 900, 20, 150), (700, 650, 64, 300)])
+def test_blocks_after_the_first_follow_the_same_skeleton(m, n, b, kmax):
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    A = colmajor(matrix("normal", m, n))
+    got = []
+    for variant in (0, 1):
+        with Handle(0) as h:
+            h.set_variant(variant)
+            r = h.column_id(A, b=b, tol=None, kmax=kmax, seed=1)
+            got.append((r.perm.cpu().numpy(), r.ranks, r.T.cpu().numpy()))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    # a Gaussian matrix of these shapes: kappa(A_S) < 30, one Gram-Schmidt pass, m eps kappa^2
+    d = np.linalg.norm(got[0][2] - got[1][2]) / np.linalg.norm(got[1][2])
+    assert d <= m * EPS * 900, d
