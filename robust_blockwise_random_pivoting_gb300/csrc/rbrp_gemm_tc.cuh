@@ -8,14 +8,13 @@
 // Both operands are K-major FP32 in global memory: X (K x M, column major, ld
 // a multiple of 4) and the hi and lo TF32 parts of Y (K x N each, same layout).
 //
-//   warp 0   TMA producer: the raw X tiles (128 x 32, 128-byte swizzled) into a
-//            10-stage ring.
+//   warp 0   TMA producer: per stage the raw X tile (128 x 32, 128-byte swizzled) and
+//            the Y hi / lo tiles (64 x 32 each) into a 6-stage ring.
 //   warp 1   MMA issuer: X hi Y hi into a large accumulator, X hi Y lo and
 //            X lo Y hi into a small one (3xTF32: the FP32 product to ~2^-22); X is
 //            read from tensor memory, Y from shared memory.
-//   warps 2-5 split each X tile by tf32_split into tensor memory (one row per
-//            thread), with two operand slots; the first split thread loads the
-//            slot's Y hi / lo tiles (64 x 32).
+//   warps 2-5 split each X tile by tf32_split into one of two slots of tensor
+//            memory (one row per thread).
 //   warps 6-13 drain the large accumulator after every RBRP_GEMM_DRAIN stages
 //            and the small one every CHUNK stages into double-float registers, then call the
 //            epilogue: thread (lane quarter q, column half ch) holds
@@ -46,15 +45,16 @@ namespace {
 constexpr int GEMM_DRAIN = RBRP_GEMM_DRAIN;
 static_assert(GEMM_DRAIN >= 1 && CHUNK % GEMM_DRAIN == 0, "drain interval");
 
-// Shared memory of k_gemm_tc: raw X tiles in a TMA ring, and per operand slot the
-// Y hi / lo tiles; the split warps write X's hi / lo parts into tensor memory (A slots
-// after the accumulators), so the MMAs read only Y from shared memory (as k_proj_w_tc).
-constexpr int GRAW = 10;
+// Shared memory of k_gemm_tc: raw X tiles and their stage's Y hi / lo tiles in one TMA
+// ring (as k_proj_w_tc: Y fetched behind a free X slot of tensor memory put its latency
+// between the MMAs); the split warps write X's hi / lo parts into tensor memory
+// (A slots after the accumulators), so the MMAs read only Y from shared memory.
+constexpr int GRAW = 6;                                  // the epilogues keep their own shared arrays
 struct __align__(1024) GemmSmem {
   uint8_t raw[GRAW][A_BYTES];
-  uint8_t ys[2][2 * B_BYTES];                            // per operand slot: Y hi, Y lo
+  uint8_t ys[GRAW][2 * B_BYTES];                         // Y hi, Y lo of the same stage
   unsigned long long rfull[GRAW], rempty[GRAW];
-  unsigned long long ofree[2], osplit[2], oy[2];
+  unsigned long long ofree[2], osplit[2];
   unsigned long long bigf[NBIG], bige[NBIG];
   unsigned long long smlf[2], smle[2];
   unsigned long long mmadone;
@@ -78,12 +78,11 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUten
   if (threadIdx.x == 0) {
     for (int s = 0; s < GRAW; ++s) {
       mbar_init(&sm.rfull[s], 1);
-      mbar_init(&sm.rempty[s], NSPLIT);
+      mbar_init(&sm.rempty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sm.ofree[b], 1);
       mbar_init(&sm.osplit[b], NSPLIT);
-      mbar_init(&sm.oy[b], 1);
     }
     for (int b = 0; b < NBIG; ++b) {
       mbar_init(&sm.bigf[b], 1);
@@ -107,38 +106,41 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUten
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = sm.tmem_base;
-  int issued = 0, yissued = 0;
+  int issued = 0;
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int s = 0; s < nk; ++s) {
-        const int rs = s % GRAW;
-        if (s >= GRAW && !mbar_wait(&sm.rempty[rs], (uint32_t)((s / GRAW) & 1) ^ 1, abort, budget)) break;
-        mbar_expect_tx(&sm.rfull[rs], A_BYTES);
+    for (int s = 0; s < nk; ++s) {
+      const int rs = s % GRAW;
+      if (s >= GRAW && !mbar_wait(&sm.rempty[rs], (uint32_t)((s / GRAW) & 1) ^ 1, abort, budget)) break;
+      if (elect_one()) {
+        mbar_expect_tx(&sm.rfull[rs], A_BYTES + 2 * B_BYTES);
         tma_load_2d(sm.raw[rs], &tmX, &sm.rfull[rs], s * BK, p0);
-        issued = s + 1;
+        tma_load_2d(sm.ys[rs], &tmYh, &sm.rfull[rs], s * BK, c0);
+        tma_load_2d(sm.ys[rs] + B_BYTES, &tmYl, &sm.rfull[rs], s * BK, c0);
       }
+      __syncwarp();
+      issued = s + 1;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      for (int s = 0; s < nk; ++s) {
-        const int os = s & 1;
-        const uint32_t ouse = (uint32_t)(s >> 1);
-        const int g = s / GEMM_DRAIN;                 // drain group of the large accumulator
-        const int b = g % NBIG;
-        const bool gfirst = (s % GEMM_DRAIN) == 0, glast = (s % GEMM_DRAIN) == GEMM_DRAIN - 1 || s == nk - 1;
-        const int chunk = s / CHUNK, sb = chunk & 1;
-        const bool first = (s % CHUNK) == 0;
-        if (gfirst && g >= NBIG && !mbar_wait(&sm.bige[b], (uint32_t)(g / NBIG - 1) & 1, abort, budget)) break;
-        if (first && chunk >= 2 && !mbar_wait(&sm.smle[sb], (uint32_t)((chunk >> 1) - 1) & 1, abort, budget)) break;
-        if (!mbar_wait(&sm.osplit[os], ouse & 1, abort, budget)) break;
-        if (!mbar_wait(&sm.oy[os], ouse & 1, abort, budget)) break;
-        tc_fence_after();
-        const uint32_t txh = tbase + TA_COL + (uint32_t)(os * 2 * BK);   // X hi: 32 columns, then X lo
-        const uint64_t dyh = sw128_desc(smem_u32(sm.ys[os]));
-        const uint64_t dyl = sw128_desc(smem_u32(sm.ys[os] + B_BYTES));
-        const uint32_t dbig = tbase + (uint32_t)(b * BN);
-        const uint32_t dsml = tbase + (uint32_t)(NBIG * BN + sb * BN);
+    for (int s = 0; s < nk; ++s) {
+      const int os = s & 1, rs = s % GRAW;
+      const uint32_t ouse = (uint32_t)(s >> 1);
+      const int g = s / GEMM_DRAIN;                 // drain group of the large accumulator
+      const int b = g % NBIG;
+      const bool gfirst = (s % GEMM_DRAIN) == 0, glast = (s % GEMM_DRAIN) == GEMM_DRAIN - 1 || s == nk - 1;
+      const int chunk = s / CHUNK, sb = chunk & 1;
+      const bool first = (s % CHUNK) == 0;
+      if (gfirst && g >= NBIG && !mbar_wait(&sm.bige[b], (uint32_t)(g / NBIG - 1) & 1, abort, budget)) break;
+      if (first && chunk >= 2 && !mbar_wait(&sm.smle[sb], (uint32_t)((chunk >> 1) - 1) & 1, abort, budget)) break;
+      if (!mbar_wait(&sm.osplit[os], ouse & 1, abort, budget)) break;
+      if (!mbar_wait(&sm.rfull[rs], (uint32_t)(s / GRAW) & 1, abort, budget)) break;
+      tc_fence_after();
+      const uint32_t txh = tbase + TA_COL + (uint32_t)(os * 2 * BK);   // X hi: 32 columns, then X lo
+      const uint64_t dyh = sw128_desc(smem_u32(sm.ys[rs]));
+      const uint64_t dyl = sw128_desc(smem_u32(sm.ys[rs] + B_BYTES));
+      const uint32_t dbig = tbase + (uint32_t)(b * BN);
+      const uint32_t dsml = tbase + (uint32_t)(NBIG * BN + sb * BN);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < BK / 8; ++k) {
           mma_tf32_ta(dbig, txh + 8 * k, dyh + 2 * k, (gfirst && k == 0) ? 0u : 1u);
@@ -146,25 +148,20 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUten
           mma_tf32_ta(dsml, txh + BK + 8 * k, dyh + 2 * k, 1u);
         }
         mma_commit(&sm.ofree[os]);
+        mma_commit(&sm.rempty[rs]);
         if (glast) mma_commit(&sm.bigf[b]);
         if ((s % CHUNK) == CHUNK - 1 || s == nk - 1) mma_commit(&sm.smlf[sb]);
       }
+      __syncwarp();
     }
   } else if (warp < 2 + NSPLIT / 32) {
     // split warps: one X row (a 128-byte swizzled row of the raw tile) per thread into
-    // TMEM lane 32 (warp % 4) + lane; the first split thread requests the Y tiles
-    const int et = threadIdx.x - 64;
+    // TMEM lane 32 (warp % 4) + lane
     const int row = 32 * (warp & 3) + lane;
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
     for (int s = 0; s < nk; ++s) {
       const int rs = s % GRAW, os = s & 1;
       if (s >= 2 && !mbar_wait(&sm.ofree[os], (uint32_t)((s >> 1) - 1) & 1, abort, budget)) break;
-      if (et == 0) {
-        mbar_expect_tx(&sm.oy[os], 2 * B_BYTES);
-        tma_load_2d(sm.ys[os], &tmYh, &sm.oy[os], s * BK, c0);
-        tma_load_2d(sm.ys[os] + B_BYTES, &tmYl, &sm.oy[os], s * BK, c0);
-        yissued = s + 1;
-      }
       if (!mbar_wait(&sm.rfull[rs], (uint32_t)(s / GRAW) & 1, abort, budget)) break;
       tc_fence_after();
       const uint8_t* rrow = sm.raw[rs] + row * 128;
@@ -182,7 +179,6 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUten
       tmem_st32(ta + BK, lo);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
-      mbar_arrive(&sm.rempty[rs]);
       mbar_arrive(&sm.osplit[os]);
     }
   } else {
@@ -224,12 +220,9 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUten
       for (int s = issued - GRAW > 0 ? issued - GRAW : 0; s < issued; ++s)
         mbar_wait(&sm.rfull[s % GRAW], (uint32_t)(s / GRAW) & 1, never);
     }
-    if (threadIdx.x == 64) {
-      for (int s = yissued - 2 > 0 ? yissued - 2 : 0; s < yissued; ++s)
-        mbar_wait(&sm.oy[s & 1], (uint32_t)(s >> 1) & 1, never);
-    }
-    if (warp == 1 && lane == 0) {
-      mma_commit(&sm.mmadone);
+    if (warp == 1) {
+      if (elect_one()) mma_commit(&sm.mmadone);
+      __syncwarp();
       mbar_wait(&sm.mmadone, 0u, never);
     }
     __syncthreads();

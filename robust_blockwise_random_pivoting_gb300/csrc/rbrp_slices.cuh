@@ -271,56 +271,61 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   auto chunk_of = [&](int h, int s) { return (s + (nh == 2 ? h : 0)) / SL_CHUNK; };
 
   if (warp == 0) {
-    if (lane == 0) {
-      bool ok = true;
-      for (int s = 0; s < nst && ok; ++s) {
-        const int b = s & 1, x = (s0 + s) * SL_BK;
-        if (s >= 2 && !mbar_wait(&sm.bempty[b], (uint32_t)((s >> 1) & 1) ^ 1, abort, budget)) break;
+    bool ok = true;
+    for (int s = 0; s < nst && ok; ++s) {
+      const int b = s & 1, x = (s0 + s) * SL_BK;
+      if (s >= 2 && !mbar_wait(&sm.bempty[b], (uint32_t)((s >> 1) & 1) ^ 1, abort, budget)) break;
+      if (elect_one()) {
         mbar_expect_tx(&sm.bfull[b], (uint32_t)(nh * SL_B_BYTES));
         for (int h = 0; h < nh; ++h)
           tma_load_2d(sm.bs[b][h], &tmB, &sm.bfull[b], x, brow + h * SL * SL_HALF);
-        bissued = s + 1;
-        for (int i = 0; i < SL; ++i) {
-          if (s >= 1 && !mbar_wait(&sm.aempty[i], (uint32_t)(s & 1) ^ 1, abort, budget)) { ok = false; break; }
+      }
+      __syncwarp();
+      bissued = s + 1;
+      for (int i = 0; i < SL; ++i) {
+        if (s >= 1 && !mbar_wait(&sm.aempty[i], (uint32_t)(s & 1) ^ 1, abort, budget)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&sm.afull[i], SL_A_BYTES);
           tma_load_2d(sm.as[i], &tmA, &sm.afull[i], x, (int)(i * a_rows) + p0);
-          aissued = s * SL + i + 1;
         }
+        __syncwarp();
+        aissued = s * SL + i + 1;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int uses[2] = {0, 0};  // chunks started per accumulator set
-      bool ok = true;
-      for (int s = 0; s < nst && ok; ++s) {
-        const int b = s & 1;
-        if (!mbar_wait(&sm.bfull[b], (uint32_t)(s >> 1) & 1, abort, budget)) break;
-        const bool starts0 = s == 0 || chunk_of(0, s) != chunk_of(0, s - 1);
-        for (int q = 0; q < nh && ok; ++q) {
-          const int h = (nh == 2 && starts0) ? 1 - q : q;
-          const int ck = chunk_of(h, s);
-          const bool first = s == 0 || ck != chunk_of(h, s - 1);
-          const bool last = s == nst - 1 || ck != chunk_of(h, s + 1);
-          const int set = nh == 2 ? h : ck & 1;
-          if (first) {
-            if (uses[set] >= 1 && !mbar_wait(&sm.acce[set], (uint32_t)(uses[set] - 1) & 1, abort, budget)) {
-              ok = false;
-              break;
-            }
-            ++uses[set];
+    int uses[2] = {0, 0};  // chunks started per accumulator set
+    bool ok = true;
+    for (int s = 0; s < nst && ok; ++s) {
+      const int b = s & 1;
+      if (!mbar_wait(&sm.bfull[b], (uint32_t)(s >> 1) & 1, abort, budget)) break;
+      const bool starts0 = s == 0 || chunk_of(0, s) != chunk_of(0, s - 1);
+      for (int q = 0; q < nh && ok; ++q) {
+        const int h = (nh == 2 && starts0) ? 1 - q : q;
+        const int ck = chunk_of(h, s);
+        const bool first = s == 0 || ck != chunk_of(h, s - 1);
+        const bool last = s == nst - 1 || ck != chunk_of(h, s + 1);
+        const int set = nh == 2 ? h : ck & 1;
+        if (first) {
+          if (uses[set] >= 1 && !mbar_wait(&sm.acce[set], (uint32_t)(uses[set] - 1) & 1, abort, budget)) {
+            ok = false;
+            break;
           }
-          const uint32_t dset = tbase + (uint32_t)(set * SL_CLASSES * SL_HALF);
-          const uint64_t db = sw128_desc(smem_u32(sm.bs[b][h]));
-          for (int i = 0; i < SL; ++i) {
-            if (!mbar_wait(&sm.afull[i], (uint32_t)s & 1, abort, budget)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint64_t da = sw128_desc(smem_u32(sm.as[i]));
-            const uint32_t d = dset + (uint32_t)(i * SL_HALF);
-            const int nsl = i == 0 ? SL : SL_CLASSES - i;   // N slices 0 .. nsl - 1: classes i .. i + nsl - 1
-            for (int k = 0; k < SL_BK / 16; ++k) {          // K = 16 BF16: 32 bytes
+          ++uses[set];
+        }
+        const uint32_t dset = tbase + (uint32_t)(set * SL_CLASSES * SL_HALF);
+        const uint64_t db = sw128_desc(smem_u32(sm.bs[b][h]));
+        for (int i = 0; i < SL; ++i) {
+          if (!mbar_wait(&sm.afull[i], (uint32_t)s & 1, abort, budget)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint64_t da = sw128_desc(smem_u32(sm.as[i]));
+          const uint32_t d = dset + (uint32_t)(i * SL_HALF);
+          const int nsl = i == 0 ? SL : SL_CLASSES - i;   // N slices 0 .. nsl - 1: classes i .. i + nsl - 1
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < SL_BK / 16; ++k) {        // K = 16 BF16: 32 bytes
               if (first && k == 0 && i == 1) {
                 // classes 1 .. 6 were started by slice 0; class 7 starts here
                 mma_bf16(d, da, db, (SL - 1) * SL_HALF, 1u);
@@ -331,10 +336,13 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               }
             }
             if (q == nh - 1) mma_commit(&sm.aempty[i]);
+            if (i == SL - 1) {
+              if (last) mma_commit(&sm.accf[set]);
+              if (q == nh - 1) mma_commit(&sm.bempty[b]);
+            }
           }
-          if (ok && last) mma_commit(&sm.accf[set]);
+          __syncwarp();
         }
-        if (ok) mma_commit(&sm.bempty[b]);
       }
     }
   } else {
@@ -403,8 +411,9 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       for (int s = bissued - 2 > 0 ? bissued - 2 : 0; s < bissued; ++s)
         mbar_wait(&sm.bfull[s & 1], (uint32_t)(s >> 1) & 1, never);
     }
-    if (warp == 1 && lane == 0) {
-      mma_commit(&sm.mmadone);
+    if (warp == 1) {
+      if (elect_one()) mma_commit(&sm.mmadone);
+      __syncwarp();
       mbar_wait(&sm.mmadone, 0u, never);
     }
     __syncthreads();

@@ -4,17 +4,16 @@
 // columns p (the MMA M dimension, TMEM lanes) and the <= 64 basis vectors a of
 // the block (MMA N), reduced over the m rows (MMA K) in stages of 32 rows.
 //
-//   warp 0   TMA producer: raw A_res tiles (128 columns x 32 rows, FP32,
-//            128-byte swizzled) into a 10-stage ring, completion on an mbarrier
-//            with a transaction count.
+//   warp 0   TMA producer: per stage the raw A_res tile (128 columns x 32 rows,
+//            FP32, 128-byte swizzled) and the Q hi / lo tiles (64 x 32 each, one
+//            box over the adjacent hi and lo arrays) into a 7-stage ring,
+//            completion on an mbarrier with a transaction count.
 //   warp 1   MMA issuer: tcgen05.mma kind::tf32 with A read from tensor memory and
 //            Q from shared memory; per K step the large product Ahi Qhi goes to
 //            one TMEM accumulator and the two small ones (Ahi Qlo, Alo Qhi) to
 //            another.
 //   warps 2-5 split each raw tile (one column per thread) by tf32_split and store
-//            the hi / lo parts into one of two A slots in tensor memory; the first
-//            of them loads that stage's Q hi / lo tiles (64 x 32 each, one TMA box
-//            over the adjacent hi and lo arrays) into the slot's shared memory.
+//            the hi / lo parts into one of two A slots in tensor memory.
 //   warps 6-13 drain the large accumulator after every stage and the small one
 //            every 512 rows with tcgen05.ld into double-float registers; two
 //            warps share each TMEM lane quarter, one per half of the 64 columns.
@@ -79,20 +78,55 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, uint32_t pa
       : "memory");
   return ok != 0;
 }
+// The same without the hardware's suspension: false at once where the phase is not complete.
+__device__ __forceinline__ bool mbar_test(unsigned long long* b, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(b)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait for the phase of parity `parity`: false once `budget` SM clocks
-// have passed (setting *abort) or another warp has set *abort.
+// have passed (setting *abort) or another warp has set *abort.  The polling loop is one
+// shared function: inlined at every wait it made the role loops several times longer.
+//
+// The lanes of a warp that wait together get the same answer, so that the instructions
+// behind a wait that need all of them (elect, tcgen05.ld) find them: a lane gives up only
+// while the whole warp is still waiting.  Where part of it has gone on, the phase is
+// complete and the rest will see that too (a bounded number of polls, should they not).
+__device__ __noinline__ bool mbar_poll(unsigned long long* b, uint32_t parity, volatile int* abort,
+                                       long long budget) {
+  const long long t0 = clock64();
+  int more = 0;
+  for (;;) {
+    if (*abort || clock64() - t0 > budget) {
+      *abort = 1;
+      if (__activemask() == 0xffffffffu || ++more > (1 << 16)) return false;
+    }
+    if (mbar_try_wait(b, parity)) return true;
+  }
+}
 __device__ __forceinline__ bool mbar_wait(unsigned long long* b, uint32_t parity, volatile int* abort,
                                           long long budget = kWaitBudgetDefault) {
-  if (mbar_try_wait(b, parity)) return true;
-  const long long t0 = clock64();
-  for (;;) {
-    if (mbar_try_wait(b, parity)) return true;
-    if (*abort) return false;
-    if (clock64() - t0 > budget) {
-      *abort = 1;
-      return false;
-    }
-  }
+  return mbar_test(b, parity) || mbar_poll(b, parity, abort, budget);
+}
+
+// One lane of a converged warp, the same one each time.  The TMA and MMA warps run their
+// loops with all lanes and issue under this predicate: as single-lane code behind a
+// divergent branch the MMA thread spent 1,600 clocks a stage beside the 700 of its MMAs
+// (the projection of a 16384 x 16384 run, k = 2000: 16.5 ms, 13.0 with uniform loops).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
@@ -179,31 +213,64 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
+
+// df_acc of two accumulators at once in packed FP32 (the same operations in the same order,
+// so the same bits): the drains are 192 FP32 operations per warp and stage, and the MMA
+// warp shares its scheduler with three that drain or split (16384 x 16384, k = 2000: the
+// projection took 13.0 ms with scalar sums, 9.7 with packed ones).
+__device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(unsigned long long r, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ void df_acc2(float& h0, float& h1, float& l0, float& l1, float x0, float x1) {
+  const unsigned long long hi = f2_pack(h0, h1), x = f2_pack(x0, x1);
+  const unsigned long long t = f2_add(hi, x);
+  const unsigned long long bb = f2_sub(t, hi);
+  const unsigned long long e = f2_add(f2_sub(hi, f2_sub(t, bb)), f2_sub(x, bb));
+  f2_unpack(f2_add(f2_pack(l0, l1), e), l0, l1);
+  f2_unpack(t, h0, h1);
+}
 __device__ __forceinline__ void drain32(uint32_t taddr, float (&hi)[32], float (&lo)[32]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float v[16];
     tmem_ld16(taddr + (uint32_t)(16 * h), v);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) df_acc(hi[16 * h + j], lo[16 * h + j], v[j]);
+    for (int j = 0; j < 16; j += 2)
+      df_acc2(hi[16 * h + j], hi[16 * h + j + 1], lo[16 * h + j], lo[16 * h + j + 1], v[j], v[j + 1]);
   }
 }
 
-// Shared memory of k_proj_w_tc.  The TMA ring holds raw A tiles only (16 KB a
-// stage: 160 KB of A in flight per SM).  The split warps write each tile's hi /
-// lo parts straight into tensor memory (the MMAs read A from there), so shared
-// memory carries only the raw tiles and, per operand slot, that stage's Q hi / lo.
-// An MMA whose A comes from shared memory re-reads its 4 KB per instruction at
-// about 128 bytes per clock (a probe: 51 clocks per M128 N64 K8 TF32 MMA); from
-// tensor memory only the 2 KB Q operand is read.
-constexpr int RAW = 10;                                  // raw A stages in flight
+// Shared memory of k_proj_w_tc: a TMA ring of raw A tiles with their stage's Q hi /
+// lo tiles (32 KB a stage).  The split warps write each A tile's hi / lo parts
+// straight into tensor memory (the MMAs read A from there), so the MMAs read only Q
+// from shared memory.  An MMA whose A comes from shared memory re-reads its 4 KB per
+// instruction at about 128 bytes per clock (a probe: 51 clocks per M128 N64 K8 TF32
+// MMA); from tensor memory only the 2 KB Q operand is read.
+// Q rides in the same ring as A instead of its own two slots, which the split
+// warps had to refill between their tiles.
+constexpr int RAW = 7;                                   // stages in flight
 constexpr uint32_t TA_COL = NBIG * BN + 2 * BN;          // TMEM columns of the A slots (after the accumulators)
 static_assert(TA_COL + 2 * 2 * BK <= TMEM_COLS, "TMEM budget: accumulators + two A slots of hi, lo");
 struct __align__(1024) ProjSmem {
   uint8_t raw[RAW][A_BYTES];
-  uint8_t qs[2][2 * B_BYTES];                            // per operand slot: Q hi, Q lo
-  unsigned long long rfull[RAW], rempty[RAW];            // raw ring: TMA done / split done
-  unsigned long long ofree[2], osplit[2], oq[2];         // operand slots: MMAs done / A in TMEM / Q landed
+  uint8_t qs[RAW][2 * B_BYTES];                          // Q hi, Q lo of the same stage
+  unsigned long long rfull[RAW], rempty[RAW];            // ring: TMA done / MMAs done
+  unsigned long long ofree[2], osplit[2];                // A slots of tensor memory: MMAs done / A stored
   unsigned long long bigf[NBIG], bige[NBIG];             // large accumulators: full (MMA done) / empty (drained)
   unsigned long long smlf[2], smle[2];                   // small accumulator
   unsigned long long mmadone;                            // abort path: every MMA this CTA issued has completed
@@ -232,12 +299,11 @@ k_proj_w_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (threadIdx.x == 0) {
     for (int s = 0; s < RAW; ++s) {
       mbar_init(&sm.rfull[s], 1);
-      mbar_init(&sm.rempty[s], NSPLIT);
+      mbar_init(&sm.rempty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sm.ofree[b], 1);
       mbar_init(&sm.osplit[b], NSPLIT);
-      mbar_init(&sm.oq[b], 1);
     }
     for (int b = 0; b < NBIG; ++b) {
       mbar_init(&sm.bigf[b], 1);
@@ -261,37 +327,38 @@ k_proj_w_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = sm.tmem_base;
-  int issued = 0;   // producer: stages whose A loads were issued
-  int qissued = 0;  // first split thread: stages whose Q loads were issued
+  int issued = 0;  // producer: stages whose loads were issued
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int s = 0; s < nk; ++s) {
-        const int rs = s % RAW;
-        if (s >= RAW && !mbar_wait(&sm.rempty[rs], (uint32_t)((s / RAW) & 1) ^ 1, abort, budget)) break;
-        mbar_expect_tx(&sm.rfull[rs], A_BYTES);
+    for (int s = 0; s < nk; ++s) {
+      const int rs = s % RAW;
+      if (s >= RAW && !mbar_wait(&sm.rempty[rs], (uint32_t)((s / RAW) & 1) ^ 1, abort, budget)) break;
+      if (elect_one()) {
+        mbar_expect_tx(&sm.rfull[rs], A_BYTES + 2 * B_BYTES);
         tma_load_2d(sm.raw[rs], &tmA, &sm.rfull[rs], (s0 + s) * BK, p0);
-        issued = s + 1;
+        tma_load_2d(sm.qs[rs], &tmQ, &sm.rfull[rs], (s0 + s) * BK, 0);   // Q hi (64 rows) then Q lo
       }
+      __syncwarp();
+      issued = s + 1;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      for (int s = 0; s < nk; ++s) {
-        const int os = s & 1;
-        const uint32_t ouse = (uint32_t)(s >> 1);
-        const int b = s % NBIG;                      // large accumulator of this stage
-        const int chunk = s / CHUNK, sb = chunk & 1;  // small accumulator of this chunk
-        const bool first = (s % CHUNK) == 0;
-        if (s >= NBIG && !mbar_wait(&sm.bige[b], (uint32_t)(s / NBIG - 1) & 1, abort, budget)) break;
-        if (first && chunk >= 2 && !mbar_wait(&sm.smle[sb], (uint32_t)((chunk >> 1) - 1) & 1, abort, budget)) break;
-        if (!mbar_wait(&sm.osplit[os], ouse & 1, abort, budget)) break;
-        if (!mbar_wait(&sm.oq[os], ouse & 1, abort, budget)) break;
-        tc_fence_after();
-        const uint32_t tah = tbase + TA_COL + (uint32_t)(os * 2 * BK);   // A hi: 32 columns, then A lo
-        const uint64_t dqh = sw128_desc(smem_u32(sm.qs[os]));
-        const uint64_t dql = sw128_desc(smem_u32(sm.qs[os] + B_BYTES));
-        const uint32_t dbig = tbase + (uint32_t)(b * BN);
-        const uint32_t dsml = tbase + (uint32_t)(NBIG * BN + sb * BN);
+    for (int s = 0; s < nk; ++s) {
+      const int os = s & 1, rs = s % RAW;
+      const uint32_t ouse = (uint32_t)(s >> 1);
+      const int b = s % NBIG;                      // large accumulator of this stage
+      const int chunk = s / CHUNK, sb = chunk & 1;  // small accumulator of this chunk
+      const bool first = (s % CHUNK) == 0;
+      if (s >= NBIG && !mbar_wait(&sm.bige[b], (uint32_t)(s / NBIG - 1) & 1, abort, budget)) break;
+      if (first && chunk >= 2 && !mbar_wait(&sm.smle[sb], (uint32_t)((chunk >> 1) - 1) & 1, abort, budget)) break;
+      if (!mbar_wait(&sm.osplit[os], ouse & 1, abort, budget)) break;
+      if (!mbar_wait(&sm.rfull[rs], (uint32_t)(s / RAW) & 1, abort, budget)) break;
+      tc_fence_after();
+      const uint32_t tah = tbase + TA_COL + (uint32_t)(os * 2 * BK);   // A hi: 32 columns, then A lo
+      const uint64_t dqh = sw128_desc(smem_u32(sm.qs[rs]));
+      const uint64_t dql = sw128_desc(smem_u32(sm.qs[rs] + B_BYTES));
+      const uint32_t dbig = tbase + (uint32_t)(b * BN);
+      const uint32_t dsml = tbase + (uint32_t)(NBIG * BN + sb * BN);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < BK / 8; ++k) {  // K = 8 TF32: 8 TMEM columns of A, 32 bytes of Q
           mma_tf32_ta(dbig, tah + 8 * k, dqh + 2 * k, k == 0 ? 0u : 1u);
@@ -299,26 +366,21 @@ k_proj_w_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           mma_tf32_ta(dsml, tah + BK + 8 * k, dqh + 2 * k, 1u);
         }
         mma_commit(&sm.ofree[os]);
+        mma_commit(&sm.rempty[rs]);
         mma_commit(&sm.bigf[b]);
         if ((s % CHUNK) == CHUNK - 1 || s == nk - 1) mma_commit(&sm.smlf[sb]);
       }
+      __syncwarp();
     }
   } else if (warp < 2 + NSPLIT / 32) {
     // split warps: TMEM lane quarter warp % 4; a thread takes one position (a 128-byte
     // row of the swizzled raw tile: 16-byte chunk c of row r sits at chunk c ^ (r % 8)),
-    // splits its 32 values and stores hi / lo into the A slot of stage s; the first split
-    // thread requests that stage's Q tiles once the slot is free
-    const int et = threadIdx.x - 64;  // 0..NSPLIT-1
+    // splits its 32 values and stores hi / lo into the A slot of stage s
     const int row = 32 * (warp & 3) + lane;
     const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
     for (int s = 0; s < nk; ++s) {
       const int rs = s % RAW, os = s & 1;
       if (s >= 2 && !mbar_wait(&sm.ofree[os], (uint32_t)((s >> 1) - 1) & 1, abort, budget)) break;
-      if (et == 0) {
-        mbar_expect_tx(&sm.oq[os], 2 * B_BYTES);   // Q hi (64 rows) then Q lo: one box of 128
-        tma_load_2d(sm.qs[os], &tmQ, &sm.oq[os], (s0 + s) * BK, 0);
-        qissued = s + 1;
-      }
       if (!mbar_wait(&sm.rfull[rs], (uint32_t)(s / RAW) & 1, abort, budget)) break;
       tc_fence_after();
       const uint8_t* rrow = sm.raw[rs] + row * 128;
@@ -336,7 +398,6 @@ k_proj_w_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       tmem_st32(ta + BK, lo);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
-      mbar_arrive(&sm.rempty[rs]);
       mbar_arrive(&sm.osplit[os]);
     }
   } else {
@@ -392,12 +453,9 @@ k_proj_w_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       for (int s = issued - RAW > 0 ? issued - RAW : 0; s < issued; ++s)
         mbar_wait(&sm.rfull[s % RAW], (uint32_t)(s / RAW) & 1, never);
     }
-    if (threadIdx.x == 64) {
-      for (int s = qissued - 2 > 0 ? qissued - 2 : 0; s < qissued; ++s)
-        mbar_wait(&sm.oq[s & 1], (uint32_t)(s >> 1) & 1, never);
-    }
-    if (warp == 1 && lane == 0) {
-      mma_commit(&sm.mmadone);
+    if (warp == 1) {
+      if (elect_one()) mma_commit(&sm.mmadone);
+      __syncwarp();
       mbar_wait(&sm.mmadone, 0u, never);
     }
     __syncthreads();

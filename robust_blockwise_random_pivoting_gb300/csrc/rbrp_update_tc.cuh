@@ -126,26 +126,30 @@ k_resid_update_tc(const __grid_constant__ CUtensorMap tmWh, const __grid_constan
   nrm.hi = nrm.lo = 0.f;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&sm.wfull, (uint32_t)(nkc * 2 * B_BYTES));
       for (int kc = 0; kc < nkc; ++kc) {
         tma_load_2d(sm.wt[kc][0], &tmWh, &sm.wfull, kc * BK, p0);
         tma_load_2d(sm.wt[kc][1], &tmWl, &sm.wfull, kc * BK, p0);
       }
-      for (int c = 0; c < nch; ++c) {
-        const int slot = c % U_STAGES;
-        const uint32_t use = (uint32_t)(c / U_STAGES);
-        if (c >= U_STAGES && !mbar_wait(&sm.qempty[slot], (use & 1) ^ 1, abort, budget)) break;
+    }
+    __syncwarp();
+    for (int c = 0; c < nch; ++c) {
+      const int slot = c % U_STAGES;
+      const uint32_t use = (uint32_t)(c / U_STAGES);
+      if (c >= U_STAGES && !mbar_wait(&sm.qempty[slot], (use & 1) ^ 1, abort, budget)) break;
+      if (elect_one()) {
         mbar_expect_tx(&sm.qfull[slot], (uint32_t)(nkc * 2 * A_BYTES));
         for (int kc = 0; kc < nkc; ++kc) {
           tma_load_2d(sm.qs[slot][kc][0], &tmQh, &sm.qfull[slot], kc * BK, rb + c * U_ROWS);
           tma_load_2d(sm.qs[slot][kc][1], &tmQl, &sm.qfull[slot], kc * BK, rb + c * U_ROWS);
         }
-        issued = c + 1;
       }
+      __syncwarp();
+      issued = c + 1;
     }
   } else if (warp == 1) {
-    if (lane == 0 && mbar_wait(&sm.wfull, 0u, abort, budget)) {
+    if (mbar_wait(&sm.wfull, 0u, abort, budget)) {
       for (int c = 0; c < nch; ++c) {
         const int slot = c % U_STAGES, buf = c & 1;
         const uint32_t use = (uint32_t)(c / U_STAGES);
@@ -153,21 +157,24 @@ k_resid_update_tc(const __grid_constant__ CUtensorMap tmWh, const __grid_constan
         if (!mbar_wait(&sm.qfull[slot], use & 1, abort, budget)) break;
         tc_fence_after();
         const uint32_t dacc = tbase + (uint32_t)(buf * U_ACC);
-        for (int kc = 0; kc < nkc; ++kc) {
-          const uint64_t dqh = sw128_desc(smem_u32(sm.qs[slot][kc][0]));
-          const uint64_t dql = sw128_desc(smem_u32(sm.qs[slot][kc][1]));
-          const uint64_t dwh = sw128_desc(smem_u32(sm.wt[kc][0]));
-          const uint64_t dwl = sw128_desc(smem_u32(sm.wt[kc][1]));
+        if (elect_one()) {
+          for (int kc = 0; kc < nkc; ++kc) {
+            const uint64_t dqh = sw128_desc(smem_u32(sm.qs[slot][kc][0]));
+            const uint64_t dql = sw128_desc(smem_u32(sm.qs[slot][kc][1]));
+            const uint64_t dwh = sw128_desc(smem_u32(sm.wt[kc][0]));
+            const uint64_t dwl = sw128_desc(smem_u32(sm.wt[kc][1]));
 #pragma unroll
-          for (int k = 0; k < BK / 8; ++k) {
-            mma_tf32(dacc + (uint32_t)(kc * U_POS), dqh + 2 * k, dwh + 2 * k, k == 0 ? 0u : 1u);
-            mma_tf32(dacc + (uint32_t)(2 * U_POS), dqh + 2 * k, dwl + 2 * k, (kc == 0 && k == 0) ? 0u : 1u);
-            mma_tf32(dacc + (uint32_t)(2 * U_POS), dql + 2 * k, dwh + 2 * k, 1u);
-            mma_tf32(dacc + (uint32_t)(2 * U_POS), dql + 2 * k, dwl + 2 * k, 1u);
+            for (int k = 0; k < BK / 8; ++k) {
+              mma_tf32(dacc + (uint32_t)(kc * U_POS), dqh + 2 * k, dwh + 2 * k, k == 0 ? 0u : 1u);
+              mma_tf32(dacc + (uint32_t)(2 * U_POS), dqh + 2 * k, dwl + 2 * k, (kc == 0 && k == 0) ? 0u : 1u);
+              mma_tf32(dacc + (uint32_t)(2 * U_POS), dql + 2 * k, dwh + 2 * k, 1u);
+              mma_tf32(dacc + (uint32_t)(2 * U_POS), dql + 2 * k, dwl + 2 * k, 1u);
+            }
           }
+          mma_commit(&sm.qempty[slot]);
+          mma_commit(&sm.accf[buf]);
         }
-        mma_commit(&sm.qempty[slot]);
-        mma_commit(&sm.accf[buf]);
+        __syncwarp();
       }
     }
   } else {
@@ -249,8 +256,9 @@ k_resid_update_tc(const __grid_constant__ CUtensorMap tmWh, const __grid_constan
       for (int c = issued - U_STAGES > 0 ? issued - U_STAGES : 0; c < issued; ++c)
         mbar_wait(&sm.qfull[c % U_STAGES], (uint32_t)(c / U_STAGES) & 1, never);
     }
-    if (warp == 1 && lane == 0) {
-      mma_commit(&sm.mmadone);
+    if (warp == 1) {
+      if (elect_one()) mma_commit(&sm.mmadone);
+      __syncwarp();
       mbar_wait(&sm.mmadone, 0u, never);
     }
     __syncthreads();
