@@ -347,8 +347,9 @@ Layout make_layout(int m, int n, int kmax, size_t elem, bool residual) {
   L.n = n;
   L.kmax = kmax;
   L.ntiles = (m + 63) / 64;
-  L.nproj = (n + 31) / 32;   // partials of the projection: 32 positions per CTA at the finest
+  L.nproj = (n + 7) / 8;     // partials of the projection: 8 positions per CTA at the finest
   L.cpart_rows = residual ? 1 : (kmax > 304 * 32 ? kmax : 304 * 32);
+  L.ptiles = (m + panel_tile_rows(m) - 1) / panel_tile_rows(m);
   L.elem = elem;
   L.residual = residual;
   L.ld_res = residual ? ((int64_t)m + 31) / 32 * 32 : 0;  // 128-byte aligned columns
@@ -408,9 +409,9 @@ rbrp_status ensure_workspace(rbrp_handle h, const Layout& L) {
       {(void**)&h->Q1, m * MAXB * 8},
       {(void**)&h->Cpart, (size_t)L.cpart_rows * MAXB * el},
       {(void**)&h->C, (L.residual ? 1 : kmax) * MAXB * el},
-      {(void**)&h->Gpart, (size_t)L.ntiles * M2 * 8},
+      {(void**)&h->Gpart, (size_t)L.ntiles * (L.residual ? M2 : (size_t)NPAIR) * 8},
       {(void**)&h->G, M2 * 8},
-      {(void**)&h->G2part, (size_t)L.ntiles * M2 * 8},
+      {(void**)&h->G2part, L.residual ? 0 : (size_t)L.ntiles * NPAIR * 8},
       {(void**)&h->G2, M2 * 8},
       {(void**)&h->R11, M2 * 8},
       {(void**)&h->R2, M2 * 8},

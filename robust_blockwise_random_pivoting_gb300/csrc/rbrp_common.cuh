@@ -24,6 +24,12 @@ constexpr int SAMPLER_GREEDY = 2;
 constexpr int SAMPLER_GIVEN = 3;  // fixed skeleton: the next columns of a given list, in list order
 constexpr int ST_ERR_NUMERIC = 5; // mirrors RBRP_ERR_NUMERIC
 
+// Panel kernels of the FP64 form (rbrp_panel64.cuh)
+constexpr int NPAIR = MAXB * (MAXB + 1) / 2;   // upper triangle of a panel's Gram matrix
+
+// Rows per CTA of the row kernels: 32, or 8 where 32 would leave SMs without a tile.
+__host__ __device__ constexpr int panel_tile_rows(int m) { return m >= 152 * 32 ? 32 : 8; }
+
 // Loop state, resident in device memory; every per-block kernel reads it, so the
 // host needs no data from the device to enqueue a block.
 struct State {

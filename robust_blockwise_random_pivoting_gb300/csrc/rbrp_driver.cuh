@@ -11,6 +11,7 @@
 
 #include "rbrp_internal.h"
 #include "rbrp_kernels.cuh"
+#include "rbrp_panel64.cuh"
 #include "rbrp_panel_df.cuh"
 #include "rbrp_slices.cuh"
 #include "rbrp_tc.cuh"
@@ -29,14 +30,13 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   rbrp_status s = ensure_workspace(h, L);
   if (s != RBRP_OK) return s;
   {  // function attributes are per device context: set them on every call (cheap)
-    for (const void* fn : {(const void*)k_pchol, (const void*)k_panel1, (const void*)k_chol2}) {
-      s = cuda_check(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PanelSmem)),
-                     "cudaFuncSetAttribute(panel)");
-      if (s != RBRP_OK) return s;
+    if constexpr (!RES) {
+      for (const void* fn : {(const void*)k_pchol, (const void*)k_chol2}) {
+        s = cuda_check(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(Panel64Smem)), "cudaFuncSetAttribute(panel)");
+        if (s != RBRP_OK) return s;
+      }
     }
-    s = cuda_check(h, cudaFuncSetAttribute(k_panel2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(PanelSmem)), "cudaFuncSetAttribute(k_panel2)");
-    if (s != RBRP_OK) return s;
     if (RES) {
       s = cuda_check(h, cudaFuncSetAttribute(k_pchol_df, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(PcholDfSmem)), "cudaFuncSetAttribute(panel df)");
@@ -76,8 +76,16 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   // FP64 form: the projection as exact BF16 slices on the tensor cores, 9 to 25 times the
   // FP64 pipe's rate for b of 30 to 64 (rbrp_slices.cuh).  Blocks of b <= 8 keep the column
   // streams: they read 8 bytes per entry of A where the slices are 14, and use one in four or
-  // fewer of the MMA's columns.  So do variant 1 and matrices whose slices would not fit.
-  const bool use_sl = !RES && h->variant == 0 && p.b > 8 && ensure_slices(h, m, n);
+  // fewer of the MMA's columns.  Fewer than 64 rows do not fill a stage (32 x 64: equal,
+  // 64 x 400, b = 16: 1.53 ms a run against 1.79; 16 x 100000, b = 12: 1.83 against 1.47).
+  // Variant 1 and matrices whose slices would not fit keep the CUDA-core kernels too.
+  //
+  // Random draws to a squared tolerance below 1e-8 keep the order of every sum as well: the
+  // weights of such a run's last blocks are differences of the order of their own rounding
+  // (eps / tol relative), and which column a draw takes follows that order.  Above, a draw
+  // moves in fewer than one run in 10^4 (b sqrt(n) eps / tol); at 1e-12 it was one in ten.
+  const bool fixed_order = p.tol > 0.0 && p.tol < 1e-8 && (p.sampler == SAMPLER_NP || p.sampler == SAMPLER_ES);
+  const bool use_sl = !RES && h->variant == 0 && p.b > 8 && m >= tc::SL_BK && !fixed_order && ensure_slices(h, m, n);
   const int64_t ldk = ((int64_t)m + tc::SL_BK - 1) / tc::SL_BK * tc::SL_BK;
   CUtensorMap tmSA, tmSQ;
   if (use_sl) {
@@ -90,12 +98,15 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
     if (s != RBRP_OK) return s;
   }
   T* Q = static_cast<T*>(h->Q);
-  T* Cpart = static_cast<T*>(h->Cpart);
   T* C = static_cast<T*>(h->C);
   const double tol = p.tol > 0.0 ? p.tol : 0.0;
   const double tol_loc = p.tol_loc > 0.0 ? p.tol_loc : 1.0 / (double)p.b;
-  const int ntiles = L.ntiles;
-  const size_t panel_smem = sizeof(PanelSmem);
+  const int ntiles = L.ntiles, ptiles = L.ptiles;
+  // the FP64 row kernels' tile height as a compile-time count
+  auto by_rows = [&](auto&& f) {
+    if (panel_tile_rows(m) == 32) f(std::integral_constant<int, 32>{});
+    else f(std::integral_constant<int, 8>{});
+  };
   h->have_result = false;
 
   const double es = (double)sizeof(T), dm = (double)m;
@@ -128,30 +139,40 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       return set_error(h, RBRP_ERR_NUMERIC, "no progress: block attempts exceeded 4*kmax+64");
     const int i = h->hst->i;
     const size_t mark0 = h->marks.size();
+    const int gram_parts = (p.b * (p.b + 1) / 2 + GRAM_PAIRS - 1) / GRAM_PAIRS;
+    const int gram_ctas = (p.b * (p.b + 1) / 2 + 63) / 64;
     ev = prof_begin(h);
     k_sample<<<1, SAMPLE_THREADS, 0, st>>>(h->st, h->diags, h->perm, n, kmax, p.b, p.seed, p.sampler,
                                            h->pbuf, h->kbuf, h->js, h->cols, h->given_order);
     prof_end(h, RBRP_PHASE_SAMPLE, ev, 28.0 * (n - i), 0.0, 1);
     ev = prof_begin(h);
-    if (!RES && i > 0) {
-      const int tiles = (i + 31) / 32;
-      int splits = splits_for(i, m);
-      int rps = ((m + splits - 1) / splits + 31) / 32 * 32;
-      splits = (m + rps - 1) / rps;
-      k_cgs_coef<T><<<dim3(tiles, 1, splits), 256, 0, st>>>(Q, m, dA, lda, h->cols, h->st, m, rps,
-                                                             (int64_t)i * MAXB, Cpart);
-      const int64_t cnt = (int64_t)i * MAXB;
-      k_reduce_parts<T><<<(int)std::min<int64_t>(1024, (cnt + 255) / 256), 256, 0, st>>>(Cpart, splits, cnt, cnt, C);
-    }
     const int dtiles = (m + DF_ROWS - 1) / DF_ROWS;   // row tiles of the double-float Gram kernel
     if (RES) {  // panel = residual columns at the sampled positions (FP32, exact), Gram in double-float
       k_gram_df<<<dtiles, 256, 0, st>>>(h->Ares, L.ld_res, h->js, h->st, m, (float*)h->V, h->Gpart);
       k_reduce_parts<double><<<16, 256, 0, st>>>(h->Gpart, dtiles, MAXB * MAXB, MAXB * MAXB, h->G);
-    } else {
-      k_cgs_update<T><<<ntiles, 256, 0, st>>>(dA, lda, h->cols, Q, m, C, h->st, m, h->V, h->Gpart, 1);
-      k_reduce_parts<double><<<16, 256, 0, st>>>(h->Gpart, ntiles, MAXB * MAXB, MAXB * MAXB, h->G);
     }
-    prof_end(h, RBRP_PHASE_CGS, ev, 0.0, 0.0, (!RES && i > 0) ? 4 : 2);
+    if constexpr (!RES) {
+      if (i > 0 && !fixed_order) {
+        k_gather_coef<<<(i + 3) / 4, 256, 0, st>>>(h->R, n, h->js, h->st, C);
+      } else if (i > 0) {
+        const int tiles = (i + 31) / 32;
+        int splits = splits_for(i, m);
+        int rps = ((m + splits - 1) / splits + 31) / 32 * 32;
+        splits = (m + rps - 1) / rps;
+        const int64_t cnt = (int64_t)i * MAXB;
+        double* Cpart = static_cast<double*>(h->Cpart);
+        k_cgs_coef<<<dim3(tiles, (p.b + COEF_COLS - 1) / COEF_COLS, splits), 256, 0, st>>>(Q, m, dA, lda, h->cols, h->st, m, rps, cnt,
+                                                                          Cpart);
+        k_reduce_parts<double><<<(int)std::min<int64_t>(1024, (cnt + 255) / 256), 256, 0, st>>>(Cpart, splits, cnt,
+                                                                                                cnt, C);
+      }
+      by_rows([&](auto tr) {
+        k_cgs_panel<decltype(tr)::value><<<ptiles, 256, 0, st>>>(dA, lda, h->cols, Q, m, C, h->st, m, h->V);
+      });
+      k_gram64<<<dim3(ntiles, gram_parts), 256, 0, st>>>(h->V, m, h->st, 0, h->Gpart);
+      k_reduce_gram<<<gram_ctas, 64, 0, st>>>(h->Gpart, ntiles, h->st, 0, h->G);
+    }
+    prof_end(h, RBRP_PHASE_CGS, ev, 0.0, 0.0, RES ? 2 : i == 0 ? 3 : fixed_order ? 5 : 4);
     ev = prof_begin(h);
     if (RES) {
       // R11 and its inverse as double-float pairs: the FP64 R11 / R2 buffers of the same
@@ -164,17 +185,23 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
           (const float*)h->V, m, h->st, Rinvdf, h->ord, (float*)Q, L.ld_res, use_tc ? h->Qh : nullptr,
           use_tc ? h->Ql : nullptr, L.ld_res, use_tc ? h->Qrh : nullptr, use_tc ? h->Qrl : nullptr);
       k_write_r11<<<1, 256, 0, st>>>(h->st, R11df, h->R, n);
-    } else {
-      k_pchol<<<1, 256, panel_smem, st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11, h->ord,
-                                          h->J, h->K1, h->K2);
-      k_panel1<<<ntiles, 256, panel_smem, st>>>(h->V, m, h->st, h->R11, h->ord, h->Q1, h->G2part);
-      k_reduce_parts<double><<<16, 256, 0, st>>>(h->G2part, ntiles, MAXB * MAXB, MAXB * MAXB, h->G2);
-      k_chol2<<<1, 256, panel_smem, st>>>(h->G2, h->st, h->R11, h->R2, h->R, n);
     }
-    if (i > 0) k_swap_R<<<(i + 127) / 128, 128, 0, st>>>(h->R, n, h->st, h->J, h->K1, h->K2);
+    if constexpr (!RES) {
+      k_pchol<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11, h->ord,
+                                                    h->J, h->K1, h->K2);
+      by_rows([&](auto tr) {
+        constexpr int TR = decltype(tr)::value;
+        k_panel_solve<TR><<<ptiles, 256, 0, st>>>(h->V, m, h->st, h->R11, h->ord, h->Q1, m, 0);
+        k_gram64<<<dim3(ntiles, gram_parts), 256, 0, st>>>(h->Q1, m, h->st, 1, h->G2part);
+        k_reduce_gram<<<gram_ctas, 64, 0, st>>>(h->G2part, ntiles, h->st, 1, h->G2);
+        k_chol2<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G2, h->st, h->R2);
+        k_panel_solve<TR><<<ptiles, 256, 0, st>>>(h->Q1, m, h->st, h->R2, nullptr, Q, m, 1);
+      });
+      k_panel_r<<<(p.b + 3) / 4, 256, 0, st>>>(h->st, h->R11, h->R2, h->R, n);
+    }
+    if (i > 0) k_swap_R<<<(i + 7) / 8, 256, 0, st>>>(h->R, n, h->st, h->J, h->K1, h->K2);
     if (RES)
       k_swap_cols<<<dim3((m + 1023) / 1024, MAXB), 256, 0, st>>>(h->Ares, L.ld_res, h->st, m, h->K1, h->K2);
-    if (!RES) k_panel2<T><<<ntiles, 256, panel_smem, st>>>(h->Q1, m, h->st, h->R2, Q, m, 1);
     if constexpr (!RES) {
       if (use_sl) {
         tc::k_slice_q<<<p.b > tc::SL_HALF ? MAXB : tc::SL_HALF, 256, 0, st>>>(Q, m, m, h->st, ldk, h->slQ,
@@ -182,7 +209,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
         tc::k_swap_slices<<<dim3(p.b, tc::SL), 256, 0, st>>>(h->slA, n, ldk, h->sl_exA, h->st, h->K1, h->K2);
       }
     }
-    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 5 : 4) : (i > 0 ? 6 : 5) + (use_sl ? 2 : 0));
+    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 5 : 4) : (i > 0 ? 8 : 7) + (use_sl ? 2 : 0));
     int nproj;
     ev = prof_begin(h);
     if (RES) {
@@ -294,9 +321,16 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       // basis tile height: the smallest KB >= b (kept <= b); b <= 8 takes the column-streaming form
       auto project = [&](auto kb) {
         constexpr int KB = decltype(kb)::value;
-        nproj = (n - i + ProjTile<KB>::PC - 1) / ProjTile<KB>::PC;
-        k_project<T, KB><<<nproj, 256, 0, st>>>(Q, m, dA, lda, h->perm, h->st, m, n, h->R, n, h->diags,
-                                                h->part_res, h->part_nnz);
+        auto run = [&](auto tile) {
+          using P = decltype(tile);
+          nproj = (n - i + P::PC - 1) / P::PC;
+          k_project<T, P><<<nproj, 256, 0, st>>>(Q, m, dA, lda, h->perm, h->st, m, n, h->R, n, h->diags, h->part_res,
+                                                 h->part_nnz);
+        };
+        // two large tiles per SM, or the small ones: the FP64 pipe bounds both, and a tile's
+        // chain over the m rows has to run on every SM
+        if ((n - i + ProjTile<KB, 4>::PC - 1) / ProjTile<KB, 4>::PC >= 2 * h->sms) run(ProjTile<KB, 4>{});
+        else run(ProjTile<KB, 1>{});
       };
       auto skinny = [&](auto kb) {
         constexpr int KB = decltype(kb)::value;

@@ -164,6 +164,7 @@ void batch_release(rbrp_handle h);
 
 struct Layout {
   int m, n, kmax, ntiles, nproj, cpart_rows;
+  int ptiles;     // row tiles of the FP64 panel kernels
   size_t elem;    // sizeof element of A / Q
   bool residual;  // FP32 residual form: Q holds one block, A_res is allocated
   int64_t ld_res;

@@ -2,12 +2,16 @@
 //
 // Per block (positions [i, i+bs) are filled), in launch order:
 //   k_sample      weighted block sampling (np-compat / exponential keys / greedy)
-//   k_cgs_coef    C = Q(:, :i)^T A(:, J)            (split-m partials)
-//   k_cgs_update  V = A(:, J) - Q(:, :i) C, Gram partials V^T V
-//   k_panel1      pivoted Cholesky of V^T V = CPQR pivots + robust filter,
-//                 Q1 = V_p R11^{-1}, Gram partials Q1^T Q1, block swap
+//   (rbrp_panel64.cuh, FP64 form)
+//   k_gather_coef C = Q(:, :i)^T A(:, J), from R
+//                 (k_cgs_coef where R holds no slice products)
+//   k_cgs_panel   V = A(:, J) - Q(:, :i) C
+//   k_gram64      V^T V, and Q1^T Q1 after the first pass
+//   k_pchol       CPQR pivots + robust filter from V^T V, R11, block swap
+//   k_panel_solve Q1 = V_p R11^{-1}, then Q_blk = Q1 R2^{-1}
+//   k_chol2       R2 = chol(Q1^T Q1);  k_panel_r  R(I2, I2) = R2 R11
+//   (here)
 //   k_swap_R      R(:i, K2) = R(:i, K1), R(:i, I2) = R(:i, J)
-//   k_panel2      second CholQR pass: Q_blk = Q1 R2^{-1}, R(I2, I2) = R2 R11
 //   k_project     W = Q_blk^T A(:, perm[p]) for the remaining positions p,
 //                 R(I2, p) = W, diags(p) -= ||W(:, p)||^2 (clipped at 0);
 //                 k_project_skinny for blocks of b <= 8 (column streams)
@@ -131,67 +135,6 @@ k_sample(State* st, const double* __restrict__ diags, const int* __restrict__ pe
   sample_block(st, diags, perm, n, kmax, b, seed, sampler, pbuf, kbuf, js, cols, order_of);
 }
 
-// ===========================================================================
-// a3: block Gram-Schmidt against the current basis (one CGS pass, as
-// python/RBRP.ipynb cell 11 line 120 and matlab/RBRP.m:55).
-// ===========================================================================
-// Cpart[z][a*MAXB + c] = sum over rows of split z of Q(r, a) * A(r, cols[c]).
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_cgs_coef(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t lda,
-           const int* __restrict__ cols, const State* __restrict__ st, int m, int rows_per_split,
-           int64_t pstride, T* __restrict__ Cpart) {
-  __shared__ T Qs[32][33];
-  __shared__ T As[32][MAXB + 1];
-  __shared__ int cs[MAXB];
-  const int tid = threadIdx.x;
-  const int i = st->i, bss = st->bs_sampled;
-  const int a0 = blockIdx.x * 32;
-  const int rb = blockIdx.z * rows_per_split, re = min(m, rb + rows_per_split);
-  if (tid < MAXB) cs[tid] = tid < bss ? cols[tid] : -1;
-  const int al = tid >> 3, cl = tid & 7;
-  const int nq = (bss + 7) >> 3;   // column groups that hold sampled columns (uniform: FP64 work only there)
-  T acc[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) acc[q] = T(0);
-  for (int r0 = rb; r0 < re; r0 += 32) {
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int idx = tid + 256 * q, kk = idx & 31, aa = idx >> 5;
-      const int r = r0 + kk, a = a0 + aa;
-      Qs[kk][aa] = (r < re && a < i) ? Q[r + (int64_t)a * ldq] : T(0);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int idx = tid + 256 * q, kk = idx & 31, cc = idx >> 5;
-      const int r = r0 + kk, c = cs[cc];
-      As[kk][cc] = (r < re && c >= 0) ? A[r + (int64_t)c * lda] : T(0);
-    }
-    __syncthreads();
-    // column groups as a compile-time count: predicated-off FP64 FMAs would still take issue slots
-    auto fmas = [&](auto nqc) {
-      constexpr int NQ = decltype(nqc)::value;
-#pragma unroll 8
-      for (int kk = 0; kk < 32; ++kk) {
-        const T qa = Qs[kk][al];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q] = fma(qa, As[kk][cl + 8 * q], acc[q]);
-      }
-    };
-    if (nq <= 1) fmas(std::integral_constant<int, 1>{});
-    else if (nq <= 2) fmas(std::integral_constant<int, 2>{});
-    else if (nq <= 4) fmas(std::integral_constant<int, 4>{});
-    else fmas(std::integral_constant<int, 8>{});
-  }
-  const int a = a0 + al;
-  if (a < i) {
-    T* out = Cpart + (int64_t)blockIdx.z * pstride + (int64_t)a * MAXB;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) out[cl + 8 * q] = acc[q];
-  }
-}
-
 // Deterministic sum of split partials: out[x] = sum_z part[z*stride + x].
 template <typename V>
 __global__ void k_reduce_parts(const V* __restrict__ part, int nparts, int64_t stride, int64_t count,
@@ -204,441 +147,30 @@ __global__ void k_reduce_parts(const V* __restrict__ part, int nparts, int64_t s
   }
 }
 
-// V(r, c) = A(r, cols[c]) - sum_a Q(r, a) C(a, c) for 64 rows; Gram partial of the tile.
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_cgs_update(const T* __restrict__ A, int64_t lda, const int* __restrict__ cols,
-             const T* __restrict__ Q, int64_t ldq, const T* __restrict__ C,
-             const State* __restrict__ st, int m, double* __restrict__ V, double* __restrict__ Gpart,
-             int use_q) {
-  // the operand tiles and the V tile are never live together
-  constexpr size_t kOps = sizeof(T) * (64 * 33 + 32 * MAXB);
-  constexpr size_t kV = sizeof(double) * 64 * (MAXB + 1);
-  __shared__ __align__(16) unsigned char raw[kOps > kV ? kOps : kV];
-  T(*Qs)[33] = reinterpret_cast<T(*)[33]>(raw);
-  T(*Cs)[MAXB] = reinterpret_cast<T(*)[MAXB]>(raw + sizeof(T) * 64 * 33);
-  double(*Vs)[MAXB + 1] = reinterpret_cast<double(*)[MAXB + 1]>(raw);
-  __shared__ int cs[MAXB];
-  const int tid = threadIdx.x;
-  const int i = use_q ? st->i : 0, bss = st->bs_sampled;
-  const int r0 = blockIdx.x * 64;
-  if (tid < MAXB) cs[tid] = tid < bss ? cols[tid] : -1;
-  const int ty = tid >> 4, tx = tid & 15;
-  const int nv = (bss + 15) >> 4;   // column groups that hold sampled columns (uniform over the CTA)
-  T acc[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = T(0);
-  for (int a0 = 0; a0 < i; a0 += 32) {
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int idx = tid + 256 * q, rr = idx & 63, aa = idx >> 6;
-      const int r = r0 + rr, a = a0 + aa;
-      Qs[rr][aa] = (r < m && a < i) ? Q[r + (int64_t)a * ldq] : T(0);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int idx = tid + 256 * q, cc = idx & 63, aa = idx >> 6;
-      Cs[aa][cc] = (a0 + aa < i) ? C[(int64_t)(a0 + aa) * MAXB + cc] : T(0);
-    }
-    __syncthreads();
-    // column groups as a compile-time count: predicated-off FP64 FMAs would still take issue slots
-    auto fmas = [&](auto nvc) {
-      constexpr int NV = decltype(nvc)::value;
-#pragma unroll 4
-      for (int aa = 0; aa < 32; ++aa) {
-        T qv[4], cv[NV];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) qv[u] = Qs[ty * 4 + u][aa];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) cv[v] = Cs[aa][tx + 16 * v];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < NV; ++v) acc[u][v] = fma(qv[u], cv[v], acc[u][v]);
-      }
-    };
-    if (nv <= 1) fmas(std::integral_constant<int, 1>{});
-    else if (nv <= 2) fmas(std::integral_constant<int, 2>{});
-    else if (nv <= 3) fmas(std::integral_constant<int, 3>{});
-    else fmas(std::integral_constant<int, 4>{});
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int rr = ty * 4 + u, r = r0 + rr;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = tx + 16 * v;
-      double val = 0.0;
-      if (r < m && c < bss) val = (double)A[r + (int64_t)cs[c] * lda] - (double)acc[u][v];
-      Vs[rr][c] = val;
-    }
-  }
-  __syncthreads();
-  // store V (column major, ld = m) coalesced along rows
-  for (int idx = tid; idx < 64 * MAXB; idx += 256) {
-    const int rr = idx & 63, c = idx >> 6, r = r0 + rr;
-    if (r < m && c < bss) V[r + (int64_t)c * m] = Vs[rr][c];
-  }
-  // Gram partial (bss x bss, stored MAXB x MAXB)
-  double* G = Gpart + (int64_t)blockIdx.x * MAXB * MAXB;
-  const int c1 = tid >> 2;
-  for (int q = 0; q < 16; ++q) {
-    const int c2 = (tid & 3) + 4 * q;
-    double s = 0.0;
-    if (c1 < bss && c2 < bss) {
-#pragma unroll 8
-      for (int rr = 0; rr < 64; ++rr) s = fma(Vs[rr][c1], Vs[rr][c2], s);
-    }
-    G[c1 * MAXB + c2] = s;
-  }
-}
-
-// ===========================================================================
-// a4 + a5: panel CPQR and robust filter.
-// CPQR of the m x bs panel V is computed as pivoted Cholesky of its Gram
-// matrix in shared memory: at step t the Schur complement's diagonal holds the
-// squared norms of the panel columns orthogonalised against the t pivots, so
-// the argmax is the CPQR pivot (LAPACK dgeqp3's greedy rule, swap semantics,
-// first index among ties), and its trace is the reverse cumulative sum of the
-// squared row norms of R that the robust filter tests
-// (python/RBRP.ipynb cell 11 lines 69-73, 122-123):
-//   keep t rows <=> trace_t / trace_0 >= tol_loc for every earlier step.
-// Q is then V_p R^{-1}, made orthonormal by a second CholQR pass (CholQR2).
-// ===========================================================================
-struct PanelSmem {
-  double S[MAXB][MAXB + 1];   // Gram / Schur complement
-  double R[MAXB][MAXB + 1];   // Cholesky factor rows
-  double W[64][MAXB + 1];     // row tile of the panel
-  int ord[MAXB];
-  int stop, piv;
-  double total;
-};
-
-// Pivoted Cholesky with the robust-filter stop; all threads of the CTA call it.
-__device__ int pivoted_chol_filter(PanelSmem& sm, int nb, int rows, double tol_loc) {
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid < MAXB) sm.ord[tid] = tid;
-  if (wid == 0) {
-    double d = 0.0;
-    for (int s = lane; s < nb; s += 32) d += sm.S[s][s];
-    d = warp_sum(d);
-    if (lane == 0) sm.total = d;
-  }
-  __syncthreads();
-  int kept = rows;
-  for (int t = 0; t < rows; ++t) {
-    if (wid == 0) {
-      double rem = 0.0, best = -1.0;
-      int bi = nb;
-      for (int s = t + lane; s < nb; s += 32) {
-        const double d = sm.S[s][s];
-        rem += d;
-        if (d > best) { best = d; bi = s; }
-      }
-      rem = warp_sum(rem);
-      rem = __shfl_sync(0xffffffffu, rem, 0);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_down_sync(0xffffffffu, best, o);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (lane == 0) {
-        const double total = sm.total;
-        const bool stop = !(total > 0.0) || (rem / total < tol_loc) || !(best > 0.0);
-        sm.stop = stop;
-        sm.piv = bi;
-      }
-    }
-    __syncthreads();
-    if (sm.stop) { kept = t; break; }
-    const int p = sm.piv;
-    if (p != t) {
-      for (int j = tid; j < nb; j += blockDim.x) {
-        const double x = sm.S[t][j]; sm.S[t][j] = sm.S[p][j]; sm.S[p][j] = x;
-      }
-      __syncthreads();
-      for (int j = tid; j < nb; j += blockDim.x) {
-        const double x = sm.S[j][t]; sm.S[j][t] = sm.S[j][p]; sm.S[j][p] = x;
-      }
-      for (int j = tid; j < t; j += blockDim.x) {
-        const double x = sm.R[j][t]; sm.R[j][t] = sm.R[j][p]; sm.R[j][p] = x;
-      }
-      if (tid == 0) { const int o = sm.ord[t]; sm.ord[t] = sm.ord[p]; sm.ord[p] = o; }
-      __syncthreads();
-    }
-    const double rtt = sqrt(sm.S[t][t]);
-    for (int s = t + tid; s < nb; s += blockDim.x) sm.R[t][s] = (s == t) ? rtt : sm.S[t][s] / rtt;
-    __syncthreads();
-    const int w = nb - t - 1;
-    for (int idx = tid; idx < w * w; idx += blockDim.x) {
-      const int s1 = t + 1 + idx / w, s2 = t + 1 + idx % w;
-      sm.S[s1][s2] -= sm.R[t][s1] * sm.R[t][s2];
-    }
-    __syncthreads();
-  }
-  return kept;
-}
-
-// Single-warp form of pivoted_chol_filter (only __syncwarp between steps): lane
-// l owns columns l and l + 32.  Returns the kept count to all 32 lanes.
-__device__ int pivoted_chol_filter_warp(PanelSmem& sm, int nb, int rows, double tol_loc) {
-  const int lane = threadIdx.x & 31;
-  sm.ord[lane] = lane;
-  sm.ord[lane + 32] = lane + 32;
-  double d = 0.0;
-  for (int s = lane; s < nb; s += 32) d += sm.S[s][s];
-  const double total = __shfl_sync(0xffffffffu, warp_sum(d), 0);
-  __syncwarp();
-  for (int t = 0; t < rows; ++t) {
-    double rem = 0.0, best = -1.0;
-    int bi = nb;
-    for (int s = t + lane; s < nb; s += 32) {
-      const double v = sm.S[s][s];
-      rem += v;
-      if (v > best) { best = v; bi = s; }
-    }
-    rem = __shfl_sync(0xffffffffu, warp_sum(rem), 0);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_down_sync(0xffffffffu, best, o);
-      const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    best = __shfl_sync(0xffffffffu, best, 0);
-    const int p = __shfl_sync(0xffffffffu, bi, 0);
-    if (!(total > 0.0) || (rem / total < tol_loc) || !(best > 0.0)) return t;
-    if (p != t) {
-      for (int j = lane; j < nb; j += 32) {
-        const double x = sm.S[t][j]; sm.S[t][j] = sm.S[p][j]; sm.S[p][j] = x;
-      }
-      __syncwarp();
-      for (int j = lane; j < nb; j += 32) {
-        const double x = sm.S[j][t]; sm.S[j][t] = sm.S[j][p]; sm.S[j][p] = x;
-      }
-      for (int j = lane; j < t; j += 32) {
-        const double x = sm.R[j][t]; sm.R[j][t] = sm.R[j][p]; sm.R[j][p] = x;
-      }
-      if (lane == 0) { const int o = sm.ord[t]; sm.ord[t] = sm.ord[p]; sm.ord[p] = o; }
-      __syncwarp();
-    }
-    const double rtt = sqrt(sm.S[t][t]);
-    for (int s = t + lane; s < nb; s += 32) sm.R[t][s] = (s == t) ? rtt : sm.S[t][s] / rtt;
-    __syncwarp();
-    for (int s2 = t + 1 + lane; s2 < nb; s2 += 32) {
-      const double r2 = sm.R[t][s2];
-      for (int s1 = t + 1; s1 < nb; ++s1) sm.S[s1][s2] = fma(-sm.R[t][s1], r2, sm.S[s1][s2]);
-    }
-    __syncwarp();
-  }
-  return rows;
-}
-
-// Single-warp plain Cholesky of S (n x n) into sm.R (upper).
-__device__ void chol_upper_warp(PanelSmem& sm, int nb) {
-  const int lane = threadIdx.x & 31;
-  for (int t = 0; t < nb; ++t) {
-    const double rtt = sqrt(fmax(sm.S[t][t], 0.0));
-    for (int s = t + lane; s < nb; s += 32) sm.R[t][s] = (s == t) ? rtt : sm.S[t][s] / rtt;
-    __syncwarp();
-    for (int s2 = t + 1 + lane; s2 < nb; s2 += 32) {
-      const double r2 = sm.R[t][s2];
-      for (int s1 = t + 1; s1 <= s2; ++s1) sm.S[s1][s2] = fma(-sm.R[t][s1], r2, sm.S[s1][s2]);
-    }
-    __syncwarp();
-  }
-}
-
-// Plain Cholesky of S (n x n) into sm.R (upper); all threads call it.
-__device__ void chol_upper(PanelSmem& sm, int nb) {
-  const int tid = threadIdx.x;
-  for (int t = 0; t < nb; ++t) {
-    const double rtt = sqrt(fmax(sm.S[t][t], 0.0));
-    for (int s = t + tid; s < nb; s += blockDim.x) sm.R[t][s] = (s == t) ? rtt : sm.S[t][s] / rtt;
-    __syncthreads();
-    const int w = nb - t - 1;
-    for (int idx = tid; idx < w * w; idx += blockDim.x) {
-      const int s1 = t + 1 + idx / w, s2 = t + 1 + idx % w;
-      sm.S[s1][s2] -= sm.R[t][s1] * sm.R[t][s2];
-    }
-    __syncthreads();
-  }
-}
-
-// Forward substitution of the CTA's 64 rows: W(r, :) <- W(r, :) R^{-1} (R upper, kept x kept).
-__device__ void rows_trsm(PanelSmem& sm, int kept) {
-  const int r = threadIdx.x;
-  if (r < 64) {
-    for (int s = 0; s < kept; ++s) {
-      double x = sm.W[r][s];
-      for (int u = 0; u < s; ++u) x = fma(-sm.W[r][u], sm.R[u][s], x);
-      sm.W[r][s] = x / sm.R[s][s];
-    }
-  }
-  __syncthreads();
-}
-
-// Gram partial of the W tile (kept x kept): upper triangle computed, mirrored.
-__device__ void tile_gram(const PanelSmem& sm, int kept, int rows_valid, double* G) {
-  const int tid = threadIdx.x, c1 = tid >> 2;
-  for (int q = 0; q < 16; ++q) {
-    const int c2 = (tid & 3) + 4 * q;
-    if (c2 < c1) continue;
-    double s = 0.0;
-    if (c1 < kept && c2 < kept)
-      for (int rr = 0; rr < rows_valid; ++rr) s = fma(sm.W[rr][c1], sm.W[rr][c2], s);
-    G[c1 * MAXB + c2] = s;
-    G[c2 * MAXB + c1] = s;
-  }
-}
-
-// k_pchol (one CTA): pivoted Cholesky of the panel Gram matrix with the robust
-// filter; publishes the pivots (ord), the kept count, R11 and performs the block
-// swap of perm and diags (matlab/RBRP.m:81-99: K1 = block positions not kept,
-// ascending; K2 = kept positions outside the block, in pivot order).
-__global__ void __launch_bounds__(256)
-k_pchol(const double* __restrict__ G, int m, State* st, double tol_loc, const int* __restrict__ js,
-        int* __restrict__ perm, double* __restrict__ diags, double* __restrict__ R11g, int* __restrict__ ordg,
-        int* __restrict__ Jg, int* __restrict__ K1g, int* __restrict__ K2g) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  PanelSmem& sm = *reinterpret_cast<PanelSmem*>(dyn_smem);
-  const int tid = threadIdx.x;
-  const int nb = st->bs_sampled, i = st->i;
-  for (int idx = tid; idx < nb * nb; idx += blockDim.x) sm.S[idx / nb][idx % nb] = G[(idx / nb) * MAXB + idx % nb];
-  __syncthreads();
-  if (tid < 32) {
-    const int kw = pivoted_chol_filter_warp(sm, nb, min(nb, m), tol_loc);
-    if (tid == 0) sm.stop = kw;
-  }
-  __syncthreads();
-  const int kept = sm.stop;
-  for (int idx = tid; idx < MAXB * MAXB; idx += blockDim.x) {
-    const int a = idx / MAXB, c = idx % MAXB;
-    R11g[idx] = (a < kept && c < kept && c >= a) ? sm.R[a][c] : 0.0;
-  }
-  if (tid < MAXB) ordg[tid] = sm.ord[tid];
-  if (tid == 0) {
-    int J[MAXB], K1[MAXB], K2[MAXB];
-    int nK = 0;
-    for (int s = 0; s < kept; ++s) J[s] = js[sm.ord[s]];
-    int nk1 = 0;
-    for (int p = i; p < i + kept; ++p) {
-      bool in = false;
-      for (int s = 0; s < kept; ++s) in |= (J[s] == p);
-      if (!in) K1[nk1++] = p;
-    }
-    for (int s = 0; s < kept; ++s)
-      if (J[s] < i || J[s] >= i + kept) K2[nK++] = J[s];
-    int Tperm[MAXB];
-    for (int s = 0; s < kept; ++s) Tperm[s] = perm[J[s]];
-    for (int t = 0; t < nK; ++t) {
-      perm[K2[t]] = perm[K1[t]];
-      diags[K2[t]] = diags[K1[t]];
-    }
-    for (int s = 0; s < kept; ++s) perm[i + s] = Tperm[s];
-    for (int s = 0; s < kept; ++s) Jg[s] = J[s];
-    for (int t = 0; t < nK; ++t) { K1g[t] = K1[t]; K2g[t] = K2[t]; }
-    st->bs = kept;
-    st->nK = nK;
-    st->zero_panel = kept == 0;
-  }
-}
-
-// Load an upper-triangular kept x kept factor (MAXB stride) into sm.R.
-__device__ __forceinline__ void load_factor(PanelSmem& sm, const double* __restrict__ Rg, int kept) {
-  for (int idx = threadIdx.x; idx < kept * kept; idx += blockDim.x) sm.R[idx / kept][idx % kept] = Rg[(idx / kept) * MAXB + idx % kept];
-}
-
-// Q1 = V(:, ord[:kept]) R11^{-1} for 64 rows per CTA, and the Gram partial of Q1.
-__global__ void __launch_bounds__(256)
-k_panel1(const double* __restrict__ V, int m, const State* __restrict__ st, const double* __restrict__ R11g,
-         const int* __restrict__ ordg, double* __restrict__ Q1, double* __restrict__ G2part) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  PanelSmem& sm = *reinterpret_cast<PanelSmem*>(dyn_smem);
-  const int tid = threadIdx.x;
-  const int kept = st->bs;
-  if (kept == 0) return;
-  load_factor(sm, R11g, kept);
-  const int r0 = blockIdx.x * 64;
-  const int rows_valid = max(0, min(64, m - r0));
-  for (int idx = tid; idx < 64 * kept; idx += blockDim.x) {
-    const int rr = idx & 63, s = idx >> 6, r = r0 + rr;
-    sm.W[rr][s] = r < m ? V[r + (int64_t)ordg[s] * m] : 0.0;
-  }
-  __syncthreads();
-  rows_trsm(sm, kept);
-  for (int idx = tid; idx < 64 * kept; idx += blockDim.x) {
-    const int rr = idx & 63, s = idx >> 6, r = r0 + rr;
-    if (r < m) Q1[r + (int64_t)s * m] = sm.W[rr][s];
-  }
-  tile_gram(sm, kept, rows_valid, G2part + (int64_t)blockIdx.x * MAXB * MAXB);
-}
-
-// k_chol2 (one CTA): R2 = chol(Q1^T Q1) and the panel R = R2 R11 into R(I2, I2)
-// (matlab/RBRP.m:78); R2 is published for the second row solve.
-__global__ void __launch_bounds__(256)
-k_chol2(const double* __restrict__ G2, const State* __restrict__ st, const double* __restrict__ R11g,
-        double* __restrict__ R2g, double* __restrict__ R, int64_t ldr) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  PanelSmem& sm = *reinterpret_cast<PanelSmem*>(dyn_smem);
-  const int tid = threadIdx.x;
-  const int kept = st->bs, i = st->i;
-  if (kept == 0) return;
-  for (int idx = tid; idx < kept * kept; idx += blockDim.x) sm.S[idx / kept][idx % kept] = G2[(idx / kept) * MAXB + idx % kept];
-  __syncthreads();
-  if (tid < 32) chol_upper_warp(sm, kept);
-  __syncthreads();
-  for (int idx = tid; idx < MAXB * MAXB; idx += blockDim.x) {
-    const int a = idx / MAXB, c = idx % MAXB;
-    R2g[idx] = (a < kept && c < kept && c >= a) ? sm.R[a][c] : 0.0;
-  }
-  for (int idx = tid; idx < kept * kept; idx += blockDim.x) {
-    const int a = idx / kept, c = idx % kept;
-    double v = 0.0;
-    if (c >= a)
-      for (int u = a; u <= c; ++u) v = fma(sm.R[a][u], R11g[u * MAXB + c], v);
-    R[(int64_t)(i + a) * ldr + (i + c)] = v;
-  }
-}
-
 // Column swap of the rows above the block: R(:i, K2) = R(:i, K1); R(:i, I2) = R(:i, J).
-__global__ void k_swap_R(double* __restrict__ R, int64_t ldr, const State* __restrict__ st,
-                         const int* __restrict__ Jg, const int* __restrict__ K1g, const int* __restrict__ K2g) {
-  const int i = st->i, kept = st->bs, nK = st->nK;
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per row, two block positions per lane, every load before the first store (a
+// thread per row walked 64 scattered columns in turn: 33 us at 640 rows of 8192 columns,
+// now 4.2).
+__global__ void __launch_bounds__(256)
+k_swap_R(double* __restrict__ R, int64_t ldr, const State* __restrict__ st, const int* __restrict__ Jg,
+         const int* __restrict__ K1g, const int* __restrict__ K2g) {
+  const int i = st->i, kept = st->bs, nK = st->nK, lane = threadIdx.x & 31;
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= i || kept == 0) return;
   double* Rr = R + (int64_t)row * ldr;
-  double tmp[MAXB];
-  for (int s = 0; s < kept; ++s) tmp[s] = Rr[Jg[s]];
-  for (int t = 0; t < nK; ++t) Rr[K2g[t]] = Rr[K1g[t]];
-  for (int s = 0; s < kept; ++s) Rr[i + s] = tmp[s];
-}
-
-// Second CholQR pass: Q_blk = Q1 R2^{-1}, 64 rows per CTA.
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_panel2(const double* __restrict__ Q1, int m, const State* __restrict__ st, const double* __restrict__ R2g,
-         T* __restrict__ Q, int64_t ldq, int q_at_i) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  PanelSmem& sm = *reinterpret_cast<PanelSmem*>(dyn_smem);
-  const int tid = threadIdx.x;
-  const int kept = st->bs, i = st->i;
-  if (kept == 0) return;
-  load_factor(sm, R2g, kept);
-  const int r0 = blockIdx.x * 64;
-  for (int idx = tid; idx < 64 * kept; idx += blockDim.x) {
-    const int rr = idx & 63, s = idx >> 6, r = r0 + rr;
-    sm.W[rr][s] = r < m ? Q1[r + (int64_t)s * m] : 0.0;
+  double tj[2], tk[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int s = lane + 32 * u;
+    tj[u] = s < kept ? Rr[Jg[s]] : 0.0;
+    tk[u] = s < nK ? Rr[K1g[s]] : 0.0;
   }
-  __syncthreads();
-  rows_trsm(sm, kept);
-  for (int idx = tid; idx < 64 * kept; idx += blockDim.x) {
-    const int rr = idx & 63, s = idx >> 6, r = r0 + rr;
-    if (r < m) Q[r + (int64_t)((q_at_i ? i : 0) + s) * ldq] = (T)sm.W[rr][s];
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int s = lane + 32 * u;
+    if (s < nK) Rr[K2g[s]] = tk[u];
+    if (s < kept) Rr[i + s] = tj[u];
   }
 }
 
@@ -647,29 +179,33 @@ k_panel2(const double* __restrict__ Q1, int m, const State* __restrict__ st, con
 // residual-norm downdate (python/RBRP.ipynb cell 11 lines 132, 154-158;
 // matlab/RBRP.m:103-104,112; the reference applies Householder reflectors to
 // the whole trailing matrix instead, gpu/rbrp.cu:297-330, 453-466).
-// CTA tile: KB basis vectors (KB >= kept, chosen on the host from b) x PC =
-// 4096 / KB positions, K loop over m in chunks of KC rows; every thread holds a
-// (KB / TY) x 4 accumulator block.  Each accumulator sums over the rows in
-// ascending order, so W is the same for every KB: KB only removes the work on
-// basis rows that do not exist (the FP64 pipe is the bound of this kernel).
+// CTA tile: KB basis vectors (KB >= kept, chosen on the host from b) x PC
+// positions, K loop over m in chunks of KC rows; every thread holds an MU x VP
+// accumulator block: 4 x 4 (PC = 4096 / KB), or 2 x 1 and PC = 8 or 16 where the
+// large tiles would not fill the SMs.  Each accumulator sums over the rows in
+// ascending order, so W is the same for every tile: the tile only spreads the
+// work and drops basis rows that do not exist (the FP64 pipe is the bound of
+// this kernel; 1000 x 1000, b = 40: 610 us a block in 16 large tiles, 120 in
+// small ones).
 // ===========================================================================
-template <int KB>
+template <int KB_, int VP_>
 struct ProjTile {
-  static constexpr int MU = KB < 4 ? KB : 4;     // basis rows per thread
+  static constexpr int KB = KB_, VP = VP_;
+  static constexpr int MU = VP == 4 ? 4 : KB >= 32 ? 2 : 1;    // basis rows per thread
   static constexpr int TY = KB / MU;             // thread rows
   static constexpr int TX = 256 / TY;            // thread columns
-  static constexpr int PC = TX * 4;              // positions per CTA
+  static constexpr int PC = TX * VP;             // positions per CTA
   static constexpr int KC = 4096 / PC < 32 ? 4096 / PC : 32;   // rows per K chunk
 };
 
-template <typename T, int KB>
+template <typename T, typename P>
 __global__ void __launch_bounds__(256)
 k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t lda,
           const int* __restrict__ perm, const State* __restrict__ st, int m, int n,
           double* __restrict__ R, int64_t ldr, double* __restrict__ diags,
           double* __restrict__ part_res, int* __restrict__ part_nnz) {
-  using P = ProjTile<KB>;
-  constexpr int PC = P::PC, KC = P::KC, TX = P::TX, TY = P::TY, MU = P::MU;
+  constexpr int KB = P::KB, VP = P::VP, PC = P::PC, KC = P::KC, TX = P::TX, TY = P::TY, MU = P::MU;
+  constexpr int NRED = PC < 64 ? 1 : PC / 64, RLEN = PC < 64 ? PC : 64;
   constexpr size_t kOps = sizeof(T) * (KC * KB + KC * (PC + 1));
   constexpr size_t kW = sizeof(double) * KB * (PC + 1);
   __shared__ __align__(16) unsigned char raw[kOps > kW ? kOps : kW];
@@ -678,8 +214,8 @@ k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t
   double(*Ws)[PC + 1] = reinterpret_cast<double(*)[PC + 1]>(raw);
   __shared__ int cs[PC];
   __shared__ double snew[PC];
-  __shared__ double red_s[PC / 64];
-  __shared__ int red_c[PC / 64];
+  __shared__ double red_s[NRED];
+  __shared__ int red_c[NRED];
   const int tid = threadIdx.x;
   // kept <= b <= KB by construction (the host picks KB from b); the clamp only keeps smem in bounds
   const int i = st->i, kept = min(st->bs, KB);
@@ -690,12 +226,13 @@ k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t
   }
   for (int t = tid; t < PC; t += 256) cs[t] = (pbase + t < n) ? perm[pbase + t] : -1;
   const int ty = tid / TX, tx = tid % TX;
-  const int me = (kept + TY - 1) / TY;   // <= MU
-  T acc[MU][4];
+  const int ty0 = (tid & ~31) / TX;      // the warp's first basis row
+  const int me = kept > ty0 ? (kept - ty0 + TY - 1) / TY : 0;   // <= MU
+  T acc[MU][VP];
 #pragma unroll
   for (int u = 0; u < MU; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = T(0);
+    for (int v = 0; v < VP; ++v) acc[u][v] = T(0);
   const T* Qb = Q + (int64_t)i * ldq;
   for (int r0 = 0; r0 < m; r0 += KC) {
     __syncthreads();
@@ -717,17 +254,18 @@ k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t
       constexpr int ME = decltype(mec)::value;
 #pragma unroll 4
       for (int kk = 0; kk < KC; ++kk) {
-        T qv[ME], av[4];
+        T qv[ME], av[VP];
 #pragma unroll
         for (int u = 0; u < ME; ++u) qv[u] = Qs[kk][ty + TY * u];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) av[v] = As[kk][tx + TX * v];
+        for (int v = 0; v < VP; ++v) av[v] = As[kk][tx + TX * v];
 #pragma unroll
         for (int u = 0; u < ME; ++u)
 #pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] = fma(qv[u], av[v], acc[u][v]);
+          for (int v = 0; v < VP; ++v) acc[u][v] = fma(qv[u], av[v], acc[u][v]);
       }
     };
+    if (me == 0) continue;
     if (MU == 1 || me <= 1) fmas(std::integral_constant<int, 1>{});
     else if (me <= 2) fmas(std::integral_constant<int, (MU < 2 ? MU : 2)>{});
     else if (me <= 3) fmas(std::integral_constant<int, (MU < 3 ? MU : 3)>{});
@@ -737,7 +275,7 @@ k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t
 #pragma unroll
   for (int u = 0; u < MU; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) Ws[ty + TY * u][tx + TX * v] = (double)acc[u][v];
+    for (int v = 0; v < VP; ++v) Ws[ty + TY * u][tx + TX * v] = (double)acc[u][v];
   __syncthreads();
   for (int idx = tid; idx < kept * PC; idx += 256) {
     const int a = idx / PC, c = idx % PC;
@@ -758,10 +296,10 @@ k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t
   __syncthreads();
   // CTA partial of the residual and of the nonzero count, positions in ascending order
   // in chunks of 64 (the sum order of the 64-position tile this kernel generalises)
-  if (tid < PC / 64) {
+  if (tid < NRED) {
     double sacc = 0.0;
     int c = 0;
-    for (int t = tid * 64; t < tid * 64 + 64; ++t) { sacc += snew[t]; c += snew[t] > 0.0; }
+    for (int t = tid * RLEN; t < (tid + 1) * RLEN; ++t) { sacc += snew[t]; c += snew[t] > 0.0; }
     red_s[tid] = sacc;
     red_c[tid] = c;
   }
@@ -769,7 +307,7 @@ k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t
   if (tid == 0) {
     double sacc = 0.0;
     int c = 0;
-    for (int t = 0; t < PC / 64; ++t) { sacc += red_s[t]; c += red_c[t]; }
+    for (int t = 0; t < NRED; ++t) { sacc += red_s[t]; c += red_c[t]; }
     part_res[blockIdx.x] = sacc;
     part_nnz[blockIdx.x] = c;
   }

@@ -7,7 +7,7 @@
 // is FP64-class arithmetic.  Here every FP64 quantity is a pair of floats
 // (hi + lo, ~48 significant bits) computed on the FP32 pipe with error-free
 // transformations: products by FMA splitting, sums by TwoSum.  The steps are
-// those of the FP64 panel kernels in rbrp_kernels.cuh (same pivot rule, same
+// those of the FP64 panel kernels in rbrp_panel64.cuh (same pivot rule, same
 // robust filter, same swap), so the FP64 path keeps its own kernels and these
 // serve the mixed-precision path.
 //
@@ -65,8 +65,8 @@ k_gram_df(const float* __restrict__ Ares, int64_t ld, const int* __restrict__ js
 
 using PcholDfSmem = PcholDfSmemT<MAXB>;
 
-// Pivoted Cholesky of the panel Gram matrix with the robust filter (same rule as
-// pivoted_chol_filter), LEAN_THREADS threads, no data movement for the swaps.  Publishes
+// Pivoted Cholesky of the panel Gram matrix with the robust filter (same rule as the
+// FP64 form's k_pchol), LEAN_THREADS threads, no data movement for the swaps.  Publishes
 // R11 (slot order, double-float pairs), ord, the kept count and performs the block swap.
 __global__ void __launch_bounds__(LEAN_THREADS)
 k_pchol_df(const double* __restrict__ G, int m, State* st, double tol_loc, const int* __restrict__ js,
@@ -125,7 +125,7 @@ k_pchol_df(const double* __restrict__ G, int m, State* st, double tol_loc, const
     }
   }
   if (tid < MAXB) ordg[tid] = sm.ord[tid];
-  block_swap_parallel(sm, i, kept, js, perm, diags, Jg, K1g, K2g, st);
+  block_swap_parallel<MAXB>(sm, i, kept, js, perm, diags, Jg, K1g, K2g, st);
 }
 
 // Q_blk = V(:, ord[:kept]) R11^{-1} in double-float as the product with the explicit

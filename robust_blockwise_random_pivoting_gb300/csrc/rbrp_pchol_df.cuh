@@ -25,8 +25,8 @@ struct PcholDfSmemT {
 // Block swap of perm and diags (matlab/RBRP.m:81-99), in parallel: K1 = block
 // positions not kept (ascending), K2 = kept positions outside the block (pivot
 // order), compacted with warp ballots.  All threads call it after `kept` is known.
-template <int BB>
-__device__ void block_swap_parallel(PcholDfSmemT<BB>& sm, int i, int kept, const int* __restrict__ js,
+template <int BB, typename Smem>
+__device__ void block_swap_parallel(Smem& sm, int i, int kept, const int* __restrict__ js,
                                     int* __restrict__ perm, double* __restrict__ diags, int* __restrict__ Jg,
                                     int* __restrict__ K1g, int* __restrict__ K2g, State* st) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;

@@ -47,6 +47,7 @@ def test_projection_matches_the_fp64_pipe(kind, m, n, b):
     # add the representation (2^-54 of each row's largest entry per value) and the dropped classes
     norm = np.array([np.linalg.norm(c / s) * s if s > 0 else 0.0 for c, s in zip(A.T, np.abs(A).max(0))])
     bound = (m + 1) * EPS * norm[:, None] + m * 2.0 ** -53 * np.abs(A).max(0)[:, None]
+    assert np.isfinite(L0).all() and np.isfinite(L1).all()
     rest = perm0[k0:]
     assert np.all(np.abs(L0 - L1)[rest] <= bound[rest])
 
@@ -65,3 +66,21 @@ def test_blocks_after_the_first_follow_the_same_skeleton(m, n, b, kmax):
     # a Gaussian matrix of these shapes: kappa(A_S) < 30, one Gram-Schmidt pass, m eps kappa^2
     d = np.linalg.norm(got[0][2] - got[1][2]) / np.linalg.norm(got[1][2])
     assert d <= m * EPS * 900, d
+
+
+def test_slice_gemm_timeout_is_clean():
+    """The projection's bounded waits run out under a budget of one clock: status 7, and the
+    same handle reproduces an untouched one's results afterwards."""
+    from robust_blockwise_random_pivoting_gb300._lib import RBRPError
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    A = colmajor(matrix("normal", 900, 700))
+    with Handle(0) as fresh:
+        want = fresh.column_id(A, b=64, tol=None, kmax=200, seed=0)
+    with Handle(0) as h:
+        h.set_wait_budget(1)
+        with pytest.raises(RBRPError) as e:
+            h.column_id(A, b=64, tol=None, kmax=200, seed=0)
+        assert e.value.status == 7
+        h.set_wait_budget(0)
+        got = h.column_id(A, b=64, tol=None, kmax=200, seed=0)
+    assert torch.equal(got.perm, want.perm) and torch.equal(got.T, want.T)
