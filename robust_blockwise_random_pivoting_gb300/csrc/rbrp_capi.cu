@@ -1,5 +1,5 @@
-// rbrp_capi.cu - C ABI, workspace management, interpolation-matrix solve
-// (a10) and ID-error kernel (a11) of the GB300 RBRP library.
+// rbrp_capi.cu - C ABI, workspace management and ID-error kernel (a11) of the
+// GB300 RBRP library.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -14,272 +14,6 @@
 #include "../../include/rbrp_gb300_testing.h"
 
 namespace rbrp {
-
-// ===========================================================================
-// a10: T = R11^{-1} R12 (matlab/driver.m:86; gpu/interp.cu:45-105 solves the
-// same triangular system after re-factoring a sketch; gpu/id_cpqr.cu:133-136).
-// R is the RBRP factor (row major, ld = n, indexed by position): R11 =
-// R[:k, :k] upper triangular, R12 = R[:k, k:].  T is k x (n-k), column major.
-// ===========================================================================
-__global__ void k_gather_T(const double* __restrict__ R, int64_t ldr, int k, int ncols, double* __restrict__ T) {
-  __shared__ double tile[32][33];
-  const int c0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int q = 0; q < 32; q += 8) {
-    const int a = a0 + ty + q, c = c0 + tx;
-    tile[ty + q][tx] = (a < k && c < ncols) ? R[(int64_t)a * ldr + k + c] : 0.0;
-  }
-  __syncthreads();
-  for (int q = 0; q < 32; q += 8) {
-    const int c = c0 + ty + q, a = a0 + tx;
-    if (a < k && c < ncols) T[a + (int64_t)c * k] = tile[tx][ty + q];
-  }
-}
-
-struct TrsmSmem {
-  double Rs[64][65];
-  double Xs[64][33];
-  double Acc[64][33];
-};
-
-// Block back substitution, 32 right-hand sides per CTA, 64-row diagonal blocks
-// from the bottom; the update of a row block by the solved blocks below it is a
-// 64 x 64 x 32 product per step.
-__global__ void __launch_bounds__(256) k_trsm_T(const double* __restrict__ R, int64_t ldr, int k, int ncols,
-                                                double* __restrict__ T) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  TrsmSmem& sm = *reinterpret_cast<TrsmSmem*>(dyn_smem);
-  const int tid = threadIdx.x;
-  const int c0 = blockIdx.x * 32;
-  const int nc = min(32, ncols - c0);
-  const int nbk = (k + 63) / 64;
-  const int x = tid >> 2;  // output row of this thread in the 64 x 32 tile
-  for (int bi = nbk - 1; bi >= 0; --bi) {
-    const int b0 = bi * 64, bl = min(64, k - b0);
-    for (int idx = tid; idx < 64 * 32; idx += 256) {
-      const int xr = idx & 63, c = idx >> 6;
-      sm.Acc[xr][c] = (xr < bl && c < nc) ? T[(b0 + xr) + (int64_t)(c0 + c) * k] : 0.0;
-    }
-    double acc[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = 0.0;
-    for (int bj = bi + 1; bj < nbk; ++bj) {
-      const int cr = bj * 64, cl = min(64, k - cr);
-      __syncthreads();
-      for (int idx = tid; idx < 64 * 64; idx += 256) {
-        const int y = idx & 63, xr = idx >> 6;
-        sm.Rs[xr][y] = (xr < bl && y < cl) ? R[(int64_t)(b0 + xr) * ldr + cr + y] : 0.0;
-      }
-      for (int idx = tid; idx < 64 * 32; idx += 256) {
-        const int y = idx & 63, c = idx >> 6;
-        sm.Xs[y][c] = (y < cl && c < nc) ? T[(cr + y) + (int64_t)(c0 + c) * k] : 0.0;
-      }
-      __syncthreads();
-#pragma unroll 4
-      for (int y = 0; y < 64; ++y) {
-        const double r = sm.Rs[x][y];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) acc[q] = fma(r, sm.Xs[y][(tid & 3) + 4 * q], acc[q]);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sm.Acc[x][(tid & 3) + 4 * q] -= acc[q];
-    for (int idx = tid; idx < 64 * 64; idx += 256) {
-      const int y = idx & 63, xr = idx >> 6;
-      sm.Rs[xr][y] = (xr < bl && y < bl && y >= xr) ? R[(int64_t)(b0 + xr) * ldr + b0 + y] : 0.0;
-    }
-    __syncthreads();
-    if (tid < nc) {
-      for (int xr = bl - 1; xr >= 0; --xr) {
-        double v = sm.Acc[xr][tid];
-        for (int y = xr + 1; y < bl; ++y) v = fma(-sm.Rs[xr][y], sm.Acc[y][tid], v);
-        sm.Acc[xr][tid] = v / sm.Rs[xr][xr];
-      }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < 64 * 32; idx += 256) {
-      const int xr = idx & 63, c = idx >> 6;
-      if (xr < bl && c < nc) T[(b0 + xr) + (int64_t)(c0 + c) * k] = sm.Acc[xr][c];
-    }
-    __syncthreads();
-  }
-}
-
-// Double-float form of the same solve.  GB300's FP64 pipe issues ~1/64 of its
-// FP32 pipe's rate, so the whole solve runs in double-float arithmetic on the
-// FP32 pipe: R11 and the right-hand sides are split once into float pairs
-// (hi + lo, ~48 significant bits) by k_split_df, the block updates use
-// error-free products (FMA split) and TwoSum, the 64 x 64 diagonal blocks are
-// solved in double-float too, and T is joined back to FP64 once at the end.
-__global__ void k_split_df(const double* __restrict__ R, int64_t ldr, int k, int ncols,
-                           float2* __restrict__ R11df, float2* __restrict__ Tdf) {
-  const int64_t total11 = (int64_t)k * k, totalT = (int64_t)k * ncols;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total11 + totalT;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    double x;
-    float2* dst;
-    if (idx < total11) {  // R11 row major (ld k), upper triangle
-      const int a = (int)(idx / k), c = (int)(idx % k);
-      x = c >= a ? R[(int64_t)a * ldr + c] : 0.0;
-      dst = R11df + idx;
-    } else {              // T column major (ld k), from R12 row major
-      const int64_t t = idx - total11;
-      const int c = (int)(t / k), a = (int)(t % k);
-      x = R[(int64_t)a * ldr + k + c];
-      dst = Tdf + t;
-    }
-    const float hi = (float)x;
-    *dst = make_float2(hi, (float)(x - (double)hi));
-  }
-}
-
-__global__ void k_join_df(const float2* __restrict__ Tdf, int64_t count, double* __restrict__ T) {
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += (int64_t)gridDim.x * blockDim.x) {
-    const float2 v = Tdf[idx];
-    T[idx] = (double)v.x + (double)v.y;
-  }
-}
-
-__device__ __forceinline__ float2 df2_two_sum(float a, float b) {
-  const float s = a + b;
-  const float bb = s - a;
-  return make_float2(s, (a - (s - bb)) + (b - bb));
-}
-__device__ __forceinline__ float2 df2_fast(float a, float b) {
-  const float s = a + b;
-  return make_float2(s, b - (s - a));
-}
-// (sh, sl) += a * b in double-float: the exact product a.x b.x = p + e (FMA split)
-// and the cross terms go into the low part by FMAs, the high parts are added by
-// TwoSum with its error into the low part (12 FP32 operations).
-__device__ __forceinline__ void df_mac(float& sh, float& sl, float2 a, float2 b) {
-  const float p = a.x * b.x;
-  const float e = fmaf(a.x, b.x, -p);
-  sl = fmaf(a.y, b.x, fmaf(a.x, b.y, sl + e));
-  const float t = sh + p;
-  const float bb = t - sh;
-  sl += (sh - (t - bb)) + (p - bb);
-  sh = t;
-}
-__device__ __forceinline__ float2 df2_add(float2 a, float2 b) {
-  float2 s = df2_two_sum(a.x, b.x);
-  s.y += a.y + b.y;
-  return df2_fast(s.x, s.y);
-}
-__device__ __forceinline__ float2 df2_mul(float2 a, float2 b) {
-  const float p = a.x * b.x;
-  float e = fmaf(a.x, b.x, -p);
-  e = fmaf(a.x, b.y, e);
-  e = fmaf(a.y, b.x, e);
-  return df2_fast(p, e);
-}
-__device__ __forceinline__ float2 df2_recip(float2 b) {
-  const float q = 1.0f / b.x;
-  const float2 r = df2_add(make_float2(1.0f, 0.0f), df2_mul(make_float2(-q, 0.0f), b));
-  return df2_fast(q, q * r.x);
-}
-
-// The double-float solve is right-looking: block row b (64 rows from the bottom
-// up) is solved for all columns at once, then its product with R11(0:b0, b) is
-// subtracted from every earlier row.  Each step has work over rows and columns,
-// so the whole GPU stays busy however few columns T has.  (A left-looking form,
-// one CTA per 32 columns for the whole solve, had as many CTAs as column tiles:
-// 120 for the adjoint's 3822 columns; it took 8.5 ms at 8192 x 8192, k = 2033,
-// against 7.6, and the same 16.2 ms at 16384.)
-//
-// k_trsm_rl_diag: X_b = R11(b, b)^{-1} B_b, one warp per column, lane l holding
-// rows l and l + 32 of the block; back substitution with the solved value
-// broadcast by shuffles, in double-float.
-__global__ void __launch_bounds__(256) k_trsm_rl_diag(const float2* __restrict__ R11, int k, int ncols, int b0, int bl,
-                                                      float2* __restrict__ T) {
-  __shared__ float2 Rd[64][65];
-  __shared__ float2 inv[64];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
-    const int xr = idx >> 6, y = idx & 63;
-    Rd[xr][y] = (xr < bl && y < bl && y >= xr) ? R11[(int64_t)(b0 + xr) * k + b0 + y] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  if (tid < bl) inv[tid] = df2_recip(Rd[tid][tid]);
-  __syncthreads();
-  const int c = blockIdx.x * 8 + w;
-  if (c >= ncols) return;
-  float2* col = T + b0 + (int64_t)c * k;
-  float2 v0 = lane < bl ? col[lane] : make_float2(0.f, 0.f);
-  float2 v1 = lane + 32 < bl ? col[lane + 32] : make_float2(0.f, 0.f);
-  for (int r = bl - 1; r >= 0; --r) {
-    // the owner of row r finishes it; every lane then removes its rows' share
-    const float2 mine = r < 32 ? v0 : v1;
-    const float2 xr = df2_mul(mine, inv[r]);
-    const float2 x = make_float2(__shfl_sync(0xffffffffu, xr.x, r & 31), __shfl_sync(0xffffffffu, xr.y, r & 31));
-    if (lane == (r & 31)) {
-      if (r < 32) v0 = x; else v1 = x;
-    }
-    if (lane < r) df_mac(v0.x, v0.y, make_float2(-Rd[lane][r].x, -Rd[lane][r].y), x);
-    if (lane + 32 < r) df_mac(v1.x, v1.y, make_float2(-Rd[lane + 32][r].x, -Rd[lane + 32][r].y), x);
-    // keep the low parts small, as the left-looking solve does after each block
-    if (lane < r) v0 = df2_fast(v0.x, v0.y);
-    if (lane + 32 < r) v1 = df2_fast(v1.x, v1.y);
-  }
-  if (lane < bl) col[lane] = v0;
-  if (lane + 32 < bl) col[lane + 32] = v1;
-}
-
-// k_trsm_rl_update: B(rows of tile, cols of tile) -= R11(rows, b) X_b for the
-// 64 x 64 tile (blockIdx.x: rows below b0, blockIdx.y: columns), in double-float:
-// each thread two rows (x, x + 32) and 8 columns, so every shared load of X feeds
-// two products; each product exact (FMA split) and summed by TwoSum.
-struct TrsmRlSmem {
-  float2 Rs[64][65];
-  float2 Xs[64][65];
-};
-__global__ void __launch_bounds__(256) k_trsm_rl_update(const float2* __restrict__ R11, int k, int ncols, int b0,
-                                                        int bl, float2* __restrict__ T) {
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  TrsmRlSmem& sm = *reinterpret_cast<TrsmRlSmem*>(dyn_smem);
-  const int tid = threadIdx.x;
-  const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
-  const int nc = min(64, ncols - c0);
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
-    const int xr = idx >> 6, y = idx & 63;
-    const float2 v = y < bl ? R11[(int64_t)(r0 + xr) * k + b0 + y] : make_float2(0.f, 0.f);
-    sm.Rs[xr][y] = make_float2(-v.x, -v.y);
-  }
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
-    const int y = idx & 63, c = idx >> 6;
-    sm.Xs[y][c] = (y < bl && c < nc) ? T[(b0 + y) + (int64_t)(c0 + c) * k] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  const int x = tid >> 3, cq = tid & 7;  // rows x and x + 32, columns cq + 8 q
-  float sh[2][8], sl[2][8];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sh[h][q] = sl[h][q] = 0.f;
-#pragma unroll 2
-  for (int y = 0; y < 64; ++y) {
-    const float2 ra = sm.Rs[x][y], rb = sm.Rs[x + 32][y];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float2 xv = sm.Xs[y][cq + 8 * q];
-      df_mac(sh[0][q], sl[0][q], ra, xv);
-      df_mac(sh[1][q], sl[1][q], rb, xv);
-    }
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int row = r0 + x + 32 * h;  // r0 + 63 < b0: every row of the tile exists
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int c = cq + 8 * q;
-      if (c < nc) {
-        float2* t = T + row + (int64_t)(c0 + c) * k;
-        *t = df2_add(*t, make_float2(sh[h][q], sl[h][q]));
-      }
-    }
-  }
-}
 
 // ===========================================================================
 // a11: ||A(:, rd) - A(:, S) T||_F^2 in FP64 (python/RBRP.ipynb cell 7 lines
@@ -370,8 +104,7 @@ rbrp_status cuda_check(rbrp_handle h, cudaError_t e, const char* what) {
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// cudaMalloc for what a run cannot do without: the slices, which it can, make room if needed.
-static rbrp_status device_alloc(rbrp_handle h, void** ptr, size_t bytes, const char* what) {
+rbrp_status device_alloc(rbrp_handle h, void** ptr, size_t bytes, const char* what) {
   cudaError_t e = cudaMalloc(ptr, bytes);
   if (e == cudaErrorMemoryAllocation && h->sl_ws) {
     cudaGetLastError();
@@ -539,55 +272,6 @@ bool ensure_slices(rbrp_handle h, int m, int n) {
   }
   h->sl_maxsplit = maxsplit;
   return true;
-}
-
-rbrp_status solve_T(rbrp_handle h, int k, int n) {
-  const size_t bytes = (size_t)k * (size_t)(n - k) * sizeof(double);
-  if (bytes > h->T_bytes) {
-    if (h->T) cudaFree(h->T);
-    h->T = nullptr;
-    h->T_bytes = 0;
-    rbrp_status s = device_alloc(h, (void**)&h->T, bytes, "cudaMalloc(T)");
-    if (s != RBRP_OK) return s;
-    h->T_bytes = bytes;
-  }
-  const int ncols = n - k;
-  rbrp_status s;
-  if (h->tsolve_fp64) {
-    dim3 g1((ncols + 31) / 32, (k + 31) / 32), b1(32, 8);
-    k_gather_T<<<g1, b1, 0, h->stream>>>(h->R, n, k, ncols, h->T);
-    s = cuda_check(h, cudaFuncSetAttribute(k_trsm_T, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(TrsmSmem)), "cudaFuncSetAttribute(k_trsm_T)");
-    if (s != RBRP_OK) return s;
-    k_trsm_T<<<(ncols + 31) / 32, 256, sizeof(TrsmSmem), h->stream>>>(h->R, n, k, ncols, h->T);
-  } else {
-    // double-float operands: R11 (k x k) and the right-hand sides (k x ncols), ~16 bytes per T entry
-    const size_t need = ((size_t)k * k + (size_t)k * ncols) * sizeof(float2);
-    if (need > h->df_bytes) {
-      if (h->df_buf) cudaFree(h->df_buf);
-      h->df_buf = nullptr;
-      h->df_bytes = 0;
-      s = device_alloc(h, &h->df_buf, need, "cudaMalloc(T solve operands)");
-      if (s != RBRP_OK) return s;
-      h->df_bytes = need;
-    }
-    float2* R11df = static_cast<float2*>(h->df_buf);
-    float2* Tdf = R11df + (size_t)k * k;
-    k_split_df<<<1216, 256, 0, h->stream>>>(h->R, n, k, ncols, R11df, Tdf);
-    s = cuda_check(h, cudaFuncSetAttribute(k_trsm_rl_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(TrsmRlSmem)), "cudaFuncSetAttribute(k_trsm_rl_update)");
-    if (s != RBRP_OK) return s;
-    const int nbk = (k + 63) / 64;
-    for (int bi = nbk - 1; bi >= 0; --bi) {
-      const int b0 = bi * 64, bl = std::min(64, k - b0);
-      k_trsm_rl_diag<<<(ncols + 7) / 8, 256, 0, h->stream>>>(R11df, k, ncols, b0, bl, Tdf);
-      if (b0 > 0)
-        k_trsm_rl_update<<<dim3(b0 / 64, (ncols + 63) / 64), 256, sizeof(TrsmRlSmem), h->stream>>>(R11df, k, ncols,
-                                                                                                   b0, bl, Tdf);
-    }
-    k_join_df<<<1216, 256, 0, h->stream>>>(Tdf, (int64_t)k * ncols, h->T);
-  }
-  return cuda_check(h, cudaGetLastError(), "T solve launch");
 }
 
 template <typename T>
@@ -851,7 +535,7 @@ rbrp_status rbrp_destroy(rbrp_handle h) {
     if (h->ws) cudaFree(h->ws);
     if (h->T) cudaFree(h->T);
     release_slices(h);
-    if (h->df_buf) cudaFree(h->df_buf);
+    if (h->ts_ws) cudaFree(h->ts_ws);
     if (h->hostA_dev) cudaFree(h->hostA_dev);
     if (h->given_order) cudaFree(h->given_order);
     if (h->adj_ws) cudaFree(h->adj_ws);

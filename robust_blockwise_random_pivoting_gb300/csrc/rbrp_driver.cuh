@@ -417,8 +417,11 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   }
   if (dPerm) cudaMemcpyAsync(dPerm, h->perm, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, st);
   cudaEventRecord(h->ev_end, st);
+  cudaMemcpyAsync(h->hst, h->st, sizeof(State), cudaMemcpyDeviceToHost, st);
   s = cuda_check(h, cudaStreamSynchronize(st), "RBRP finalisation");
   if (s != RBRP_OK) return s;
+  if (h->hst->status == tc::ST_ERR_TIMEOUT)
+    return set_error(h, RBRP_ERR_DEVICE_TIMEOUT, "a device-side wait timed out; the kernel aborted cleanly");
 
   prof_collect(h);
   const int nb = h->hst->nblocks;

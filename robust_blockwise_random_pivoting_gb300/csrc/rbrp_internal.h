@@ -85,8 +85,8 @@ struct rbrp_handle_st {
   // interpolation matrix of the last run
   double* T = nullptr;
   size_t T_bytes = 0;
-  void* df_buf = nullptr;      // double-float operands of the T solve
-  size_t df_bytes = 0;
+  void* ts_ws = nullptr;       // operands of the T solve (rbrp_tsolve.cu)
+  size_t ts_bytes = 0;
 
   // Gaussian sketch matrix (rbrp_sketch.cu)
   void* sketch_ws = nullptr;
@@ -179,6 +179,9 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
                      int* dPerm, rbrp_result* out);
 
 rbrp_status solve_T(rbrp_handle h, int k, int n);
+
+// cudaMalloc for what a run cannot do without (the slices of A, which it can, make room).
+rbrp_status device_alloc(rbrp_handle h, void** ptr, size_t bytes, const char* what);
 
 // 2-D FP32 TMA descriptor (inner dimension contiguous, 128-byte swizzle).
 rbrp_status make_tmap_f32(rbrp_handle h, void* map, const float* base, uint64_t inner, uint64_t outer,

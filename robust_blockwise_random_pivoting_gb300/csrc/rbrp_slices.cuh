@@ -67,6 +67,16 @@ __device__ __forceinline__ int slice_exponent(unsigned hi) {
   return (ex ? ex : 1) - 1022;
 }
 
+// Slice s of eight consecutive values, 16 bytes.
+__device__ __forceinline__ void store_slice8(unsigned short* dst, const unsigned short (&d)[8][SL], int s) {
+  uint4 v;
+  v.x = d[0][s] | ((unsigned)d[1][s] << 16);
+  v.y = d[2][s] | ((unsigned)d[3][s] << 16);
+  v.z = d[4][s] | ((unsigned)d[5][s] << 16);
+  v.w = d[6][s] | ((unsigned)d[7][s] << 16);
+  *reinterpret_cast<uint4*>(dst) = v;
+}
+
 // Slices of the columns of an FP64 matrix: column c into rows s * srows + c of out
 // (ldk BF16 values each, zero past m), its exponent into ex[c].  One warp per column:
 // a pass for the largest entry, then a second one (L2) that writes 16 bytes per lane
@@ -89,14 +99,7 @@ k_slice_cols(const double* __restrict__ A, int64_t lda, int m, int n, int64_t sr
 #pragma unroll
     for (int u = 0; u < 8; ++u) slice_digits(r0 + u < m ? col[r0 + u] : 0.0, e, d[u]);
 #pragma unroll
-    for (int s = 0; s < SL; ++s) {
-      uint4 v;
-      v.x = d[0][s] | ((unsigned)d[1][s] << 16);
-      v.y = d[2][s] | ((unsigned)d[3][s] << 16);
-      v.z = d[4][s] | ((unsigned)d[5][s] << 16);
-      v.w = d[6][s] | ((unsigned)d[7][s] << 16);
-      *reinterpret_cast<uint4*>(out + ((int64_t)s * srows + c) * ldk + r0) = v;
-    }
+    for (int s = 0; s < SL; ++s) store_slice8(out + ((int64_t)s * srows + c) * ldk + r0, d, s);
   }
 }
 
@@ -237,8 +240,8 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   extern __shared__ uint8_t sl_raw[];
   SliceSmem& sm = *reinterpret_cast<SliceSmem*>((reinterpret_cast<uintptr_t>(sl_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int p0, brow, s0, nst, nh;   // first M row, first N row, stage range, halves
-  if (!epi.tile(p0, brow, s0, nst, nh)) return;  // uniform over the CTA
+  int p0, brow, s0, nst, nh, ax;   // first M row, first N row, stage range, halves, M's first value of k
+  if (!epi.tile(p0, brow, s0, nst, nh, ax)) return;  // uniform over the CTA
   volatile int* abort = &sm.abort;
   if (threadIdx.x == 0) {
     for (int s = 0; s < SL; ++s) {
@@ -286,7 +289,7 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         if (s >= 1 && !mbar_wait(&sm.aempty[i], (uint32_t)(s & 1) ^ 1, abort, budget)) { ok = false; break; }
         if (elect_one()) {
           mbar_expect_tx(&sm.afull[i], SL_A_BYTES);
-          tma_load_2d(sm.as[i], &tmA, &sm.afull[i], x, (int)(i * a_rows) + p0);
+          tma_load_2d(sm.as[i], &tmA, &sm.afull[i], ax + x, (int)(i * a_rows) + p0);
         }
         __syncwarp();
         aissued = s * SL + i + 1;
@@ -435,8 +438,9 @@ struct ProjEpi {
   const int* exA;
   const int* exQ;
   double* Wpart;
-  __device__ bool tile(int& p0, int& brow, int& s0, int& nst, int& nh) const {
+  __device__ bool tile(int& p0, int& brow, int& s0, int& nst, int& nh, int& ax) const {
     const int kept = st->bs;
+    ax = 0;
     p0 = st->i + kept + blockIdx.x * BM;
     brow = 0;
     s0 = blockIdx.y * sps;

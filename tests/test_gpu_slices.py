@@ -68,6 +68,30 @@ def test_blocks_after_the_first_follow_the_same_skeleton(m, n, b, kmax):
     assert d <= m * EPS * 900, d
 
 
+@pytest.mark.parametrize("k,n", [(1, 40), (63, 95), (64, 129), (65, 128), (255, 400), (256, 257), (257, 700),
+                                 (520, 66200), (900, 1000)])
+def test_T_solve_matches_the_fp64_pipe(k, n):
+    """T = R11^{-1} R12 as slice products against the substitution on the FP64 pipe, at the
+    edges of its blocks of 256 rows, tiles of 128 x 64 and passes of 65536 columns."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    rng = torch.Generator(device="cuda").manual_seed(k)
+    m = k + 40
+    A = torch.randn(n, m, generator=rng, device="cuda", dtype=torch.float64).t()
+    A = (A * 2.0 ** -(torch.arange(n, device="cuda") % 50)).t().contiguous().t()     # graded columns
+    Ts = []
+    for fp64 in (True, False):
+        with Handle(0) as h:
+            h.set_tsolve_fp64(fp64)
+            r = h.column_id(A, b=min(64, k), tol=None, kmax=k, sampler="greedy")
+            assert r.k == k
+            Ts.append(r.T)
+    # substitution: |dT| <= c k eps |R^-1| |R| |T|, row by row; greedy pivots keep |R^-1| |R| of these
+    # Gaussian factors below 20 sqrt(k)
+    scale = Ts[0].abs().amax(0).clamp_min(1e-300)
+    d = ((Ts[1] - Ts[0]).abs().amax(0) / scale).max().item()
+    assert d <= 4 * k * EPS * 20 * k ** 0.5, d
+
+
 def test_slice_gemm_timeout_is_clean():
     """The projection's bounded waits run out under a budget of one clock: status 7, and the
     same handle reproduces an untouched one's results afterwards."""
