@@ -310,9 +310,9 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
           sps = s_w;
         }
       }
-      tc::k_gemm_slices<<<dim3(ctiles, nsplit), tc::SL_THREADS, tc::SL_SMEM, st>>>(
+      tc::k_gemm_slices<<<std::min(h->sms, ctiles * nsplit), tc::SL_THREADS, tc::SL_SMEM, st>>>(
           tmSA, tmSQ, (int64_t)n, h->wait_budget > 0 ? h->wait_budget : kWaitBudgetDefault,
-          tc::ProjEpi{h->st, n, nst, sps, h->sl_exA, h->sl_exQ, h->sl_Wpart});
+          tc::ProjEpi{h->st, n, nst, sps, h->sl_exA, h->sl_exQ, h->sl_Wpart, 0, 0, 0});
       nproj = (n - i + 31) / 32;
       tc::k_proj_finish<<<nproj, 256, 0, st>>>(h->st, h->sl_Wpart, nsplit, n, h->R, n, h->diags, h->part_res,
                                                h->part_nnz);

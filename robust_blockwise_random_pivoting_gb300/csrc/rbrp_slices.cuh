@@ -168,36 +168,36 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
   for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// (hi 2^24 + lo) 2^e rounded to the nearest FP64 value, on the integer pipe (the same
-// conversions and a scaling on the FP64 pipe cost ~25,000 clocks per 128 x 64 tile).
+// (hi 2^24 + lo) 2^e rounded to the nearest FP64 value (ties away from zero), on 32-bit
+// words: conversions on the FP64 pipe would cost 25,000 clocks per 128 x 64 tile, and 64-bit
+// shifts with a normalisation by cases did cost 20,000 (T solve, k = 2000, 14,384 columns:
+// 3.9 ms; 2.7 with this and the persistent grid).
 __device__ __forceinline__ double slice_value(long long hi, long long lo, int e) {
   hi += lo >> 24;
-  lo &= 0xFFFFFF;                       // now 0 <= lo < 2^24
-  const bool neg = hi < 0;
-  if (neg) {
-    hi = lo ? ~hi : -hi;
-    lo = lo ? 0x1000000 - lo : 0;
-  }
-  if (hi == 0) {                        // at most 24 significant bits
-    if (lo == 0) return 0.0;
-    hi = lo;
-    lo = 0;
-    e -= 24;
-  }
-  const int n = __clzll(hi);            // hi < 2^62: n >= 1
-  const unsigned long long lo40 = (unsigned long long)lo << 40;
-  unsigned long long t = ((unsigned long long)hi << n) | (lo40 >> (64 - n));
-  const bool rest = (lo40 << n) != 0;
-  unsigned long long m = t >> 11;
-  const unsigned r = (unsigned)t & 0x7FFu;
-  m += (r > 0x400u || (r == 0x400u && (rest || (m & 1)))) ? 1u : 0u;
-  const int be = 35 - n + e + 52 + 1023;   // value = m 2^(35 - n + e), 2^52 <= m <= 2^53
-  if (be >= 1 && be <= 2045) {
-    const long long bits = ((long long)be << 52) + (long long)(m - (1ull << 52));
-    return __longlong_as_double(neg ? bits | (long long)(1ull << 63) : bits);
-  }
-  const double v = ldexp((double)m, 35 - n + e);   // subnormal or out of range
-  return neg ? -v : v;
+  // |hi 2^32 + (lo mod 2^24) 2^8| as three words
+  unsigned w2 = (unsigned)((unsigned long long)hi >> 32), w1 = (unsigned)hi, w0 = (unsigned)lo << 8;
+  const unsigned neg = (unsigned)((int)w2 >> 31);
+  w0 = (w0 ^ neg) - neg;
+  const unsigned c0 = neg & (w0 == 0u ? 1u : 0u);   // the carry of -x = ~x + 1
+  w1 = (w1 ^ neg) + c0;
+  const unsigned c1 = c0 & (w1 == 0u ? 1u : 0u);
+  w2 = (w2 ^ neg) + c1;
+  // leading one into bit 31 of w2
+  int p = 95;
+  if (w2 == 0u) { w2 = w1; w1 = w0; w0 = 0u; p -= 32; }
+  if (w2 == 0u) { w2 = w1; w1 = 0u; p -= 32; }
+  const int n = __clz((int)w2);
+  w2 = __funnelshift_lc(w1, w2, n);
+  w1 = __funnelshift_lc(w0, w1, n);
+  // 53 bits of w2 : w1, rounded; a carry out of them raises the exponent by itself
+  const unsigned r = (w1 >> 10) & 1u;
+  unsigned ml = __funnelshift_r(w1, w2, 11), mh = w2 >> 11;
+  ml += r;
+  mh += r & (ml == 0u ? 1u : 0u);
+  const int be = 1023 + p - n - 8 + e;
+  if (w2 == 0u) return 0.0;
+  if (be < 1 || be > 2045) return ldexp(__hiloint2double((int)(mh + (1022u << 20) | (neg & 0x80000000u)), (int)ml), be - 1023);
+  return __hiloint2double((int)((mh + ((unsigned)(be - 1) << 20)) | (neg & 0x80000000u)), (int)ml);
 }
 
 // Shared memory: the seven slices of the stage's M tile, each its own slot of a ring,
@@ -212,8 +212,8 @@ struct __align__(1024) SliceSmem {
 constexpr size_t SL_SMEM = sizeof(SliceSmem) + 1024;
 static_assert(SL_SMEM <= 232448, "227 KB of shared memory per CTA");
 
-// One 128 x 64 tile (128 x 32 when one half holds every column): D(p, a) over the
-// stages [s0, s0 + nst) of 64 values of k.
+// Tiles of 128 x 64 (128 x 32 where one half holds every column) of D(p, a), each over the
+// stages [s0, s0 + nst) of 64 values of k: a persistent grid, tile t = blockIdx.x, + gridDim.x, ...
 //
 //   warp 0    TMA: per stage the N operand's halves, then the M operand's slices.
 //   warp 1    MMAs.  Slice i of M meets slices 0 .. min(6, 7 - i) of N at once: those sit
@@ -224,15 +224,18 @@ static_assert(SL_SMEM <= 232448, "227 KB of shared memory per CTA");
 //             that its drain hides behind the other's MMAs.  With one half, chunks
 //             alternate between the sets.
 //   warps 2-9 drain a set each (four lane quarters): FP32 integers to int, folded into
-//             two 64-bit integers per column (weights 256^3 and 1, in units of class 6).
+//             two 64-bit integers per column (weights 256^3 and 1, in units of class 6);
+//             with one half, warps 2-5 drain both sets.  A tile's results leave the
+//             registers while the next tile's MMAs run.
 //
 // What bounds it: the MMAs, 568 clocks per 16 values of k and half (N = 32 x 34 classes
 // at half a clock per column, or the shared-memory reads of the short ones), against
-// 1.75 KB of slices per value of k from HBM.  8192 x 8192, 64 columns: 0.37 ms a block
+// 1.75 KB of slices per value of k from HBM.  8192 x 8192, 64 columns: 0.23 ms a block
 // against 8.8 ms on the FP64 pipe; 1000 x 1000, 40 columns: 0.034 against 0.61 ms.
 //
-// epi.part(h, p, a0, hi, lo): the thread's 32 columns a0 .. a0 + 31 of row p, with
-// D = 2^(ex + ey - 60) (hi 2^24 + lo).
+// epi.init(): halves of every tile, 0 for nothing to do; epi.tile(t, ...): the t-th tile,
+// false past the last; epi.part(t, p, a0, hi, lo): the thread's 32 columns a0 .. a0 + 31 of
+// row p, with D = 2^(ex + ey - 60) (hi 2^24 + lo).
 template <typename Epi>
 __global__ void __launch_bounds__(SL_THREADS, 1)
 k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int64_t a_rows,
@@ -240,8 +243,9 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   extern __shared__ uint8_t sl_raw[];
   SliceSmem& sm = *reinterpret_cast<SliceSmem*>((reinterpret_cast<uintptr_t>(sl_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int p0, brow, s0, nst, nh, ax;   // first M row, first N row, stage range, halves, M's first value of k
-  if (!epi.tile(p0, brow, s0, nst, nh, ax)) return;  // uniform over the CTA
+  const int nh = epi.init();
+  int p0, brow, s0, nst, ax;   // first M row, first N row, stage range, M's first value of k
+  if (nh == 0 || !epi.tile(blockIdx.x, p0, brow, s0, nst, ax)) return;  // uniform over the CTA
   volatile int* abort = &sm.abort;
   if (threadIdx.x == 0) {
     for (int s = 0; s < SL; ++s) {
@@ -268,139 +272,128 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = sm.tmem_base;
+  int g = 0;                     // stages so far, over the tiles (ring positions)
   int aissued = 0, bissued = 0;  // producer: slices and N stages whose loads were issued
+  bool ok = true;
 
-  // chunk of half h at stage s: with two halves the second one's chunks start a stage early
+  // chunk of half h at stage s of a tile: with two halves the second one's chunks start a stage early
   auto chunk_of = [&](int h, int s) { return (s + (nh == 2 ? h : 0)) / SL_CHUNK; };
 
   if (warp == 0) {
-    bool ok = true;
-    for (int s = 0; s < nst && ok; ++s) {
-      const int b = s & 1, x = (s0 + s) * SL_BK;
-      if (s >= 2 && !mbar_wait(&sm.bempty[b], (uint32_t)((s >> 1) & 1) ^ 1, abort, budget)) break;
-      if (elect_one()) {
-        mbar_expect_tx(&sm.bfull[b], (uint32_t)(nh * SL_B_BYTES));
-        for (int h = 0; h < nh; ++h)
-          tma_load_2d(sm.bs[b][h], &tmB, &sm.bfull[b], x, brow + h * SL * SL_HALF);
-      }
-      __syncwarp();
-      bissued = s + 1;
-      for (int i = 0; i < SL; ++i) {
-        if (s >= 1 && !mbar_wait(&sm.aempty[i], (uint32_t)(s & 1) ^ 1, abort, budget)) { ok = false; break; }
+    for (int t = blockIdx.x; ok && epi.tile(t, p0, brow, s0, nst, ax); t += gridDim.x) {
+      for (int s = 0; s < nst && ok; ++s, ++g) {
+        const int b = g & 1, x = (s0 + s) * SL_BK;
+        if (g >= 2 && !mbar_wait(&sm.bempty[b], (uint32_t)((g >> 1) & 1) ^ 1, abort, budget)) { ok = false; break; }
         if (elect_one()) {
-          mbar_expect_tx(&sm.afull[i], SL_A_BYTES);
-          tma_load_2d(sm.as[i], &tmA, &sm.afull[i], ax + x, (int)(i * a_rows) + p0);
+          mbar_expect_tx(&sm.bfull[b], (uint32_t)(nh * SL_B_BYTES));
+          for (int h = 0; h < nh; ++h)
+            tma_load_2d(sm.bs[b][h], &tmB, &sm.bfull[b], x, brow + h * SL * SL_HALF);
         }
         __syncwarp();
-        aissued = s * SL + i + 1;
+        bissued = g + 1;
+        for (int i = 0; i < SL; ++i) {
+          if (g >= 1 && !mbar_wait(&sm.aempty[i], (uint32_t)(g & 1) ^ 1, abort, budget)) { ok = false; break; }
+          if (elect_one()) {
+            mbar_expect_tx(&sm.afull[i], SL_A_BYTES);
+            tma_load_2d(sm.as[i], &tmA, &sm.afull[i], ax + x, (int)(i * a_rows) + p0);
+          }
+          __syncwarp();
+          aissued = g * SL + i + 1;
+        }
       }
     }
   } else if (warp == 1) {
     int uses[2] = {0, 0};  // chunks started per accumulator set
-    bool ok = true;
-    for (int s = 0; s < nst && ok; ++s) {
-      const int b = s & 1;
-      if (!mbar_wait(&sm.bfull[b], (uint32_t)(s >> 1) & 1, abort, budget)) break;
-      const bool starts0 = s == 0 || chunk_of(0, s) != chunk_of(0, s - 1);
-      for (int q = 0; q < nh && ok; ++q) {
-        const int h = (nh == 2 && starts0) ? 1 - q : q;
-        const int ck = chunk_of(h, s);
-        const bool first = s == 0 || ck != chunk_of(h, s - 1);
-        const bool last = s == nst - 1 || ck != chunk_of(h, s + 1);
-        const int set = nh == 2 ? h : ck & 1;
-        if (first) {
-          if (uses[set] >= 1 && !mbar_wait(&sm.acce[set], (uint32_t)(uses[set] - 1) & 1, abort, budget)) {
-            ok = false;
-            break;
+    for (int t = blockIdx.x; ok && epi.tile(t, p0, brow, s0, nst, ax); t += gridDim.x) {
+      for (int s = 0; s < nst && ok; ++s, ++g) {
+        const int b = g & 1;
+        if (!mbar_wait(&sm.bfull[b], (uint32_t)(g >> 1) & 1, abort, budget)) { ok = false; break; }
+        const bool starts0 = s == 0 || chunk_of(0, s) != chunk_of(0, s - 1);
+        for (int q = 0; q < nh && ok; ++q) {
+          const int h = (nh == 2 && starts0) ? 1 - q : q;
+          const int ck = chunk_of(h, s);
+          const bool first = s == 0 || ck != chunk_of(h, s - 1);
+          const bool last = s == nst - 1 || ck != chunk_of(h, s + 1);
+          const int set = nh == 2 ? h : ck & 1;
+          if (first) {
+            const int u = set ? uses[1] : uses[0];
+            if (u >= 1 && !mbar_wait(&sm.acce[set], (uint32_t)(u - 1) & 1, abort, budget)) {
+              ok = false;
+              break;
+            }
+            if (set) ++uses[1]; else ++uses[0];
           }
-          ++uses[set];
-        }
-        const uint32_t dset = tbase + (uint32_t)(set * SL_CLASSES * SL_HALF);
-        const uint64_t db = sw128_desc(smem_u32(sm.bs[b][h]));
-        for (int i = 0; i < SL; ++i) {
-          if (!mbar_wait(&sm.afull[i], (uint32_t)s & 1, abort, budget)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t da = sw128_desc(smem_u32(sm.as[i]));
-          const uint32_t d = dset + (uint32_t)(i * SL_HALF);
-          const int nsl = i == 0 ? SL : SL_CLASSES - i;   // N slices 0 .. nsl - 1: classes i .. i + nsl - 1
-          if (elect_one()) {
+          const uint32_t dset = tbase + (uint32_t)(set * SL_CLASSES * SL_HALF);
+          const uint64_t db = sw128_desc(smem_u32(sm.bs[b][h]));
+          for (int i = 0; i < SL; ++i) {
+            if (!mbar_wait(&sm.afull[i], (uint32_t)g & 1, abort, budget)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t da = sw128_desc(smem_u32(sm.as[i]));
+            const uint32_t d = dset + (uint32_t)(i * SL_HALF);
+            const int nsl = i == 0 ? SL : SL_CLASSES - i;   // N slices 0 .. nsl - 1: classes i .. i + nsl - 1
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < SL_BK / 16; ++k) {        // K = 16 BF16: 32 bytes
-              if (first && k == 0 && i == 1) {
-                // classes 1 .. 6 were started by slice 0; class 7 starts here
-                mma_bf16(d, da, db, (SL - 1) * SL_HALF, 1u);
-                mma_bf16(d + (uint32_t)((SL - 1) * SL_HALF), da,
-                         db + (uint64_t)(((SL - 1) * SL_HALF * SL_BK * 2) >> 4), SL_HALF, 0u);
-              } else {
-                mma_bf16(d, da + 2 * k, db + 2 * k, nsl * SL_HALF, (first && k == 0 && i == 0) ? 0u : 1u);
+              for (int k = 0; k < SL_BK / 16; ++k) {        // K = 16 BF16: 32 bytes
+                if (first && k == 0 && i == 1) {
+                  // classes 1 .. 6 were started by slice 0; class 7 starts here
+                  mma_bf16(d, da, db, (SL - 1) * SL_HALF, 1u);
+                  mma_bf16(d + (uint32_t)((SL - 1) * SL_HALF), da,
+                           db + (uint64_t)(((SL - 1) * SL_HALF * SL_BK * 2) >> 4), SL_HALF, 0u);
+                } else {
+                  mma_bf16(d, da + 2 * k, db + 2 * k, nsl * SL_HALF, (first && k == 0 && i == 0) ? 0u : 1u);
+                }
+              }
+              if (q == nh - 1) mma_commit(&sm.aempty[i]);
+              if (i == SL - 1) {
+                if (last) mma_commit(&sm.accf[set]);
+                if (q == nh - 1) mma_commit(&sm.bempty[b]);
               }
             }
-            if (q == nh - 1) mma_commit(&sm.aempty[i]);
-            if (i == SL - 1) {
-              if (last) mma_commit(&sm.accf[set]);
-              if (q == nh - 1) mma_commit(&sm.bempty[b]);
-            }
+            __syncwarp();
           }
-          __syncwarp();
         }
       }
     }
-  } else {
-    const int q = warp & 3, set = (warp - 2) >> 2;
-    const uint32_t ta = tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(set * SL_CLASSES * SL_HALF);
-    long long hi[SL_HALF], lo[SL_HALF];
+  } else if (nh == 2 || warp < 6) {
+    const int q = warp & 3, grp = (warp - 2) >> 2;
+    const uint32_t tq = tbase + ((uint32_t)(32 * q) << 16);
+    int uses[2] = {0, 0};
+    for (int t = blockIdx.x; ok && epi.tile(t, p0, brow, s0, nst, ax); t += gridDim.x) {
+      long long hi[SL_HALF], lo[SL_HALF];
 #pragma unroll
-    for (int j = 0; j < SL_HALF; ++j) hi[j] = lo[j] = 0;
-    const int nchunk = nst > 0 ? chunk_of(set, nst - 1) + 1 : 0;
-    bool ok = true;
-    int use = 0;
-    for (int c = nh == 2 ? 0 : set; c < nchunk; c += nh == 2 ? 1 : 2, ++use) {
-      if (!mbar_wait(&sm.accf[set], (uint32_t)use & 1, abort, budget)) { ok = false; break; }
-      tc_fence_after();
+      for (int j = 0; j < SL_HALF; ++j) hi[j] = lo[j] = 0;
+      const int nchunk = chunk_of(grp, nst - 1) + 1;
+      for (int c = 0; c < nchunk; ++c) {
+        const int set = nh == 2 ? grp : c & 1;
+        const int u = set ? uses[1] : uses[0];
+        if (!mbar_wait(&sm.accf[set], (uint32_t)u & 1, abort, budget)) { ok = false; break; }
+        if (set) ++uses[1]; else ++uses[0];
+        tc_fence_after();
+        const uint32_t ta = tq + (uint32_t)(set * SL_CLASSES * SL_HALF);
 #pragma unroll
-      for (int j0 = 0; j0 < SL_HALF; j0 += 4) {
-        float v[SL_CLASSES][4];
+        for (int j0 = 0; j0 < SL_HALF; j0 += 4) {
+          float v[SL_CLASSES][4];
 #pragma unroll
-        for (int k = 0; k < SL_CLASSES; ++k) tmem_ld4(ta + (uint32_t)(k * SL_HALF + j0), v[k]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int k = 0; k < SL_CLASSES; ++k) tmem_ld4(ta + (uint32_t)(k * SL_HALF + j0), v[k]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int s01 = __float2int_rn(v[0][j]) * 256 + __float2int_rn(v[1][j]);   // < 2^28
-          const int s23 = __float2int_rn(v[2][j]) * 256 + __float2int_rn(v[3][j]);   // < 2^31
-          hi[j0 + j] += (long long)s01 * 65536 + s23;
-          // class 7 joins class 6, rounded to its unit
-          lo[j0 + j] += (long long)__float2int_rn(v[4][j]) * 65536 + (long long)__float2int_rn(v[5][j]) * 256 +
-                        __float2int_rn(fmaf(v[7][j], 0.00390625f, v[6][j]));
+          for (int j = 0; j < 4; ++j) {
+            const int s01 = __float2int_rn(v[0][j]) * 256 + __float2int_rn(v[1][j]);   // < 2^28
+            const int s23 = __float2int_rn(v[2][j]) * 256 + __float2int_rn(v[3][j]);   // < 2^31
+            hi[j0 + j] += (long long)s01 * 65536 + s23;
+            // class 7 joins class 6, rounded to its unit
+            lo[j0 + j] += (long long)__float2int_rn(v[4][j]) * 65536 + (long long)__float2int_rn(v[5][j]) * 256 +
+                          __float2int_rn(fmaf(v[7][j], 0.00390625f, v[6][j]));
+          }
         }
+        tc_fence_before();
+        mbar_arrive(&sm.acce[set]);
       }
-      tc_fence_before();
-      mbar_arrive(&sm.acce[set]);
+      if (ok && !*abort) epi.part(t, p0 + 32 * q + lane, SL_HALF * grp, hi, lo);
     }
-    // one half: its chunks alternated between the sets, whose sums meet in shared memory
-    // (behind the barrier the last chunk of each set is drained: no load or MMA is left)
-    if (nh == 1) {
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      long long* sh = reinterpret_cast<long long*>(sm.as) + (32 * q + lane);
-      if (set == 1 && ok) {
-#pragma unroll
-        for (int j = 0; j < SL_HALF; ++j) {
-          sh[(2 * j) * BM] = hi[j];
-          sh[(2 * j + 1) * BM] = lo[j];
-        }
-      }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (set == 0 && ok) {
-#pragma unroll
-        for (int j = 0; j < SL_HALF; ++j) {
-          hi[j] += sh[(2 * j) * BM];
-          lo[j] += sh[(2 * j + 1) * BM];
-        }
-      }
-    }
-    if (ok && !*abort && (nh == 2 || set == 0)) epi.part(p0 + 32 * q + lane, nh == 2 ? SL_HALF * set : 0, hi, lo);
   }
   __syncthreads();
   if (*abort) {
@@ -438,20 +431,25 @@ struct ProjEpi {
   const int* exA;
   const int* exQ;
   double* Wpart;
-  __device__ bool tile(int& p0, int& brow, int& s0, int& nst, int& nh, int& ax) const {
-    const int kept = st->bs;
-    ax = 0;
-    p0 = st->i + kept + blockIdx.x * BM;
-    brow = 0;
-    s0 = blockIdx.y * sps;
-    nst = min(sps, nstages - s0);
-    nh = kept > SL_HALF ? 2 : 1;
-    return kept > 0 && p0 < n && nst > 0;
+  int pb, kept, ctiles;   // set by init
+  __device__ int init() {
+    kept = st->bs;
+    pb = st->i + kept;
+    ctiles = (n - pb + BM - 1) / BM;
+    return kept == 0 || pb >= n ? 0 : kept > SL_HALF ? 2 : 1;
   }
-  __device__ void part(int p, int a0, const long long (&hi)[SL_HALF], const long long (&lo)[SL_HALF]) const {
+  __device__ bool tile(int t, int& p0, int& brow, int& s0, int& nst, int& ax) const {
+    const int z = t / ctiles;
+    ax = brow = 0;
+    p0 = pb + (t - z * ctiles) * BM;
+    s0 = z * sps;
+    nst = min(sps, nstages - s0);
+    return nst > 0;
+  }
+  __device__ void part(int t, int p, int a0, const long long (&hi)[SL_HALF], const long long (&lo)[SL_HALF]) const {
     if (p >= n) return;
-    const int kept = st->bs, e = exA[p] - 60;
-    double* w = Wpart + ((int64_t)blockIdx.y * MAXB + a0) * n + p;
+    const int e = exA[p] - 60;
+    double* w = Wpart + ((int64_t)(t / ctiles) * MAXB + a0) * n + p;
 #pragma unroll
     for (int j = 0; j < SL_HALF; ++j)
       if (a0 + j < kept) w[(int64_t)j * n] = slice_value(hi[j], lo[j], e + exQ[a0 + j]);

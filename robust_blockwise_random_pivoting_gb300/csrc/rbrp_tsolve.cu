@@ -107,10 +107,10 @@ __global__ void __launch_bounds__(256) k_trsm_T(const double* __restrict__ R, in
 // loses nothing: 55 bits below each row's largest entry, where the double-float solve this
 // replaces carried 48 throughout.
 //
-// What bounds it: a 128 x 64 tile over 256 values of k is 18,000 clocks of MMAs and some
-// 8,000 of setup, drain and epilogue; the double-float solve needed 12 FP32 operations per
+// What bounds it: a 128 x 64 tile over 256 values of k is 18,000 clocks of MMAs, which its
+// epilogue (one FP64 subtraction per entry) runs beside; the double-float solve needed 12 FP32 operations per
 // product and a warp per column in the diagonal blocks (k = 2000, 14,384 columns: 15.9 ms,
-// now 3.9; k = 1000, 64,536 columns: 19.5, now 4.9).
+// now 2.7; k = 1000, 64,536 columns: 19.5, now 3.4).
 // ===========================================================================
 namespace tc {
 namespace {
@@ -257,29 +257,31 @@ struct TsEpi {
   int row0, rows, ncols, nst, ax, sub;
   const int* exM;
   const int* exX;
-  __device__ bool tile(int& p0, int& brow, int& s0, int& n, int& nh, int& a_x) const {
-    p0 = row0 + blockIdx.x * BM;
-    brow = blockIdx.y * 2 * SL * SL_HALF;
+  __device__ int mtiles() const { return (rows + BM - 1) / BM; }
+  __device__ int init() const { return ncols > SL_HALF ? 2 : 1; }
+  __device__ bool tile(int t, int& p0, int& brow, int& s0, int& n, int& a_x) const {
+    const int y = t / mtiles();
+    p0 = row0 + (t - y * mtiles()) * BM;
+    brow = y * 2 * SL * SL_HALF;
     s0 = 0;
     n = nst;
-    nh = ncols - (int)blockIdx.y * 64 > SL_HALF ? 2 : 1;
     a_x = ax;
-    return true;
+    return y * 64 < ncols;
   }
-  __device__ void part(int p, int a0, const long long (&hi)[SL_HALF], const long long (&lo)[SL_HALF]) const {
+  __device__ void part(int t, int p, int a0, const long long (&hi)[SL_HALF], const long long (&lo)[SL_HALF]) const {
     if (p >= row0 + rows) return;
-    const int c0 = blockIdx.y * 64 + a0, e = exM[p] - 60;
-    double* t = T + p + (int64_t)c0 * ldt;
+    const int c0 = t / mtiles() * 64 + a0, e = exM[p] - 60;
+    double* x = T + p + (int64_t)c0 * ldt;
 #pragma unroll
     for (int j0 = 0; j0 < SL_HALF; j0 += 8) {
       double old[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) old[j] = sub && c0 + j0 + j < ncols ? t[(int64_t)(j0 + j) * ldt] : 0.0;
+      for (int j = 0; j < 8; ++j) old[j] = sub && c0 + j0 + j < ncols ? x[(int64_t)(j0 + j) * ldt] : 0.0;
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (c0 + j0 + j < ncols) {
           const double v = slice_value(hi[j0 + j], lo[j0 + j], e + exX[c0 + j0 + j]);
-          t[(int64_t)(j0 + j) * ldt] = sub ? old[j] - v : v;
+          x[(int64_t)(j0 + j) * ldt] = sub ? old[j] - v : v;
         }
     }
   }
@@ -314,7 +316,7 @@ rbrp_status solve_T(rbrp_handle h, int k, int n) {
   using namespace tc;
   // the chain of ob steps of the inverses against fewer, larger products: k = 270, 1730 columns:
   // 0.26 ms with blocks of 128, 0.34 with 256; 640, 7552: 0.61 and 0.63; 900, 300: 0.54 and 0.50;
-  // 2000, 14384: 5.7 and 3.9
+  // 2000, 14384: 5.7 and 3.9 (before the grid was persistent)
   const int ob = k <= 640 ? TS_OB / 2 : TS_OB;
   const int nblk = (k + ob - 1) / ob;
   const size_t ldk = ((size_t)k + 63) / 64 * 64, ldi = std::min((size_t)ob, ldk);
@@ -370,11 +372,11 @@ rbrp_status solve_T(rbrp_handle h, int k, int n) {
     for (int J = nblk - 1; J >= 0; --J) {
       const int j0 = J * ob, len = std::min(ob, k - j0), nst = (len + SL_BK - 1) / SL_BK;
       k_ts_slice_x<<<(nc + 7) / 8, 256, 0, st>>>(T, k, j0, len, nc, (int)ldi, sX, eX);
-      k_gemm_slices<<<dim3((len + BM - 1) / BM, ntile), SL_THREADS, SL_SMEM, st>>>(
+      k_gemm_slices<<<std::min(h->sms, (len + BM - 1) / BM * ntile), SL_THREADS, SL_SMEM, st>>>(
           tmI, tmX, (int64_t)k, budget, TsEpi{h->st, T, k, j0, len, nc, nst, 0, 0, eI, eX});
       if (J > 0) {
         k_ts_slice_x<<<(nc + 7) / 8, 256, 0, st>>>(T, k, j0, len, nc, (int)ldi, sX, eX);
-        k_gemm_slices<<<dim3(j0 / BM, ntile), SL_THREADS, SL_SMEM, st>>>(
+        k_gemm_slices<<<std::min(h->sms, j0 / BM * ntile), SL_THREADS, SL_SMEM, st>>>(
             tmR, tmX, (int64_t)k, budget, TsEpi{h->st, T, k, 0, j0, nc, nst, j0, 1, eR, eX});
       }
     }
