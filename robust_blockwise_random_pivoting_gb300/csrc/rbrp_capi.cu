@@ -127,6 +127,9 @@ rbrp_status ensure_workspace(rbrp_handle h, const Layout& L) {
       {(void**)&h->perm, n * 4},
       {(void**)&h->pbuf, 2 * n * 8},
       {(void**)&h->kbuf, n * 8},
+      {(void**)&h->samp_part, 1024 * 8},
+      {(void**)&h->samp_tot, 1024 * 8},
+      {(void**)&h->samp_pos, 1024 * 4},
       {(void**)&h->Q, (L.residual ? (size_t)L.ld_res * MAXB : m * kmax) * el},
       {(void**)&h->part_norm, L.residual ? (size_t)P2_MAX_SPLIT_WS * n * 8 : 0},
       {(void**)&h->Wpart, L.residual ? (size_t)P1_MAX_SPLIT * MAXB * n * 8 : 0},

@@ -30,6 +30,19 @@ constexpr int NPAIR = MAXB * (MAXB + 1) / 2;   // upper triangle of a panel's Gr
 // Rows per CTA of the row kernels: 32, or 8 where 32 would leave SMs without a tile.
 __host__ __device__ constexpr int panel_tile_rows(int m) { return m >= 152 * 32 ? 32 : 8; }
 
+// Pair x of the upper triangle of a w x w matrix (rows folded in pairs r, w - 1 - r of w + 1
+// entries together), 0 <= x < w (w + 1) / 2.
+__device__ __forceinline__ void tri_pair(int x, int w, int& a, int& b) {
+  const int r = x / (w + 1), c = x % (w + 1);
+  if (c < w - r) {
+    a = r;
+    b = r + c;
+  } else {
+    a = w - 1 - r;
+    b = a + c - (w - r);
+  }
+}
+
 // Loop state, resident in device memory; every per-block kernel reads it, so the
 // host needs no data from the device to enqueue a block.
 struct State {

@@ -142,14 +142,22 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
     const int gram_parts = (p.b * (p.b + 1) / 2 + GRAM_PAIRS - 1) / GRAM_PAIRS;
     const int gram_ctas = (p.b * (p.b + 1) / 2 + 63) / 64;
     ev = prof_begin(h);
-    k_sample<<<1, SAMPLE_THREADS, 0, st>>>(h->st, h->diags, h->perm, n, kmax, p.b, p.seed, p.sampler,
-                                           h->pbuf, h->kbuf, h->js, h->cols, h->given_order);
-    prof_end(h, RBRP_PHASE_SAMPLE, ev, 28.0 * (n - i), 0.0, 1);
+    const bool pre = p.sampler == SAMPLER_NP && n - i >= SAMPLE_PRE_MIN;
+    if (pre) {
+      k_sample_sums<<<SAMPLE_THREADS / 32, 32, 0, st>>>(h->st, h->diags, n, h->samp_part);
+      k_sample_probs<<<SAMPLE_THREADS / 32, 32, 0, st>>>(h->st, h->diags, n, h->samp_part, h->pbuf, h->samp_tot,
+                                                         h->samp_pos);
+    }
+    k_sample<<<1, SAMPLE_THREADS, 0, st>>>(h->st, h->diags, h->perm, n, kmax, p.b, p.seed, p.sampler, h->pbuf, h->kbuf,
+                                           h->js, h->cols, h->given_order, pre ? h->samp_tot : nullptr,
+                                           pre ? h->samp_pos : nullptr);
+    prof_end(h, RBRP_PHASE_SAMPLE, ev, 28.0 * (n - i), 0.0, pre ? 3 : 1);
     ev = prof_begin(h);
     const int dtiles = (m + DF_ROWS - 1) / DF_ROWS;   // row tiles of the double-float Gram kernel
     if (RES) {  // panel = residual columns at the sampled positions (FP32, exact), Gram in double-float
-      k_gram_df<<<dtiles, 256, 0, st>>>(h->Ares, L.ld_res, h->js, h->st, m, (float*)h->V, h->Gpart);
-      k_reduce_parts<double><<<16, 256, 0, st>>>(h->Gpart, dtiles, MAXB * MAXB, MAXB * MAXB, h->G);
+      const int parts = (p.b * (p.b + 1) / 2 + GRAM_DF_PAIRS - 1) / GRAM_DF_PAIRS;
+      k_gram_df<<<dim3(dtiles, parts), 256, 0, st>>>(h->Ares, L.ld_res, h->js, h->st, m, (float*)h->V, h->Gpart);
+      k_reduce_parts<double><<<64, 64, 0, st>>>(h->Gpart, dtiles, MAXB * MAXB, MAXB * MAXB, h->G);
     }
     if constexpr (!RES) {
       if (i > 0 && !fixed_order) {
@@ -175,16 +183,14 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
     prof_end(h, RBRP_PHASE_CGS, ev, 0.0, 0.0, RES ? 2 : i == 0 ? 3 : fixed_order ? 5 : 4);
     ev = prof_begin(h);
     if (RES) {
-      // R11 and its inverse as double-float pairs: the FP64 R11 / R2 buffers of the same
-      // size (R2 serves only the FP64 form's second CholQR pass), reinterpreted
-      float2* R11df = reinterpret_cast<float2*>(h->R11);
+      // the inverse of R11 as double-float pairs: the FP64 R2 buffer of the same size (it
+      // serves only the FP64 form's second CholQR pass), reinterpreted
       float2* Rinvdf = reinterpret_cast<float2*>(h->R2);
       k_pchol_df<<<1, LEAN_THREADS, sizeof(PcholDfSmem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags,
-                                                               R11df, Rinvdf, h->ord, h->J, h->K1, h->K2);
+                                                               h->R, n, Rinvdf, h->ord, h->J, h->K1, h->K2);
       k_panel_q_df<<<(m + QS_ROWS - 1) / QS_ROWS, 256, sizeof(QSolveSmem), st>>>(
           (const float*)h->V, m, h->st, Rinvdf, h->ord, (float*)Q, L.ld_res, use_tc ? h->Qh : nullptr,
           use_tc ? h->Ql : nullptr, L.ld_res, use_tc ? h->Qrh : nullptr, use_tc ? h->Qrl : nullptr);
-      k_write_r11<<<1, 256, 0, st>>>(h->st, R11df, h->R, n);
     }
     if constexpr (!RES) {
       k_pchol<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11, h->ord,
@@ -209,7 +215,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
         tc::k_swap_slices<<<dim3(p.b, tc::SL), 256, 0, st>>>(h->slA, n, ldk, h->sl_exA, h->st, h->K1, h->K2);
       }
     }
-    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 5 : 4) : (i > 0 ? 8 : 7) + (use_sl ? 2 : 0));
+    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 4 : 3) : (i > 0 ? 8 : 7) + (use_sl ? 2 : 0));
     int nproj;
     ev = prof_begin(h);
     if (RES) {

@@ -46,6 +46,9 @@ struct rbrp_handle_st {
   int* ord = nullptr;
   double* pbuf = nullptr;      // 2n: weights and cdf
   unsigned long long* kbuf = nullptr;
+  double* samp_part = nullptr; // the sampler's chunk sums, totals and counts (1024 each)
+  double* samp_tot = nullptr;
+  int* samp_pos = nullptr;
   int* js = nullptr;
   int* cols = nullptr;
   int* J = nullptr;

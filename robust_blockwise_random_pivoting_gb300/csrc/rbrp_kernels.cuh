@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS)
 k_sample(State* st, const double* __restrict__ diags, const int* __restrict__ perm, int n, int kmax,
          int b, uint64_t seed, int sampler, double* __restrict__ pbuf,
          unsigned long long* __restrict__ kbuf, int* __restrict__ js, int* __restrict__ cols,
-         const int* __restrict__ order_of) {
-  sample_block(st, diags, perm, n, kmax, b, seed, sampler, pbuf, kbuf, js, cols, order_of);
+         const int* __restrict__ order_of, const double* __restrict__ pre_tot, const int* __restrict__ pre_pos) {
+  sample_block(st, diags, perm, n, kmax, b, seed, sampler, pbuf, kbuf, js, cols, order_of, pre_tot, pre_pos);
 }
 
 // Deterministic sum of split partials: out[x] = sum_z part[z*stride + x].
@@ -142,6 +142,7 @@ __global__ void k_reduce_parts(const V* __restrict__ part, int nparts, int64_t s
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < count;
        x += (int64_t)gridDim.x * blockDim.x) {
     V s = V(0);
+#pragma unroll 8
     for (int z = 0; z < nparts; ++z) s += part[(int64_t)z * stride + x];
     out[x] = s;
   }

@@ -17,19 +17,6 @@
 namespace rbrp {
 namespace {
 
-// Pair x of the upper triangle of a w x w matrix (rows folded in pairs r, w - 1 - r of w + 1
-// entries together), 0 <= x < w (w + 1) / 2.
-__device__ __forceinline__ void tri_pair(int x, int w, int& a, int& b) {
-  const int r = x / (w + 1), c = x % (w + 1);
-  if (c < w - r) {
-    a = r;
-    b = r + c;
-  } else {
-    a = w - 1 - r;
-    b = a + c - (w - r);
-  }
-}
-
 // ===========================================================================
 // a3: block Gram-Schmidt against the current basis (one CGS pass, as
 // python/RBRP.ipynb cell 11 line 120 and matlab/RBRP.m:55).

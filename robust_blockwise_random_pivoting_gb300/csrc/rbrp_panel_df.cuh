@@ -24,42 +24,51 @@ namespace {
 
 constexpr int DF_ROWS = 128;  // panel rows per CTA of the Gram kernel
 
-// V = A_res(:, J) (FP32, exact) for 128 rows per CTA, and the tile's Gram partial V^T V
-// (upper triangle, mirrored) in double-float, stored as FP64.
+// V = A_res(:, J) (FP32, exact) for 128 rows (gridDim.x), and the tile's Gram partial V^T V in
+// double-float, stored as FP64: a fifth of the upper triangle's pairs per CTA (gridDim.y),
+// mirrored (the products are exact and commute).  A pair is one chain of 128 dependent
+// double-float sums; 16 pairs a thread in one CTA per row tile took 57 us at 1000 rows, this 20.
+constexpr int GRAM_DF_PARTS = 5;
+constexpr int GRAM_DF_PAIRS = NPAIR / GRAM_DF_PARTS;
 __global__ void __launch_bounds__(256)
 k_gram_df(const float* __restrict__ Ares, int64_t ld, const int* __restrict__ js, const State* __restrict__ st,
           int m, float* __restrict__ V, double* __restrict__ Gpart) {
-  __shared__ float Vs[DF_ROWS][MAXB + 1];
-  __shared__ int cs[MAXB];
+  __shared__ float Vs[MAXB][DF_ROWS + 1];
   const int tid = threadIdx.x;
   const int bss = st->bs_sampled;
+  const int x0 = blockIdx.y * GRAM_DF_PAIRS, x1 = min(bss * (bss + 1) / 2, x0 + GRAM_DF_PAIRS);
+  if (x0 >= x1) return;
   const int r0 = blockIdx.x * DF_ROWS;
-  if (tid < MAXB) cs[tid] = tid < bss ? js[tid] : -1;
-  __syncthreads();
-  for (int idx = tid; idx < DF_ROWS * MAXB; idx += 256) {
+  for (int idx = tid; idx < DF_ROWS * bss; idx += 256) {
     const int rr = idx % DF_ROWS, c = idx / DF_ROWS, r = r0 + rr;
-    const float v = (r < m && cs[c] >= 0) ? Ares[r + (int64_t)cs[c] * ld] : 0.f;
-    Vs[rr][c] = v;
-    if (r < m && c < bss) V[r + (int64_t)c * m] = v;
+    const float v = r < m ? Ares[r + (int64_t)js[c] * ld] : 0.f;
+    Vs[c][rr] = v;
+    if (blockIdx.y == 0 && r < m) V[r + (int64_t)c * m] = v;
   }
   __syncthreads();
   double* G = Gpart + (int64_t)blockIdx.x * MAXB * MAXB;
-  const int c1 = tid >> 2;
-  dfl acc[16];
+  static_assert(GRAM_DF_PAIRS <= 512, "two pairs per thread");
+  int a[2], b[2];
+  bool in[2];
 #pragma unroll
-  for (int q = 0; q < 16; ++q) acc[q] = {0.f, 0.f};
-  if (c1 < bss) {
-    for (int rr = 0; rr < DF_ROWS; ++rr) {
-      const float x = Vs[rr][c1];
-#pragma unroll
-      for (int q = 0; q < 16; ++q) df_acc_prod(acc[q], x, Vs[rr][(tid & 3) + 4 * q]);
-    }
+  for (int q = 0; q < 2; ++q) {
+    const int x = x0 + tid + 256 * q;
+    in[q] = x < x1;
+    tri_pair(in[q] ? x : x0, bss, a[q], b[q]);
+  }
+  dfl acc[2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+  for (int rr = 0; rr < DF_ROWS; ++rr) {
+    df_acc_prod(acc[0], Vs[a[0]][rr], Vs[b[0]][rr]);
+    if (in[1]) df_acc_prod(acc[1], Vs[a[1]][rr], Vs[b[1]][rr]);
   }
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int c2 = (tid & 3) + 4 * q;
-    const double g = (c1 < bss && c2 < bss) ? df_dbl(acc[q]) : 0.0;
-    G[c1 * MAXB + c2] = g;
+  for (int q = 0; q < 2; ++q) {
+    if (in[q]) {
+      const double g = df_dbl(acc[q]);
+      G[a[q] * MAXB + b[q]] = g;
+      G[b[q] * MAXB + a[q]] = g;
+    }
   }
 }
 
@@ -67,11 +76,12 @@ using PcholDfSmem = PcholDfSmemT<MAXB>;
 
 // Pivoted Cholesky of the panel Gram matrix with the robust filter (same rule as the
 // FP64 form's k_pchol), LEAN_THREADS threads, no data movement for the swaps.  Publishes
-// R11 (slot order, double-float pairs), ord, the kept count and performs the block swap.
+// R11 (slot order) as R(I2, I2), the panel R of a single CholQR pass, its inverse as
+// double-float pairs, ord and the kept count, and performs the block swap.
 __global__ void __launch_bounds__(LEAN_THREADS)
 k_pchol_df(const double* __restrict__ G, int m, State* st, double tol_loc, const int* __restrict__ js,
-           int* __restrict__ perm, double* __restrict__ diags, float2* __restrict__ R11g, float2* __restrict__ Rinvg,
-           int* __restrict__ ordg, int* __restrict__ Jg, int* __restrict__ K1g, int* __restrict__ K2g) {
+           int* __restrict__ perm, double* __restrict__ diags, double* __restrict__ R, int64_t ldr,
+           float2* __restrict__ Rinvg, int* __restrict__ ordg, int* __restrict__ Jg, int* __restrict__ K1g, int* __restrict__ K2g) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   PcholDfSmem& sm = *reinterpret_cast<PcholDfSmem*>(dyn_smem);
   const int tid = threadIdx.x;
@@ -81,18 +91,14 @@ k_pchol_df(const double* __restrict__ G, int m, State* st, double tol_loc, const
     const int a = idx / MAXB, c = idx % MAXB;
     sm.S[a][c] = (a < nb && c < nb) ? df_of(G[a * MAXB + c]) : dfl{0.f, 0.f};
   }
-  if (tid < MAXB) {
-    sm.ord[tid] = tid;
-    sm.alive[tid] = tid < nb;
-  }
+  if (tid < MAXB) sm.ord[tid] = tid;
   __syncthreads();
   static_assert(MAXB == 64, "the lean factorization is written for 64-column panels");
   const int kept = pchol_filter_df_lean(sm, nb, rows, tol_loc);
   // R11 in slot order: R11[a][c] = R[a][ord[c]] for c >= a
   for (int idx = tid; idx < MAXB * MAXB; idx += blockDim.x) {
     const int a = idx / MAXB, c = idx % MAXB;
-    const dfl v = (a < kept && c < kept && c >= a) ? sm.R[a][sm.ord[c]] : dfl{0.f, 0.f};
-    R11g[idx] = make_float2(v.hi, v.lo);
+    if (a < kept && c < kept) R[(int64_t)(i + a) * ldr + i + c] = c >= a ? df_dbl(sm.R[a][sm.ord[c]]) : 0.0;
   }
   // R11^{-1} (upper triangular, slot order) by columns: 16 threads per column c solve
   // R11 x = e_c from the bottom, the dot products split over the 16 lanes.  The Schur
@@ -209,17 +215,6 @@ k_panel_q_df(const float* __restrict__ V, int m, const State* __restrict__ st, c
         Qrl[(int64_t)rw * MAXB + s] = sm.Lr[rr][s];
       }
     }
-  }
-}
-
-// R(I2, I2) = R11, the panel R of a single CholQR pass (upper triangle, slot order).
-__global__ void k_write_r11(const State* __restrict__ st, const float2* __restrict__ R11g, double* __restrict__ R,
-                            int64_t ldr) {
-  const int kept = st->bs, i = st->i;
-  for (int idx = threadIdx.x; idx < kept * kept; idx += blockDim.x) {
-    const int a = idx / kept, c = idx % kept;
-    const float2 v = R11g[a * MAXB + c];
-    R[(int64_t)(i + a) * ldr + (i + c)] = c >= a ? (double)v.x + (double)v.y : 0.0;
   }
 }
 

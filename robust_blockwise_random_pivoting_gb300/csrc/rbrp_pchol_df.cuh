@@ -13,13 +13,10 @@ struct PcholDfSmemT {
   dfl S[BB][BB + 1];  // Schur complement, indexed by panel column
   dfl R[BB][BB + 1];  // R[t][j]: row t of the factor, by panel column j
   int ord[BB];        // slot -> panel column
-  int slot[BB];       // panel column -> slot (pchol_filter_df_lean)
   int alive[BB];
   int J[BB], K1[BB], K2[BB], inblk[BB], Tperm[BB];
   int stop, piv, nK;
   dfl inv;
-  dfl cval[32], crem[32];  // per diagonal owner: best live diagonal and live diagonal sum
-  int cslot[32], ccol[32];
 };
 
 // Block swap of perm and diags (matlab/RBRP.m:81-99), in parallel: K1 = block
@@ -167,17 +164,17 @@ __device__ int pchol_filter_df(PcholDfSmemT<BB>& sm, int nb, int rows, double to
 }
 
 // The same factorization and filter as pchol_filter_df<64>, by 1024 threads
-// (LEAN_THREADS): thread (ty, tx) of a 32 x 32 grid owns the Schur entries of
-// rows ty + 32u and columns tx + 32v (u, v < 2), so a warp touches one row pair
-// of consecutive entries (no bank conflicts) and each thread's update is four
-// independent double-float chains.  Two barriers per step instead of three and
-// a 32-way pivot search: the 32 threads that own diagonal entries (ty == tx)
-// rank their live diagonals right after updating them, and every thread forms
-// its own factor-row values S(pv, j) / r from the pivot row, which no thread
-// writes during the update.  Each Schur entry gets the same double-float
-// operation on the same inputs and pivots tie to the first slot as before;
-// only the remaining-trace sum of the stop test is added in another order.
+// (LEAN_THREADS).  A step: warp 0 finds the pivot among the diagonal entries
+// (reductions of the bit patterns, first slot on ties), takes its square root and
+// reciprocal and scales its row; warp 1 sums the remaining trace for the filter;
+// a barrier; warp w updates the active slots t + 1 + w and t + 33 + w, lanes over
+// the active columns; a barrier.  Each Schur entry gets the same double-float
+// operation on the same inputs as in the 256-thread form, both triangles (the
+// low parts of an entry and its mirror differ with the order of the factors).
 // Square root and reciprocal start from the correctly rounded FP32 intrinsics.
+// Latency bound on one SM: 64 steps of two barriers and the pivot's chain.  With
+// every thread scaling its own rows, a pivot search by shuffles and no
+// compaction a step took 4,000 clocks (64 columns: 128 us with the inverse, now about 60).
 constexpr int LEAN_THREADS = 1024;
 
 __device__ __forceinline__ dfl df_sqrt_lean(dfl a) {
@@ -193,101 +190,87 @@ __device__ __forceinline__ dfl df_recip_lean(dfl b) {
 }
 
 __device__ int pchol_filter_df_lean(PcholDfSmemT<64>& sm, int nb, int rows, double tol_loc) {
-  constexpr int BB = 64, U = 2, G = 32;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int ty = wid, tx = lane;
-  const bool owner = ty == tx;  // owns the diagonal entries ty + 32u
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  bool a0 = lane < nb, a1 = lane + 32 < nb;   // warp 1: its columns still active
   bool have_total = false;
   dfl thr = {0.f, 0.f};
-  if (tid < BB) sm.slot[tid] = tid;
-  auto rank_diag = [&]() {
-    dfl best = {-1.f, 0.f}, rem = {0.f, 0.f};
-    int bs = BB, bc = -1;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = ty + G * u;
-      if (j < nb && sm.alive[j]) {
-        const dfl d = sm.S[j][j];
-        rem = df_add(rem, d);
-        const int sj = sm.slot[j];
-        if (df_gt(d, best) || (df_eq(d, best) && sj < bs)) { best = d; bs = sj; bc = j; }
-      }
-    }
-    sm.cval[ty] = best;
-    sm.crem[ty] = rem;
-    sm.cslot[ty] = bs;
-    sm.ccol[ty] = bc;
-  };
-  __syncthreads();
-  if (owner) rank_diag();
-  __syncthreads();
-  if (wid == 0) {
-    dfl t = sm.crem[lane];
+  auto trace = [&]() {   // remaining trace, valid in lane 0
+    dfl rem = {0.f, 0.f};
+    if (a0) rem = df_add(rem, sm.S[lane][lane]);
+    if (a1) rem = df_add(rem, sm.S[lane + 32][lane + 32]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
-      t = df_add(t, {__shfl_down_sync(0xffffffffu, t.hi, o), __shfl_down_sync(0xffffffffu, t.lo, o)});
-    const double total = __shfl_sync(0xffffffffu, df_dbl(t), 0);
+      rem = df_add(rem, {__shfl_down_sync(0xffffffffu, rem.hi, o), __shfl_down_sync(0xffffffffu, rem.lo, o)});
+    return rem;
+  };
+  if (tid == 0) sm.stop = 0;
+  __syncthreads();
+  if (w == 1) {
+    const double total = __shfl_sync(0xffffffffu, df_dbl(trace()), 0);
     have_total = total > 0.0;
     thr = df_of(tol_loc * total);
   }
-  int kept = rows;
   for (int t = 0; t < rows; ++t) {
-    if (wid == 0) {
-      dfl best = sm.cval[lane], rem = sm.crem[lane];
-      int bs = sm.cslot[lane], bc = sm.ccol[lane];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        rem = df_add(rem, {__shfl_down_sync(0xffffffffu, rem.hi, o), __shfl_down_sync(0xffffffffu, rem.lo, o)});
-        const dfl ob = {__shfl_down_sync(0xffffffffu, best.hi, o), __shfl_down_sync(0xffffffffu, best.lo, o)};
-        const int os = __shfl_down_sync(0xffffffffu, bs, o), oc = __shfl_down_sync(0xffffffffu, bc, o);
-        if (df_gt(ob, best) || (df_eq(ob, best) && os < bs)) { best = ob; bs = os; bc = oc; }
+    if (w == 0) {
+      const int c0 = sm.ord[lane], c1 = sm.ord[lane + 32];
+      dfl best = {-1.f, 0.f};
+      int slot = 64;
+      if (lane >= t && lane < nb) { best = sm.S[c0][c0]; slot = lane; }
+      if (lane + 32 >= t && lane + 32 < nb) {
+        const dfl d = sm.S[c1][c1];
+        if (slot == 64 || df_gt(d, best)) { best = d; slot = lane + 32; }
       }
+      const unsigned hi = best.hi > 0.f ? __float_as_uint(best.hi) : 0u;
+      const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+      const unsigned lb = __float_as_uint(best.lo + 0.f);   // -0 as +0
+      const unsigned lo = hi == mh ? ((lb & 0x80000000u) ? ~lb : (lb | 0x80000000u)) : 0u;
+      const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+      const unsigned sl = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (unsigned)slot : 64u);
+      const int bs = mh ? (int)sl : t;
+      const int o = sm.ord[t], pv = sm.ord[bs];
+      __syncwarp();
       if (lane == 0) {
-        const bool stop = !have_total || df_gt(thr, rem) || !(best.hi > 0.f) || bc < 0;
-        sm.stop = stop;
-        if (!stop) {
-          // LAPACK order: the pivot column moves to slot t, slot t's column to the pivot's slot
-          const int o = sm.ord[t];
-          sm.ord[t] = bc;
-          sm.ord[bs] = o;
-          sm.slot[o] = bs;
-          sm.slot[bc] = t;
-          sm.alive[bc] = 0;
-          const dfl r = df_sqrt_lean(sm.S[bc][bc]);
-          sm.R[t][bc] = r;
-          sm.inv = df_recip_lean(r);
-          sm.piv = bc;
+        if (!mh) sm.stop = 1;
+        // LAPACK order: the pivot column moves to slot t, slot t's column to the pivot's slot
+        sm.ord[t] = pv;
+        sm.ord[bs] = o;
+      }
+      __syncwarp();
+      const dfl r = df_sqrt_lean(sm.S[pv][pv]);
+      const dfl inv = df_recip_lean(r);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int s = lane + 32 * u;
+        if (s > t && s < nb) {
+          const int c = sm.ord[s];
+          sm.R[t][c] = df_mul(sm.S[pv][c], inv);
         }
       }
+      if (lane == 0) {
+        sm.R[t][pv] = r;
+        sm.piv = pv;
+      }
+    } else if (w == 1) {
+      const dfl rem = trace();
+      if (lane == 0 && (!have_total || df_gt(thr, rem))) sm.stop = 1;
     }
     __syncthreads();
-    if (sm.stop) { kept = t; break; }
-    const int pv = sm.piv;
-    const dfl inv = sm.inv;
-    dfl ru[U], rv[U];
-    bool au[U], av[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = ty + G * u, c = tx + G * u;
-      au[u] = j < nb && sm.alive[j];
-      av[u] = c < nb && sm.alive[c];
-      ru[u] = au[u] ? df_mul(sm.S[pv][j], inv) : dfl{0.f, 0.f};
-      rv[u] = av[u] ? df_mul(sm.S[pv][c], inv) : dfl{0.f, 0.f};
+    if (sm.stop) return t;
+    if (w == 1) {
+      a0 = a0 && sm.piv != lane;
+      a1 = a1 && sm.piv != lane + 32;
     }
-    if (ty == 0) {
-#pragma unroll
-      for (int v = 0; v < U; ++v)
-        if (av[v]) sm.R[t][tx + G * v] = rv[v];
+    for (int ss = t + 1 + w; ss < nb; ss += 32) {
+      const int c = sm.ord[ss];
+      const dfl rc = sm.R[t][c];
+      for (int s2 = t + 1 + lane; s2 < nb; s2 += 32) {
+        const int c2 = sm.ord[s2];
+        sm.S[c][c2] = df_fms(sm.S[c][c2], rc, sm.R[t][c2]);
+      }
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int v = 0; v < U; ++v)
-        if (au[u] && av[v]) sm.S[ty + G * u][tx + G * v] = df_fms(sm.S[ty + G * u][tx + G * v], ru[u], rv[v]);
-    if (owner) rank_diag();
     __syncthreads();
   }
-  return kept;
+  return rows;
 }
 
 }  // namespace

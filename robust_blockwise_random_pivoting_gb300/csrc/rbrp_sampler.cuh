@@ -24,13 +24,54 @@ namespace {
 // ===========================================================================
 constexpr int SAMPLE_THREADS = 1024;
 
+// Weights, probabilities and cdf values are never negative: their bit patterns order as they
+// do, and a comparison on the FP64 pipe takes a warp 20 clocks.
+__device__ __forceinline__ bool nonneg_gt(double a, double b) {
+  return __double_as_longlong(a) > __double_as_longlong(b);
+}
+
+// block_exclusive_scan of one value per thread where `any` tells which warps hold some (the
+// others' zeros would only take the FP64 pipe): the same sums in the same order.
+__device__ __forceinline__ double scan_active(double v, bool any, double* sh) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  double x = v;
+  if (any) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+  }
+  __syncthreads();
+  if (lane == 31) sh[wid] = x;
+  __syncthreads();
+  if (wid == 0) {
+    double w = lane < nw ? sh[lane] : 0.0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    sh[lane] = w;
+  }
+  __syncthreads();
+  const double off = wid ? sh[wid - 1] : 0.0;
+  __syncthreads();
+  double excl = __shfl_up_sync(0xffffffffu, x, 1);
+  if (lane == 0) excl = 0.0;
+  return off + excl;
+}
+
 // Block-wide sampler body (any block size from 64 to MAXT); k_sample runs it with
-// 1024 threads, the batched kernel with its CTA.
+// 1024 threads, the batched kernel with its CTA.  pre_tot / pre_pos (one entry per thread,
+// or NULL): the NP sampler's probabilities are in pbuf already, with the chunk totals and
+// counts (k_sample_probs, which spreads their FP64 work over 32 SMs).
 template <int MAXT = SAMPLE_THREADS>
 __device__ void sample_block(State* st, const double* __restrict__ diags, const int* __restrict__ perm, int n,
                              int kmax, int b, uint64_t seed, int sampler, double* __restrict__ pbuf,
                              unsigned long long* __restrict__ kbuf, int* __restrict__ js, int* __restrict__ cols,
-                             const int* __restrict__ order_of = nullptr) {
+                             const int* __restrict__ order_of = nullptr, const double* __restrict__ pre_tot = nullptr,
+                             const int* __restrict__ pre_pos = nullptr) {
   __shared__ double shd[32];
   __shared__ int shi[32];
   __shared__ unsigned int hist[256];
@@ -56,20 +97,24 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
 
   if (sampler == SAMPLER_NP) {
     // p = w / sum(w)
-    double part = 0.0;
-    for (int j = lo; j < hi; ++j) part += w[j];
-    const double S = block_sum(part, shd);
-    // one FP64 division for the block, shared: per-thread or per-entry divisions are
-    // ~1/64-rate work on GB300
-    __shared__ double s_invS;
-    if (tid == 0) s_invS = 1.0 / S;
-    __syncthreads();
-    const double invS = s_invS;
     int npos = 0;
-    for (int j = lo; j < hi; ++j) {
-      const double pj = w[j] * invS;
-      pbuf[j] = pj;
-      npos += pj > 0.0;
+    if (pre_tot) {
+      npos = pre_pos[tid];
+    } else {
+      double part = 0.0;
+      for (int j = lo; j < hi; ++j) part += w[j];
+      const double S = block_sum(part, shd);
+      // one FP64 division for the block, shared: per-thread or per-entry divisions are
+      // ~1/64-rate work on GB300
+      __shared__ double s_invS;
+      if (tid == 0) s_invS = 1.0 / S;
+      __syncthreads();
+      const double invS = s_invS;
+      for (int j = lo; j < hi; ++j) {
+        const double pj = w[j] * invS;
+        pbuf[j] = pj;
+        npos += nonneg_gt(pj, 0.0);
+      }
     }
     npos = block_sum(npos, shi);
     if (tid == 0) {
@@ -85,22 +130,22 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
     __shared__ double s_end[MAXT];
     __shared__ double s_off[MAXT];
     __shared__ double s_last, s_inv_last;
-    double tot = 0.0;
+    __shared__ unsigned s_new[2];
+    double tot = pre_tot ? pre_tot[tid] : 0.0;
+    const bool warp_any = (tid & ~31) * chunk < nrem;   // some thread of this warp holds entries
     __syncthreads();
     // Rejection rounds.  Each round draws at least one new index unless every
     // remaining positive weight is absorbed by rounding in the cdf; the cap
     // turns that (pathological) case into a smaller sample instead of a spin.
     for (int round = 0; s_found < s_size && round < 4096; ++round) {
       const int found = s_found, need = s_size - s_found;
-      if (tid < found) pbuf[s_rel[tid]] = 0.0;
+      if (tid < found) {
+        pbuf[s_rel[tid]] = 0.0;
+        s_end[s_rel[tid] / chunk] = -1.0;   // that chunk's total is to be formed again
+      }
       __syncthreads();
       // chunk totals: every chunk in the first round, afterwards the chunks holding a drawn index
-      bool dirty = round == 0;
-      for (int u = 0; u < found && !dirty; ++u) {
-        const int jr = s_rel[u];
-        dirty = jr >= lo && jr < hi;
-      }
-      if (dirty) {
+      if (round == 0 ? pre_tot == nullptr : __double_as_longlong(s_end[tid]) < 0) {
         double run = 0.0;
         int j = lo;
         for (; j + 8 <= hi; j += 8) {
@@ -113,7 +158,7 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
         for (; j < hi; ++j) run += pbuf[j];
         tot = run;
       }
-      const double off = block_exclusive_scan(tot, shd, (double*)nullptr);
+      const double off = scan_active(tot, warp_any, shd);
       if (lo < hi && hi == nrem) {
         s_last = off + tot;
         s_inv_last = 1.0 / s_last;  // once, by the thread holding the last chunk
@@ -128,7 +173,7 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
         int a = 0, z = (int)blockDim.x;  // first chunk whose last cdf entry is > x
         while (a < z) {
           const int mid = (a + z) >> 1;
-          if (s_end[mid] <= x) a = mid + 1; else z = mid;
+          if (!nonneg_gt(s_end[mid], x)) a = mid + 1; else z = mid;
         }
         const int t = min(a, (int)blockDim.x - 1);
         const int clo = min(nrem, t * chunk), chi = min(nrem, clo + chunk);
@@ -146,7 +191,7 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
             if (!hit && j < chi) {
               run += v[q];
               const double c = j == nrem - 1 ? 1.0 : (co + run) * inv_last;
-              if (c > x) {
+              if (nonneg_gt(c, x)) {
                 pick = j;
                 hit = true;
               }
@@ -156,15 +201,26 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
         s_cand[tid] = pick < nrem ? pick : nrem - 1;
       }
       __syncthreads();
-      if (tid == 0) {
-        int f = found;
-        for (int t = 0; t < need; ++t) {
-          const int c = s_cand[t];
-          bool dup = false;
-          for (int u = 0; u < t; ++u) dup |= (s_cand[u] == c);
-          if (!dup) s_rel[f++] = c;
+      // first occurrences in draw order, 64 threads side by side (one thread comparing all
+      // pairs took 8 of a 64-column block's 41 us)
+      bool fresh = tid < need;
+      int mine = -1;
+      if (tid < MAXB) {
+        if (fresh) {
+          mine = s_cand[tid];
+          for (int u = 0; u < tid; ++u) fresh = fresh && s_cand[u] != mine;
         }
-        s_found = f;
+        const unsigned bal = __ballot_sync(0xffffffffu, fresh);
+        if ((tid & 31) == 0) s_new[tid >> 5] = bal;
+      }
+      __syncthreads();
+      const unsigned n0 = s_new[0], n1 = s_new[1];
+      if (fresh) {
+        const unsigned before = (1u << (tid & 31)) - 1u;
+        s_rel[found + (tid < 32 ? __popc(n0 & before) : __popc(n0) + __popc(n1 & before))] = mine;
+      }
+      if (tid == 0) {
+        s_found = found + __popc(n0) + __popc(n1);
         s_draws += (unsigned long long)need;
       }
       __syncthreads();
@@ -307,6 +363,55 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
     st->draws = s_draws;
   }
   __syncthreads();
+}
+
+// The NP sampler's FP64 passes for many columns: thread t of k_sample's 1024 owns the chunk
+// [t chunk, (t + 1) chunk) of the remaining positions; here chunk t belongs to thread t % 32 of
+// CTA t / 32, so the sums keep their order and take 32 SMs' FP64 pipes instead of one's.
+constexpr int SAMPLE_PRE_MIN = 8192;   // remaining positions from which the two launches pay (64,500
+// columns: 180 us a block in one launch, 50 in three; 15,000: 70 and 40)
+
+// part[t] = sum of the chunk's weights
+__global__ void __launch_bounds__(32)
+k_sample_sums(const State* __restrict__ st, const double* __restrict__ diags, int n, double* __restrict__ part) {
+  const int nrem = n - st->i, t = blockIdx.x * 32 + threadIdx.x;
+  const int chunk = (nrem + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
+  const int lo = min(nrem, t * chunk), hi = min(nrem, lo + chunk);
+  const double* w = diags + st->i;
+  double s = 0.0;
+#pragma unroll 8
+  for (int j = lo; j < hi; ++j) s += w[j];
+  part[t] = s;
+}
+
+// p = w / sum(w) into pbuf, chunk totals of p and counts of positive p.  Every CTA adds up the
+// 1024 partial sums as block_sum does.
+__global__ void __launch_bounds__(32)
+k_sample_probs(const State* __restrict__ st, const double* __restrict__ diags, int n, const double* __restrict__ part,
+               double* __restrict__ pbuf, double* __restrict__ tot, int* __restrict__ pos) {
+  const int nrem = n - st->i, lane = threadIdx.x, t = blockIdx.x * 32 + lane;
+  const int chunk = (nrem + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
+  const int lo = min(nrem, t * chunk), hi = min(nrem, lo + chunk);
+  const double* w = diags + st->i;
+  double mine = 0.0;
+#pragma unroll 4
+  for (int q = 0; q < 32; ++q) {
+    const double s = __shfl_sync(0xffffffffu, warp_sum(part[32 * q + lane]), 0);
+    if (lane == q) mine = s;
+  }
+  const double S = __shfl_sync(0xffffffffu, warp_sum(mine), 0);
+  const double invS = 1.0 / S;
+  double run = 0.0;
+  int np = 0;
+#pragma unroll 8
+  for (int j = lo; j < hi; ++j) {
+    const double pj = w[j] * invS;
+    pbuf[j] = pj;
+    np += nonneg_gt(pj, 0.0);
+    run += pj;
+  }
+  tot[t] = run;
+  pos[t] = np;
 }
 
 }  // namespace
