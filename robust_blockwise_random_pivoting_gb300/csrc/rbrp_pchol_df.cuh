@@ -168,7 +168,9 @@ __device__ int pchol_filter_df(PcholDfSmemT<BB>& sm, int nb, int rows, double to
 // (reductions of the bit patterns, first slot on ties), takes its square root and
 // reciprocal and scales its row; warp 1 sums the remaining trace for the filter;
 // a barrier; warp w updates the active slots t + 1 + w and t + 33 + w, lanes over
-// the active columns; a barrier.  Each Schur entry gets the same double-float
+// the columns as they are stored (active ones; by slot, the permuted columns cost
+// four times the shared-memory wavefronts and 1,600 of a step's 3,300 clocks); a
+// barrier.  Each Schur entry gets the same double-float
 // operation on the same inputs as in the 256-thread form, both triangles (the
 // low parts of an entry and its mirror differ with the order of the factors).
 // Square root and reciprocal start from the correctly rounded FP32 intrinsics.
@@ -191,7 +193,7 @@ __device__ __forceinline__ dfl df_recip_lean(dfl b) {
 
 __device__ int pchol_filter_df_lean(PcholDfSmemT<64>& sm, int nb, int rows, double tol_loc) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  bool a0 = lane < nb, a1 = lane + 32 < nb;   // warp 1: its columns still active
+  bool a0 = lane < nb, a1 = lane + 32 < nb;   // the lane's columns still active
   bool have_total = false;
   dfl thr = {0.f, 0.f};
   auto trace = [&]() {   // remaining trace, valid in lane 0
@@ -238,35 +240,31 @@ __device__ int pchol_filter_df_lean(PcholDfSmemT<64>& sm, int nb, int rows, doub
       __syncwarp();
       const dfl r = df_sqrt_lean(sm.S[pv][pv]);
       const dfl inv = df_recip_lean(r);
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int s = lane + 32 * u;
-        if (s > t && s < nb) {
-          const int c = sm.ord[s];
-          sm.R[t][c] = df_mul(sm.S[pv][c], inv);
-        }
-      }
-      if (lane == 0) {
-        sm.R[t][pv] = r;
-        sm.piv = pv;
-      }
+      if (a0) sm.R[t][lane] = pv == lane ? r : df_mul(sm.S[pv][lane], inv);
+      if (a1) sm.R[t][lane + 32] = pv == lane + 32 ? r : df_mul(sm.S[pv][lane + 32], inv);
+      if (lane == 0) sm.piv = pv;
     } else if (w == 1) {
       const dfl rem = trace();
       if (lane == 0 && (!have_total || df_gt(thr, rem))) sm.stop = 1;
     }
     __syncthreads();
     if (sm.stop) return t;
-    if (w == 1) {
-      a0 = a0 && sm.piv != lane;
-      a1 = a1 && sm.piv != lane + 32;
-    }
-    for (int ss = t + 1 + w; ss < nb; ss += 32) {
-      const int c = sm.ord[ss];
-      const dfl rc = sm.R[t][c];
-      for (int s2 = t + 1 + lane; s2 < nb; s2 += 32) {
-        const int c2 = sm.ord[s2];
-        sm.S[c][c2] = df_fms(sm.S[c][c2], rc, sm.R[t][c2]);
-      }
+    a0 = a0 && sm.piv != lane;
+    a1 = a1 && sm.piv != lane + 32;
+    if (t + 1 + w < nb) {
+      const bool two = t + 33 + w < nb;
+      const int r0 = sm.ord[t + 1 + w], r1 = sm.ord[two ? t + 33 + w : t + 1 + w];
+      const dfl f0 = sm.R[t][r0], f1 = sm.R[t][r1];
+      const dfl g0 = a0 ? sm.R[t][lane] : dfl{0.f, 0.f}, g1 = a1 ? sm.R[t][lane + 32] : dfl{0.f, 0.f};
+      dfl x00 = {0.f, 0.f}, x01 = x00, x10 = x00, x11 = x00;
+      if (a0) x00 = sm.S[r0][lane];
+      if (a1) x01 = sm.S[r0][lane + 32];
+      if (two && a0) x10 = sm.S[r1][lane];
+      if (two && a1) x11 = sm.S[r1][lane + 32];
+      if (a0) sm.S[r0][lane] = df_fms(x00, f0, g0);
+      if (a1) sm.S[r0][lane + 32] = df_fms(x01, f0, g1);
+      if (two && a0) sm.S[r1][lane] = df_fms(x10, f1, g0);
+      if (two && a1) sm.S[r1][lane + 32] = df_fms(x11, f1, g1);
     }
     __syncthreads();
   }
