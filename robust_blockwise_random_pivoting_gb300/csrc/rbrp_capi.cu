@@ -159,6 +159,9 @@ rbrp_status ensure_workspace(rbrp_handle h, const Layout& L) {
       {(void**)&h->K2, MAXB * 4},
       {(void**)&h->part_res, (size_t)L.nproj * 8},
       {(void**)&h->part_nnz, (size_t)L.nproj * 4},
+      {(void**)&h->fix_q, L.residual ? 0 : m * 8 * 2 * 4},
+      {(void**)&h->fix_exQ, MAXB * 4},
+      {(void**)&h->fix_exA, L.residual ? 0 : n * 4},
       {(void**)&h->trace_rank, kmax * 4},
       {(void**)&h->trace_err, kmax * 8},
       {(void**)&h->trace_samp, kmax * 4},
@@ -239,6 +242,27 @@ void release_slices(rbrp_handle h) {
   h->sl_bytes = 0;
 }
 
+// sl_ws with room for `total` bytes, if that is at most half of what is free.
+static bool ensure_sl_ws(rbrp_handle h, size_t total) {
+  if (total <= h->sl_bytes) return true;
+  release_slices(h);
+  size_t avail = 0, all = 0;
+  if (cudaMemGetInfo(&avail, &all) != cudaSuccess || total > avail / 2 ||
+      cudaMalloc(&h->sl_ws, total) != cudaSuccess) {
+    cudaGetLastError();
+    h->sl_ws = nullptr;
+    return false;
+  }
+  h->sl_bytes = total;
+  return true;
+}
+
+bool ensure_fixed(rbrp_handle h, int m, int n) {
+  if (!ensure_sl_ws(h, (size_t)m * n * sizeof(int2))) return false;
+  h->fix_A = static_cast<int2*>(h->sl_ws);
+  return true;
+}
+
 bool ensure_slices(rbrp_handle h, int m, int n) {
   const size_t ldk = ((size_t)m + 63) / 64 * 64;
   // row ranges of the projection: enough CTAs for four waves at the most, 16 ranges at the most
@@ -256,17 +280,7 @@ bool ensure_slices(rbrp_handle h, int m, int n) {
   };
   size_t total = 0;
   for (auto& it : items) total += align_up(it.bytes);
-  if (total > h->sl_bytes) {
-    release_slices(h);
-    size_t avail = 0, all = 0;
-    if (cudaMemGetInfo(&avail, &all) != cudaSuccess || total > avail / 2 ||
-        cudaMalloc(&h->sl_ws, total) != cudaSuccess) {
-      cudaGetLastError();
-      h->sl_ws = nullptr;
-      return false;
-    }
-    h->sl_bytes = total;
-  }
+  if (!ensure_sl_ws(h, total)) return false;
   char* base = static_cast<char*>(h->sl_ws);
   size_t off = 0;
   for (auto& it : items) {

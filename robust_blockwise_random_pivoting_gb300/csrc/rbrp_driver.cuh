@@ -13,6 +13,7 @@
 #include "rbrp_kernels.cuh"
 #include "rbrp_panel64.cuh"
 #include "rbrp_panel_df.cuh"
+#include "rbrp_fixed.cuh"
 #include "rbrp_slices.cuh"
 #include "rbrp_tc.cuh"
 #include "rbrp_update_tc.cuh"
@@ -86,6 +87,10 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   // moves in fewer than one run in 10^4 (b sqrt(n) eps / tol); at 1e-12 it was one in ten.
   const bool fixed_order = p.tol > 0.0 && p.tol < 1e-8 && (p.sampler == SAMPLER_NP || p.sampler == SAMPLER_ES);
   const bool use_sl = !RES && h->variant == 0 && p.b > 8 && m >= tc::SL_BK && !fixed_order && ensure_slices(h, m, n);
+  // Blocks of b <= 8 whose sums may be reordered: the column streams in fixed point, from four
+  // blocks on (the conversion of A costs what two of them gain).
+  const bool use_fix = !RES && h->variant == 0 && p.b <= 8 && m <= FIX_MAX_ROWS && !fixed_order && kmax >= 4 * p.b &&
+                       ensure_fixed(h, m, n);
   const int64_t ldk = ((int64_t)m + tc::SL_BK - 1) / tc::SL_BK * tc::SL_BK;
   CUtensorMap tmSA, tmSQ;
   if (use_sl) {
@@ -118,8 +123,10 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   if (RES)  // the residual starts as A, in position (= column) order
     cudaMemcpy2DAsync(h->Ares, (size_t)L.ld_res * sizeof(float), dA, (size_t)lda * sizeof(T), (size_t)m * sizeof(T),
                       n, cudaMemcpyDeviceToDevice, st);
-  k_colnorm<T><<<(n + 7) / 8, 256, 0, st>>>(dA, lda, m, n, h->diags, h->perm, h->st);
+  k_colnorm<T><<<(n + 7) / 8, 256, 0, st>>>(dA, lda, m, n, h->diags, h->perm, h->st, use_fix ? h->fix_exA : nullptr);
   k_init<<<1, 1024, 0, st>>>(h->st, h->diags, n, kmax);
+  if constexpr (!RES)
+    if (use_fix) k_fix_cols<<<(n + 7) / 8, 256, 0, st>>>(dA, lda, m, n, h->fix_exA, h->fix_A);
   if constexpr (!RES)
     if (use_sl)
       tc::k_slice_cols<<<(n + 7) / 8, 256, 0, st>>>(dA, lda, m, n, n, ldk, h->slA, h->sl_exA);
@@ -139,6 +146,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       return set_error(h, RBRP_ERR_NUMERIC, "no progress: block attempts exceeded 4*kmax+64");
     const int i = h->hst->i;
     const size_t mark0 = h->marks.size();
+    const bool panel_one = use_fix && p.b == 1;
     const int gram_parts = (p.b * (p.b + 1) / 2 + GRAM_PAIRS - 1) / GRAM_PAIRS;
     const int gram_ctas = (p.b * (p.b + 1) / 2 + 63) / 64;
     ev = prof_begin(h);
@@ -177,8 +185,10 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       by_rows([&](auto tr) {
         k_cgs_panel<decltype(tr)::value><<<ptiles, 256, 0, st>>>(dA, lda, h->cols, Q, m, C, h->st, m, h->V);
       });
-      k_gram64<<<dim3(ntiles, gram_parts), 256, 0, st>>>(h->V, m, h->st, 0, h->Gpart);
-      k_reduce_gram<<<gram_ctas, 64, 0, st>>>(h->Gpart, ntiles, h->st, 0, h->G);
+      if (!panel_one) {
+        k_gram64<<<dim3(ntiles, gram_parts), 256, 0, st>>>(h->V, m, h->st, 0, h->Gpart);
+        k_reduce_gram<<<gram_ctas, 64, 0, st>>>(h->Gpart, ntiles, h->st, 0, h->G);
+      }
     }
     prof_end(h, RBRP_PHASE_CGS, ev, 0.0, 0.0, RES ? 2 : i == 0 ? 3 : fixed_order ? 5 : 4);
     ev = prof_begin(h);
@@ -193,17 +203,23 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
           use_tc ? h->Ql : nullptr, L.ld_res, use_tc ? h->Qrh : nullptr, use_tc ? h->Qrl : nullptr);
     }
     if constexpr (!RES) {
-      k_pchol<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11, h->ord,
-                                                    h->J, h->K1, h->K2);
-      by_rows([&](auto tr) {
-        constexpr int TR = decltype(tr)::value;
-        k_panel_solve<TR><<<ptiles, 256, 0, st>>>(h->V, m, h->st, h->R11, h->ord, h->Q1, m, 0);
-        k_gram64<<<dim3(ntiles, gram_parts), 256, 0, st>>>(h->Q1, m, h->st, 1, h->G2part);
-        k_reduce_gram<<<gram_ctas, 64, 0, st>>>(h->G2part, ntiles, h->st, 1, h->G2);
-        k_chol2<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G2, h->st, h->R2);
-        k_panel_solve<TR><<<ptiles, 256, 0, st>>>(h->Q1, m, h->st, h->R2, nullptr, Q, m, 1);
-      });
-      k_panel_r<<<(p.b + 3) / 4, 256, 0, st>>>(h->st, h->R11, h->R2, h->R, n);
+      if (panel_one) {
+        k_panel_one<<<1, 1024, 0, st>>>(h->V, m, h->st, tol_loc, h->js, h->perm, h->diags, Q, m, h->R, n, h->fix_q,
+                                        h->fix_exQ, h->J, h->K1, h->K2);
+      } else {
+        k_pchol<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11, h->ord,
+                                                      h->J, h->K1, h->K2);
+        by_rows([&](auto tr) {
+          constexpr int TR = decltype(tr)::value;
+          k_panel_solve<TR><<<ptiles, 256, 0, st>>>(h->V, m, h->st, h->R11, h->ord, h->Q1, m, 0);
+          k_gram64<<<dim3(ntiles, gram_parts), 256, 0, st>>>(h->Q1, m, h->st, 1, h->G2part);
+          k_reduce_gram<<<gram_ctas, 64, 0, st>>>(h->G2part, ntiles, h->st, 1, h->G2);
+          k_chol2<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G2, h->st, h->R2);
+          k_panel_solve<TR><<<ptiles, 256, 0, st>>>(h->Q1, m, h->st, h->R2, nullptr, Q, m, 1);
+        });
+        k_panel_r<<<(p.b + 3) / 4, 256, 0, st>>>(h->st, h->R11, h->R2, h->R, n);
+        if (use_fix) k_fix_q<<<p.b, 256, 0, st>>>(Q, m, m, h->st, h->fix_q, h->fix_exQ);
+      }
     }
     if (i > 0) k_swap_R<<<(i + 7) / 8, 256, 0, st>>>(h->R, n, h->st, h->J, h->K1, h->K2);
     if (RES)
@@ -340,6 +356,14 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       };
       auto skinny = [&](auto kb) {
         constexpr int KB = decltype(kb)::value;
+        if constexpr (!RES) {
+          if (use_fix) {
+            nproj = (n - i + FixTile<KB>::COLS - 1) / FixTile<KB>::COLS;
+            k_project_fix<KB><<<nproj, 256, 0, st>>>(h->fix_q, h->fix_exQ, h->fix_A, h->fix_exA, h->perm, h->st, m, n,
+                                                     h->R, n, h->diags, h->part_res, h->part_nnz);
+            return;
+          }
+        }
         nproj = (n - i + SKINNY_COLS - 1) / SKINNY_COLS;
         k_project_skinny<T, KB><<<nproj, 256, 0, st>>>(Q, m, dA, lda, h->perm, h->st, m, n, h->R, n, h->diags,
                                                        h->part_res, h->part_nnz);

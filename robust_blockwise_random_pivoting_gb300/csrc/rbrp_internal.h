@@ -81,6 +81,11 @@ struct rbrp_handle_st {
   int* sl_exQ = nullptr;
   double* sl_Wpart = nullptr;
   int sl_maxsplit = 0;
+  // FP64 form, b <= 8 (rbrp_fixed.cuh): limbs of the block's basis, exponents of it and of A's columns
+  int2* fix_A = nullptr;       // A in fixed point (in sl_ws: a run uses one of the two)
+  int* fix_q = nullptr;
+  int* fix_exQ = nullptr;
+  int* fix_exA = nullptr;
   int variant = 0;             // 0: tensor-core projection and update, 1: CUDA-core ones
   bool tsolve_fp64 = false;    // T solve on the FP64 pipe instead of double-float
   long long wait_budget = 0;   // clock64 limit of bounded device waits (0: the default, ~2 s)
@@ -197,6 +202,7 @@ rbrp_status make_tmap_bf16(rbrp_handle h, void* map, const unsigned short* base,
 // Slice workspace of the FP64 form for an m x n matrix; false (and none held) where it would
 // take more than half of the free memory, which the CUDA-core projection then keeps.
 bool ensure_slices(rbrp_handle h, int m, int n);
+bool ensure_fixed(rbrp_handle h, int m, int n);   // the same for the fixed-point copy of A
 void release_slices(rbrp_handle h);
 
 template <typename T>

@@ -31,9 +31,13 @@ namespace {
 // a1: squared column norms (initial weights) - one HBM pass over A.
 // gpu/rbrp.cu:82-99,352-356; python/RBRP.ipynb cell 11 lines 93-94.
 // One warp per column, 16-byte vector loads when the column starts are
-// 16-byte aligned, four loads in flight per lane.
+// 16-byte aligned, four loads in flight per lane.  The FP64 form also keeps
+// the exponent of each column's largest entry (exps, or NULL).
 // ===========================================================================
-__device__ __forceinline__ double col_sumsq(const double* __restrict__ col, int m, int lane, bool vec) {
+__device__ __forceinline__ void max_hi(unsigned& mx, double v) {
+  mx = max(mx, (unsigned)__double2hiint(v) & 0x7FFFFFFFu);
+}
+__device__ __forceinline__ double col_sumsq(const double* __restrict__ col, int m, int lane, bool vec, unsigned& mx) {
   double s0 = 0.0, s1 = 0.0;
   if (vec) {
     const double2* c2 = reinterpret_cast<const double2*>(col);
@@ -45,19 +49,22 @@ __device__ __forceinline__ double col_sumsq(const double* __restrict__ col, int 
       s0 = fma(b.x, b.x, s0); s1 = fma(b.y, b.y, s1);
       s0 = fma(c.x, c.x, s0); s1 = fma(c.y, c.y, s1);
       s0 = fma(d.x, d.x, s0); s1 = fma(d.y, d.y, s1);
+      max_hi(mx, a.x); max_hi(mx, a.y); max_hi(mx, b.x); max_hi(mx, b.y);
+      max_hi(mx, c.x); max_hi(mx, c.y); max_hi(mx, d.x); max_hi(mx, d.y);
     }
     for (; r < m2; r += 32) {
       const double2 a = __ldg(c2 + r);
       s0 = fma(a.x, a.x, s0); s1 = fma(a.y, a.y, s1);
+      max_hi(mx, a.x); max_hi(mx, a.y);
     }
-    if ((m & 1) && lane == 0) { const double v = col[m - 1]; s0 = fma(v, v, s0); }
+    if ((m & 1) && lane == 0) { const double v = col[m - 1]; s0 = fma(v, v, s0); max_hi(mx, v); }
   } else {
-    for (int r = lane; r < m; r += 32) { const double v = col[r]; s0 = fma(v, v, s0); }
+    for (int r = lane; r < m; r += 32) { const double v = col[r]; s0 = fma(v, v, s0); max_hi(mx, v); }
   }
   return warp_sum(s0 + s1);
 }
 
-__device__ __forceinline__ double col_sumsq(const float* __restrict__ col, int m, int lane, bool vec) {
+__device__ __forceinline__ double col_sumsq(const float* __restrict__ col, int m, int lane, bool vec, unsigned&) {
   DF acc{0.f, 0.f};
   if (vec) {
     const float4* c4 = reinterpret_cast<const float4*>(col);
@@ -84,12 +91,17 @@ __device__ __forceinline__ double col_sumsq(const float* __restrict__ col, int m
 template <typename T>
 __global__ void __launch_bounds__(256) k_colnorm(const T* __restrict__ A, int64_t lda, int m, int n,
                                                  double* __restrict__ diags, int* __restrict__ perm,
-                                                 State* st) {
+                                                 State* st, int* __restrict__ exps) {
   const int lane = threadIdx.x & 31;
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= n) return;
   const bool vec = ((reinterpret_cast<uintptr_t>(A) & 15) == 0) && ((lda * (int64_t)sizeof(T)) % 16 == 0);
-  const double s = col_sumsq(A + (int64_t)c * lda, m, lane, vec);
+  unsigned mx = 0u;
+  const double s = col_sumsq(A + (int64_t)c * lda, m, lane, vec, mx);
+  if (exps) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) exps[c] = (int)max(mx >> 20, 1u) - 1022;   // |a| < 2^exps
+  }
   if (lane == 0) {
     diags[c] = s;
     perm[c] = c;
