@@ -145,12 +145,15 @@ rbrp_status ensure_workspace(rbrp_handle h, const Layout& L) {
       {(void**)&h->Q1, m * MAXB * 8},
       {(void**)&h->Cpart, (size_t)L.cpart_rows * MAXB * el},
       {(void**)&h->C, (L.residual ? 1 : kmax) * MAXB * el},
-      {(void**)&h->Gpart, (size_t)L.ntiles * (L.residual ? M2 : (size_t)NPAIR) * 8},
+      {(void**)&h->Gpart, L.residual ? (size_t)L.ntiles * M2 * 8 : (size_t)L.ptiles * NPAIR * 8},
       {(void**)&h->G, M2 * 8},
-      {(void**)&h->G2part, L.residual ? 0 : (size_t)L.ntiles * NPAIR * 8},
+      {(void**)&h->G2part, L.residual ? 0 : (size_t)L.ptiles * NPAIR * 8},
       {(void**)&h->G2, M2 * 8},
       {(void**)&h->R11, M2 * 8},
       {(void**)&h->R2, M2 * 8},
+      {(void**)&h->X11, M2 * 8},
+      {(void**)&h->U2, M2 * 4},
+      {(void**)&h->chol2_full, 4},
       {(void**)&h->ord, MAXB * 4},
       {(void**)&h->js, MAXB * 4},
       {(void**)&h->cols, MAXB * 4},

@@ -12,6 +12,7 @@
 #include "rbrp_internal.h"
 #include "rbrp_kernels.cuh"
 #include "rbrp_panel64.cuh"
+#include "rbrp_panel64f.cuh"
 #include "rbrp_panel_df.cuh"
 #include "rbrp_fixed.cuh"
 #include "rbrp_slices.cuh"
@@ -32,6 +33,16 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   if (s != RBRP_OK) return s;
   {  // function attributes are per device context: set them on every call (cheap)
     if constexpr (!RES) {
+      for (const void* fn : {(const void*)k_pchol_ldl, (const void*)k_chol2_fast}) {
+        s = cuda_check(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LdlSmem)),
+                       "cudaFuncSetAttribute(panel)");
+        if (s != RBRP_OK) return s;
+      }
+      for (const void* fn : {(const void*)k_panel1_fast<32>, (const void*)k_panel2_fast<32>}) {
+        s = cuda_check(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)panel_rows_smem<32>()), "cudaFuncSetAttribute(panel rows)");
+        if (s != RBRP_OK) return s;
+      }
       for (const void* fn : {(const void*)k_pchol, (const void*)k_chol2}) {
         s = cuda_check(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)sizeof(Panel64Smem)), "cudaFuncSetAttribute(panel)");
@@ -185,7 +196,12 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       by_rows([&](auto tr) {
         k_cgs_panel<decltype(tr)::value><<<ptiles, 256, 0, st>>>(dA, lda, h->cols, Q, m, C, h->st, m, h->V);
       });
-      if (!panel_one) {
+      if (!panel_one && !fixed_order) {
+        by_rows([&](auto tr) {
+          k_gram_tiles<decltype(tr)::value><<<ptiles, 256, 0, st>>>(h->V, m, h->st, h->Gpart);
+        });
+        k_reduce_gram_fast<<<2 * gram_ctas, 256, 0, st>>>(h->Gpart, ptiles, h->st, 0, h->G);
+      } else if (!panel_one) {
         k_gram64<<<dim3(ntiles, gram_parts), 256, 0, st>>>(h->V, m, h->st, 0, h->Gpart);
         k_reduce_gram<<<gram_ctas, 64, 0, st>>>(h->Gpart, ntiles, h->st, 0, h->G);
       }
@@ -206,6 +222,19 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       if (panel_one) {
         k_panel_one<<<1, 1024, 0, st>>>(h->V, m, h->st, tol_loc, h->js, h->perm, h->diags, Q, m, h->R, n, h->fix_q,
                                         h->fix_exQ, h->J, h->K1, h->K2);
+      } else if (!fixed_order) {
+        k_pchol_ldl<<<1, 1024, sizeof(LdlSmem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11,
+                                                      h->X11, h->ord, h->J, h->K1, h->K2);
+        by_rows([&](auto tr) {
+          constexpr int TR = decltype(tr)::value;
+          k_panel1_fast<TR><<<ptiles, 256, panel_rows_smem<TR>(), st>>>(h->V, m, h->st, h->X11, h->ord, h->Q1,
+                                                                       h->G2part);
+          k_reduce_gram_fast<<<2 * gram_ctas, 256, 0, st>>>(h->G2part, ptiles, h->st, 1, h->G2);
+          k_chol2_fast<<<1, 1024, sizeof(LdlSmem), st>>>(h->G2, h->st, h->R11, h->R2, h->U2, h->chol2_full, h->R, n);
+          k_panel2_fast<TR><<<ptiles, 256, panel_rows_smem<TR>(), st>>>(h->Q1, m, h->st, h->R2, h->U2, h->chol2_full,
+                                                                       Q, m);
+        });
+        if (use_fix) k_fix_q<<<p.b, 256, 0, st>>>(Q, m, m, h->st, h->fix_q, h->fix_exQ);
       } else {
         k_pchol<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11, h->ord,
                                                       h->J, h->K1, h->K2);
@@ -218,7 +247,6 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
           k_panel_solve<TR><<<ptiles, 256, 0, st>>>(h->Q1, m, h->st, h->R2, nullptr, Q, m, 1);
         });
         k_panel_r<<<(p.b + 3) / 4, 256, 0, st>>>(h->st, h->R11, h->R2, h->R, n);
-        if (use_fix) k_fix_q<<<p.b, 256, 0, st>>>(Q, m, m, h->st, h->fix_q, h->fix_exQ);
       }
     }
     if (i > 0) k_swap_R<<<(i + 7) / 8, 256, 0, st>>>(h->R, n, h->st, h->J, h->K1, h->K2);
@@ -231,7 +259,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
         tc::k_swap_slices<<<dim3(p.b, tc::SL), 256, 0, st>>>(h->slA, n, ldk, h->sl_exA, h->st, h->K1, h->K2);
       }
     }
-    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 4 : 3) : (i > 0 ? 8 : 7) + (use_sl ? 2 : 0));
+    prof_end(h, RBRP_PHASE_PANEL, ev, 0.0, 0.0, RES ? (i > 0 ? 4 : 3) : (panel_one ? 1 : fixed_order ? 7 : 5) + (i > 0) + (use_sl ? 2 : 0));
     int nproj;
     ev = prof_begin(h);
     if (RES) {

@@ -42,7 +42,10 @@ struct rbrp_handle_st {
   double* G2part = nullptr;
   double* G2 = nullptr;
   double* R11 = nullptr;
-  double* R2 = nullptr;
+  double* R2 = nullptr;        // FP64 form: R2 of the second CholQR pass, or its inverse
+  double* X11 = nullptr;       // FP64 form, free order: R11^{-1}
+  float* U2 = nullptr;         // FP64 form, free order: R2 - I where it is small, and which of the two holds
+  int* chol2_full = nullptr;
   int* ord = nullptr;
   double* pbuf = nullptr;      // 2n: weights and cdf
   unsigned long long* kbuf = nullptr;
