@@ -266,7 +266,7 @@ bool ensure_fixed(rbrp_handle h, int m, int n) {
   return true;
 }
 
-bool ensure_slices(rbrp_handle h, int m, int n) {
+bool ensure_slices(rbrp_handle h, int m, int n, int kmax) {
   const size_t ldk = ((size_t)m + 63) / 64 * 64;
   // row ranges of the projection: enough CTAs for four waves at the most, 16 ranges at the most
   const int ctiles = (n + 127) / 128;
@@ -277,6 +277,10 @@ bool ensure_slices(rbrp_handle h, int m, int n) {
   } items[] = {
       {(void**)&h->slA, 7 * ldk * (size_t)n * 2},
       {(void**)&h->slQ, 7 * ldk * MAXB * 2},
+      {(void**)&h->slH, 7 * ldk * (size_t)kmax * 2},
+      {(void**)&h->slC, 7 * (((size_t)kmax + 63) / 64 * 64) * MAXB * 2},
+      {(void**)&h->sl_exH, (size_t)kmax * 4},
+      {(void**)&h->sl_exC, MAXB * 4},
       {(void**)&h->sl_exA, (size_t)n * 4},
       {(void**)&h->sl_exQ, MAXB * 4},
       {(void**)&h->sl_Wpart, (size_t)maxsplit * MAXB * n * 8},

@@ -97,16 +97,24 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   // (eps / tol relative), and which column a draw takes follows that order.  Above, a draw
   // moves in fewer than one run in 10^4 (b sqrt(n) eps / tol); at 1e-12 it was one in ten.
   const bool fixed_order = p.tol > 0.0 && p.tol < 1e-8 && (p.sampler == SAMPLER_NP || p.sampler == SAMPLER_ES);
-  const bool use_sl = !RES && h->variant == 0 && p.b > 8 && m >= tc::SL_BK && !fixed_order && ensure_slices(h, m, n);
+  const bool use_sl = !RES && h->variant == 0 && p.b > 8 && m >= tc::SL_BK && !fixed_order &&
+                      ensure_slices(h, m, n, kmax);
   // Blocks of b <= 8 whose sums may be reordered: the column streams in fixed point, from four
   // blocks on (the conversion of A costs what two of them gain).
   const bool use_fix = !RES && h->variant == 0 && p.b <= 8 && m <= FIX_MAX_ROWS && !fixed_order && kmax >= 4 * p.b &&
                        ensure_fixed(h, m, n);
   const int64_t ldk = ((int64_t)m + tc::SL_BK - 1) / tc::SL_BK * tc::SL_BK;
-  CUtensorMap tmSA, tmSQ;
+  CUtensorMap tmSA, tmSQ, tmSH, tmSC;
+  const int64_t ldc = ((int64_t)kmax + 63) / 64 * 64;
   if (use_sl) {
     s = make_tmap_bf16(h, &tmSA, h->slA, ldk, (uint64_t)tc::SL * n, tc::BM);
     if (s == RBRP_OK) s = make_tmap_bf16(h, &tmSQ, h->slQ, ldk, tc::SL * MAXB, tc::SL * tc::SL_HALF);
+    if (s == RBRP_OK) s = make_tmap_bf16(h, &tmSH, h->slH, ldk, (uint64_t)tc::SL * kmax, tc::SL_BK);
+    if (s == RBRP_OK) s = make_tmap_bf16(h, &tmSC, h->slC, ldc, tc::SL * MAXB, tc::SL * tc::SL_HALF);
+    if (s == RBRP_OK)
+      s = cuda_check(h, cudaFuncSetAttribute(tc::k_gemm_slices<tc::CgsEpi>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SL_SMEM),
+                     "cudaFuncSetAttribute(k_gemm_slices)");
     if (s == RBRP_OK)
       s = cuda_check(h, cudaFuncSetAttribute(tc::k_gemm_slices<tc::ProjEpi>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SL_SMEM),
@@ -179,7 +187,16 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       k_reduce_parts<double><<<64, 64, 0, st>>>(h->Gpart, dtiles, MAXB * MAXB, MAXB * MAXB, h->G);
     }
     if constexpr (!RES) {
-      if (i > 0 && !fixed_order) {
+      // Q C as slice products where the FP64 pipe would take longer than their two launches:
+      // 2e7 products are 40 us of it, and the launches take 25 to 50
+      const bool cgs_sl = use_sl && (double)m * i * p.b >= 2e7;
+      if (cgs_sl) {
+        tc::k_slice_coef<<<p.b > tc::SL_HALF ? MAXB : tc::SL_HALF, 256, 0, st>>>(h->R, n, h->js, h->st, h->sl_exH, ldc,
+                                                                                 h->slC, h->sl_exC);
+        tc::k_gemm_slices<<<std::min(h->sms, (m + tc::BM - 1) / tc::BM), tc::SL_THREADS, tc::SL_SMEM, st>>>(
+            tmSH, tmSC, (int64_t)kmax, h->wait_budget > 0 ? h->wait_budget : kWaitBudgetDefault,
+            tc::CgsEpi{h->st, m, dA, lda, h->cols, h->sl_exC, h->V, 0, 0});
+      } else if (i > 0 && !fixed_order) {
         k_gather_coef<<<(i + 3) / 4, 256, 0, st>>>(h->R, n, h->js, h->st, C);
       } else if (i > 0) {
         const int tiles = (i + 31) / 32;
@@ -193,7 +210,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
         k_reduce_parts<double><<<(int)std::min<int64_t>(1024, (cnt + 255) / 256), 256, 0, st>>>(Cpart, splits, cnt,
                                                                                                 cnt, C);
       }
-      by_rows([&](auto tr) {
+      if (!cgs_sl) by_rows([&](auto tr) {
         k_cgs_panel<decltype(tr)::value><<<ptiles, 256, 0, st>>>(dA, lda, h->cols, Q, m, C, h->st, m, h->V);
       });
       if (!panel_one && !fixed_order) {
@@ -254,8 +271,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       k_swap_cols<<<dim3((m + 1023) / 1024, MAXB), 256, 0, st>>>(h->Ares, L.ld_res, h->st, m, h->K1, h->K2);
     if constexpr (!RES) {
       if (use_sl) {
-        tc::k_slice_q<<<p.b > tc::SL_HALF ? MAXB : tc::SL_HALF, 256, 0, st>>>(Q, m, m, h->st, ldk, h->slQ,
-                                                                              h->sl_exQ);
+        tc::k_slice_q<<<2 * MAXB, 256, 0, st>>>(Q, m, m, h->st, ldk, h->slQ, h->sl_exQ, h->slH, kmax, h->sl_exH);
         tc::k_swap_slices<<<dim3(p.b, tc::SL), 256, 0, st>>>(h->slA, n, ldk, h->sl_exA, h->st, h->K1, h->K2);
       }
     }

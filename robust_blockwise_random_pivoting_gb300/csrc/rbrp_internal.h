@@ -80,6 +80,10 @@ struct rbrp_handle_st {
   size_t sl_bytes = 0;
   unsigned short* slA = nullptr;
   unsigned short* slQ = nullptr;
+  unsigned short* slH = nullptr;   // slices of the basis so far, and of the sampled columns' coefficients
+  unsigned short* slC = nullptr;
+  int* sl_exH = nullptr;
+  int* sl_exC = nullptr;
   int* sl_exA = nullptr;
   int* sl_exQ = nullptr;
   double* sl_Wpart = nullptr;
@@ -204,7 +208,7 @@ rbrp_status make_tmap_bf16(rbrp_handle h, void* map, const unsigned short* base,
 
 // Slice workspace of the FP64 form for an m x n matrix; false (and none held) where it would
 // take more than half of the free memory, which the CUDA-core projection then keeps.
-bool ensure_slices(rbrp_handle h, int m, int n);
+bool ensure_slices(rbrp_handle h, int m, int n, int kmax);
 bool ensure_fixed(rbrp_handle h, int m, int n);   // the same for the fixed-point copy of A
 void release_slices(rbrp_handle h);
 

@@ -105,13 +105,19 @@ k_slice_cols(const double* __restrict__ A, int64_t lda, int m, int n, int64_t sr
 
 // Slices of the block's basis columns Q(:, i .. i + kept) as the N operand: rows
 // (half, slice, column within the half), zero beyond the kept columns (up to 32, or 64
-// where more than 32 are kept).  One CTA per column.
+// where more than 32 are kept).  One CTA per column.  Also into row i + a of the basis
+// history (hist_rows per slice; its rows up to the next multiple of 64 are zeroed: the
+// Gram-Schmidt products read whole stages).
 __global__ void __launch_bounds__(256)
 k_slice_q(const double* __restrict__ Q, int64_t ldq, int m, const State* __restrict__ st, int64_t ldk,
-          unsigned short* __restrict__ out, int* __restrict__ exps) {
+          unsigned short* __restrict__ out, int* __restrict__ exps, unsigned short* __restrict__ hist, int hist_rows,
+          int* __restrict__ hist_exps) {
   __shared__ unsigned s_mx[8];
   const int tid = threadIdx.x, a = blockIdx.x, i = st->i, kept = st->bs;
-  if (kept == 0 || a >= (kept > SL_HALF ? 2 * SL_HALF : SL_HALF)) return;
+  const bool oper = a < (kept > SL_HALF ? 2 * SL_HALF : SL_HALF);
+  const bool keep = i + a < hist_rows && i + a < (i + kept + 63) / 64 * 64;
+  if (kept == 0 || (!oper && !keep)) return;
+  unsigned short* hdst = hist + (int64_t)(i + a) * ldk;
   unsigned short* dst = out + ((int64_t)(a / SL_HALF) * SL * SL_HALF + a % SL_HALF) * ldk;
   const double* col = Q + (int64_t)(i + (a < kept ? a : 0)) * ldq;
   unsigned mx = 0u;
@@ -122,14 +128,47 @@ k_slice_q(const double* __restrict__ Q, int64_t ldq, int m, const State* __restr
   __syncthreads();
   for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w]);
   const int e = slice_exponent(mx);
-  if (tid == 0) exps[a] = e;
+  if (tid == 0 && oper) exps[a] = e;
+  if (tid == 0 && keep) hist_exps[i + a] = e;
   for (int r0 = 2 * tid; r0 < ldk; r0 += 512) {
     unsigned short d0[SL], d1[SL];
     slice_digits(a < kept && r0 < m ? col[r0] : 0.0, e, d0);
     slice_digits(a < kept && r0 + 1 < m ? col[r0 + 1] : 0.0, e, d1);
 #pragma unroll
-    for (int s = 0; s < SL; ++s)
-      *reinterpret_cast<unsigned*>(dst + (int64_t)s * SL_HALF * ldk + r0) = d0[s] | ((unsigned)d1[s] << 16);
+    for (int s = 0; s < SL; ++s) {
+      const unsigned v = d0[s] | ((unsigned)d1[s] << 16);
+      if (oper) *reinterpret_cast<unsigned*>(dst + (int64_t)s * SL_HALF * ldk + r0) = v;
+      if (keep) *reinterpret_cast<unsigned*>(hdst + (int64_t)s * hist_rows * ldk + r0) = v;
+    }
+  }
+}
+
+// Slices of the sampled columns' coefficients R(0:i, js[c]) as the N operand of Q C, K = the
+// basis index, each scaled by its basis column's exponent (2^ex of the history's rows).  One CTA
+// per column, zero beyond the sampled ones.
+__global__ void __launch_bounds__(256)
+k_slice_coef(const double* __restrict__ R, int64_t ldr, const int* __restrict__ js, const State* __restrict__ st,
+             const int* __restrict__ hist_exps, int64_t ldk, unsigned short* __restrict__ out, int* __restrict__ exps) {
+  __shared__ int s_mx[8];
+  const int tid = threadIdx.x, c = blockIdx.x, i = st->i;
+  const bool in = c < st->bs_sampled;
+  unsigned short* dst = out + ((int64_t)(c / SL_HALF) * SL * SL_HALF + c % SL_HALF) * ldk;
+  const double* col = R + (in ? js[c] : 0);
+  int mx = -4096;
+  for (int a = tid; a < i && in; a += 256)
+    mx = max(mx, slice_exponent((unsigned)__double2hiint(col[(int64_t)a * ldr]) & 0x7FFFFFFFu) + hist_exps[a]);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((tid & 31) == 0) s_mx[tid >> 5] = mx;
+  __syncthreads();
+  for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w]);
+  if (tid == 0) exps[c] = mx;
+  const int kend = (i + SL_BK - 1) / SL_BK * SL_BK;
+  for (int a = tid; a < kend; a += 256) {
+    unsigned short d[SL];
+    const bool ok = in && a < i;
+    slice_digits(ok ? col[(int64_t)a * ldr] : 0.0, ok ? mx - hist_exps[a] : 0, d);
+#pragma unroll
+    for (int s = 0; s < SL; ++s) dst[(int64_t)s * SL_HALF * ldk + a] = d[s];
   }
 }
 
@@ -147,10 +186,24 @@ k_swap_slices(unsigned short* __restrict__ out, int64_t srows, int64_t ldk, int*
   if (blockIdx.y == 0 && threadIdx.x == 0) exps[b] = exps[a];
 }
 
+// A tile stored [k][128-byte row of 64 values of M] (two such blocks, 64 k rows each): the
+// descriptor of an M-major operand, 128-byte swizzle.  Leading offset: the next 64 values of
+// M; stride offset: the next 8 values of k.
+__device__ __forceinline__ uint64_t sw128_desc_m(uint32_t saddr) {
+  uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((SL_BK * 128) >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
+template <bool A_M_MAJOR>
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, int n, uint32_t accumulate) {
-  // D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1), K-major, N >> 3, M >> 4
-  const uint32_t idesc =
-      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+  // D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1), A K-major or M-major (bit 15),
+  // B K-major, N >> 3, M >> 4
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (A_M_MAJOR ? 1u << 15 : 0u) |
+                         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
@@ -233,6 +286,9 @@ static_assert(SL_SMEM <= 232448, "227 KB of shared memory per CTA");
 // 1.75 KB of slices per value of k from HBM.  8192 x 8192, 64 columns: 0.23 ms a block
 // against 8.8 ms on the FP64 pipe; 1000 x 1000, 40 columns: 0.034 against 0.61 ms.
 //
+// The M operand is K-major (slices of rows along k), or M-major (Epi::A_M_MAJOR: slices of
+// columns along M, k the slice's row).
+//
 // epi.init(): halves of every tile, 0 for nothing to do; epi.tile(t, ...): the t-th tile,
 // false past the last; epi.part(t, p, a0, hi, lo): the thread's 32 columns a0 .. a0 + 31 of
 // row p, with D = 2^(ex + ey - 60) (hi 2^24 + lo).
@@ -295,7 +351,12 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           if (g >= 1 && !mbar_wait(&sm.aempty[i], (uint32_t)(g & 1) ^ 1, abort, budget)) { ok = false; break; }
           if (elect_one()) {
             mbar_expect_tx(&sm.afull[i], SL_A_BYTES);
-            tma_load_2d(sm.as[i], &tmA, &sm.afull[i], ax + x, (int)(i * a_rows) + p0);
+            if constexpr (Epi::A_M_MAJOR) {
+              tma_load_2d(sm.as[i], &tmA, &sm.afull[i], p0, (int)(i * a_rows) + x);
+              tma_load_2d(sm.as[i] + SL_A_BYTES / 2, &tmA, &sm.afull[i], p0 + 64, (int)(i * a_rows) + x);
+            } else {
+              tma_load_2d(sm.as[i], &tmA, &sm.afull[i], ax + x, (int)(i * a_rows) + p0);
+            }
           }
           __syncwarp();
           aissued = g * SL + i + 1;
@@ -331,7 +392,8 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               break;
             }
             tc_fence_after();
-            const uint64_t da = sw128_desc(smem_u32(sm.as[i]));
+            const uint64_t da = Epi::A_M_MAJOR ? sw128_desc_m(smem_u32(sm.as[i])) : sw128_desc(smem_u32(sm.as[i]));
+            constexpr int AK = Epi::A_M_MAJOR ? 16 * 128 / 16 : 2;   // 16 values of k further on, in 16 bytes
             const uint32_t d = dset + (uint32_t)(i * SL_HALF);
             const int nsl = i == 0 ? SL : SL_CLASSES - i;   // N slices 0 .. nsl - 1: classes i .. i + nsl - 1
             if (elect_one()) {
@@ -339,11 +401,12 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               for (int k = 0; k < SL_BK / 16; ++k) {        // K = 16 BF16: 32 bytes
                 if (first && k == 0 && i == 1) {
                   // classes 1 .. 6 were started by slice 0; class 7 starts here
-                  mma_bf16(d, da, db, (SL - 1) * SL_HALF, 1u);
-                  mma_bf16(d + (uint32_t)((SL - 1) * SL_HALF), da,
+                  mma_bf16<Epi::A_M_MAJOR>(d, da, db, (SL - 1) * SL_HALF, 1u);
+                  mma_bf16<Epi::A_M_MAJOR>(d + (uint32_t)((SL - 1) * SL_HALF), da,
                            db + (uint64_t)(((SL - 1) * SL_HALF * SL_BK * 2) >> 4), SL_HALF, 0u);
                 } else {
-                  mma_bf16(d, da + 2 * k, db + 2 * k, nsl * SL_HALF, (first && k == 0 && i == 0) ? 0u : 1u);
+                  mma_bf16<Epi::A_M_MAJOR>(d, da + AK * k, db + 2 * k, nsl * SL_HALF,
+                                           (first && k == 0 && i == 0) ? 0u : 1u);
                 }
               }
               if (q == nh - 1) mma_commit(&sm.aempty[i]);
@@ -426,6 +489,7 @@ k_gemm_slices(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
 // gridDim.y; FP64 partials per row range, summed by k_proj_finish.
 // ---------------------------------------------------------------------------
 struct ProjEpi {
+  static constexpr bool A_M_MAJOR = false;
   State* st;
   int n, nstages, sps;
   const int* exA;
@@ -453,6 +517,43 @@ struct ProjEpi {
 #pragma unroll
     for (int j = 0; j < SL_HALF; ++j)
       if (a0 + j < kept) w[(int64_t)j * n] = slice_value(hi[j], lo[j], e + exQ[a0 + j]);
+  }
+  __device__ void timeout() const { atomicExch(&st->status, ST_ERR_TIMEOUT); }
+};
+
+// ---------------------------------------------------------------------------
+// a3 of the FP64 form: V(r, c) = A(r, cols[c]) - (Q C)(r, c), M = rows (the basis history's
+// columns, M-major), N = the sampled columns, K = the i basis vectors.  8192 rows, 64 columns,
+// 288 basis vectors on average: 288 us on the FP64 pipe, 40 here.
+// ---------------------------------------------------------------------------
+struct CgsEpi {
+  static constexpr bool A_M_MAJOR = true;
+  State* st;
+  int m;
+  const double* A;
+  int64_t lda;
+  const int* cols;
+  const int* exC;
+  double* V;
+  int nst, bss;   // set by init
+  __device__ int init() {
+    bss = st->bs_sampled;
+    nst = (st->i + SL_BK - 1) / SL_BK;
+    return bss == 0 || nst == 0 ? 0 : bss > SL_HALF ? 2 : 1;
+  }
+  __device__ bool tile(int t, int& p0, int& brow, int& s0, int& n, int& ax) const {
+    p0 = t * BM;
+    brow = s0 = ax = 0;
+    n = nst;
+    return p0 < m;
+  }
+  __device__ void part(int, int r, int c0, const long long (&hi)[SL_HALF], const long long (&lo)[SL_HALF]) const {
+    if (r >= m) return;
+#pragma unroll
+    for (int j = 0; j < SL_HALF; ++j) {
+      const int c = c0 + j;
+      if (c < bss) V[r + (int64_t)c * m] = A[r + (int64_t)cols[c] * lda] - slice_value(hi[j], lo[j], exC[c] - 60);
+    }
   }
   __device__ void timeout() const { atomicExch(&st->status, ST_ERR_TIMEOUT); }
 };

@@ -251,6 +251,7 @@ k_ts_slice_x(const double* __restrict__ T, int64_t ldt, int j0, int len, int nco
 // M = rows row0 .. row0 + rows of the sliced matrix (its K starts at column ax), N = columns
 // of T; stores the product in T, or subtracts it (sub).
 struct TsEpi {
+  static constexpr bool A_M_MAJOR = false;
   State* st;
   double* T;
   int64_t ldt;

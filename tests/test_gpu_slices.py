@@ -57,7 +57,10 @@ def test_projection_matches_the_fp64_pipe(kind, m, n, b):
     assert np.all(np.abs(L0 - L1)[rest] <= bound[rest])
 
 
-@pytest.mark.parametrize("m,n,b,kmax", [(300, 900, 20, 150), (700, 650, 64, 300)])
+# (the last three take the Gram-Schmidt products as slices: m i b >= 2e7, one and two column halves,
+# ragged row tiles and blocks of the basis)
+@pytest.mark.parametrize("m,n,b,kmax", [(300, 900, 20, 150), (700, 650, 64, 300), (5000, 400, 40, 250),
+                                        (9000, 500, 30, 330), (6401, 700, 64, 600)])
 def test_blocks_after_the_first_follow_the_same_skeleton(m, n, b, kmax):
     from robust_blockwise_random_pivoting_gb300.rbrp import Handle
     A = colmajor(matrix("normal", m, n))
