@@ -164,19 +164,19 @@ __device__ int pchol_filter_df(PcholDfSmemT<BB>& sm, int nb, int rows, double to
 }
 
 // The same factorization and filter as pchol_filter_df<64>, by 1024 threads
-// (LEAN_THREADS).  A step: warp 0 finds the pivot among the diagonal entries
-// (reductions of the bit patterns, first slot on ties), takes its square root and
-// reciprocal and scales its row; warp 1 sums the remaining trace for the filter;
-// a barrier; warp w updates the active slots t + 1 + w and t + 33 + w, lanes over
-// the columns as they are stored (active ones; by slot, the permuted columns cost
-// four times the shared-memory wavefronts and 1,600 of a step's 3,300 clocks); a
-// barrier.  Each Schur entry gets the same double-float
+// (LEAN_THREADS).  A step: warp 0 scales the pivot's row, warp 1 applies the filter; a
+// barrier; warps 2 .. 31 update the active slots, lanes over the columns as they are
+// stored (active ones; by slot, the permuted columns cost several shared-memory
+// wavefronts), while warps 0 and 1, which carry the diagonal in registers, find the next
+// pivot with its square root and reciprocal (reductions of the bit patterns, first slot on
+// ties) and the remaining trace; a barrier.  Each Schur entry gets the same double-float
 // operation on the same inputs as in the 256-thread form, both triangles (the
 // low parts of an entry and its mirror differ with the order of the factors).
 // Square root and reciprocal start from the correctly rounded FP32 intrinsics.
 // Latency bound on one SM: 64 steps of two barriers and the pivot's chain.  With
 // every thread scaling its own rows, a pivot search by shuffles and no
-// compaction a step took 4,000 clocks (64 columns: 128 us with the inverse, now about 60).
+// compaction a step took 4,000 clocks, with the pivot found at its start 3,300, now 2,800
+// (an adjoint call's 64 panels at 8192 rows: 11.0 -> 9.9 ms).
 constexpr int LEAN_THREADS = 1024;
 
 __device__ __forceinline__ dfl df_sqrt_lean(dfl a) {
@@ -194,77 +194,100 @@ __device__ __forceinline__ dfl df_recip_lean(dfl b) {
 __device__ int pchol_filter_df_lean(PcholDfSmemT<64>& sm, int nb, int rows, double tol_loc) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   bool a0 = lane < nb, a1 = lane + 32 < nb;   // the lane's columns still active
+  // warps 0 and 1: the lane's diagonal entries, kept up beside the update of the matrix, so
+  // that the next pivot and the remaining trace are found while the other warps update
+  dfl d0 = {0.f, 0.f}, d1 = {0.f, 0.f};
+  int s0 = lane, s1 = lane + 32;              // warp 0: the slots of the lane's columns
+  int pv = 0, bs = 0;                         // warp 0: the next pivot column and its slot
+  bool none = false;
+  dfl r = {0.f, 0.f}, inv = {0.f, 0.f}, rem = {0.f, 0.f}, thr = {0.f, 0.f};
   bool have_total = false;
-  dfl thr = {0.f, 0.f};
   auto trace = [&]() {   // remaining trace, valid in lane 0
-    dfl rem = {0.f, 0.f};
-    if (a0) rem = df_add(rem, sm.S[lane][lane]);
-    if (a1) rem = df_add(rem, sm.S[lane + 32][lane + 32]);
+    dfl t = {0.f, 0.f};
+    if (a0) t = df_add(t, d0);
+    if (a1) t = df_add(t, d1);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
-      rem = df_add(rem, {__shfl_down_sync(0xffffffffu, rem.hi, o), __shfl_down_sync(0xffffffffu, rem.lo, o)});
-    return rem;
+      t = df_add(t, {__shfl_down_sync(0xffffffffu, t.hi, o), __shfl_down_sync(0xffffffffu, t.lo, o)});
+    return t;
+  };
+  auto find = [&]() {    // largest active diagonal entry, lowest slot on ties
+    dfl best = {-1.f, 0.f};
+    int slot = 64, col = 0;
+    if (a0) { best = d0; slot = s0; col = lane; }
+    if (a1 && (slot == 64 || df_gt(d1, best) || (df_eq(d1, best) && s1 < slot))) { best = d1; slot = s1; col = lane + 32; }
+    const unsigned hi = best.hi > 0.f ? __float_as_uint(best.hi) : 0u;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lb = __float_as_uint(best.lo + 0.f);   // -0 as +0
+    const unsigned lo = hi == mh ? ((lb & 0x80000000u) ? ~lb : (lb | 0x80000000u)) : 0u;
+    const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+    const bool mine = hi == mh && lo == ml;
+    const unsigned key = __reduce_min_sync(0xffffffffu, mine ? ((unsigned)slot << 6) | (unsigned)col : 0xffffffffu);
+    none = mh == 0u;
+    bs = (int)(key >> 6);
+    pv = (int)(key & 63u);
+    // every matching lane holds the same value
+    const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+    const dfl v = {__shfl_sync(0xffffffffu, best.hi, src), __shfl_sync(0xffffffffu, best.lo, src)};
+    r = df_sqrt_lean(v);
+    inv = df_recip_lean(r);
   };
   if (tid == 0) sm.stop = 0;
   __syncthreads();
-  if (w == 1) {
-    const double total = __shfl_sync(0xffffffffu, df_dbl(trace()), 0);
-    have_total = total > 0.0;
-    thr = df_of(tol_loc * total);
+  if (w < 2) {
+    if (a0) d0 = sm.S[lane][lane];
+    if (a1) d1 = sm.S[lane + 32][lane + 32];
+    if (w == 0) find();
+    if (w == 1) {
+      rem = trace();
+      const double total = __shfl_sync(0xffffffffu, df_dbl(rem), 0);
+      have_total = total > 0.0;
+      thr = df_of(tol_loc * total);
+    }
   }
   for (int t = 0; t < rows; ++t) {
     if (w == 0) {
-      const int c0 = sm.ord[lane], c1 = sm.ord[lane + 32];
-      dfl best = {-1.f, 0.f};
-      int slot = 64;
-      if (lane >= t && lane < nb) { best = sm.S[c0][c0]; slot = lane; }
-      if (lane + 32 >= t && lane + 32 < nb) {
-        const dfl d = sm.S[c1][c1];
-        if (slot == 64 || df_gt(d, best)) { best = d; slot = lane + 32; }
+      if (none) {
+        if (lane == 0) sm.stop = 1;
+      } else {
+        if (lane == 0) {
+          // LAPACK order: the pivot column moves to slot t, slot t's column to the pivot's slot
+          const int o = sm.ord[t];
+          sm.ord[t] = pv;
+          sm.ord[bs] = o;
+          sm.piv = pv;
+        }
+        if (a0) sm.R[t][lane] = pv == lane ? r : df_mul(sm.S[pv][lane], inv);
+        if (a1) sm.R[t][lane + 32] = pv == lane + 32 ? r : df_mul(sm.S[pv][lane + 32], inv);
       }
-      const unsigned hi = best.hi > 0.f ? __float_as_uint(best.hi) : 0u;
-      const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-      const unsigned lb = __float_as_uint(best.lo + 0.f);   // -0 as +0
-      const unsigned lo = hi == mh ? ((lb & 0x80000000u) ? ~lb : (lb | 0x80000000u)) : 0u;
-      const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
-      const unsigned sl = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (unsigned)slot : 64u);
-      const int bs = mh ? (int)sl : t;
-      const int o = sm.ord[t], pv = sm.ord[bs];
-      __syncwarp();
-      if (lane == 0) {
-        if (!mh) sm.stop = 1;
-        // LAPACK order: the pivot column moves to slot t, slot t's column to the pivot's slot
-        sm.ord[t] = pv;
-        sm.ord[bs] = o;
-      }
-      __syncwarp();
-      const dfl r = df_sqrt_lean(sm.S[pv][pv]);
-      const dfl inv = df_recip_lean(r);
-      if (a0) sm.R[t][lane] = pv == lane ? r : df_mul(sm.S[pv][lane], inv);
-      if (a1) sm.R[t][lane + 32] = pv == lane + 32 ? r : df_mul(sm.S[pv][lane + 32], inv);
-      if (lane == 0) sm.piv = pv;
     } else if (w == 1) {
-      const dfl rem = trace();
       if (lane == 0 && (!have_total || df_gt(thr, rem))) sm.stop = 1;
     }
     __syncthreads();
     if (sm.stop) return t;
     a0 = a0 && sm.piv != lane;
     a1 = a1 && sm.piv != lane + 32;
-    if (t + 1 + w < nb) {
-      const bool two = t + 33 + w < nb;
-      const int r0 = sm.ord[t + 1 + w], r1 = sm.ord[two ? t + 33 + w : t + 1 + w];
-      const dfl f0 = sm.R[t][r0], f1 = sm.R[t][r1];
-      const dfl g0 = a0 ? sm.R[t][lane] : dfl{0.f, 0.f}, g1 = a1 ? sm.R[t][lane + 32] : dfl{0.f, 0.f};
-      dfl x00 = {0.f, 0.f}, x01 = x00, x10 = x00, x11 = x00;
-      if (a0) x00 = sm.S[r0][lane];
-      if (a1) x01 = sm.S[r0][lane + 32];
-      if (two && a0) x10 = sm.S[r1][lane];
-      if (two && a1) x11 = sm.S[r1][lane + 32];
-      if (a0) sm.S[r0][lane] = df_fms(x00, f0, g0);
-      if (a1) sm.S[r0][lane + 32] = df_fms(x01, f0, g1);
-      if (two && a0) sm.S[r1][lane] = df_fms(x10, f1, g0);
-      if (two && a1) sm.S[r1][lane + 32] = df_fms(x11, f1, g1);
+    const dfl g0 = a0 ? sm.R[t][lane] : dfl{0.f, 0.f}, g1 = a1 ? sm.R[t][lane + 32] : dfl{0.f, 0.f};
+    if (w < 2) {
+      if (a0) d0 = df_fms(d0, g0, g0);
+      if (a1) d1 = df_fms(d1, g1, g1);
+      if (w == 0) {
+        if (s0 == t) s0 = bs;   // slot t's column took the pivot's slot
+        if (s1 == t) s1 = bs;
+        find();
+      } else {
+        rem = trace();
+      }
+    } else {
+      for (int ss = t + w - 1; ss < nb; ss += LEAN_THREADS / 32 - 2) {
+        const int c = sm.ord[ss];
+        const dfl f = sm.R[t][c];
+        dfl x0 = {0.f, 0.f}, x1 = {0.f, 0.f};
+        if (a0) x0 = sm.S[c][lane];
+        if (a1) x1 = sm.S[c][lane + 32];
+        if (a0) sm.S[c][lane] = df_fms(x0, f, g0);
+        if (a1) sm.S[c][lane + 32] = df_fms(x1, f, g1);
+      }
     }
     __syncthreads();
   }
