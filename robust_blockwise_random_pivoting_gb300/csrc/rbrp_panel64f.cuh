@@ -79,6 +79,43 @@ struct LdlSmem {
   unsigned cmax[MAXB];        // k_chol2_fast: largest upper word of |R11(:, c)|
 };
 
+// Warp 0 of ldl64: the diagonal by stored column (lane, lane + 32) in registers, with the
+// columns' slots, and the next pivot: the largest active entry, lowest slot on ties (integer
+// reductions: the diagonal is positive where it matters).
+struct Pivot64 {
+  double d0, d1;
+  int s0, s1;
+  bool a0, a1;
+  double best;      // the pivot's diagonal entry
+  int pv, slot;     // its column and slot
+  bool none;
+  __device__ void find() {
+    const int lane = threadIdx.x & 31;
+    double v = 0.0;
+    int s = 64, c = 0;
+    if (a0) { v = d0; s = s0; c = lane; }
+    if (a1 && (s == 64 || d1 > v || (d1 == v && s1 < s))) { v = d1; s = s1; c = lane + 32; }
+    const bool pos = s < 64 && v > 0.0;
+    const unsigned hi = pos ? (unsigned)__double2hiint(v) : 0u, lo = pos ? (unsigned)__double2loint(v) : 0u;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    none = mh == 0u && ml == 0u;
+    const unsigned key =
+        __reduce_min_sync(0xffffffffu, pos && hi == mh && lo == ml ? ((unsigned)s << 6) | (unsigned)c : 0xffffffffu);
+    slot = (int)(key >> 6);
+    pv = (int)(key & 63u);
+    best = __hiloint2double((int)mh, (int)ml);
+  }
+  // the pivot of step t is gone: the column of slot t has its slot
+  __device__ void taken(int t) {
+    const int lane = threadIdx.x & 31;
+    a0 = a0 && pv != lane;
+    a1 = a1 && pv != lane + 32;
+    if (s0 == t) s0 = slot;
+    if (s1 == t) s1 = slot;
+  }
+};
+
 // L D L^T of the nb x nb matrix in sm.S with L^{-1} carried along, 1024 threads.  With
 // PIVOT the step takes the largest remaining diagonal entry (LAPACK dgeqp3's rule on the
 // panel, first slot on ties; swaps are virtual: ord maps slot -> column) and stops where
@@ -86,91 +123,101 @@ struct LdlSmem {
 // 69-73).  Returns the number of steps taken; R = D^{1/2} L^T and R^{-1} = L^{-T} D^{-1/2}
 // follow from U, M and d, so no square root sits in the chain of steps.
 //
-// A step: warp 0 finds the pivot (integer comparisons: the diagonal is positive where it
-// matters), takes its reciprocal and scales the row, warp 1 sums the trace; a barrier; each
-// warp updates the rows (slots) ww, ww + 32 that are still active, lanes over the row's
-// entries of L^{-1} and of the Schur complement together; a barrier.
+// A step: warp 0 scales the pivot's row, warp 1 applies the filter; a barrier; warps 2 .. 31
+// update the active rows (slots), lanes over the row's entries of L^{-1} and of the Schur
+// complement together, while warps 0 and 1, which carry the diagonal in registers, find the
+// next pivot with its reciprocal and the remaining trace; a barrier.  k_pchol_ldl at 64
+// columns: 103 us with the pivot found at the start of the step, now 89.
 template <bool PIVOT>
 __device__ int ldl64(LdlSmem& sm, int nb, int rows, double tol_loc) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  double thr = 0.0;                   // warp 1: the filter's threshold, and its columns still active
-  bool a0 = lane < nb, a1 = lane + 32 < nb;
+  Pivot64 pz;
+  pz.a0 = lane < nb;
+  pz.a1 = lane + 32 < nb;
+  pz.d0 = pz.d1 = 0.0;
+  pz.s0 = lane;
+  pz.s1 = lane + 32;
+  pz.none = false;
+  pz.slot = 0;
+  double thr = 0.0, rem = 0.0, inv = 0.0;
   if (tid < MAXB) sm.ord[tid] = tid;
   if (tid == 0) sm.stop = 0;
   __syncthreads();
-  auto diag = [&](int slot) { return slot < nb ? sm.S[sm.ord[slot]][sm.ord[slot]] : 0.0; };
-  if (PIVOT && w == 1) {
-    double t = warp_sum((a0 ? sm.S[lane][lane] : 0.0) + (a1 ? sm.S[lane + 32][lane + 32] : 0.0));
-    t = __shfl_sync(0xffffffffu, t, 0);
-    thr = tol_loc * t;
-    if (!(t > 0.0)) thr = INFINITY;   // a zero or NaN panel keeps nothing
+  // the pivot of step t is known: its reciprocal
+  auto next = [&](int t) {
+    if (PIVOT) {
+      pz.find();
+    } else if (t < nb) {   // natural order
+      pz.pv = pz.slot = t;
+      pz.best = __shfl_sync(0xffffffffu, t < 32 ? pz.d0 : pz.d1, t & 31);
+    }
+    inv = 1.0 / pz.best;
+  };
+  if (w < 2) {
+    if (pz.a0) pz.d0 = sm.S[lane][lane];
+    if (pz.a1) pz.d1 = sm.S[lane + 32][lane + 32];
+    if (w == 0) next(0);
+    if (PIVOT && w == 1) {
+      rem = __shfl_sync(0xffffffffu, warp_sum(pz.d0 + pz.d1), 0);
+      thr = tol_loc * rem;
+      if (!(rem > 0.0)) thr = INFINITY;   // a zero or NaN panel keeps nothing
+    }
   }
   for (int t = 0; t < rows; ++t) {
     if (w == 0) {
-      int pv = t;
-      if (PIVOT) {
-        // (value, lowest slot) of the largest positive diagonal entry among the slots >= t
-        const double d0 = lane >= t ? diag(lane) : 0.0, d1 = lane + 32 >= t ? diag(lane + 32) : 0.0;
-        const double best = d1 > d0 ? d1 : d0;
-        const unsigned hi = best > 0.0 ? (unsigned)__double2hiint(best) : 0u;
-        const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)__double2loint(best) : 0u);
-        const double mx = __hiloint2double((int)mh, (int)ml);
-        const unsigned b0 = __ballot_sync(0xffffffffu, d0 == mx), b1 = __ballot_sync(0xffffffffu, d1 == mx);
-        const int slot = mh == 0u ? t : b0 ? __ffs(b0) - 1 : 31 + __ffs(b1);
-        if (mh == 0u && lane == 0) sm.stop = 1;
-        __syncwarp();
+      const int pv = pz.pv;
+      if (PIVOT && pz.none) {
+        if (lane == 0) sm.stop = 1;
+      } else {
         if (lane == 0) {
           const int o = sm.ord[t];
-          sm.ord[t] = sm.ord[slot];
-          sm.ord[slot] = o;
+          sm.ord[t] = pv;
+          sm.ord[pz.slot] = o;
+          sm.piv = pv;
+          sm.d[t] = pz.best;
         }
-        __syncwarp();
-        pv = sm.ord[t];
-      }
-      const double d = sm.S[pv][pv];
-      const double inv = 1.0 / d;
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int s = lane + 32 * u;
-        if (s > t && s < nb) {
-          const int c = sm.ord[s];
-          const double v = sm.S[min(pv, c)][max(pv, c)];
-          sm.U[t][c] = v;
-          sm.l[c] = v * inv;
+        for (int u = 0; u < 2; ++u) {
+          const int c = lane + 32 * u;
+          if ((u ? pz.a1 : pz.a0) && c != pv) {
+            const double v = sm.S[min(pv, c)][max(pv, c)];
+            sm.U[t][c] = v;
+            sm.l[c] = v * inv;
+          }
         }
-      }
-      if (lane == 0) {
-        sm.piv = pv;
-        sm.d[t] = d;
       }
     } else if (PIVOT && w == 1) {
-      // by column, not by slot: warp 0 is moving the slots
-      const double rem = warp_sum((a0 ? sm.S[lane][lane] : 0.0) + (a1 ? sm.S[lane + 32][lane + 32] : 0.0));
       if (lane == 0 && !(rem >= thr)) sm.stop = 1;
     }
     __syncthreads();
     if (sm.stop) return t;
     const int pv = sm.piv;
-    a0 = a0 && pv != lane;
-    a1 = a1 && pv != lane + 32;
-    for (int ss = t + 1 + w; ss < nb; ss += 32) {
-      const int c = sm.ord[ss];
-      const double lc = sm.l[c];
-      const int len = t + nb - ss;               // t entries of L^{-1}, then the slots ss .. nb - 1
-      for (int e = lane; e < len; e += 32) {
-        double *p, q;
-        if (e < t) {
-          p = &sm.M[c][e];
-          q = sm.M[pv][e];
-        } else {
-          const int c2 = sm.ord[ss + e - t];
-          p = &sm.S[min(c, c2)][max(c, c2)];
-          q = sm.U[t][c2];
+    if (w < 2) {
+      if (w == 1) pz.pv = pv;
+      pz.taken(t);
+      if (pz.a0) pz.d0 = fma(-sm.l[lane], sm.U[t][lane], pz.d0);
+      if (pz.a1) pz.d1 = fma(-sm.l[lane + 32], sm.U[t][lane + 32], pz.d1);
+      if (w == 0) next(t + 1);
+      else if (PIVOT) rem = warp_sum((pz.a0 ? pz.d0 : 0.0) + (pz.a1 ? pz.d1 : 0.0));
+    } else {
+      for (int ss = t + w - 1; ss < nb; ss += 30) {
+        const int c = sm.ord[ss];
+        const double lc = sm.l[c];
+        const int len = t + nb - ss;               // t entries of L^{-1}, then the slots ss .. nb - 1
+        for (int e = lane; e < len; e += 32) {
+          double *p, q;
+          if (e < t) {
+            p = &sm.M[c][e];
+            q = sm.M[pv][e];
+          } else {
+            const int c2 = sm.ord[ss + e - t];
+            p = &sm.S[min(c, c2)][max(c, c2)];
+            q = sm.U[t][c2];
+          }
+          *p = fma(-lc, q, *p);
         }
-        *p = fma(-lc, q, *p);
+        if (lane == 0) sm.M[c][t] = -lc;
       }
-      if (lane == 0) sm.M[c][t] = -lc;
     }
     __syncthreads();
   }
