@@ -16,7 +16,7 @@
 // tensor cores (tcgen05, 3xTF32, rbrp_gemm_tc.cuh) with the loss terms, E w and
 // the rank-one terms fused into their epilogues (the handle's variant 1 keeps
 // them as 128 x 128-tiled FP32 FFMA GEMMs); z is a double-float triangular
-// solve.
+// solve by one cluster of CTAs.
 //
 // Tensor-core operand layouts (K-major, leading dimensions rounded up to 4
 // floats for TMA):
@@ -25,6 +25,8 @@
 //                 written as E^T (nc x m, ld ncp): the drain lanes run along c
 //   E T^T:        M = rows r, N = skeleton index t, K = rd columns c
 //                 X = E^T, Y = T^T (nc x k, ld ncp, TF32 hi / lo)
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 
@@ -32,6 +34,8 @@
 #include "rbrp_df.cuh"
 #include "rbrp_gemm.cuh"
 #include "rbrp_gemm_tc.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace rbrp {
 namespace {
@@ -111,123 +115,140 @@ __global__ void k_adj_sum_rows(const float2* __restrict__ part, int nparts, int 
   out[i] = df_two_sum(s.hi, s.lo).hi;
 }
 
-// R11 (FP64, row major, ld ldr, upper) as double-float pairs, row major ld k.
+// R11 (FP64, row major, ld ldr, upper) as double-float pairs, row major ld k, with R11^T
+// in the lower triangle: both directions of the solve then read rows.
 __global__ void k_adj_split_r(const double* __restrict__ R, int64_t ldr, int k, float2* __restrict__ Rdf) {
-  const int64_t total = (int64_t)k * k;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int a = (int)(idx / k), c = (int)(idx % k);
-    const double x = c >= a ? R[(int64_t)a * ldr + c] : 0.0;
-    const float hi = (float)x;
-    Rdf[idx] = make_float2(hi, (float)(x - (double)hi));
-  }
-}
-
-// z = R11^{-1} R11^{-T} u in double-float, by 32-row blocks, one launch per block
-// and direction.  In every CTA warp 0 solves the block's 32 x 32 triangle from the
-// right-hand side rhs (lane-parallel: the lane of row i finishes x_i, every later
-// lane subtracts its term), CTA 0 stores it in sol, and all CTAs subtract the
-// block's contribution from their share of the remaining rows of rhs.  No CTA
-// writes what another reads in the same launch: the block's rhs rows are only
-// read, its solution goes to sol.
-__device__ __forceinline__ dfl r_df(const float2* __restrict__ R, int k, int a, int c) {
-  const float2 v = R[(int64_t)a * k + c];
-  return dfl{v.x, v.y};
-}
-
-// forward step: R11^T y = u for rows [j0, j0 + 32): y(j0..) into sol, rhs(j) for j >= j0 + 32
-__global__ void __launch_bounds__(256) k_adj_zf_step(const float2* __restrict__ R, int k, int j0,
-                                                     float2* __restrict__ rhs, float2* __restrict__ sol) {
-  __shared__ dfl xb[32];
-  __shared__ dfl Rb[32][33];  // the block's diagonal 32 x 32 of R, staged once
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int jl = min(32, k - j0);
-  for (int e = tid; e < 32 * 32; e += blockDim.x) {
-    const int a = e >> 5, c = e & 31;
-    Rb[a][c] = (a < jl && c < jl) ? r_df(R, k, j0 + a, j0 + c) : dfl{1.f, 0.f};
+  __shared__ float2 tile[32][33];
+  const int c0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
+  if (a0 > c0) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int q = ty; q < 32; q += 8) {
+    const int a = a0 + q, c = c0 + tx;
+    if (a < k && c < k && c >= a) {
+      const double x = R[(int64_t)a * ldr + c];
+      const float hi = (float)x;
+      const float2 v = make_float2(hi, (float)(x - (double)hi));
+      Rdf[(int64_t)a * k + c] = v;
+      tile[q][tx] = v;
+    }
   }
   __syncthreads();
-  if (tid < 32) {
-    dfl b = {0.f, 0.f};
-    if (lane < jl) {
-      const float2 v = rhs[j0 + lane];
-      b = {v.x, v.y};
-    }
-    dfl x = {0.f, 0.f};
-    for (int i = 0; i < jl; ++i) {
-      if (lane == i) x = df_mul(b, df_recip(Rb[i][i]));
-      const dfl xi = {__shfl_sync(0xffffffffu, x.hi, i), __shfl_sync(0xffffffffu, x.lo, i)};
-      if (lane > i && lane < jl) b = df_fms(b, Rb[i][lane], xi);
-    }
-    xb[lane] = x;
-  }
-  __syncthreads();
-  if (blockIdx.x == 0 && tid < jl) sol[j0 + tid] = make_float2(xb[tid].hi, xb[tid].lo);
-  for (int j = j0 + jl + blockIdx.x * blockDim.x + tid; j < k; j += gridDim.x * blockDim.x) {
-    const float2 w0 = rhs[j];
-    dfl v = {w0.x, w0.y};
-    for (int ii = 0; ii < jl; ++ii) v = df_fms(v, r_df(R, k, j0 + ii, j), xb[ii]);
-    rhs[j] = make_float2(v.hi, v.lo);
+  for (int q = ty; q < 32; q += 8) {
+    const int c = c0 + q, a = a0 + tx;
+    if (c < k && a < c) Rdf[(int64_t)c * k + a] = tile[tx][q];
   }
 }
 
-// backward step: R11 z = y for rows [i0, i0 + il): z(i0..) into sol, rhs(i) for i < i0
-__global__ void __launch_bounds__(256) k_adj_zb_step(const float2* __restrict__ R, int k, int i0, int il,
-                                                     float2* __restrict__ rhs, float2* __restrict__ sol) {
-  __shared__ dfl xb[32];
-  __shared__ dfl Rb[32][33];  // the block's diagonal il x il of R, staged once
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (int e = tid; e < 32 * 32; e += blockDim.x) {
-    const int a = e >> 5, c = e & 31;
-    Rb[a][c] = (a < il && c < il) ? r_df(R, k, i0 + a, i0 + c) : dfl{1.f, 0.f};
-  }
-  __syncthreads();
-  if (tid < 32) {
-    dfl b = {0.f, 0.f};
-    if (lane < il) {
-      const float2 v = rhs[i0 + lane];
-      b = {v.x, v.y};
+// z = R11^{-1} R11^{-T} u in double-float, one kernel per direction.  Rows are taken in the
+// order of the substitution (q = row, backward k - 1 - row) in blocks of 32; thread g of a
+// cluster of 8 CTAs has the rows q = g, g + 4096, ... in shared memory.  A step: the warp
+// whose lanes have the block's rows solves the 32 x 32 triangle (the lane of row q finishes
+// x_q, every later lane subtracts its term) and sends the solution to all 8 CTAs; one
+// cluster barrier; every thread subtracts the block's terms from its later rows.  The
+// triangle of the next block, its reciprocals and the entries that a thread's first later
+// row needs are loaded before the barrier.
+// Bound by the chain of k substitutions (about 3,500 clocks per 32).  A launch per block
+// and direction, every CTA solving the triangle for itself, took 17.6 and 14.3 us a block
+// (4.1 ms at k = 4096); each row's operations and their order are the same.
+constexpr int ZC = 8;              // CTAs of the cluster
+constexpr int ZT = 512;            // threads per CTA
+constexpr int ZG = ZC * ZT;
+
+template <bool BACK>
+__global__ void __cluster_dims__(ZC, 1, 1) __launch_bounds__(ZT)
+k_adj_zsolve(const float2* __restrict__ R, int k, const float2* __restrict__ rhs, float2* __restrict__ sol,
+             float* __restrict__ z) {
+  extern __shared__ float2 zr[];                // [row of the thread][thread]: right-hand side
+  __shared__ dfl xb[2][32];                     // the block's solution, by step parity
+  __shared__ dfl tri[2][32][33];                // coefficient of solved a in row c
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = (int)cl.block_rank() * ZT + tid;
+  const int nt = (k + 31) / 32;
+  auto row = [&](int q) { return BACK ? k - 1 - q : q; };
+  // what row q (later) takes of the solved p
+  auto coef = [&](int p, int q) { return __ldg(R + (int64_t)row(p) * k + row(q)); };
+  for (int r = 0; g + r * ZG < k; ++r) zr[r * ZT + tid] = rhs[row(g + r * ZG)];
+  dfl rinv = {0.f, 0.f};
+  auto mine = [&](int t) { return (32 * t) % ZG / 32 == g / 32; };   // the warp has block t
+  auto load_tri = [&](int t) {
+    const int q0 = 32 * t, q = q0 + lane;
+    for (int a = 0; a < 32; ++a) {
+      const float2 v = q < k && a <= lane ? coef(q0 + a, q) : make_float2(a == lane ? 1.f : 0.f, 0.f);
+      tri[t & 1][a][lane] = {v.x, v.y};
     }
-    dfl x = {0.f, 0.f};
-    for (int i = il - 1; i >= 0; --i) {
-      if (lane == i) x = df_mul(b, df_recip(Rb[i][i]));
-      const dfl xi = {__shfl_sync(0xffffffffu, x.hi, i), __shfl_sync(0xffffffffu, x.lo, i)};
-      if (lane < i) b = df_fms(b, Rb[lane][i], xi);
+    rinv = df_recip(tri[t & 1][lane][lane]);
+    __syncwarp();
+  };
+  if (mine(0)) load_tri(0);
+  cl.sync();                                    // every CTA runs before anything is sent to it
+  for (int t = 0; t < nt; ++t) {
+    const int q0 = 32 * t, jl = min(32, k - q0);
+    if (mine(t)) {
+      dfl b = {0.f, 0.f};
+      if (lane < jl) {
+        const float2 v = zr[q0 / ZG * ZT + tid];
+        b = {v.x, v.y};
+      }
+      dfl x = {0.f, 0.f};
+      for (int a = 0; a < jl; ++a) {
+        if (lane == a) x = df_mul(b, rinv);
+        const dfl xa = {__shfl_sync(0xffffffffu, x.hi, a), __shfl_sync(0xffffffffu, x.lo, a)};
+        if (lane > a && lane < jl) b = df_fms(b, tri[t & 1][a][lane], xa);
+      }
+#pragma unroll
+      for (int c = 0; c < ZC; ++c) cl.map_shared_rank(&xb[0][0], c)[32 * (t & 1) + lane] = x;
+      if (lane < jl) {
+        const int o = row(q0 + lane);
+        if (BACK) z[o] = x.hi;
+        else sol[o] = make_float2(x.hi, x.lo);
+      }
     }
-    xb[lane] = x;
+    if (t + 1 < nt && mine(t + 1)) load_tri(t + 1);
+    // the first of the thread's rows behind the block
+    int r = q0 / ZG;
+    if (g + r * ZG < q0 + 32) ++r;
+    const int q1 = g + r * ZG;
+    float2 cf[32];
+    if (q1 < k) {
+#pragma unroll
+      for (int a = 0; a < 32; ++a) cf[a] = coef(q0 + a, q1);   // a block before a later row is whole
+    }
+    cl.sync();
+    auto apply = [&](int at) {                  // in order of rising rows, both directions
+      const float2 w = zr[at];
+      dfl v = {w.x, w.y};
+#pragma unroll
+      for (int a = 0; a < 32; ++a) {
+        const int aa = BACK ? 31 - a : a;
+        v = df_fms(v, {cf[aa].x, cf[aa].y}, xb[t & 1][aa]);
+      }
+      zr[at] = make_float2(v.hi, v.lo);
+    };
+    if (q1 < k) apply(r * ZT + tid);
+    for (++r; g + r * ZG < k; ++r) {
+#pragma unroll
+      for (int a = 0; a < 32; ++a) cf[a] = coef(q0 + a, g + r * ZG);
+      apply(r * ZT + tid);
+    }
   }
-  __syncthreads();
-  if (blockIdx.x == 0 && tid < il) sol[i0 + tid] = make_float2(xb[tid].hi, xb[tid].lo);
-  for (int i = blockIdx.x * blockDim.x + tid; i < i0; i += gridDim.x * blockDim.x) {
-    const float2 w0 = rhs[i];
-    dfl v = {w0.x, w0.y};
-    for (int jj = 0; jj < il; ++jj) v = df_fms(v, r_df(R, k, i, i0 + jj), xb[jj]);
-    rhs[i] = make_float2(v.hi, v.lo);
-  }
+  cl.sync();                                    // no CTA leaves while another may still send to it
 }
 
-__global__ void k_adj_copy_df(const float2* __restrict__ in, float2* __restrict__ out, int k) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < k) out[i] = in[i];
-}
-
-__global__ void k_adj_z_out(const float2* __restrict__ zdf, float* __restrict__ z, int k) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < k) z[i] = zdf[i].x;
-}
-
-// z (FP32) = R11^{-1} R11^{-T} u; work and ys are k double-float scratch vectors each.
-void solve_z(cudaStream_t st, int sms, const float2* Rdf, int k, const float2* udf, float2* work, float2* ys,
-             float* z) {
-  const int grid = std::max(1, std::min((k + 255) / 256, 2 * sms));
-  k_adj_copy_df<<<(k + 255) / 256, 256, 0, st>>>(udf, work, k);
-  for (int j0 = 0; j0 < k; j0 += 32) k_adj_zf_step<<<grid, 256, 0, st>>>(Rdf, k, j0, work, ys);
-  // backward: the right-hand side is y (ys, updated in place), the solution goes to work
-  for (int i1 = k; i1 > 0; i1 -= 32) {
-    const int i0 = std::max(0, i1 - 32);
-    k_adj_zb_step<<<grid, 256, 0, st>>>(Rdf, k, i0, i1 - i0, ys, work);
-  }
-  k_adj_z_out<<<(k + 255) / 256, 256, 0, st>>>(work, z, k);
+// z (FP32) = R11^{-1} R11^{-T} u; ys holds k double-float scratch values.
+rbrp_status solve_z(rbrp_handle h, const float2* Rdf, int k, const float2* udf, float2* ys, float* z) {
+  const size_t smem = (size_t)((k + ZG - 1) / ZG) * ZT * sizeof(float2);
+  // one limit for every k (the attribute is the process's): k <= 196608, whose R11 alone is 309 GB
+  constexpr int lim = 192 * 1024;
+  rbrp_status s = cuda_check(h, cudaFuncSetAttribute(k_adj_zsolve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     lim), "cudaFuncSetAttribute(k_adj_zsolve)");
+  if (s == RBRP_OK)
+    s = cuda_check(h, cudaFuncSetAttribute(k_adj_zsolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim),
+                   "cudaFuncSetAttribute(k_adj_zsolve)");
+  if (s != RBRP_OK) return s;
+  k_adj_zsolve<false><<<ZC, ZT, smem, h->stream>>>(Rdf, k, udf, ys, nullptr);
+  k_adj_zsolve<true><<<ZC, ZT, smem, h->stream>>>(Rdf, k, ys, nullptr, z);
+  return cuda_check(h, cudaGetLastError(), "k_adj_zsolve");
 }
 
 // czpart[p][r] = sum over the part-p skeleton columns t of A[r, perm[t]] z[t]
@@ -528,7 +549,7 @@ namespace {
 // The tensor-core form of the loss and gradient (same outputs as the FFMA kernels).
 rbrp_status adjoint_tc(rbrp_handle h, int m, int k, int nc, int kp, int ncp, const float* dA, int64_t lda,
                        const float* dW, float scale, float* dG, int64_t ldg, double* loss, float* Trh, float* Trl,
-                       float* Tx, float* wr, float2* up, float* u, float2* udf, float* z, float2* Rdf, float2* wk,
+                       float* Tx, float* wr, float2* up, float* u, float2* udf, float* z, float2* Rdf,
                        float2* ys, float2* czp, float* cz, float* Et, float2* ewp, float* ew, float2* lp, double* lout,
                        float* Cth, float* Ctl, int* dstatus) {
   cudaStream_t st = h->stream;
@@ -557,8 +578,9 @@ rbrp_status adjoint_tc(rbrp_handle h, int m, int k, int nc, int kp, int ncp, con
   k_adj_u<<<dim3((k + 255) / 256, PARTS), 256, 0, st>>>(Tx, kp, k, nc, wr, up);
   k_adj_sum_parts<<<(k + 255) / 256, 256, 0, st>>>(up, k, u, udf);
   if (dG) {
-    k_adj_split_r<<<1216, 256, 0, st>>>(h->R, n, k, Rdf);
-    solve_z(st, h->sms, Rdf, k, udf, wk, ys, z);
+    k_adj_split_r<<<dim3((k + 31) / 32, (k + 31) / 32), 256, 0, st>>>(h->R, n, k, Rdf);
+    s = solve_z(h, Rdf, k, udf, ys, z);
+    if (s != RBRP_OK) return s;
     k_adj_cz<<<dim3((m + 255) / 256, PARTS), 256, 0, st>>>(dA, lda, m, k, h->perm, z, czp);
     k_adj_sum_parts<<<(m + 255) / 256, 256, 0, st>>>(czp, m, cz, nullptr);
   }
@@ -622,7 +644,7 @@ extern "C" rbrp_status rbrp_fixed_id_adjoint_f32(rbrp_handle h, int m, int n, co
   const size_t o_Tr = take(4 * (use_tc ? (size_t)ncp * k : kn)), o_Tc = take(4 * (use_tc ? (size_t)kp * nc : kn));
   const size_t o_wr = take(4 * (size_t)nc);
   const size_t o_up = take(8 * (size_t)PARTS * k), o_u = take(4 * (size_t)k), o_udf = take(8 * (size_t)k);
-  const size_t o_z = take(4 * (size_t)k), o_R = take(8 * (size_t)k * k), o_wk = take(8 * (size_t)k);
+  const size_t o_z = take(4 * (size_t)k), o_R = take(8 * (size_t)k * k);
   const size_t o_ys = take(8 * (size_t)k);
   const size_t o_czp = take(8 * (size_t)PARTS * m), o_cz = take(4 * (size_t)m);
   const size_t o_E = take(4 * (use_tc ? (size_t)ncp * m : (size_t)m * nc)), o_ewp = take(8 * (size_t)gy1 * m);
@@ -649,7 +671,6 @@ extern "C" rbrp_status rbrp_fixed_id_adjoint_f32(rbrp_handle h, int m, int n, co
   float2* udf = reinterpret_cast<float2*>(w + o_udf);
   float* z = reinterpret_cast<float*>(w + o_z);
   float2* Rdf = reinterpret_cast<float2*>(w + o_R);
-  float2* wk = reinterpret_cast<float2*>(w + o_wk);
   float2* ys = reinterpret_cast<float2*>(w + o_ys);
   float2* czp = reinterpret_cast<float2*>(w + o_czp);
   float* cz = reinterpret_cast<float*>(w + o_cz);
@@ -661,15 +682,16 @@ extern "C" rbrp_status rbrp_fixed_id_adjoint_f32(rbrp_handle h, int m, int n, co
   int* dstatus = reinterpret_cast<int*>(w + o_st);
 
   if (use_tc) return adjoint_tc(h, m, k, nc, kp, ncp, dA, lda, dW, scale, dG, ldg, loss, Tr /* T^T hi */,
-                                reinterpret_cast<float*>(w + o_Trl), Tc /* Tx */, wr, up, u, udf, z, Rdf, wk, ys, czp,
+                                reinterpret_cast<float*>(w + o_Trl), Tc /* Tx */, wr, up, u, udf, z, Rdf, ys, czp,
                                 cz, E /* E^T */, ewp, ew, lp, lout, reinterpret_cast<float*>(w + o_Cth),
                                 reinterpret_cast<float*>(w + o_Ctl), dstatus);
   k_adj_prep<<<dim3((k + 31) / 32, (nc + 31) / 32), 256, 0, st>>>(h->T, k, nc, dW, h->perm, Tr, Tc, wr);
   k_adj_u<<<dim3((k + 255) / 256, PARTS), 256, 0, st>>>(Tc, k, k, nc, wr, up);
   k_adj_sum_parts<<<(k + 255) / 256, 256, 0, st>>>(up, k, u, udf);
   if (dG) {
-    k_adj_split_r<<<1216, 256, 0, st>>>(h->R, n, k, Rdf);
-    solve_z(st, h->sms, Rdf, k, udf, wk, ys, z);
+    k_adj_split_r<<<dim3((k + 31) / 32, (k + 31) / 32), 256, 0, st>>>(h->R, n, k, Rdf);
+    rbrp_status s = solve_z(h, Rdf, k, udf, ys, z);
+    if (s != RBRP_OK) return s;
     k_adj_cz<<<dim3((m + 255) / 256, PARTS), 256, 0, st>>>(dA, lda, m, k, h->perm, z, czp);
     k_adj_sum_parts<<<(m + 255) / 256, 256, 0, st>>>(czp, m, cz, nullptr);
   }

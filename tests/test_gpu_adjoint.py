@@ -221,3 +221,28 @@ def test_tensor_core_adjoint_matches_ffma(handle):
     # core / FFMA; at squared tol 1e-8 this skeleton is less well conditioned than the others)
     assert out[0][0] <= 1.5 * out[1][0] + 1e-5 and out[0][0] <= 5e-4, out
     assert out[0][1] <= 1.5 * out[1][1] + 1e-4 and out[0][1] <= 1e-2, out
+
+
+@pytest.mark.parametrize("m,k", [(40, 1), (90, 31), (90, 32), (90, 33), (700, 300), (6000, 4130)])
+def test_triangular_solves_of_the_gradient(handle, m, k):
+    """The cluster kernel of z = R11^{-1} R11^{-T} u at the edges of its blocks of 32 rows and
+    with more than one row per thread (k > 4096).  A is Gaussian and w large, so that the terms
+    with z lead the gradient; the FP32 operands and 3xTF32 products give about 1e-6 relative,
+    times a condition number below 12 squared."""
+    from robust_blockwise_random_pivoting_gb300.adjoint import fixed_skeleton_loss_and_grad
+    gen = torch.Generator(device="cpu").manual_seed(m + k)
+    n = k + 37
+    A = colmajor(torch.randn(m, n, generator=gen).cuda())
+    w = 30.0 * torch.randn(n, generator=gen).cuda()
+    S = torch.arange(k, dtype=torch.int32, device="cuda")
+    _, G = fixed_skeleton_loss_and_grad(handle, A, S, w, b=64)
+    D, wr = A.double(), w.double()[k:]
+    C, B = D[:, :k], D[:, k:]
+    R = torch.linalg.qr(C, mode="r")[1]
+    T = torch.cholesky_solve(C.t() @ B, R, upper=True)
+    E = B - C @ T
+    u = T @ wr
+    z = torch.cholesky_solve(u[:, None], R, upper=True)[:, 0]
+    ref = torch.cat([-2 * E @ T.t() - 2 * torch.outer(C @ z, u) + 2 * torch.outer(E @ wr, z),
+                     2 * E + 2 * torch.outer(C @ z, wr)], 1)
+    assert (torch.linalg.norm(G.double() - ref) / torch.linalg.norm(ref)).item() <= 2e-4
