@@ -246,3 +246,26 @@ def test_triangular_solves_of_the_gradient(handle, m, k):
     ref = torch.cat([-2 * E @ T.t() - 2 * torch.outer(C @ z, u) + 2 * torch.outer(E @ wr, z),
                      2 * E + 2 * torch.outer(C @ z, wr)], 1)
     assert (torch.linalg.norm(G.double() - ref) / torch.linalg.norm(ref)).item() <= 2e-4
+
+
+@pytest.mark.parametrize("m,pad", [(96, 0), (97, 0), (96, 1), (130, 2), (200, 4)])
+def test_residual_epilogue_by_vectors_and_elements(handle, m, pad):
+    """E = B - C T's epilogue reads and writes whole 32-row pieces by 16 bytes where the columns
+    start on 16: leading dimensions that are multiples of 4 and not, and ragged rows.  The
+    arithmetic is the same, so padding the columns changes neither loss nor gradient."""
+    from robust_blockwise_random_pivoting_gb300.adjoint import fixed_skeleton_loss_and_grad
+    gen = torch.Generator(device="cpu").manual_seed(m)
+    n, k = 150, 40
+    A = torch.randn(n, m, generator=gen).cuda()
+    w = torch.randn(n, generator=gen).cuda()
+    S = torch.arange(k, dtype=torch.int32, device="cuda")
+    loss0, G0 = fixed_skeleton_loss_and_grad(handle, A.clone().t(), S, w, b=64)
+    B = torch.zeros(n, m + pad, device="cuda")
+    B[:, :m] = A
+    loss, G = fixed_skeleton_loss_and_grad(handle, B[:, :m].t(), S, w, b=64)
+    assert loss == loss0 and torch.equal(G, G0)
+    D, wr = A.t().double(), w.double()[k:]
+    T = torch.linalg.lstsq(D[:, :k], D[:, k:]).solution
+    E = D[:, k:] - D[:, :k] @ T
+    ref = ((E * E).sum() + ((T @ wr) ** 2).sum()).item()
+    assert abs(loss - ref) <= 1e-5 * ref
