@@ -56,7 +56,7 @@ typedef enum {
 typedef enum {
   RBRP_PREC_F64 = 0,        /* FP64 throughout: the plain form */
   RBRP_PREC_F32_MIXED = 1   /* FP32 storage and projections; double-float (pairs of FP32,
-                               ~48-bit) panels, sums and T solve; FP64 sampler weights */
+                               ~48-bit) panels and sums; FP64 sampler weights */
 } rbrp_precision;
 
 typedef struct {

@@ -21,8 +21,8 @@ extern "C" {
  * ~1e-8 relative. */
 rbrp_status rbrp_set_variant(rbrp_handle h, int variant);
 
-/* T = R11^{-1} R12 block updates: 0 = double-float on the FP32 pipe (default,
- * ~48 significant bits), 1 = FP64 pipe. */
+/* T = R11^{-1} R12 block updates: 0 = exact BF16 slice products on the tensor cores
+ * (default; FP64-accurate), 1 = FP64 pipe. */
 rbrp_status rbrp_set_tsolve_fp64(rbrp_handle h, int on);
 
 /* Limit, in SM clock cycles, of the bounded device-side waits of kernels launched

@@ -219,7 +219,7 @@ class Handle:
         check(self.lib.rbrp_set_variant(self.h, int(variant)), self.h)
 
     def set_tsolve_fp64(self, on=True):
-        """T solve on the FP64 pipe (True) or in double-float on the FP32 pipe (False, default)."""
+        """T solve on the FP64 pipe (True) or as exact BF16 slice products (False, default)."""
         check(self.lib.rbrp_set_tsolve_fp64(self.h, int(bool(on))), self.h)
 
     def set_wait_budget(self, cycles=0):
