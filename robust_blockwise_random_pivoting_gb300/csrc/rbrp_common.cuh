@@ -57,6 +57,7 @@ struct State {
   int nK;           // |K1| = |K2| of the block swap
   int recomputes;
   int attempts;     // block attempts (also counts zero panels): exponential-key stream index
+  int t_hard;       // T solve: a factor for the FP64 pipe (rbrp_tsolve.cu)
   unsigned long long draws;  // uniforms consumed from the np-compat stream
   double res0;      // ||A||_F^2
   double residual;  // sum of diags over remaining positions

@@ -484,10 +484,11 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   h->kmax = kmax;
   if (p.compute_T && k > 0 && k < n) {
     ev = prof_begin(h);
-    s = solve_T(h, k, n);
+    int launches = 0;
+    s = solve_T(h, k, n, &launches);
     if (s != RBRP_OK) return s;
     const double dk = k, nc = (double)n - k;
-    prof_end(h, RBRP_PHASE_TSOLVE, ev, 16.0 * dk * nc + 4.0 * dk * dk, dk * dk * nc, 2);
+    prof_end(h, RBRP_PHASE_TSOLVE, ev, 16.0 * dk * nc + 4.0 * dk * dk, dk * dk * nc, launches);
   }
   if (dPerm) cudaMemcpyAsync(dPerm, h->perm, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, st);
   cudaEventRecord(h->ev_end, st);
@@ -496,6 +497,16 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   if (s != RBRP_OK) return s;
   if (h->hst->status == tc::ST_ERR_TIMEOUT)
     return set_error(h, RBRP_ERR_DEVICE_TIMEOUT, "a device-side wait timed out; the kernel aborted cleanly");
+  if (h->hst->t_hard) {   // a factor that the slice products do not solve: T anew on the FP64 pipe
+    ev = prof_begin(h);
+    int launches = 0;
+    s = solve_T_fp64(h, k, n, &launches);
+    if (s != RBRP_OK) return s;
+    prof_end(h, RBRP_PHASE_TSOLVE, ev, 0.0, 0.0, launches);
+    cudaEventRecord(h->ev_end, st);
+    s = cuda_check(h, cudaStreamSynchronize(st), "T solve");
+    if (s != RBRP_OK) return s;
+  }
 
   prof_collect(h);
   const int nb = h->hst->nblocks;

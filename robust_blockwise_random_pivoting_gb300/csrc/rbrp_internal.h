@@ -193,7 +193,10 @@ template <typename T>
 rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, const rbrp_params& p,
                      int* dPerm, rbrp_result* out);
 
-rbrp_status solve_T(rbrp_handle h, int k, int n);
+// T of the run's factor; adds its launches.  State::t_hard is set on the device where the slice
+// products do not do and the second has to solve anew.
+rbrp_status solve_T(rbrp_handle h, int k, int n, int* launches);
+rbrp_status solve_T_fp64(rbrp_handle h, int k, int n, int* launches);
 
 // cudaMalloc for what a run cannot do without (the slices of A, which it can, make room).
 rbrp_status device_alloc(rbrp_handle h, void** ptr, size_t bytes, const char* what);

@@ -102,74 +102,63 @@ __global__ void __launch_bounds__(256) k_trsm_T(const double* __restrict__ R, in
 // ===========================================================================
 // The same solve as slice products (rbrp_slices.cuh): blocks of 256 (or 128) rows from the bottom up,
 // X_J = inv(R11(J, J)) B_J and then B(0:j0) -= R11(0:j0, J) X_J, both on the tensor cores.
-// Rows are scaled by the power of two of their diagonal entry (which leaves T alone), so the
-// entries of the scaled R11, of its blocks' inverses and of T are of one size and a slice
-// loses nothing: 55 bits below each row's largest entry, where the double-float solve this
-// replaces carried 48 throughout.
+//
+// A slice keeps 55 bits below the largest entry of its row (M) or column (N).  The skeleton's
+// columns may differ in size by any factor and nearly depend on one another, so the terms of a
+// product are brought to one size first, by what the data are: term a of the solve by the power
+// of two of the largest entry of B_J(a, :), term j of the update by that of X_J(j, :).  A row i of
+// X then carries 2^-55 of max_a |inv(i, a)| |B_J(a, :)|, and where that is not much more than
+// |X_J(i, :)| it is as good as a substitution's.  Where it is (2^6 and more: the inverse's
+// products cancel), one step of refinement for the block, X_J += inv (B_J - R11(J, J) X_J); past
+// 2^44, and where something is not finite, the substitution on the FP64 pipe solves anew
+// (State::t_hard).  Residuals |R11 T - R12| against |R11| |T| of kernel, Gaussian, sparse and
+// nearly dependent skeletons, and of columns scaled from 2^0 to 2^60: at most 5e-16, of the FP64
+// substitution 5e-16 too, of the 48-bit one 3e-15.  Scaled by R11's diagonal instead, which supposes
+// that its rows and columns are ordered by size, a skeleton of pairs 1e-8 apart had 1e-9.
 //
 // What bounds it: a 128 x 64 tile over 256 values of k is 18,000 clocks of MMAs, which its
 // epilogue (one FP64 subtraction per entry) runs beside; the double-float solve needed 12 FP32 operations per
 // product and a warp per column in the diagonal blocks (k = 2000, 14,384 columns: 15.9 ms,
-// now 2.7; k = 1000, 64,536 columns: 19.5, now 3.4).
+// now 3.1; k = 1000, 64,536 columns: 19.5, now 3.9; 0.4 and 0.5 of these are the scales, the
+// copies of X and the launches of a refinement that is not needed).
 // ===========================================================================
 namespace tc {
 namespace {
 
 constexpr int TS_OB = 256;            // rows per block at the most
 constexpr int TS_CHUNK = 65536;       // columns of T per pass: bounds the sliced copy to 235 MB
+constexpr int TS_REFINE = 6;          // log2 of the cancellation from which X_J is refined
+constexpr int TS_HARD = 44;           // and from which the FP64 pipe solves
 
-__device__ __forceinline__ int diag_exponent(const double* R, int64_t ldr, int a) {
-  return slice_exponent((unsigned)__double2hiint(R[(int64_t)a * ldr + a]) & 0x7FFFFFFFu);
-}
+__device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
 
-// T(a, c) = R(a, k + c) 2^(-e_a), transposed; e_a into ed.
+// Exponent of a row from the upper word of its largest entry; 0 for a zero row.
+__device__ __forceinline__ int row_exponent(unsigned hi) { return hi ? slice_exponent(hi) : 0; }
+
+// T(a, c) = R(a, c0 + c), transposed; the rows' largest entries (upper words) into rho from row a_rho on.
 __global__ void k_ts_gather(const double* __restrict__ R, int64_t ldr, int k, int ncols, double* __restrict__ T,
-                            int* __restrict__ ed) {
+                            int a_rho, unsigned* __restrict__ rho) {
   __shared__ double tile[32][33];
   const int c0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
   for (int q = 0; q < 32; q += 8) {
     const int a = a0 + ty + q, c = c0 + tx;
-    tile[ty + q][tx] = (a < k && c < ncols) ? R[(int64_t)a * ldr + k + c] : 0.0;
+    tile[ty + q][tx] = (a < k && c < ncols) ? R[(int64_t)a * ldr + c] : 0.0;
   }
   __syncthreads();
   const int a = a0 + tx;
   if (a >= k) return;
-  const int e = diag_exponent(R, ldr, a);
-  if (blockIdx.x == 0 && ty == 0) ed[a] = e;
-  // 2^(-e) as an FP64 value (a subnormal one only beside a diagonal of 2^1022 and more)
-  const double sc = ldexp(1.0, -e);
+  unsigned mx = 0u;
   for (int q = 0; q < 32; q += 8) {
     const int c = c0 + ty + q;
-    if (c < ncols) T[a + (int64_t)c * k] = tile[tx][ty + q] * sc;
+    const double v = tile[tx][ty + q];
+    mx = max(mx, abs_hi(v));
+    if (c < ncols) T[a + (int64_t)c * k] = v;
   }
+  if (a >= a_rho) atomicMax(rho + a, mx);
 }
 
-// Slices of R11's rows right of their own block of ob rows (one warp per row), K-major; the
-// exponents are those of the scaled rows.
-__global__ void __launch_bounds__(256)
-k_ts_slice_r(const double* __restrict__ R, int64_t ldr, int k, int ob, int64_t ldk, unsigned short* __restrict__ out,
-             int* __restrict__ exps) {
-  const int lane = threadIdx.x & 31;
-  const int a = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int jb = (a / ob + 1) * ob;
-  if (a >= k || jb >= k) return;
-  const double* row = R + (int64_t)a * ldr;
-  unsigned mx = 0u;
-  for (int j = jb + lane; j < k; j += 32) mx = max(mx, (unsigned)__double2hiint(row[j]) & 0x7FFFFFFFu);
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  const int e = slice_exponent(mx);
-  if (lane == 0) exps[a] = e - diag_exponent(R, ldr, a);
-  for (int j0 = jb + 8 * lane; j0 < ldk; j0 += 256) {
-    unsigned short d[8][SL];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) slice_digits(j0 + u < k ? row[j0 + u] : 0.0, e, d[u]);
-#pragma unroll
-    for (int s = 0; s < SL; ++s) store_slice8(out + ((int64_t)s * k + a) * ldk + j0, d, s);
-  }
-}
-
-// Inverses of the scaled diagonal blocks, row major (ld ldi): CTA (g, J) finds columns 8g ..
+// Inverses of the diagonal blocks, row major (ld ldi): CTA (g, J) finds columns 8g ..
 // 8g + 7 of block J by back substitution, thread = row, the columns still to come updated
 // as soon as an entry is known.
 __global__ void __launch_bounds__(TS_OB)
@@ -184,8 +173,7 @@ k_ts_inv(const double* __restrict__ R, int64_t ldr, int k, double* __restrict__ 
     return;
   }
   const double* Ra = R + (int64_t)(j0 + a) * ldr + j0;
-  const double sc = row ? ldexp(1.0, -diag_exponent(R, ldr, j0 + a)) : 0.0;
-  const double rinv = row ? 1.0 / (Ra[a] * sc) : 0.0;
+  const double rinv = row ? 1.0 / Ra[a] : 0.0;
   double x[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) x[q] = a == cb + q ? 1.0 : 0.0;
@@ -194,7 +182,7 @@ k_ts_inv(const double* __restrict__ R, int64_t ldr, int k, double* __restrict__ 
   for (int jt = cb; jt >= 0; jt -= 8) {      // columns jt .. jt + 7 of R, from the last
     if (w0 < jt + 8) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) r[u] = (row && jt + u < len && a < jt + u) ? Ra[jt + u] * sc : 0.0;
+      for (int u = 0; u < 8; ++u) r[u] = (row && jt + u < len && a < jt + u) ? Ra[jt + u] : 0.0;
     }
 #pragma unroll
     for (int u = 7; u >= 0; --u) {
@@ -220,71 +208,134 @@ k_ts_inv(const double* __restrict__ R, int64_t ldr, int k, double* __restrict__ 
   }
 }
 
-// Slices of rows j0 .. j0 + len of T's columns (one warp per column, its entries in registers)
-// as the N operand: rows (64-column tile, half, slice, column within the half), ldk values.
+// Vectors of up to 256 FP64 values (rows of R11 or of an inverse for M, columns of T for N) whose
+// entry u is taken times 2^(sign * row_exponent(scale[u])), as slices of kpad values.
+struct TsVec {
+  const double* src;
+  int64_t ld;
+  int count;               // vectors
+  int sign;
+  int tri;                 // vector c starts at entry c - tri (rows of R11 from its diagonal on)
+  bool n_operand;          // rows (64-column tile, half, slice, column within the half), else slice by slice
+  int64_t rows;            // M: vectors per slice
+  unsigned short* out;
+  int* exps;
+  double* copy;            // N: the values themselves too (or NULL), ld ldc
+  int64_t ldc;
+};
+
+// What a launch has to know of the refinement of its block.
+struct TsNeed {
+  int* flag;               // NULL: no condition
+  const int* eI;           // not NULL: find the flag from the inverse's exponents and X's rows
+  const unsigned* sig;
+};
+
+// One warp per vector, its entries in registers; first the M vectors' CTAs, then the N vectors'.
 __global__ void __launch_bounds__(256)
-k_ts_slice_x(const double* __restrict__ T, int64_t ldt, int j0, int len, int ncols, int ldk,
-             unsigned short* __restrict__ out, int* __restrict__ exps) {
+k_ts_slices(TsVec vm, TsVec vn, const unsigned* __restrict__ scale, int len, int kpad, TsNeed need,
+            State* __restrict__ st) {
+  bool refine = false;
+  if (need.eI) {           // every CTA for itself, the first one for the launches to come
+    const int t = threadIdx.x;
+    const int kappa = t < len && need.sig[t] ? need.eI[t] - slice_exponent(need.sig[t]) : 0;
+    refine = __syncthreads_or(kappa > TS_REFINE);
+    const bool hard = __syncthreads_or(kappa > TS_HARD);
+    if (blockIdx.x == 0 && t == 0) {
+      *need.flag = refine;
+      if (hard) st->t_hard = 1;
+    }
+  } else if (need.flag && *need.flag == 0) {
+    return;
+  }
+  const int mctas = (vm.count + 7) / 8;
+  const bool m_part = (int)blockIdx.x < mctas;
+  const TsVec& v = m_part ? vm : vn;
   const int lane = threadIdx.x & 31;
-  const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (c >= ncols) return;
-  const double* col = T + (int64_t)c * ldt + j0;
+  const int c = ((int)blockIdx.x - (m_part ? 0 : mctas)) * 8 + (threadIdx.x >> 5);
+  if (c >= v.count) return;
+  const double* src = v.src + (int64_t)c * v.ld;
+  constexpr int NONE = -8192;
   double x[8];
-  unsigned mx = 0u;
+  int f[8];
+  int mx = NONE;
+  bool bad = false;
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
-    x[u] = 8 * lane + u < len ? col[8 * lane + u] : 0.0;
-    mx = max(mx, (unsigned)__double2hiint(x[u]) & 0x7FFFFFFFu);
+    const int a = 8 * lane + u;
+    const bool in = a < len && a >= c - v.tri;
+    x[u] = in ? src[a] : 0.0;
+    f[u] = in ? v.sign * row_exponent(scale[a]) : 0;
+    const unsigned hi = abs_hi(x[u]);
+    bad = bad || hi >= 0x7FF00000u;
+    if (x[u] != 0.0) mx = max(mx, slice_exponent(hi) + f[u]);
   }
+  if (v.copy && !refine) {   // coalesced, the values once more from the cache
+    double* dst = v.copy + (int64_t)c * v.ldc;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (lane + 32 * u < len) dst[lane + 32 * u] = src[lane + 32 * u];
+  }
+  if (bad) st->t_hard = 1;
   mx = __reduce_max_sync(0xffffffffu, mx);
-  const int e = slice_exponent(mx);
-  if (lane == 0) exps[c] = e;
-  if (8 * lane >= ldk) return;
+  const int e = mx == NONE ? 0 : mx;
+  if (lane == 0) v.exps[c] = e;
+  if (8 * lane >= kpad) return;
   unsigned short d[8][SL];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) slice_digits(x[u], e, d[u]);
-  unsigned short* dst = out + ((int64_t)(c / SL_HALF) * SL * SL_HALF + c % SL_HALF) * ldk + 8 * lane;
+  for (int u = 0; u < 8; ++u) slice_digits(x[u], max(e - f[u], -1021), d[u]);
+  const int64_t step = (v.n_operand ? SL_HALF : v.rows) * (int64_t)kpad;
+  const int64_t at = v.n_operand ? (int64_t)(c / SL_HALF) * SL * SL_HALF + c % SL_HALF : (int64_t)c;
+  unsigned short* dst = v.out + at * kpad + 8 * lane;
 #pragma unroll
-  for (int s = 0; s < SL; ++s) store_slice8(dst + (int64_t)s * SL_HALF * ldk, d, s);
+  for (int s = 0; s < SL; ++s) store_slice8(dst + s * step, d, s);
 }
 
-// M = rows row0 .. row0 + rows of the sliced matrix (its K starts at column ax), N = columns
-// of T; stores the product in T, or subtracts it (sub).
+// M = rows row0 .. row0 + rows of the sliced matrix, N = columns of T, K = a block's rows; row
+// p of the product at T(p, :), stored, subtracted from it or added to it.  The rows' largest
+// entries into mx(p) for p >= mx0.
+enum { TS_SET, TS_SUB, TS_ADD };
 struct TsEpi {
   static constexpr bool A_M_MAJOR = false;
   State* st;
   double* T;
   int64_t ldt;
-  int row0, rows, ncols, nst, ax, sub;
+  int row0, rows, ncols, nst, mode;
   const int* exM;
   const int* exX;
+  int mx0;
+  unsigned* mx;
+  const int* flag;         // not NULL: only where it is set
   __device__ int mtiles() const { return (rows + BM - 1) / BM; }
-  __device__ int init() const { return ncols > SL_HALF ? 2 : 1; }
-  __device__ bool tile(int t, int& p0, int& brow, int& s0, int& n, int& a_x) const {
+  __device__ int init() const { return flag && *flag == 0 ? 0 : ncols > SL_HALF ? 2 : 1; }
+  __device__ bool tile(int t, int& p0, int& brow, int& s0, int& n, int& ax) const {
     const int y = t / mtiles();
     p0 = row0 + (t - y * mtiles()) * BM;
     brow = y * 2 * SL * SL_HALF;
-    s0 = 0;
+    s0 = ax = 0;
     n = nst;
-    a_x = ax;
     return y * 64 < ncols;
   }
   __device__ void part(int t, int p, int a0, const long long (&hi)[SL_HALF], const long long (&lo)[SL_HALF]) const {
     if (p >= row0 + rows) return;
     const int c0 = t / mtiles() * 64 + a0, e = exM[p] - 60;
     double* x = T + p + (int64_t)c0 * ldt;
+    unsigned m = 0u;
 #pragma unroll
     for (int j0 = 0; j0 < SL_HALF; j0 += 8) {
       double old[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) old[j] = sub && c0 + j0 + j < ncols ? x[(int64_t)(j0 + j) * ldt] : 0.0;
+      for (int j = 0; j < 8; ++j) old[j] = mode != TS_SET && c0 + j0 + j < ncols ? x[(int64_t)(j0 + j) * ldt] : 0.0;
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (c0 + j0 + j < ncols) {
-          const double v = slice_value(hi[j0 + j], lo[j0 + j], e + exX[c0 + j0 + j]);
-          x[(int64_t)(j0 + j) * ldt] = sub ? old[j] - v : v;
+          double v = slice_value(hi[j0 + j], lo[j0 + j], e + exX[c0 + j0 + j]);
+          if (mode != TS_SET) v = mode == TS_SUB ? old[j] - v : old[j] + v;
+          x[(int64_t)(j0 + j) * ldt] = v;
+          m = max(m, abs_hi(v));
         }
     }
+    if (p >= mx0) atomicMax(mx + p, m);
   }
   __device__ void timeout() const { atomicExch(&st->status, ST_ERR_TIMEOUT); }
 };
@@ -292,7 +343,20 @@ struct TsEpi {
 }  // namespace
 }  // namespace tc
 
-rbrp_status solve_T(rbrp_handle h, int k, int n) {
+rbrp_status solve_T_fp64(rbrp_handle h, int k, int n, int* launches) {
+  const int ncols = n - k;
+  cudaStream_t st = h->stream;
+  *launches += 2;
+  k_gather_T<<<dim3((ncols + 31) / 32, (k + 31) / 32), dim3(32, 8), 0, st>>>(h->R, n, k, ncols, h->T);
+  rbrp_status s = cuda_check(h, cudaFuncSetAttribute(k_trsm_T, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)sizeof(TrsmSmem)), "cudaFuncSetAttribute(k_trsm_T)");
+  if (s != RBRP_OK) return s;
+  k_trsm_T<<<(ncols + 31) / 32, 256, sizeof(TrsmSmem), st>>>(h->R, n, k, ncols, h->T);
+  return cuda_check(h, cudaGetLastError(), "T solve launch");
+}
+
+rbrp_status solve_T(rbrp_handle h, int k, int n, int* launches) {
+  *launches = 0;
   const size_t bytes = (size_t)k * (size_t)(n - k) * sizeof(double);
   if (bytes > h->T_bytes) {
     if (h->T) cudaFree(h->T);
@@ -302,42 +366,39 @@ rbrp_status solve_T(rbrp_handle h, int k, int n) {
     if (s != RBRP_OK) return s;
     h->T_bytes = bytes;
   }
+  if (h->tsolve_fp64) return solve_T_fp64(h, k, n, launches);
   const int ncols = n - k;
   cudaStream_t st = h->stream;
   rbrp_status s;
-  if (h->tsolve_fp64) {
-    dim3 g1((ncols + 31) / 32, (k + 31) / 32), b1(32, 8);
-    k_gather_T<<<g1, b1, 0, st>>>(h->R, n, k, ncols, h->T);
-    s = cuda_check(h, cudaFuncSetAttribute(k_trsm_T, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(TrsmSmem)), "cudaFuncSetAttribute(k_trsm_T)");
-    if (s != RBRP_OK) return s;
-    k_trsm_T<<<(ncols + 31) / 32, 256, sizeof(TrsmSmem), st>>>(h->R, n, k, ncols, h->T);
-    return cuda_check(h, cudaGetLastError(), "T solve launch");
-  }
   using namespace tc;
   // the chain of ob steps of the inverses against fewer, larger products: k = 270, 1730 columns:
   // 0.26 ms with blocks of 128, 0.34 with 256; 640, 7552: 0.61 and 0.63; 900, 300: 0.54 and 0.50;
   // 2000, 14384: 5.7 and 3.9 (before the grid was persistent)
   const int ob = k <= 640 ? TS_OB / 2 : TS_OB;
   const int nblk = (k + ob - 1) / ob;
-  const size_t ldk = ((size_t)k + 63) / 64 * 64, ldi = std::min((size_t)ob, ldk);
+  const size_t ldi = std::min((size_t)ob, ((size_t)k + 63) / 64 * 64);
   const size_t chunk = std::min(ncols, TS_CHUNK), cpad = (chunk + 63) / 64 * 64;
   struct Item {
     void** ptr;
     size_t bytes;
   };
-  int *ed, *eR, *eI, *eX;
+  unsigned *rho, *rho2, *sig;   // largest entries of the rows of B, of a block's residual, of X
+  int *flag, *eR, *eI, *eX;
   unsigned short *sR, *sI, *sX;
-  double* inv;
+  double *inv, *X;
   Item items[] = {
-      {(void**)&ed, (size_t)k * 4},
+      {(void**)&rho, (size_t)k * 4},
+      {(void**)&rho2, (size_t)k * 4},
+      {(void**)&sig, (size_t)k * 4},
+      {(void**)&flag, 4},
       {(void**)&eR, (size_t)k * 4},
-      {(void**)&eI, (size_t)k * 4},
+      {(void**)&eI, ldi * 4},
       {(void**)&eX, cpad * 4},
-      {(void**)&sR, nblk > 1 ? (size_t)SL * k * ldk * 2 : 0},
+      {(void**)&sR, (size_t)SL * k * ldi * 2},
       {(void**)&inv, (size_t)k * ldi * 8},
-      {(void**)&sI, (size_t)SL * k * ldi * 2},
+      {(void**)&sI, (size_t)SL * ldi * ldi * 2},
       {(void**)&sX, (size_t)SL * cpad * ldi * 2},
+      {(void**)&X, cpad * ldi * 8},
   };
   size_t need = 0;
   for (auto& it : items) need += (it.bytes + 255) & ~(size_t)255;
@@ -355,31 +416,52 @@ rbrp_status solve_T(rbrp_handle h, int k, int n) {
     base += (it.bytes + 255) & ~(size_t)255;
   }
   CUtensorMap tmR, tmI, tmX;
-  s = make_tmap_bf16(h, &tmI, sI, ldi, (uint64_t)SL * k, BM);
-  if (s == RBRP_OK && nblk > 1) s = make_tmap_bf16(h, &tmR, sR, ldk, (uint64_t)SL * k, BM);
+  s = make_tmap_bf16(h, &tmI, sI, ldi, (uint64_t)SL * ldi, BM);
+  if (s == RBRP_OK) s = make_tmap_bf16(h, &tmR, sR, ldi, (uint64_t)SL * k, BM);
   if (s == RBRP_OK) s = make_tmap_bf16(h, &tmX, sX, ldi, (uint64_t)SL * cpad, SL * SL_HALF);
   if (s == RBRP_OK)
     s = cuda_check(h, cudaFuncSetAttribute(k_gemm_slices<TsEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)SL_SMEM), "cudaFuncSetAttribute(k_gemm_slices)");
   if (s != RBRP_OK) return s;
   const long long budget = h->wait_budget > 0 ? h->wait_budget : kWaitBudgetDefault;
-  k_ts_gather<<<dim3((ncols + 31) / 32, (k + 31) / 32), dim3(32, 8), 0, st>>>(h->R, n, k, ncols, h->T, ed);
-  if (nblk > 1) k_ts_slice_r<<<(k + 7) / 8, 256, 0, st>>>(h->R, n, k, ob, ldk, sR, eR);
-  k_ts_inv<<<dim3((int)ldi / 8, nblk), ob, 0, st>>>(h->R, n, k, inv, (int)ldi);
-  k_slice_cols<<<(k + 7) / 8, 256, 0, st>>>(inv, ldi, (int)ldi, k, k, ldi, sI, eI);
+  const int kpad = (int)ldi;
+  k_ts_inv<<<dim3(kpad / 8, nblk), ob, 0, st>>>(h->R, n, k, inv, kpad);
+  *launches += 1;
   for (int c0 = 0; c0 < ncols; c0 += TS_CHUNK) {
     const int nc = std::min(TS_CHUNK, ncols - c0), ntile = (nc + 63) / 64;
     double* T = h->T + (size_t)c0 * k;
+    const int jlast = (nblk - 1) * ob;
+    // rho, rho2 and sig lie together
+    cudaMemsetAsync(rho, 0, (size_t)((char*)flag - (char*)rho), st);
+    k_ts_gather<<<dim3((nc + 31) / 32, (k + 31) / 32), dim3(32, 8), 0, st>>>(h->R + k + c0, n, k, nc, T, jlast, rho);
+    *launches += 1;
     for (int J = nblk - 1; J >= 0; --J) {
       const int j0 = J * ob, len = std::min(ob, k - j0), nst = (len + SL_BK - 1) / SL_BK;
-      k_ts_slice_x<<<(nc + 7) / 8, 256, 0, st>>>(T, k, j0, len, nc, (int)ldi, sX, eX);
-      k_gemm_slices<<<std::min(h->sms, (len + BM - 1) / BM * ntile), SL_THREADS, SL_SMEM, st>>>(
-          tmI, tmX, (int64_t)k, budget, TsEpi{h->st, T, k, j0, len, nc, nst, 0, 0, eI, eX});
-      if (J > 0) {
-        k_ts_slice_x<<<(nc + 7) / 8, 256, 0, st>>>(T, k, j0, len, nc, (int)ldi, sX, eX);
-        k_gemm_slices<<<std::min(h->sms, j0 / BM * ntile), SL_THREADS, SL_SMEM, st>>>(
-            tmR, tmX, (int64_t)k, budget, TsEpi{h->st, T, k, 0, j0, nc, nst, j0, 1, eR, eX});
-      }
+      auto slices = [&](const TsVec& vm, const TsVec& vn, const unsigned* scale, const TsNeed& nd) {
+        k_ts_slices<<<(vm.count + 7) / 8 + (vn.count + 7) / 8, 256, 0, st>>>(vm, vn, scale + j0, len, kpad, nd, h->st);
+      };
+      auto gemm = [&](const CUtensorMap& tm, int64_t a_rows, const TsEpi& e) {
+        k_gemm_slices<<<std::min(h->sms, (e.rows + BM - 1) / BM * ntile), SL_THREADS, SL_SMEM, st>>>(tm, tmX, a_rows,
+                                                                                                    budget, e);
+      };
+      const TsVec vI{inv + (size_t)j0 * ldi, (int64_t)ldi, len, 1, len, false, (int64_t)ldi, sI, eI, nullptr, 0};
+      const TsVec vB{T + j0, k, nc, -1, nc, true, 0, sX, eX, nullptr, 0};
+      const TsVec vR{h->R + j0, n, j0 + len, 1, j0, false, k, sR, eR, nullptr, 0};
+      const TsVec vX{X, (int64_t)ldi, nc, -1, nc, true, 0, sX, eX, T + j0, k};
+      TsVec none = vI;
+      none.count = 0;
+      // X = inv B_J, and from it the flag and the operands of the update; T takes X if it stands
+      slices(vI, vB, rho, TsNeed{nullptr, nullptr, nullptr});
+      gemm(tmI, (int64_t)ldi, TsEpi{h->st, X, (int64_t)ldi, 0, len, nc, nst, TS_SET, eI, eX, 0, sig + j0, nullptr});
+      slices(vR, vX, sig, TsNeed{flag, eI, sig + j0});
+      // the refinement: launches that return at once where the flag is not set
+      gemm(tmR, k, TsEpi{h->st, T, k, j0, len, nc, nst, TS_SUB, eR, eX, 0, rho2, flag});
+      slices(vI, vB, rho2, TsNeed{flag, nullptr, nullptr});
+      gemm(tmI, (int64_t)ldi, TsEpi{h->st, X, (int64_t)ldi, 0, len, nc, nst, TS_ADD, eI, eX, len, nullptr, flag});
+      slices(none, vX, sig, TsNeed{flag, nullptr, nullptr});
+      if (J > 0)
+        gemm(tmR, k, TsEpi{h->st, T, k, 0, j0, nc, nst, TS_SUB, eR, eX, j0 - ob, rho, nullptr});
+      *launches += J > 0 ? 8 : 7;
     }
   }
   return cuda_check(h, cudaGetLastError(), "T solve launch");

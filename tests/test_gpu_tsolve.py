@@ -1,0 +1,56 @@
+"""T = R11^{-1} R12 of given skeletons whose columns differ in size or nearly depend on one another."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+def skeleton_matrix(kind, k, n):
+    """n columns, the first k of them (in this order) the skeleton."""
+    rng = np.random.Generator(np.random.Philox(key=k))
+    A = rng.standard_normal((k + 40, n))
+    j = np.arange(k)
+    if kind == "ascending":          # 2^0 in the first block of 64 columns up to 2^60 in the last
+        A[:, :k] *= 2.0 ** (60 * (j // 64) // ((k - 1) // 64))
+    elif kind == "descending":
+        A[:, :k] *= 2.0 ** -(60 * (j // 64) // ((k - 1) // 64))
+    elif kind == "mixed":            # sizes without any order
+        A[:, :k] *= 2.0 ** rng.integers(-30, 31, k)
+    elif kind == "pairs":            # every second column its neighbour's within 1e-6
+        A[:, 1:k:2] = A[:, 0:k - k % 2:2] + 1e-6 * A[:, 1:k:2]
+    elif kind == "blocks":           # a block of 64 columns follows the one before within 1e-6
+        A[:, 64:k] = A[:, :k - 64] + 1e-6 * A[:, 64:k]
+    return A
+
+
+def substitution(R, B):
+    R, X = R.astype(np.longdouble), B.astype(np.longdouble)
+    for i in range(len(R) - 1, -1, -1):
+        X[i] /= R[i, i]
+        X[:i] -= np.outer(R[:i, i], X[i])
+    return X
+
+
+@pytest.mark.parametrize("kind", ["ascending", "descending", "mixed", "pairs", "blocks"])
+@pytest.mark.parametrize("k", [128, 130, 257, 700])    # one block of 128 rows, two, three, three of 256
+def test_T_of_skeletons_in_any_order_and_scale(kind, k):
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
+    n = k + 33
+    A = torch.from_numpy(skeleton_matrix(kind, k, n)).cuda().t().contiguous().t()
+    with Handle(0) as h:
+        perm, T = fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=64)
+        R = h.L().cpu().numpy()[perm.cpu().numpy()].T
+    T, k = T.cpu().numpy(), T.shape[0]      # (columns whose residual norm is lost in rounding are not taken)
+    R11 = R[:, :k]
+    want = substitution(R11, R[:, k:])
+    # in the scaling 2^-f of R11's columns: a residual of (4 k + 256) eps of the row's largest entry
+    # times the largest of T's column - the slices' cuts and the sums over k, and the block inverses
+    # that are not refined (largest entry 128) - carried through |R11^-1|
+    f = np.abs(R11).max(0)
+    Rs, Y = R11 / f, np.abs(T) * f[:, None]
+    inv = np.abs(substitution(Rs, np.eye(k))).astype(np.float64)
+    bound = (4 * k + 256) * EPS * (inv @ np.abs(Rs).max(1))[:, None] * Y.max(0) / f[:, None]
+    assert np.all(np.abs(T - want) <= bound), float((np.abs(T - want) / bound).max())
