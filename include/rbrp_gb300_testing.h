@@ -35,6 +35,11 @@ rbrp_status rbrp_set_tsolve_fp64(rbrp_handle h, int on);
  * aborting kernel's own copies and MMAs finish keep the default limit. */
 rbrp_status rbrp_set_wait_budget(rbrp_handle h, long long cycles);
 
+/* Device memory, in bytes, that the handle's allocations find free from now on (0: what
+ * there is): an allocation of more fails as it would on a full device, without filling one.
+ * Memory that the handle already holds and could release counts against it. */
+rbrp_status rbrp_set_memory_limit(rbrp_handle h, size_t bytes);
+
 #ifdef __cplusplus
 }
 #endif

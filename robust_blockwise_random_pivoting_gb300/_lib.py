@@ -103,6 +103,7 @@ _SIGS = {
     "rbrp_set_variant": (c_int, [c_void_p, c_int]),
     "rbrp_set_tsolve_fp64": (c_int, [c_void_p, c_int]),
     "rbrp_set_wait_budget": (c_int, [c_void_p, ctypes.c_longlong]),
+    "rbrp_set_memory_limit": (c_int, [c_void_p, ctypes.c_size_t]),
     "rbrp_matdivide_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_double,
                                    c_void_p, c_int64, ctypes.POINTER(c_int)]),
     "rbrp_T_matdivide": (c_int, [c_void_p, c_double, ctypes.POINTER(c_int)]),

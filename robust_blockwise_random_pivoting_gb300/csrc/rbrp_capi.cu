@@ -105,13 +105,18 @@ rbrp_status cuda_check(rbrp_handle h, cudaError_t e, const char* what) {
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 rbrp_status device_alloc(rbrp_handle h, void** ptr, size_t bytes, const char* what) {
-  cudaError_t e = cudaMalloc(ptr, bytes);
+  // mem_limit: what the slices leave of it is there (rbrp_set_memory_limit)
+  auto take = [&] {
+    return h->mem_limit && bytes + h->sl_bytes > h->mem_limit ? cudaErrorMemoryAllocation : cudaMalloc(ptr, bytes);
+  };
+  cudaError_t e = take();
   if (e == cudaErrorMemoryAllocation && h->sl_ws) {
     cudaGetLastError();
     cudaStreamSynchronize(h->stream);
     release_slices(h);
-    e = cudaMalloc(ptr, bytes);
+    e = take();
   }
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // reported here, not by a later launch check
   return cuda_check(h, e, what);
 }
 
@@ -250,7 +255,8 @@ static bool ensure_sl_ws(rbrp_handle h, size_t total) {
   if (total <= h->sl_bytes) return true;
   release_slices(h);
   size_t avail = 0, all = 0;
-  if (cudaMemGetInfo(&avail, &all) != cudaSuccess || total > avail / 2 ||
+  if (cudaMemGetInfo(&avail, &all) != cudaSuccess ||
+      total > (h->mem_limit ? std::min(avail, h->mem_limit) : avail) / 2 ||
       cudaMalloc(&h->sl_ws, total) != cudaSuccess) {
     cudaGetLastError();
     h->sl_ws = nullptr;
@@ -731,6 +737,12 @@ rbrp_status rbrp_set_variant(rbrp_handle h, int variant) {
 rbrp_status rbrp_set_wait_budget(rbrp_handle h, long long cycles) {
   if (!h || cycles < 0) return RBRP_ERR_INVALID_ARG;
   h->wait_budget = cycles;
+  return RBRP_OK;
+}
+
+rbrp_status rbrp_set_memory_limit(rbrp_handle h, size_t bytes) {
+  if (!h) return RBRP_ERR_INVALID_ARG;
+  h->mem_limit = bytes;
   return RBRP_OK;
 }
 

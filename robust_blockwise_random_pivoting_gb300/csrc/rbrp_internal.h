@@ -95,6 +95,7 @@ struct rbrp_handle_st {
   int* fix_exA = nullptr;
   int variant = 0;             // 0: tensor-core projection and update, 1: CUDA-core ones
   bool tsolve_fp64 = false;    // T solve on the FP64 pipe instead of slice products
+  size_t mem_limit = 0;        // device memory that allocations find free (0: what there is)
   long long wait_budget = 0;   // clock64 limit of bounded device waits (0: the default, ~2 s)
 
   // interpolation matrix of the last run

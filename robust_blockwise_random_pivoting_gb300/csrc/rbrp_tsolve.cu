@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(256) k_trsm_T(const double* __restrict__ R, in
 // products cancel), one step of refinement for the block, X_J += inv (B_J - R11(J, J) X_J); past
 // 2^44, and where something is not finite, the substitution on the FP64 pipe solves anew
 // (State::t_hard).  Residuals |R11 T - R12| against |R11| |T| of kernel, Gaussian, sparse and
-// nearly dependent skeletons, and of columns scaled from 2^0 to 2^60: at most 5e-16, of the FP64
-// substitution 5e-16 too, of the 48-bit one 3e-15.  Scaled by R11's diagonal instead, which supposes
+// nearly dependent skeletons, and of columns scaled from 2^0 to 2^60: at most 2e-15, of the FP64
+// substitution 5e-16, of the 48-bit one 3e-15.  Scaled by R11's diagonal instead, which supposes
 // that its rows and columns are ordered by size, a skeleton of pairs 1e-8 apart had 1e-9.
 //
 // What bounds it: a 128 x 64 tile over 256 values of k is 18,000 clocks of MMAs, which its
@@ -406,8 +406,10 @@ rbrp_status solve_T(rbrp_handle h, int k, int n, int* launches) {
     if (h->ts_ws) cudaFree(h->ts_ws);
     h->ts_ws = nullptr;
     h->ts_bytes = 0;
-    s = device_alloc(h, &h->ts_ws, need, "cudaMalloc(T solve operands)");
-    if (s != RBRP_OK) return s;
+    if (device_alloc(h, &h->ts_ws, need, "cudaMalloc(T solve operands)") != RBRP_OK) {
+      h->ts_ws = nullptr;   // no room for them: the substitution needs none
+      return solve_T_fp64(h, k, n, launches);
+    }
     h->ts_bytes = need;
   }
   char* base = static_cast<char*>(h->ts_ws);

@@ -228,6 +228,11 @@ class Handle:
         A few cycles makes them run out: calls then raise status 7 (device wait timed out)."""
         check(self.lib.rbrp_set_wait_budget(self.h, int(cycles)), self.h)
 
+    def set_memory_limit(self, nbytes=0):
+        """Device memory that this handle's allocations find free (0: what there is): for tests
+        of what a call does on a full device."""
+        check(self.lib.rbrp_set_memory_limit(self.h, int(nbytes)), self.h)
+
     def reset_phase_stats(self):
         check(self.lib.rbrp_reset_phase_stats(self.h), self.h)
 

@@ -54,3 +54,56 @@ def test_T_of_skeletons_in_any_order_and_scale(kind, k):
     inv = np.abs(substitution(Rs, np.eye(k))).astype(np.float64)
     bound = (4 * k + 256) * EPS * (inv @ np.abs(Rs).max(1))[:, None] * Y.max(0) / f[:, None]
     assert np.all(np.abs(T - want) <= bound), float((np.abs(T - want) / bound).max())
+
+
+def test_T_without_room_for_its_operands():
+    """The T solve on a device that has no room for the slices' operands takes the FP64 pipe."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    A = torch.from_numpy(skeleton_matrix("pairs", 300, 340)).cuda().t().contiguous().t()
+    with Handle(0) as h:
+        h.set_tsolve_fp64(True)
+        want = h.column_id(A, b=50, tol=None, kmax=300, seed=2)
+    with Handle(0) as h:
+        h.column_id(A, b=50, tol=None, kmax=300, seed=2, compute_T=False)
+        h.set_memory_limit(300 * 40 * 8)       # room for T alone
+        got = h.column_id(A, b=50, tol=None, kmax=300, seed=2)
+    assert torch.equal(got.perm, want.perm) and torch.equal(got.T, want.T)
+
+
+def test_T_of_a_factor_that_slices_do_not_solve():
+    """R11 = 1 on the diagonal, -1 above: the inverse grows as 2^k and its products with R12 = R11 X
+    cancel past any refinement; the FP64 pipe's substitution gives T."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
+    k, n = 128, 160
+    rng = np.random.Generator(np.random.Philox(key=1))
+    Q = np.linalg.qr(rng.standard_normal((200, k)))[0]
+    R = np.eye(k) - np.triu(np.ones((k, k)), 1)
+    A = Q @ np.hstack([R, R @ rng.uniform(-1, 1, (k, n - k))])
+    A = torch.from_numpy(A).cuda().t().contiguous().t()
+    Ts = []
+    for fp64 in (False, True):
+        with Handle(0) as h:
+            h.set_tsolve_fp64(fp64)
+            Ts.append(fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=1)[1])
+    assert torch.equal(Ts[0], Ts[1])
+
+
+@pytest.mark.parametrize("k", [128, 300, 600])
+def test_T_of_smooth_kernel_skeletons(k):
+    """Skeletons in no order of a smooth kernel: blocks whose inverses cancel and are refined."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
+    rng = np.random.Generator(np.random.Philox(key=k))
+    x, y = rng.random((k + 60, 3)), rng.random((k + 40, 3))
+    A = np.exp(-2.0 * ((x[:, None] - y[None]) ** 2).sum(-1)) + 1e-10 * rng.standard_normal((k + 60, k + 40))
+    A = torch.from_numpy(A).cuda().t().contiguous().t()
+    with Handle(0) as h:
+        perm, T = fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=64)
+        R = h.L().cpu().numpy()[perm.cpu().numpy()].T.astype(np.longdouble)
+    T = T.cpu().numpy()
+    k = len(T)
+    # per column, against the largest entry of |R11| |T|: the sums over k of the substitution (eps
+    # each) and what a cancellation of 2^6 may leave of a block that is not refined
+    res = np.abs(R[:, :k] @ T - R[:, k:]).max(0)
+    assert np.all(res <= (k + 64) * EPS * (np.abs(R[:, :k]) @ np.abs(T)).max(0))
