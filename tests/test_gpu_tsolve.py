@@ -71,22 +71,20 @@ def test_T_without_room_for_its_operands():
 
 
 def test_T_of_a_factor_that_slices_do_not_solve():
-    """R11 = 1 on the diagonal, -1 above: the inverse grows as 2^k and its products with R12 = R11 X
-    cancel past any refinement; the FP64 pipe's substitution gives T."""
+    """A_S = R11 with 1 on the diagonal and -1 above, R12 = R11 X, all of it exact: the inverse's
+    entries grow as 2^k and their products cancel past any refinement; the substitution on the
+    FP64 pipe, which has to solve, gives X itself."""
     from robust_blockwise_random_pivoting_gb300.rbrp import Handle
     from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
     k, n = 128, 160
-    rng = np.random.Generator(np.random.Philox(key=1))
-    Q = np.linalg.qr(rng.standard_normal((200, k)))[0]
     R = np.eye(k) - np.triu(np.ones((k, k)), 1)
-    A = Q @ np.hstack([R, R @ rng.uniform(-1, 1, (k, n - k))])
+    X = np.random.Generator(np.random.Philox(key=1)).integers(-1000, 1001, (k, n - k)).astype(np.float64)
+    A = np.zeros((200, n))
+    A[:k] = np.hstack([R, R @ X])
     A = torch.from_numpy(A).cuda().t().contiguous().t()
-    Ts = []
-    for fp64 in (False, True):
-        with Handle(0) as h:
-            h.set_tsolve_fp64(fp64)
-            Ts.append(fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=1)[1])
-    assert torch.equal(Ts[0], Ts[1])
+    with Handle(0) as h:
+        perm, T = fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=1)
+    assert np.array_equal(perm.cpu().numpy(), np.arange(n)) and np.array_equal(T.cpu().numpy(), X)
 
 
 @pytest.mark.parametrize("k", [128, 300, 600])
