@@ -251,7 +251,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
           k_panel2_fast<TR><<<ptiles, 256, panel_rows_smem<TR>(), st>>>(h->Q1, m, h->st, h->R2, h->U2, h->chol2_full,
                                                                        Q, m);
         });
-        if (use_fix) k_fix_q<<<p.b, 256, 0, st>>>(Q, m, m, h->st, h->fix_q, h->fix_exQ);
+        if (use_fix) k_fix_q<<<p.b, 256, 0, st>>>(Q, m, m, n, h->st, h->fix_q, h->fix_exQ);
       } else {
         k_pchol<<<1, 1024, sizeof(Panel64Smem), st>>>(h->G, m, h->st, tol_loc, h->js, h->perm, h->diags, h->R11, h->ord,
                                                       h->J, h->K1, h->K2);
@@ -271,7 +271,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       k_swap_cols<<<dim3((m + 1023) / 1024, MAXB), 256, 0, st>>>(h->Ares, L.ld_res, h->st, m, h->K1, h->K2);
     if constexpr (!RES) {
       if (use_sl) {
-        tc::k_slice_q<<<2 * MAXB, 256, 0, st>>>(Q, m, m, h->st, ldk, h->slQ, h->sl_exQ, h->slH, kmax, h->sl_exH);
+        tc::k_slice_q<<<2 * MAXB, 256, 0, st>>>(Q, m, m, n, h->st, ldk, h->slQ, h->sl_exQ, h->slH, kmax, h->sl_exH);
         tc::k_swap_slices<<<dim3(p.b, tc::SL), 256, 0, st>>>(h->slA, n, ldk, h->sl_exA, h->st, h->K1, h->K2);
       }
     }

@@ -54,9 +54,10 @@ k_fix_cols(const double* __restrict__ A, int64_t lda, int m, int n, const int* _
   }
 }
 
-// Limbs and exponents of the block's basis columns: FIX layout [column][limb][row].
+// Limbs and exponents of the block's basis columns: FIX layout [column][limb][row].  Columns that
+// are not finite end the run as in k_slice_q.
 __global__ void __launch_bounds__(256)
-k_fix_q(const double* __restrict__ Q, int64_t ldq, int m, const State* __restrict__ st, int* __restrict__ lim,
+k_fix_q(const double* __restrict__ Q, int64_t ldq, int m, int n, State* __restrict__ st, int* __restrict__ lim,
         int* __restrict__ exps) {
   __shared__ unsigned s_mx[8];
   const int tid = threadIdx.x, a = blockIdx.x;
@@ -69,6 +70,7 @@ k_fix_q(const double* __restrict__ Q, int64_t ldq, int m, const State* __restric
   __syncthreads();
   for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w]);
   const int e = tc::slice_exponent(mx);
+  if (tid == 0 && mx >= 0x7FF00000u && st->i + st->bs < n) atomicCAS(&st->status, 0, ST_ERR_NUMERIC);
   if (tid == 0) exps[a] = e;
   for (int r = tid; r < m; r += 256) {
     int h, l;

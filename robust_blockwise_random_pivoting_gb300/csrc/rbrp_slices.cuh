@@ -107,9 +107,10 @@ k_slice_cols(const double* __restrict__ A, int64_t lda, int m, int n, int64_t sr
 // (half, slice, column within the half), zero beyond the kept columns (up to 32, or 64
 // where more than 32 are kept).  One CTA per column.  Also into row i + a of the basis
 // history (hist_rows per slice; its rows up to the next multiple of 64 are zeroed: the
-// Gram-Schmidt products read whole stages).
+// Gram-Schmidt products read whole stages).  A column that is not finite has no digits: the run
+// ends with the status that its products would have brought about (remaining positions: n).
 __global__ void __launch_bounds__(256)
-k_slice_q(const double* __restrict__ Q, int64_t ldq, int m, const State* __restrict__ st, int64_t ldk,
+k_slice_q(const double* __restrict__ Q, int64_t ldq, int m, int n, State* __restrict__ st, int64_t ldk,
           unsigned short* __restrict__ out, int* __restrict__ exps, unsigned short* __restrict__ hist, int hist_rows,
           int* __restrict__ hist_exps) {
   __shared__ unsigned s_mx[8];
@@ -128,6 +129,7 @@ k_slice_q(const double* __restrict__ Q, int64_t ldq, int m, const State* __restr
   __syncthreads();
   for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w]);
   const int e = slice_exponent(mx);
+  if (tid == 0 && mx >= 0x7FF00000u && i + kept < n) atomicCAS(&st->status, 0, ST_ERR_NUMERIC);
   if (tid == 0 && oper) exps[a] = e;
   if (tid == 0 && keep) hist_exps[i + a] = e;
   for (int r0 = 2 * tid; r0 < ldk; r0 += 512) {

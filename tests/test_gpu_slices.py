@@ -116,3 +116,31 @@ def test_slice_gemm_timeout_is_clean():
         h.set_wait_budget(0)
         got = h.column_id(A, b=64, tol=None, kmax=200, seed=0)
     assert torch.equal(got.perm, want.perm) and torch.equal(got.T, want.T)
+
+
+@pytest.mark.parametrize("b", [1, 8, 48])
+def test_a_basis_that_is_not_finite_is_an_error(b):
+    """Given skeletons of exactly dependent columns: where the second Cholesky factorisation of a
+    panel breaks down the run says so (status 5), as with the FP64 pipe's products, and otherwise
+    |q^T a| <= ||a|| for its basis vectors of norm 1."""
+    from robust_blockwise_random_pivoting_gb300._lib import RBRPError
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
+    S = torch.arange(48, dtype=torch.int32)
+    with Handle(0) as h:
+        for seed in range(400):
+            rng = np.random.default_rng(seed)
+            r, m = int(rng.integers(1, 20)), int(rng.integers(64, 300))
+            if seed % 2:
+                A = rng.standard_normal((m, r)) @ rng.standard_normal((r, 80))
+            else:
+                A = rng.integers(-3, 4, (m, r)).astype(float) @ rng.integers(-3, 4, (r, 80))
+            A[:, 48:] += rng.standard_normal((m, 32))
+            try:
+                fixed_skeleton(h, colmajor(A), S, b=b)
+            except RBRPError as e:
+                assert e.status == 5, seed
+                continue
+            L = h.L().cpu().numpy()
+            assert np.isfinite(L).all(), seed
+            assert np.all(np.abs(L) <= 1.01 * np.linalg.norm(A, axis=0)[:, None]), seed
