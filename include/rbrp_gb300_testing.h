@@ -40,6 +40,19 @@ rbrp_status rbrp_set_wait_budget(rbrp_handle h, long long cycles);
  * Memory that the handle already holds and could release counts against it. */
 rbrp_status rbrp_set_memory_limit(rbrp_handle h, size_t bytes);
 
+/* The arithmetic of the last successful single-matrix run, as a sum of RBRP_FORM_*: results are
+ * reproducible bit for bit within one form.  Which of them a run takes follows from its
+ * parameters and sizes and, for the first three, from whether their scratch fits into half of
+ * the free device memory. */
+enum {
+  RBRP_FORM_SLICES = 1,        /* FP64 projection as BF16 slices on the tensor cores */
+  RBRP_FORM_SLICED_CGS = 2,    /* with room for the basis: Gram-Schmidt products too, where large */
+  RBRP_FORM_FIXED_POINT = 4,   /* FP64 projection of b <= 8 from a fixed-point copy of A */
+  RBRP_FORM_FIXED_ORDER = 8,   /* FP64: every sum in one order whatever the launch */
+  RBRP_FORM_T_FP64 = 16        /* T by substitution on the FP64 pipe */
+};
+rbrp_status rbrp_last_form(rbrp_handle h, int* form);
+
 #ifdef __cplusplus
 }
 #endif

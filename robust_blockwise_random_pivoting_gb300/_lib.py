@@ -42,6 +42,7 @@ class PhaseStats(ctypes.Structure):
                 ("launches", c_int * NPHASES)]
 
 
+FORMS = {"slices": 1, "sliced_cgs": 2, "fixed_point": 4, "fixed_order": 8, "T_fp64": 16}
 BATCH_PHASES = ["norms", "sample", "gram", "pivot", "basis", "project", "update", "finish", "tsolve"]
 
 
@@ -104,6 +105,7 @@ _SIGS = {
     "rbrp_set_tsolve_fp64": (c_int, [c_void_p, c_int]),
     "rbrp_set_wait_budget": (c_int, [c_void_p, ctypes.c_longlong]),
     "rbrp_set_memory_limit": (c_int, [c_void_p, ctypes.c_size_t]),
+    "rbrp_last_form": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
     "rbrp_matdivide_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_double,
                                    c_void_p, c_int64, ctypes.POINTER(c_int)]),
     "rbrp_T_matdivide": (c_int, [c_void_p, c_double, ctypes.POINTER(c_int)]),

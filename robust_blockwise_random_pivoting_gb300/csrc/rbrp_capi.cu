@@ -746,6 +746,13 @@ rbrp_status rbrp_set_memory_limit(rbrp_handle h, size_t bytes) {
   return RBRP_OK;
 }
 
+rbrp_status rbrp_last_form(rbrp_handle h, int* form) {
+  if (!h || !form) return RBRP_ERR_INVALID_ARG;
+  if (!h->have_result) return set_error(h, RBRP_ERR_NOT_COMPUTED, "no successful run");
+  *form = h->form;
+  return RBRP_OK;
+}
+
 rbrp_status rbrp_set_tsolve_fp64(rbrp_handle h, int on) {
   if (!h) return RBRP_ERR_INVALID_ARG;
   h->tsolve_fp64 = on != 0;

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "../../include/rbrp_gb300_testing.h"
 #include "rbrp_internal.h"
 #include "rbrp_kernels.cuh"
 #include "rbrp_panel64.cuh"
@@ -103,6 +104,8 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   // blocks on (the conversion of A costs what two of them gain).
   const bool use_fix = !RES && h->variant == 0 && p.b <= 8 && m <= FIX_MAX_ROWS && !fixed_order && kmax >= 4 * p.b &&
                        ensure_fixed(h, m, n);
+  h->form = (use_sl ? RBRP_FORM_SLICES | RBRP_FORM_SLICED_CGS : 0) | (use_fix ? RBRP_FORM_FIXED_POINT : 0) |
+            (!RES && fixed_order ? RBRP_FORM_FIXED_ORDER : 0);
   const int64_t ldk = ((int64_t)m + tc::SL_BK - 1) / tc::SL_BK * tc::SL_BK;
   CUtensorMap tmSA, tmSQ, tmSH, tmSC;
   const int64_t ldc = ((int64_t)kmax + 63) / 64 * 64;

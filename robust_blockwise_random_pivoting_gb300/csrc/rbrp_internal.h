@@ -132,6 +132,7 @@ struct rbrp_handle_st {
   // last-run results
   bool have_result = false;
   int m = 0, n = 0, k = 0, kmax = 0, prec = 0;
+  int form = 0;                // RBRP_FORM_*
   rbrp_result res{};
   std::vector<int> h_ranks;
   std::vector<double> h_err;

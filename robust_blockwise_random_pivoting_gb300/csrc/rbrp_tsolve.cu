@@ -3,6 +3,7 @@
 
 #include <cuda.h>
 
+#include "../../include/rbrp_gb300_testing.h"
 #include "rbrp_internal.h"
 #include "rbrp_slices.cuh"
 
@@ -347,6 +348,7 @@ rbrp_status solve_T_fp64(rbrp_handle h, int k, int n, int* launches) {
   const int ncols = n - k;
   cudaStream_t st = h->stream;
   *launches += 2;
+  h->form |= RBRP_FORM_T_FP64;
   k_gather_T<<<dim3((ncols + 31) / 32, (k + 31) / 32), dim3(32, 8), 0, st>>>(h->R, n, k, ncols, h->T);
   rbrp_status s = cuda_check(h, cudaFuncSetAttribute(k_trsm_T, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)sizeof(TrsmSmem)), "cudaFuncSetAttribute(k_trsm_T)");

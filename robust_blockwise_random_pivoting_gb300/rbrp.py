@@ -233,6 +233,14 @@ class Handle:
         of what a call does on a full device."""
         check(self.lib.rbrp_set_memory_limit(self.h, int(nbytes)), self.h)
 
+    def form(self):
+        """The arithmetic that the last single-matrix run took: a set of names out of
+        ``_lib.FORMS`` (``include/rbrp_gb300_testing.h``).  Results are reproducible bit for bit
+        within one form."""
+        f = ctypes.c_int()
+        check(self.lib.rbrp_last_form(self.h, ctypes.byref(f)), self.h)
+        return {name for name, bit in _lib.FORMS.items() if f.value & bit}
+
     def reset_phase_stats(self):
         check(self.lib.rbrp_reset_phase_stats(self.h), self.h)
 

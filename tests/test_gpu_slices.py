@@ -144,3 +144,27 @@ def test_a_basis_that_is_not_finite_is_an_error(b):
             L = h.L().cpu().numpy()
             assert np.isfinite(L).all(), seed
             assert np.all(np.abs(L) <= 1.01 * np.linalg.norm(A, axis=0)[:, None]), seed
+
+
+def test_the_form_of_a_run_is_told():
+    """Which arithmetic a run took, with and without room for its scratch (256 x 400 slices: 2 MB)."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    A = colmajor(matrix("normal", 256, 400))
+
+    def form(h, **kw):
+        h.column_id(A, kmax=100, **kw)
+        return h.form()
+    for limit in (0, 1 << 20):
+        room = limit == 0
+        with Handle(0) as h:
+            form(h, b=20, tol=1e-10)               # the workspace that every run has to have
+            h.set_memory_limit(limit)
+            f = form(h, b=20, tol=1e-4)
+            assert ("slices" in f) == room and "fixed_point" not in f and "fixed_order" not in f
+            f = form(h, b=4, tol=None, sampler="greedy")
+            assert ("fixed_point" in f) == (room or 256 * 400 * 8 <= limit // 2) and "slices" not in f
+            f = form(h, b=20, tol=1e-10)
+            assert "fixed_order" in f and "slices" not in f
+    with Handle(0) as h:
+        h.column_id(A.float(), b=20, tol=1e-10, kmax=100)
+        assert not h.form()
