@@ -22,9 +22,17 @@
 
 namespace rbrp {
 
+// Squared relative residual below which the weights of a run are differences of the order of
+// their own rounding (eps over it, relative), and which column a random or greedy draw takes
+// follows the order of the sums behind them.  Above, a draw moves in fewer than one run in 10^4
+// (b sqrt(n) eps over the residual); at 1e-12 it was one in ten.
+constexpr double ORDER_DEPTH = 1e-8;
+
+// One pass of the loop.  again (NULL: sums in fixed order from the start): set, and the pass left,
+// where draws are to follow from a residual below ORDER_DEPTH.
 template <typename T>
-rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, const rbrp_params& p,
-                     int* dPerm, rbrp_result* out) {
+rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, const rbrp_params& p,
+                     int* dPerm, rbrp_result* out, bool* again) {
   // FP64: the notebook's implicit form (projections of A, downdated norms) -
   // the parity path.  FP32: the explicit residual form (see k_proj_w).
   constexpr bool RES = sizeof(T) == sizeof(float);
@@ -93,11 +101,16 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   // 64 x 400, b = 16: 1.53 ms a run against 1.79; 16 x 100000, b = 12: 1.83 against 1.47).
   // Variant 1 and matrices whose slices would not fit keep the CUDA-core kernels too.
   //
-  // Random draws to a squared tolerance below 1e-8 keep the order of every sum as well: the
-  // weights of such a run's last blocks are differences of the order of their own rounding
-  // (eps / tol relative), and which column a draw takes follows that order.  Above, a draw
-  // moves in fewer than one run in 10^4 (b sqrt(n) eps / tol); at 1e-12 it was one in ten.
-  const bool fixed_order = p.tol > 0.0 && p.tol < 1e-8 && (p.sampler == SAMPLER_NP || p.sampler == SAMPLER_ES);
+  // Draws below ORDER_DEPTH keep the order of every sum as well.  Random ones to a tolerance
+  // below it do from the start (they get there, or to kmax); the others that may get there (greedy
+  // draws, and any to no tolerance) from the first block that does, in a second pass of run_rbrp.
+  // With b <= 8 and nothing but the numerical rank to end the run that pass would be most of
+  // the time (400 x 400 to rank 229, b = 8: 12.1 ms in two passes, 8.8 in fixed order; b = 40: 5.0 and 3.8,
+  // but 2.9 where the spectrum stays above): from the start too.  A given skeleton draws nothing.
+  const bool random = p.sampler == SAMPLER_NP || p.sampler == SAMPLER_ES;
+  const bool fixed_order = !again || (p.tol < ORDER_DEPTH && p.sampler != SAMPLER_GIVEN &&
+                                      ((random && p.tol > 0.0) || (p.b <= 8 && kmax == std::min(m, n))));
+  const bool watch = !RES && !fixed_order && p.sampler != SAMPLER_GIVEN;
   const bool use_sl = !RES && h->variant == 0 && p.b > 8 && m >= tc::SL_BK && !fixed_order &&
                       ensure_slices(h, m, n, kmax);
   // Blocks of b <= 8 whose sums may be reordered: the column streams in fixed point, from four
@@ -139,7 +152,7 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   const double es = (double)sizeof(T), dm = (double)m;
   h->marks.clear();
   h->prof_next = 0;
-  cudaEventRecord(h->ev_start, st);
+  if (again) cudaEventRecord(h->ev_start, st);
   cudaMemsetAsync(h->st, 0, sizeof(State), st);
   int ev = prof_begin(h);
   if (RES)  // the residual starts as A, in position (= column) order
@@ -478,6 +491,10 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       }
     }
     ++attempts;
+    if (watch && !h->hst->done && h->hst->residual < ORDER_DEPTH * h->hst->res0) {
+      *again = true;
+      return RBRP_OK;
+    }
   }
   cudaEventRecord(h->ev_loop, st);
   const int k = h->hst->i;
@@ -546,6 +563,14 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   h->have_result = true;
   if (out) *out = r;
   return cuda_check(h, cudaGetLastError(), "RBRP kernels");
+}
+
+template <typename T>
+rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, const rbrp_params& p,
+                     int* dPerm, rbrp_result* out) {
+  bool again = false;
+  const rbrp_status s = run_pass<T>(h, m, n, dA, lda, p, dPerm, out, &again);
+  return s == RBRP_OK && again ? run_pass<T>(h, m, n, dA, lda, p, dPerm, out, nullptr) : s;
 }
 
 }  // namespace rbrp

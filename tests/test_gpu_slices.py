@@ -168,3 +168,26 @@ def test_the_form_of_a_run_is_told():
     with Handle(0) as h:
         h.column_id(A.float(), b=20, tol=1e-10, kmax=100)
         assert not h.form()
+
+
+@pytest.mark.parametrize("sampler", ["np", "es", "greedy"])
+@pytest.mark.parametrize("b,kmax", [(8, None), (8, 220), (24, None), (40, 215)])
+def test_draws_past_the_depth_follow_the_fixed_order(sampler, b, kmax):
+    """Draws from weights below 1e-8 of the start (the spectrum exp(-i / 12) has its numerical rank
+    near 230) follow the order of the sums: a run without a tolerance that gets there takes the
+    columns, bit for bit, that one to a tolerance below any residual takes."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    from robust_blockwise_random_pivoting_gb300.workloads import gaussian_exp
+    A = colmajor(gaussian_exp(400, 400, decay=12.0, seed=0))
+    with Handle(0) as h:
+        for seed in range(3):
+            got = h.column_id(A, b=b, tol=None, kmax=kmax, seed=seed, sampler=sampler)
+            assert "fixed_order" in h.form()
+            want = h.column_id(A, b=b, tol=1e-30, kmax=kmax, seed=seed, sampler=sampler)
+            assert "fixed_order" in h.form()
+            assert torch.equal(got.perm, want.perm) and np.array_equal(got.ranks, want.ranks)
+            assert np.array_equal(got.residuals, want.residuals) and got.draws == want.draws
+            assert torch.equal(got.T, want.T)
+            if kmax:     # above the depth the order is free
+                h.column_id(A, b=b, tol=None, kmax=40, seed=seed, sampler=sampler)
+                assert "fixed_order" not in h.form()
