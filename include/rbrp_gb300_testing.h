@@ -40,6 +40,10 @@ rbrp_status rbrp_set_wait_budget(rbrp_handle h, long long cycles);
  * Memory that the handle already holds and could release counts against it. */
 rbrp_status rbrp_set_memory_limit(rbrp_handle h, size_t bytes);
 
+/* Device memory, in bytes, that the handle holds for the slices or the fixed-point copy of the
+ * last FP64 matrix: scratch that any of its allocations that finds no room gives back. */
+rbrp_status rbrp_scratch_bytes(rbrp_handle h, size_t* bytes);
+
 /* The arithmetic of the last successful single-matrix run, as a sum of RBRP_FORM_*: results are
  * reproducible bit for bit within one form.  Which of them a run takes follows from its
  * parameters and sizes and, for the first three, from whether their scratch fits into half of

@@ -105,6 +105,7 @@ _SIGS = {
     "rbrp_set_tsolve_fp64": (c_int, [c_void_p, c_int]),
     "rbrp_set_wait_budget": (c_int, [c_void_p, ctypes.c_longlong]),
     "rbrp_set_memory_limit": (c_int, [c_void_p, ctypes.c_size_t]),
+    "rbrp_scratch_bytes": (c_int, [c_void_p, ctypes.POINTER(ctypes.c_size_t)]),
     "rbrp_last_form": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
     "rbrp_matdivide_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_double,
                                    c_void_p, c_int64, ctypes.POINTER(c_int)]),

@@ -704,7 +704,7 @@ extern "C" rbrp_status rbrp_fixed_id_adjoint_f32(rbrp_handle h, int m, int n, co
     if (h->adj_ws) cudaFree(h->adj_ws);
     h->adj_ws = nullptr;
     h->adj_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&h->adj_ws, off), "cudaMalloc(adjoint workspace)");
+    rbrp_status s = device_alloc(h, (void**)&h->adj_ws, off, "cudaMalloc(adjoint workspace)");
     if (s != RBRP_OK) return s;
     h->adj_bytes = off;
   }

@@ -1461,14 +1461,14 @@ rbrp_status batch_alloc(rbrp_handle h, BatchState& B, size_t slot_bytes, int gri
     B.d_order = nullptr;
     B.d_res = nullptr;
     B.cap_probs = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&B.d_probs, sizeof(rbrp_batch_problem) * B.nprob), "cudaMalloc(batch)");
-    if (s == RBRP_OK) s = cuda_check(h, cudaMalloc(&B.d_order, sizeof(int) * B.nprob), "cudaMalloc(batch order)");
-    if (s == RBRP_OK) s = cuda_check(h, cudaMalloc(&B.d_res, sizeof(rbrp_batch_result) * B.nprob), "cudaMalloc(batch results)");
+    rbrp_status s = device_alloc(h, (void**)&B.d_probs, sizeof(rbrp_batch_problem) * B.nprob, "cudaMalloc(batch)");
+    if (s == RBRP_OK) s = device_alloc(h, (void**)&B.d_order, sizeof(int) * B.nprob, "cudaMalloc(batch order)");
+    if (s == RBRP_OK) s = device_alloc(h, (void**)&B.d_res, sizeof(rbrp_batch_result) * B.nprob, "cudaMalloc(batch results)");
     if (s != RBRP_OK) return s;
     B.cap_probs = B.nprob;
   }
   if (!B.d_queue) {
-    rbrp_status s = cuda_check(h, cudaMalloc(&B.d_queue, sizeof(int)), "cudaMalloc(queue)");
+    rbrp_status s = device_alloc(h, (void**)&B.d_queue, sizeof(int), "cudaMalloc(queue)");
     if (s != RBRP_OK) return s;
   }
   const size_t need = slot_bytes * (size_t)grid;
@@ -1476,7 +1476,7 @@ rbrp_status batch_alloc(rbrp_handle h, BatchState& B, size_t slot_bytes, int gri
     cudaFree(B.slots);
     B.slots = nullptr;
     B.slots_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&B.slots, need), "cudaMalloc(batch workspace)");
+    rbrp_status s = device_alloc(h, (void**)&B.slots, need, "cudaMalloc(batch workspace)");
     if (s != RBRP_OK) return s;
     B.slots_bytes = need;
   }
@@ -1739,7 +1739,7 @@ rbrp_status rbrp_batch_set_profiling(rbrp_handle h, int on) {
   BatchState& B = *h->batch;
   DeviceGuard g(h->device);
   if (on && !B.d_prof) {
-    rbrp_status s = cuda_check(h, cudaMalloc(&B.d_prof, sizeof(unsigned long long) * BPH_N), "cudaMalloc(profile)");
+    rbrp_status s = device_alloc(h, (void**)&B.d_prof, sizeof(unsigned long long) * BPH_N, "cudaMalloc(profile)");
     if (s != RBRP_OK) return s;
   }
   B.profiling = on != 0;

@@ -405,7 +405,7 @@ rbrp_status host_run(rbrp_handle h, int m, int n, const T* hA, int64_t lda, cons
     if (h->hostA_dev) cudaFree(h->hostA_dev);
     h->hostA_dev = nullptr;
     h->hostA_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&h->hostA_dev, bytes), "cudaMalloc(A copy)");
+    rbrp_status s = device_alloc(h, (void**)&h->hostA_dev, bytes, "cudaMalloc(A copy)");
     if (s != RBRP_OK) return s;
     h->hostA_bytes = bytes;
   }
@@ -481,7 +481,7 @@ rbrp_status fixed_id(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
     if (h->given_order) cudaFree(h->given_order);
     h->given_order = nullptr;
     h->given_cap = 0;
-    s = cuda_check(h, cudaMalloc((void**)&h->given_order, sizeof(int) * (size_t)n), "cudaMalloc(skeleton order)");
+    s = device_alloc(h, (void**)&h->given_order, sizeof(int) * (size_t)n, "cudaMalloc(skeleton order)");
     if (s != RBRP_OK) return s;
     h->given_cap = n;
   }
@@ -746,6 +746,12 @@ rbrp_status rbrp_set_memory_limit(rbrp_handle h, size_t bytes) {
   return RBRP_OK;
 }
 
+rbrp_status rbrp_scratch_bytes(rbrp_handle h, size_t* bytes) {
+  if (!h || !bytes) return RBRP_ERR_INVALID_ARG;
+  *bytes = h->sl_bytes;
+  return RBRP_OK;
+}
+
 rbrp_status rbrp_last_form(rbrp_handle h, int* form) {
   if (!h || !form) return RBRP_ERR_INVALID_ARG;
   if (!h->have_result) return set_error(h, RBRP_ERR_NOT_COMPUTED, "no successful run");
@@ -806,10 +812,10 @@ rbrp_status rbrp_RandAdapRBRP(const double* dA, int m, int n, int** sk, int** rd
   if (s == RBRP_OK) {
     const int k = r.k, nc = n - k;
     *rank = k;
-    if (cudaMalloc((void**)sk, sizeof(int) * (size_t)(k > 0 ? k : 1)) != cudaSuccess ||
-        cudaMalloc((void**)rd, sizeof(int) * (size_t)(nc > 0 ? nc : 1)) != cudaSuccess ||
-        cudaMalloc((void**)T, sizeof(double) * (size_t)(k > 0 && nc > 0 ? (size_t)k * nc : 1)) != cudaSuccess) {
-      cudaGetLastError();
+    if (device_alloc(h, (void**)sk, sizeof(int) * (size_t)(k > 0 ? k : 1), "cudaMalloc(sk)") != RBRP_OK ||
+        device_alloc(h, (void**)rd, sizeof(int) * (size_t)(nc > 0 ? nc : 1), "cudaMalloc(rd)") != RBRP_OK ||
+        device_alloc(h, (void**)T, sizeof(double) * (size_t)(k > 0 && nc > 0 ? (size_t)k * nc : 1),
+                     "cudaMalloc(T)") != RBRP_OK) {
       if (*sk) cudaFree(*sk);
       if (*rd) cudaFree(*rd);
       if (*T) cudaFree(*T);

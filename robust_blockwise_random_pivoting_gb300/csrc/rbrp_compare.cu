@@ -52,14 +52,12 @@ int grid_for(int64_t count) { return (int)std::max<int64_t>(1, std::min<int64_t>
 
 // Device scratch freed on scope exit.
 struct Scratch {
+  rbrp_handle h;
   std::vector<void*> ptrs;
   template <typename T>
   T* get(size_t count) {
     void* p = nullptr;
-    if (cudaMalloc(&p, std::max<size_t>(1, count) * sizeof(T)) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
+    if (device_alloc(h, &p, std::max<size_t>(1, count) * sizeof(T), "cudaMalloc(scratch)") != RBRP_OK) return nullptr;
     ptrs.push_back(p);
     return static_cast<T*>(p);
   }
@@ -127,19 +125,17 @@ extern "C" rbrp_status rbrp_RandLUPP_OS(const double* dA, int m, int n, int k, i
   if ((s = rbrp_create(&h, dev)) != RBRP_OK) return s;
   const int nc = n - k;
   {
-    Scratch sc;
+    Scratch sc{h, {}};
     double* Y64 = nullptr;
     int* perm = sc.get<int>(n);
     s = perm ? sketch_f64(h, sc, dA, m, n, k, seed, &Y64) : RBRP_ERR_ALLOC;
     if (s == RBRP_OK) s = rbrp_lupp_pivots_f64(h, k, n, Y64, 2 * k, perm, nullptr);
     double* Tout = nullptr;
     if (s == RBRP_OK) {
-      if (cudaMalloc((void**)sk, sizeof(int) * (size_t)k) != cudaSuccess ||
-          cudaMalloc((void**)rd, sizeof(int) * (size_t)std::max(nc, 1)) != cudaSuccess ||
-          cudaMalloc((void**)&Tout, sizeof(double) * std::max<size_t>(1, (size_t)k * nc)) != cudaSuccess) {
-        cudaGetLastError();
+      if (device_alloc(h, (void**)sk, sizeof(int) * (size_t)k, "cudaMalloc(sk)") != RBRP_OK ||
+          device_alloc(h, (void**)rd, sizeof(int) * (size_t)std::max(nc, 1), "cudaMalloc(rd)") != RBRP_OK ||
+          device_alloc(h, (void**)&Tout, sizeof(double) * std::max<size_t>(1, (size_t)k * nc), "cudaMalloc(T)") != RBRP_OK)
         s = RBRP_ERR_ALLOC;
-      }
     }
     if (s == RBRP_OK) s = interpolation_on_sketch(h, sc, Y64, k, n, perm, Tout);
     if (s == RBRP_OK) {
@@ -175,7 +171,7 @@ extern "C" rbrp_status rbrp_RandCPQR_OS(const double* dA, int m, int n, int k, i
   if ((s = rbrp_create(&h, dev)) != RBRP_OK) return s;
   const int nc = n - k;
   {
-    Scratch sc;
+    Scratch sc{h, {}};
     double* Y64 = nullptr;
     int* perm = sc.get<int>(n);
     s = perm ? sketch_f64(h, sc, dA, m, n, k, seed, &Y64) : RBRP_ERR_ALLOC;
@@ -193,10 +189,9 @@ extern "C" rbrp_status rbrp_RandCPQR_OS(const double* dA, int m, int n, int k, i
       if (s == RBRP_OK && r.k != k) s = set_error(h, RBRP_ERR_NUMERIC, "the sketch has rank below k");
     }
     double* Tout = nullptr;
-    if (s == RBRP_OK && cudaMalloc((void**)&Tout, sizeof(double) * std::max<size_t>(1, (size_t)k * nc)) != cudaSuccess) {
-      cudaGetLastError();
+    if (s == RBRP_OK && device_alloc(h, (void**)&Tout, sizeof(double) * std::max<size_t>(1, (size_t)k * nc),
+                                     "cudaMalloc(T)") != RBRP_OK)
       s = RBRP_ERR_ALLOC;
-    }
     if (s == RBRP_OK) s = interpolation_on_sketch(h, sc, Y64, k, n, perm, Tout);
     if (s == RBRP_OK) {
       cudaMemcpy(h_sk, perm, sizeof(int) * (size_t)k, cudaMemcpyDeviceToHost);

@@ -200,7 +200,8 @@ rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
 rbrp_status solve_T(rbrp_handle h, int k, int n, int* launches);
 rbrp_status solve_T_fp64(rbrp_handle h, int k, int n, int* launches);
 
-// cudaMalloc for what a run cannot do without (the slices of A, which it can, make room).
+// cudaMalloc for what a call cannot do without: the slices of A, which it can, make room.  Every
+// allocation made on a handle goes through it (none while a run's blocks use the slices).
 rbrp_status device_alloc(rbrp_handle h, void** ptr, size_t bytes, const char* what);
 
 // 2-D FP32 TMA descriptor (inner dimension contiguous, 128-byte swizzle).

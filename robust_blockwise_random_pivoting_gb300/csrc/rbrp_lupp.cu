@@ -307,7 +307,7 @@ extern "C" rbrp_status rbrp_lupp_pivots_f64(rbrp_handle h, int k, int n, const d
     if (h->lupp_ws) cudaFree(h->lupp_ws);
     h->lupp_ws = nullptr;
     h->lupp_bytes = 0;
-    s = cuda_check(h, cudaMalloc(&h->lupp_ws, bytes), "cudaMalloc(LU workspace)");
+    s = device_alloc(h, (void**)&h->lupp_ws, bytes, "cudaMalloc(LU workspace)");
     if (s != RBRP_OK) return s;
     h->lupp_bytes = bytes;
   }

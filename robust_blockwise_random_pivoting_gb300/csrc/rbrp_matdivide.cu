@@ -268,7 +268,7 @@ rbrp_status matdivide(rbrp_handle h, int p, int q, int nc, const double* dB, int
     if (h->md_ws) cudaFree(h->md_ws);
     h->md_ws = nullptr;
     h->md_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&h->md_ws, bytes), "cudaMalloc(matdivide workspace)");
+    rbrp_status s = device_alloc(h, (void**)&h->md_ws, bytes, "cudaMalloc(matdivide workspace)");
     if (s != RBRP_OK) return s;
     h->md_bytes = bytes;
   }
@@ -359,7 +359,7 @@ extern "C" rbrp_status rbrp_T_matdivide(rbrp_handle h, double tol, int* rank) {
     if (h->T) cudaFree(h->T);
     h->T = nullptr;
     h->T_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc((void**)&h->T, tbytes), "cudaMalloc(T)");
+    rbrp_status s = device_alloc(h, (void**)&h->T, tbytes, "cudaMalloc(T)");
     if (s != RBRP_OK) return s;
     h->T_bytes = tbytes;
   }
@@ -368,7 +368,7 @@ extern "C" rbrp_status rbrp_T_matdivide(rbrp_handle h, double tol, int* rank) {
     if (h->md_aux) cudaFree(h->md_aux);
     h->md_aux = nullptr;
     h->md_aux_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&h->md_aux, abytes), "cudaMalloc(matdivide operands)");
+    rbrp_status s = device_alloc(h, (void**)&h->md_aux, abytes, "cudaMalloc(matdivide operands)");
     if (s != RBRP_OK) return s;
     h->md_aux_bytes = abytes;
   }
@@ -401,7 +401,7 @@ rbrp_status refine_T(rbrp_handle h, int m, int n, const T* dA, int64_t lda, int 
     if (h->md_aux) cudaFree(h->md_aux);
     h->md_aux = nullptr;
     h->md_aux_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&h->md_aux, bytes), "cudaMalloc(refinement operands)");
+    rbrp_status s = device_alloc(h, (void**)&h->md_aux, bytes, "cudaMalloc(refinement operands)");
     if (s != RBRP_OK) return s;
     h->md_aux_bytes = bytes;
   }

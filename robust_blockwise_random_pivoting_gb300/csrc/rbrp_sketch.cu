@@ -130,7 +130,7 @@ extern "C" rbrp_status rbrp_sketch_gaussian_f32(rbrp_handle h, int l, int m, int
     if (h->sketch_ws) cudaFree(h->sketch_ws);
     h->sketch_ws = nullptr;
     h->sketch_bytes = 0;
-    rbrp_status s = cuda_check(h, cudaMalloc(&h->sketch_ws, bytes), "cudaMalloc(sketch matrix)");
+    rbrp_status s = device_alloc(h, (void**)&h->sketch_ws, bytes, "cudaMalloc(sketch matrix)");
     if (s != RBRP_OK) return s;
     h->sketch_bytes = bytes;
   }

@@ -233,6 +233,13 @@ class Handle:
         of what a call does on a full device."""
         check(self.lib.rbrp_set_memory_limit(self.h, int(nbytes)), self.h)
 
+    def scratch_bytes(self):
+        """Device memory that this handle holds for the slices or the fixed-point copy of its last
+        FP64 matrix (given back to any of its allocations that finds no room)."""
+        b = ctypes.c_size_t()
+        check(self.lib.rbrp_scratch_bytes(self.h, ctypes.byref(b)), self.h)
+        return b.value
+
     def form(self):
         """The arithmetic that the last single-matrix run took: a set of names out of
         ``_lib.FORMS`` (``include/rbrp_gb300_testing.h``).  Results are reproducible bit for bit

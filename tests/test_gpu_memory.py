@@ -1,0 +1,62 @@
+"""Device memory that a handle keeps between calls, seen on a device that is (said to be) nearly full."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+M, N = 512, 1100
+
+
+def matrix(dtype=torch.float64):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    return torch.randn(N, M, generator=g, device="cuda", dtype=torch.float64).to(dtype).t()
+
+
+def later_batch(h, A):
+    from robust_blockwise_random_pivoting_gb300.rbrp import Batch
+    Batch(h, [matrix(torch.float32)[:64, :64].t().contiguous().t()], b=16).run()
+
+
+def later_adjoint(h, A):
+    from robust_blockwise_random_pivoting_gb300.adjoint import fixed_skeleton_id_loss
+    B = A[:200, :300].float().t().contiguous().t().requires_grad_()
+    fixed_skeleton_id_loss(B, torch.arange(100, dtype=torch.int32), torch.ones(300, device="cuda"), 50, h).backward()
+
+
+def later_sketch(h, A):
+    from robust_blockwise_random_pivoting_gb300.sketch_ids import gaussian_sketch
+    gaussian_sketch(A.float(), 64, handle=h)
+
+
+def later_lupp(h, A):
+    from robust_blockwise_random_pivoting_gb300.sketch_ids import lupp_pivots
+    lupp_pivots(A[:50], handle=h)
+
+
+LATER = {
+    "host run": lambda h, A: h.column_id_host(A.cpu(), b=32, tol=None, kmax=100, sampler="greedy"),
+    "T_matdivide": lambda h, A: h.T_matdivide(),
+    "refine_T": lambda h, A: h.refine_T(A),
+    "batch": later_batch,
+    "adjoint": later_adjoint,
+    "sketch": later_sketch,
+    "lupp": later_lupp,
+}
+
+
+@pytest.mark.parametrize("name", list(LATER))
+def test_every_allocation_gets_the_slices_memory(name):
+    """After an FP64 run its slices (9 MB here) fill what the device has: the next call on the handle
+    takes their memory instead of failing."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    A = matrix()
+    with Handle(0) as h:
+        r = h.column_id(A, b=32, tol=None, kmax=100)
+        assert r.k == 100 and "slices" in h.form()
+        held = h.scratch_bytes()
+        assert held > 8 * MB
+        h.set_memory_limit(held)
+        LATER[name](h, A)
+        assert h.scratch_bytes() != held
+        torch.cuda.synchronize()
