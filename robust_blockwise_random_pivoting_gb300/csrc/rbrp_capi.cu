@@ -547,13 +547,15 @@ rbrp_status rbrp_create(rbrp_handle* out, int device) {
   if (!h) return RBRP_ERR_ALLOC;
   h->device = device;
   DeviceGuard g(device);
-  if (!g.ok || cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+  size_t avail = 0, all = 0;
+  if (!g.ok || cudaMemGetInfo(&avail, &all) != cudaSuccess || cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
       cudaEventCreate(&h->ev_start) != cudaSuccess || cudaEventCreate(&h->ev_loop) != cudaSuccess ||
       cudaEventCreate(&h->ev_end) != cudaSuccess) {
     cudaGetLastError();
     delete h;
     return RBRP_ERR_CUDA;
   }
+  h->sl_keep = all / 16;
   *out = h;
   return RBRP_OK;
 }

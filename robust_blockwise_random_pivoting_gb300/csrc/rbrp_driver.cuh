@@ -569,8 +569,10 @@ template <typename T>
 rbrp_status run_rbrp(rbrp_handle h, int m, int n, const T* dA, int64_t lda, const rbrp_params& p,
                      int* dPerm, rbrp_result* out) {
   bool again = false;
-  const rbrp_status s = run_pass<T>(h, m, n, dA, lda, p, dPerm, out, &again);
-  return s == RBRP_OK && again ? run_pass<T>(h, m, n, dA, lda, p, dPerm, out, nullptr) : s;
+  rbrp_status s = run_pass<T>(h, m, n, dA, lda, p, dPerm, out, &again);
+  if (s == RBRP_OK && again) s = run_pass<T>(h, m, n, dA, lda, p, dPerm, out, nullptr);
+  if (h->sl_bytes > h->sl_keep) release_slices(h);
+  return s;
 }
 
 }  // namespace rbrp

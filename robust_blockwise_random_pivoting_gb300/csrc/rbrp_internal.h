@@ -78,6 +78,9 @@ struct rbrp_handle_st {
   // block's basis, their exponents, and the row-split FP64 partials of the projection
   void* sl_ws = nullptr;
   size_t sl_bytes = 0;
+  // kept from run to run up to a sixteenth of the device's memory (17 GiB: 34000 x 34000); a
+  // larger run allocates it anew (4.5 GB: 3 ms, of a run of 25 to rank 640)
+  size_t sl_keep = 0;
   unsigned short* slA = nullptr;
   unsigned short* slQ = nullptr;
   unsigned short* slH = nullptr;   // slices of the basis so far, and of the sampled columns' coefficients

@@ -60,3 +60,21 @@ def test_every_allocation_gets_the_slices_memory(name):
         LATER[name](h, A)
         assert h.scratch_bytes() != held
         torch.cuda.synchronize()
+
+
+def test_a_handle_keeps_scratch_of_up_to_a_sixteenth_of_the_device():
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    total = torch.cuda.get_device_properties(0).total_memory
+    m = 32000
+    n = total // 16 // (14 * m) + 64           # 14 bytes of slices an entry
+    for n, keep in ((1000, True), (n, False)):
+        A = torch.randn(n, m, device="cuda", dtype=torch.float64).t()
+        free = torch.cuda.mem_get_info()[0]
+        with Handle(0) as h:
+            for _ in range(2):
+                h.column_id(A, b=16, tol=None, kmax=32, compute_T=False)
+                assert "slices" in h.form() and (h.scratch_bytes() > 0) == keep
+            if not keep:
+                assert free - torch.cuda.mem_get_info()[0] < 1 << 30
+        del A
+        torch.cuda.empty_cache()
