@@ -250,29 +250,33 @@ void release_slices(rbrp_handle h) {
   h->sl_bytes = 0;
 }
 
-// sl_ws with room for `total` bytes, if that is at most half of what is free.
-static bool ensure_sl_ws(rbrp_handle h, size_t total) {
-  if (total <= h->sl_bytes) return true;
+// sl_ws with room for `total` bytes and, as far as they fit, `extra` more, if that is at most half
+// of what is free; the extra bytes it has, or -1.
+static int64_t ensure_sl_ws(rbrp_handle h, size_t total, size_t extra) {
+  if (total + extra <= h->sl_bytes) return (int64_t)extra;
   release_slices(h);
   size_t avail = 0, all = 0;
-  if (cudaMemGetInfo(&avail, &all) != cudaSuccess ||
-      total > (h->mem_limit ? std::min(avail, h->mem_limit) : avail) / 2 ||
-      cudaMalloc(&h->sl_ws, total) != cudaSuccess) {
-    cudaGetLastError();
-    h->sl_ws = nullptr;
-    return false;
+  if (cudaMemGetInfo(&avail, &all) != cudaSuccess) avail = 0;
+  const size_t half = (h->mem_limit ? std::min(avail, h->mem_limit) : avail) / 2;
+  if (total <= half) {
+    extra = std::min(extra, half - total);
+    if (cudaMalloc(&h->sl_ws, total + extra) == cudaSuccess) {
+      h->sl_bytes = total + extra;
+      return (int64_t)extra;
+    }
   }
-  h->sl_bytes = total;
-  return true;
+  cudaGetLastError();
+  h->sl_ws = nullptr;
+  return -1;
 }
 
 bool ensure_fixed(rbrp_handle h, int m, int n) {
-  if (!ensure_sl_ws(h, (size_t)m * n * sizeof(int2))) return false;
+  if (ensure_sl_ws(h, (size_t)m * n * sizeof(int2), 0) < 0) return false;
   h->fix_A = static_cast<int2*>(h->sl_ws);
   return true;
 }
 
-bool ensure_slices(rbrp_handle h, int m, int n, int kmax) {
+bool ensure_slices(rbrp_handle h, int m, int n, int kmax, int hist_rows) {
   const size_t ldk = ((size_t)m + 63) / 64 * 64;
   // row ranges of the projection: enough CTAs for four waves at the most, 16 ranges at the most
   const int ctiles = (n + 127) / 128;
@@ -283,23 +287,26 @@ bool ensure_slices(rbrp_handle h, int m, int n, int kmax) {
   } items[] = {
       {(void**)&h->slA, 7 * ldk * (size_t)n * 2},
       {(void**)&h->slQ, 7 * ldk * MAXB * 2},
-      {(void**)&h->slH, 7 * ldk * (size_t)kmax * 2},
-      {(void**)&h->slC, 7 * (((size_t)kmax + 63) / 64 * 64) * MAXB * 2},
-      {(void**)&h->sl_exH, (size_t)kmax * 4},
+      {(void**)&h->slC, hist_rows ? 7 * (((size_t)kmax + 63) / 64 * 64) * MAXB * 2 : 0},
+      {(void**)&h->sl_exH, (size_t)hist_rows * 4},
       {(void**)&h->sl_exC, MAXB * 4},
       {(void**)&h->sl_exA, (size_t)n * 4},
       {(void**)&h->sl_exQ, MAXB * 4},
       {(void**)&h->sl_Wpart, (size_t)maxsplit * MAXB * n * 8},
+      {(void**)&h->slH, 0},     // last: as many rows as fit
   };
   size_t total = 0;
   for (auto& it : items) total += align_up(it.bytes);
-  if (!ensure_sl_ws(h, total)) return false;
+  const size_t row = 7 * ldk * 2;
+  const int64_t extra = ensure_sl_ws(h, total, row * hist_rows);
+  if (extra < 0) return false;
   char* base = static_cast<char*>(h->sl_ws);
   size_t off = 0;
   for (auto& it : items) {
     *it.ptr = base + off;
     off += align_up(it.bytes);
   }
+  h->sl_hist = (int)std::min<int64_t>(hist_rows, extra / (int64_t)row);
   h->sl_maxsplit = maxsplit;
   return true;
 }

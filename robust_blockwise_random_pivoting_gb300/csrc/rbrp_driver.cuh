@@ -111,13 +111,19 @@ rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   const bool fixed_order = !again || (p.tol < ORDER_DEPTH && p.sampler != SAMPLER_GIVEN &&
                                       ((random && p.tol > 0.0) || (p.b <= 8 && kmax == std::min(m, n))));
   const bool watch = !RES && !fixed_order && p.sampler != SAMPLER_GIVEN;
+  //
+  // Gram-Schmidt products Q C as slice products where the FP64 pipe would take longer than their
+  // two launches: 2e7 products are 40 us of it, and the launches take 25 to 50.  Runs that cannot
+  // get there keep no slices of the basis.
+  auto cgs_pays = [&](int i) { return (double)m * i * p.b >= 2e7; };
   const bool use_sl = !RES && h->variant == 0 && p.b > 8 && m >= tc::SL_BK && !fixed_order &&
-                      ensure_slices(h, m, n, kmax);
+                      ensure_slices(h, m, n, kmax, cgs_pays(kmax - 1) ? kmax : 0);
   // Blocks of b <= 8 whose sums may be reordered: the column streams in fixed point, from four
   // blocks on (the conversion of A costs what two of them gain).
   const bool use_fix = !RES && h->variant == 0 && p.b <= 8 && m <= FIX_MAX_ROWS && !fixed_order && kmax >= 4 * p.b &&
                        ensure_fixed(h, m, n);
-  h->form = (use_sl ? RBRP_FORM_SLICES | RBRP_FORM_SLICED_CGS : 0) | (use_fix ? RBRP_FORM_FIXED_POINT : 0) |
+  const int hist = use_sl ? h->sl_hist : 0;
+  h->form = (use_sl ? RBRP_FORM_SLICES : 0) | (hist ? RBRP_FORM_SLICED_CGS : 0) | (use_fix ? RBRP_FORM_FIXED_POINT : 0) |
             (!RES && fixed_order ? RBRP_FORM_FIXED_ORDER : 0);
   const int64_t ldk = ((int64_t)m + tc::SL_BK - 1) / tc::SL_BK * tc::SL_BK;
   CUtensorMap tmSA, tmSQ, tmSH, tmSC;
@@ -125,8 +131,8 @@ rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   if (use_sl) {
     s = make_tmap_bf16(h, &tmSA, h->slA, ldk, (uint64_t)tc::SL * n, tc::BM);
     if (s == RBRP_OK) s = make_tmap_bf16(h, &tmSQ, h->slQ, ldk, tc::SL * MAXB, tc::SL * tc::SL_HALF);
-    if (s == RBRP_OK) s = make_tmap_bf16(h, &tmSH, h->slH, ldk, (uint64_t)tc::SL * kmax, tc::SL_BK);
-    if (s == RBRP_OK) s = make_tmap_bf16(h, &tmSC, h->slC, ldc, tc::SL * MAXB, tc::SL * tc::SL_HALF);
+    if (s == RBRP_OK && hist) s = make_tmap_bf16(h, &tmSH, h->slH, ldk, (uint64_t)tc::SL * hist, tc::SL_BK);
+    if (s == RBRP_OK && hist) s = make_tmap_bf16(h, &tmSC, h->slC, ldc, tc::SL * MAXB, tc::SL * tc::SL_HALF);
     if (s == RBRP_OK)
       s = cuda_check(h, cudaFuncSetAttribute(tc::k_gemm_slices<tc::CgsEpi>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SL_SMEM),
@@ -203,14 +209,12 @@ rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       k_reduce_parts<double><<<64, 64, 0, st>>>(h->Gpart, dtiles, MAXB * MAXB, MAXB * MAXB, h->G);
     }
     if constexpr (!RES) {
-      // Q C as slice products where the FP64 pipe would take longer than their two launches:
-      // 2e7 products are 40 us of it, and the launches take 25 to 50
-      const bool cgs_sl = use_sl && (double)m * i * p.b >= 2e7;
+      const bool cgs_sl = i <= hist && cgs_pays(i);
       if (cgs_sl) {
         tc::k_slice_coef<<<p.b > tc::SL_HALF ? MAXB : tc::SL_HALF, 256, 0, st>>>(h->R, n, h->js, h->st, h->sl_exH, ldc,
                                                                                  h->slC, h->sl_exC);
         tc::k_gemm_slices<<<std::min(h->sms, (m + tc::BM - 1) / tc::BM), tc::SL_THREADS, tc::SL_SMEM, st>>>(
-            tmSH, tmSC, (int64_t)kmax, h->wait_budget > 0 ? h->wait_budget : kWaitBudgetDefault,
+            tmSH, tmSC, (int64_t)hist, h->wait_budget > 0 ? h->wait_budget : kWaitBudgetDefault,
             tc::CgsEpi{h->st, m, dA, lda, h->cols, h->sl_exC, h->V, 0, 0});
       } else if (i > 0 && !fixed_order) {
         k_gather_coef<<<(i + 3) / 4, 256, 0, st>>>(h->R, n, h->js, h->st, C);
@@ -287,7 +291,7 @@ rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       k_swap_cols<<<dim3((m + 1023) / 1024, MAXB), 256, 0, st>>>(h->Ares, L.ld_res, h->st, m, h->K1, h->K2);
     if constexpr (!RES) {
       if (use_sl) {
-        tc::k_slice_q<<<2 * MAXB, 256, 0, st>>>(Q, m, m, n, h->st, ldk, h->slQ, h->sl_exQ, h->slH, kmax, h->sl_exH);
+        tc::k_slice_q<<<2 * MAXB, 256, 0, st>>>(Q, m, m, n, h->st, ldk, h->slQ, h->sl_exQ, h->slH, hist, h->sl_exH);
         tc::k_swap_slices<<<dim3(p.b, tc::SL), 256, 0, st>>>(h->slA, n, ldk, h->sl_exA, h->st, h->K1, h->K2);
       }
     }

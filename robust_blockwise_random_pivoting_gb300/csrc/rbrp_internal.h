@@ -91,6 +91,7 @@ struct rbrp_handle_st {
   int* sl_exQ = nullptr;
   double* sl_Wpart = nullptr;
   int sl_maxsplit = 0;
+  int sl_hist = 0;             // basis vectors that slH has room for
   // FP64 form, b <= 8 (rbrp_fixed.cuh): limbs of the block's basis, exponents of it and of A's columns
   int2* fix_A = nullptr;       // A in fixed point (in sl_ws: a run uses one of the two)
   int* fix_q = nullptr;
@@ -216,8 +217,9 @@ rbrp_status make_tmap_bf16(rbrp_handle h, void* map, const unsigned short* base,
                            uint32_t box_outer);
 
 // Slice workspace of the FP64 form for an m x n matrix; false (and none held) where it would
-// take more than half of the free memory, which the CUDA-core projection then keeps.
-bool ensure_slices(rbrp_handle h, int m, int n, int kmax);
+// take more than half of the free memory, which the CUDA-core projection then keeps.  The basis
+// history gets up to hist_rows rows of what is left of that half (sl_hist).
+bool ensure_slices(rbrp_handle h, int m, int n, int kmax, int hist_rows);
 bool ensure_fixed(rbrp_handle h, int m, int n);   // the same for the fixed-point copy of A
 void release_slices(rbrp_handle h);
 

@@ -78,3 +78,23 @@ def test_a_handle_keeps_scratch_of_up_to_a_sixteenth_of_the_device():
                 assert free - torch.cuda.mem_get_info()[0] < 1 << 30
         del A
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("mb,sliced_cgs", [(0, True), (72, True), (61, False)])
+def test_the_basis_gets_what_the_slices_of_A_leave(mb, sliced_cgs):
+    """2000 x 800 to rank 700: 32 MB for the slices of A and what goes with them, 20 MB for those of the
+    whole basis.  Half of 72 MB holds 200 basis vectors' too, half of 61 MB none: the products
+    with A stay on the tensor cores, those with the basis go there as far as there is room."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    g = torch.Generator(device="cuda").manual_seed(7)
+    A = torch.randn(800, 2000, generator=g, device="cuda", dtype=torch.float64).t()
+    with Handle(0) as h:
+        h.set_variant(1)
+        want = h.column_id(A, b=64, tol=None, kmax=700)
+    with Handle(0) as h:
+        h.set_memory_limit(mb * MB)
+        got = h.column_id(A, b=64, tol=None, kmax=700)
+        assert h.form() - {"T_fp64"} == ({"slices", "sliced_cgs"} if sliced_cgs else {"slices"})
+    assert torch.equal(got.perm, want.perm) and np.array_equal(got.ranks, want.ranks)
+    # a Gaussian matrix: kappa(A_S) < 10, one Gram-Schmidt pass, m eps kappa^2
+    assert (got.T - want.T).norm() <= 2000 * 2.0 ** -53 * 100 * want.T.norm()
