@@ -191,3 +191,34 @@ def test_draws_past_the_depth_follow_the_fixed_order(sampler, b, kmax):
             if kmax:     # above the depth the order is free
                 h.column_id(A, b=b, tol=None, kmax=40, seed=seed, sampler=sampler)
                 assert "fixed_order" not in h.form()
+
+
+@pytest.mark.parametrize("m,n,b", [(64, 120, 16), (193, 150, 33), (300, 400, 40), (1100, 333, 64), (777, 100, 48),
+                                   (500, 200, 8), (600, 150, 3), (900, 100, 1)])
+def test_projection_error_is_that_of_the_operands_digits(m, n, b):
+    """The first block's products against exact ones.  Unit columns e_j beside the data give its basis,
+    Q(j, :) = Q^T e_j.  What may be off: entries of q and a cut 55 bits below 2^e > |.|max, uniformly, their
+    products' dropped classes, Q(j, :) read back in 53 bits and one rounding of the result: four times the
+    root mean square of that (without its lowest class of 2^-60 products the error is ten times)."""
+    rng = np.random.Generator(np.random.Philox(key=m))
+    B = rng.standard_normal((m, n))
+    A = np.hstack([B, np.eye(m)])
+    err = []
+    for variant in (0, 1):
+        perm, L, k1 = first_block(A, b, variant)
+        assert (perm[:k1] < n).all()               # the data's norms are far above the unit columns'
+        rest = np.setdiff1d(np.arange(n), perm[:k1])
+        Q = L[n:].astype(np.longdouble)
+        exact = B[:, rest].T.astype(np.longdouble) @ Q
+        err.append((L[rest] - exact).astype(np.float64))
+    Q, X = Q.astype(np.float64), B[:, rest]
+    eq, ea = 2.0 ** np.frexp(np.abs(Q).max(0))[1], 2.0 ** np.frexp(np.abs(X).max(0))[1]
+    u = 1.0 / np.sqrt(12.0)                        # of a unit, uniform
+    var = (u * 2.0 ** -54 * ea[:, None] * np.linalg.norm(Q, axis=0)) ** 2 \
+        + (u * 2.0 ** -54 * eq * np.linalg.norm(X, axis=0)[:, None]) ** 2 \
+        + (u * 2.0 ** -52) ** 2 * ((X ** 2).T @ Q ** 2) \
+        + (u * 2.0 ** -52 * np.abs(X.T @ Q)) ** 2 \
+        + (2.0 ** -60 * ea[:, None] * eq * np.sqrt(5.0 * m) * 128 ** 2 / 3 / 256 ** 2) ** 2
+    rms = lambda e: float(np.sqrt(np.mean(e ** 2)))
+    assert rms(err[0]) <= 4 * np.sqrt(var.mean())
+    assert rms(err[0]) <= rms(err[1])              # and no more than the FP64 pipe's
