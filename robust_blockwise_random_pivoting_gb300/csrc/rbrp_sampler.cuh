@@ -368,8 +368,9 @@ __device__ void sample_block(State* st, const double* __restrict__ diags, const 
 // The NP sampler's FP64 passes for many columns: thread t of k_sample's 1024 owns the chunk
 // [t chunk, (t + 1) chunk) of the remaining positions; here chunk t belongs to thread t % 32 of
 // CTA t / 32, so the sums keep their order and take 32 SMs' FP64 pipes instead of one's.
-constexpr int SAMPLE_PRE_MIN = 8192;   // remaining positions from which the two launches pay (64,500
-// columns: 180 us a block in one launch, 50 in three; 15,000: 70 and 40)
+constexpr int SAMPLE_PRE_MIN = 15 * SAMPLE_THREADS + 1;   // remaining positions from which the two launches
+// pay: 16 a thread (us a block in one launch and in three: 8,300 columns 48 and 63, 13,000 61 and 66, 15,000
+// 68 and 68, 15,424 104 and 65, 32,000 186 and 80)
 
 // part[t] = sum of the chunk's weights
 __global__ void __launch_bounds__(32)
