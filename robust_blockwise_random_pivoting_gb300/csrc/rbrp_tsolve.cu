@@ -373,10 +373,11 @@ rbrp_status solve_T(rbrp_handle h, int k, int n, int* launches) {
   cudaStream_t st = h->stream;
   rbrp_status s;
   using namespace tc;
-  // the chain of ob steps of the inverses against fewer, larger products: k = 270, 1730 columns:
-  // 0.26 ms with blocks of 128, 0.34 with 256; 640, 7552: 0.61 and 0.63; 900, 300: 0.54 and 0.50;
-  // 2000, 14384: 5.7 and 3.9 (before the grid was persistent)
-  const int ob = k <= 640 ? TS_OB / 2 : TS_OB;
+  // blocks of 256 rows, but two or three of 128 where those shorten the chain of steps in the
+  // inverses and the columns are too few to hide it (ms with 128 and with 256): k = 208, 4747 columns
+  // 0.25 and 0.24, 256 0.25 and 0.29, 384, 3000 columns 0.32 and 0.35, 385 0.39 and 0.36, 1000, 15,000
+  // columns 1.69 and 1.30; 60,000 columns, 256 0.88 and 0.85, 384 1.37 and 1.26
+  const int ob = k > 208 && k <= 384 && ncols <= 32768 ? TS_OB / 2 : TS_OB;
   const int nblk = (k + ob - 1) / ob;
   const size_t ldi = std::min((size_t)ob, ((size_t)k + 63) / 64 * 64);
   const size_t chunk = std::min(ncols, TS_CHUNK), cpad = (chunk + 63) / 64 * 64;

@@ -34,7 +34,7 @@ def substitution(R, B):
 
 
 @pytest.mark.parametrize("kind", ["ascending", "descending", "mixed", "pairs", "blocks"])
-@pytest.mark.parametrize("k", [128, 130, 257, 700])    # one block of 128 rows, two, three, three of 256
+@pytest.mark.parametrize("k", [128, 130, 257, 700])    # one block, three of 128 rows, three of 256
 def test_T_of_skeletons_in_any_order_and_scale(kind, k):
     from robust_blockwise_random_pivoting_gb300.rbrp import Handle
     from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
