@@ -7,6 +7,7 @@
 // lines 76-173, with the stopping rule of cell 11 line 164 (squared tol).
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "../../include/rbrp_gb300_testing.h"
@@ -104,13 +105,22 @@ rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   // Draws below ORDER_DEPTH keep the order of every sum as well.  Random ones to a tolerance
   // below it do from the start (they get there, or to kmax); the others that may get there (greedy
   // draws, and any to no tolerance) from the first block that does, in a second pass of run_rbrp.
-  // With b <= 8 and nothing but the numerical rank to end the run that pass would be most of
-  // the time (400 x 400 to rank 229, b = 8: 12.1 ms in two passes, 8.8 in fixed order; b = 40: 5.0 and 3.8,
-  // but 2.9 where the spectrum stays above): from the start too.  A given skeleton draws nothing.
-  const bool random = p.sampler == SAMPLER_NP || p.sampler == SAMPLER_ES;
-  const bool fixed_order = !again || (p.tol < ORDER_DEPTH && p.sampler != SAMPLER_GIVEN &&
-                                      ((random && p.tol > 0.0) || (p.b <= 8 && kmax == std::min(m, n))));
+  // A given skeleton draws nothing.
+  const bool fixed_order = !again || (p.tol > 0.0 && p.tol < ORDER_DEPTH &&
+                                      (p.sampler == SAMPLER_NP || p.sampler == SAMPLER_ES));
   const bool watch = !RES && !fixed_order && p.sampler != SAMPLER_GIVEN;
+  // With b <= 8 a block in fixed order takes 1.5 times as long as in free order (2.5 to 4 times with
+  // larger b), and the pass given up is a good part of the whole: there, where nothing but the
+  // numerical rank ends the run, it is given up from an eighth of the ranks on where the residual so
+  // far falls at twice the pace that would reach the depth at the last (400 x 400, spectrum exp(-i / 12),
+  // greedy b = 1: 44 ms when it waits for the depth, 36 so, 33 in fixed order from the start, which would
+  // take Gaussian columns, whose residuals stay above to the end, from 36 ms to 58).
+  const bool foresee = watch && p.b <= 8 && kmax == std::min(m, n) && p.tol < ORDER_DEPTH;
+  auto deep = [&](const State& q) {
+    const double at = (double)q.i / kmax;
+    return q.residual < ORDER_DEPTH * q.res0 ||
+           (foresee && at >= 0.125 && q.residual < std::pow(ORDER_DEPTH, 2.0 * at) * q.res0);
+  };
   //
   // Gram-Schmidt products Q C as slice products where the FP64 pipe would take longer than their
   // two launches: 2e7 products are 40 us of it, and the launches take 25 to 50.  Runs that cannot
@@ -495,7 +505,7 @@ rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
       }
     }
     ++attempts;
-    if (watch && !h->hst->done && h->hst->residual < ORDER_DEPTH * h->hst->res0) {
+    if (watch && !h->hst->done && deep(*h->hst)) {
       *again = true;
       return RBRP_OK;
     }
