@@ -100,6 +100,50 @@ __global__ void __launch_bounds__(256) k_trsm_T(const double* __restrict__ R, in
   }
 }
 
+// Back substitution for small ranks, k <= 32 NR: a warp per right-hand side, row 32 q + lane in
+// register q, R11 in shared memory with its rows divided by their diagonal, so that a step is a
+// shuffle and the updates.  Bound by the FP64 pipe, about ncols k^2 / 10^6 us, or the load of R11 and the
+// chain of k steps (k = 64, 500 columns: 17 us).  The slice products below take some ten launches.
+constexpr int TS_SMALL = 128;
+template <int NR>
+__global__ void __launch_bounds__(256)
+k_trsm_small(const double* __restrict__ R, int64_t ldr, int k, int ncols, double* __restrict__ T) {
+  extern __shared__ __align__(16) double small_smem[];
+  constexpr int LD = 32 * NR + 1;
+  double(*Rs)[LD] = reinterpret_cast<double(*)[LD]>(small_smem);              // [row][column], k rows
+  double(*Bs)[LD] = reinterpret_cast<double(*)[LD]>(small_smem + k * LD);     // [right-hand side][row]
+  double* ri = small_smem + (k + 8) * LD;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, c0 = blockIdx.x * 8;
+  if (tid < k) ri[tid] = 1.0 / R[(int64_t)tid * ldr + tid];
+  __syncthreads();
+  for (int x = tid; x < k * k; x += 256) {
+    const int a = x / k, j = x % k;
+    if (j > a) Rs[a][j] = R[(int64_t)a * ldr + j] * ri[a];
+  }
+  for (int x = tid; x < 8 * k; x += 256) {
+    const int a = x / 8, c = x % 8;
+    Bs[c][a] = c0 + c < ncols ? R[(int64_t)a * ldr + k + c0 + c] * ri[a] : 0.0;
+  }
+  __syncthreads();
+  if (c0 + w >= ncols) return;
+  double x[NR];
+#pragma unroll
+  for (int q = 0; q < NR; ++q) x[q] = 32 * q + lane < k ? Bs[w][32 * q + lane] : 0.0;
+#pragma unroll
+  for (int r = NR - 1; r >= 0; --r) {
+    for (int jj = min(31, k - 1 - 32 * r); jj >= 0; --jj) {
+      const int j = 32 * r + jj;
+      const double xj = __shfl_sync(0xffffffffu, x[r], jj);
+#pragma unroll
+      for (int q = 0; q < r; ++q) x[q] = fma(-Rs[32 * q + lane][j], xj, x[q]);
+      if (lane < jj) x[r] = fma(-Rs[32 * r + lane][j], xj, x[r]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NR; ++q)
+    if (32 * q + lane < k) T[32 * q + lane + (int64_t)(c0 + w) * k] = x[q];
+}
+
 // ===========================================================================
 // The same solve as slice products (rbrp_slices.cuh): blocks of 256 (or 128) rows from the bottom up,
 // X_J = inv(R11(J, J)) B_J and then B(0:j0) -= R11(0:j0, J) X_J, both on the tensor cores.
@@ -357,6 +401,20 @@ rbrp_status solve_T_fp64(rbrp_handle h, int k, int n, int* launches) {
   return cuda_check(h, cudaGetLastError(), "T solve launch");
 }
 
+template <int NR>
+static rbrp_status solve_T_small(rbrp_handle h, int k, int n, int* launches) {
+  const size_t smem = ((size_t)(k + 8) * (32 * NR + 1) + k) * sizeof(double);
+  const rbrp_status s =
+      cuda_check(h, cudaFuncSetAttribute(k_trsm_small<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(((32 * NR + 8) * (32 * NR + 1) + 32 * NR) * sizeof(double))),
+                 "cudaFuncSetAttribute(k_trsm_small)");
+  if (s != RBRP_OK) return s;
+  *launches += 1;
+  h->form |= RBRP_FORM_T_FP64;
+  k_trsm_small<NR><<<(n - k + 7) / 8, 256, smem, h->stream>>>(h->R, n, k, n - k, h->T);
+  return cuda_check(h, cudaGetLastError(), "T solve launch");
+}
+
 rbrp_status solve_T(rbrp_handle h, int k, int n, int* launches) {
   *launches = 0;
   const size_t bytes = (size_t)k * (size_t)(n - k) * sizeof(double);
@@ -370,6 +428,14 @@ rbrp_status solve_T(rbrp_handle h, int k, int n, int* launches) {
   }
   if (h->tsolve_fp64) return solve_T_fp64(h, k, n, launches);
   const int ncols = n - k;
+  // where the FP64 pipe is the shorter way (us, substitution and slice products): k = 16, 500 columns 8 and
+  // 67, 64, 500 columns 17 and 100, 20,000 140 and 192, 128, 2000 71 and 155, 5000 162 and 167, 10,000 285
+  // and 202, 100, 10,000 186 and 177
+  if (k <= TS_SMALL && (double)ncols * k * k <= 9e7)
+    return k <= 32   ? solve_T_small<1>(h, k, n, launches)
+           : k <= 64 ? solve_T_small<2>(h, k, n, launches)
+           : k <= 96 ? solve_T_small<3>(h, k, n, launches)
+                     : solve_T_small<4>(h, k, n, launches);
   cudaStream_t st = h->stream;
   rbrp_status s;
   using namespace tc;

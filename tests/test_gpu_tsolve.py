@@ -34,11 +34,12 @@ def substitution(R, B):
 
 
 @pytest.mark.parametrize("kind", ["ascending", "descending", "mixed", "pairs", "blocks"])
-@pytest.mark.parametrize("k", [128, 130, 257, 700])    # one block, three of 128 rows, three of 256
-def test_T_of_skeletons_in_any_order_and_scale(kind, k):
+@pytest.mark.parametrize("k,nc", [(128, 33), (130, 33), (257, 33), (700, 33),    # substitution, one block, 3 of 128, 3 of 256
+                                  (100, 9100), (128, 5600)])
+def test_T_of_skeletons_in_any_order_and_scale(kind, k, nc):
     from robust_blockwise_random_pivoting_gb300.rbrp import Handle
     from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
-    n = k + 33
+    n = k + nc
     A = torch.from_numpy(skeleton_matrix(kind, k, n)).cuda().t().contiguous().t()
     with Handle(0) as h:
         perm, T = fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=64)
@@ -70,20 +71,22 @@ def test_T_without_room_for_its_operands():
     assert torch.equal(got.perm, want.perm) and torch.equal(got.T, want.T)
 
 
-def test_T_of_a_factor_that_slices_do_not_solve():
+@pytest.mark.parametrize("k", [128, 200])      # (the first by its rank, the second after the slices)
+def test_T_of_a_factor_that_slices_do_not_solve(k):
     """A_S = R11 with 1 on the diagonal and -1 above, R12 = R11 X, all of it exact: the inverse's
     entries grow as 2^k and their products cancel past any refinement; the substitution on the
     FP64 pipe, which has to solve, gives X itself."""
     from robust_blockwise_random_pivoting_gb300.rbrp import Handle
     from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
-    k, n = 128, 160
+    n = k + 32
     R = np.eye(k) - np.triu(np.ones((k, k)), 1)
     X = np.random.Generator(np.random.Philox(key=1)).integers(-1000, 1001, (k, n - k)).astype(np.float64)
-    A = np.zeros((200, n))
+    A = np.zeros((k + 72, n))
     A[:k] = np.hstack([R, R @ X])
     A = torch.from_numpy(A).cuda().t().contiguous().t()
     with Handle(0) as h:
         perm, T = fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=1)
+        assert "T_fp64" in h.form()
     assert np.array_equal(perm.cpu().numpy(), np.arange(n)) and np.array_equal(T.cpu().numpy(), X)
 
 
@@ -105,3 +108,23 @@ def test_T_of_smooth_kernel_skeletons(k):
     # each) and what a cancellation of 2^6 may leave of a block that is not refined
     res = np.abs(R[:, :k] @ T - R[:, k:]).max(0)
     assert np.all(res <= (k + 64) * EPS * (np.abs(R[:, :k]) @ np.abs(T)).max(0))
+
+
+@pytest.mark.parametrize("k", [1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 128])
+@pytest.mark.parametrize("nc", [1, 7, 8, 9, 300])
+def test_T_of_small_ranks(k, nc):
+    """Up to rank 128 the substitution on the FP64 pipe, a warp per column: entry by entry within the
+    rounding of k + 3 operations on rows that were divided by their diagonal first, twice over for the
+    reciprocal."""
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    from robust_blockwise_random_pivoting_gb300.sketch_ids import fixed_skeleton
+    A = torch.from_numpy(skeleton_matrix("mixed", k, k + nc)).cuda().t().contiguous().t()
+    with Handle(0) as h:
+        perm, T = fixed_skeleton(h, A, torch.arange(k, dtype=torch.int32), b=min(k, 16))
+        assert "T_fp64" in h.form() and T.shape == (k, nc)
+        R = h.L().cpu().numpy()[perm.cpu().numpy()].T
+    R11, T = R[:, :k], T.cpu().numpy()
+    want = substitution(R11, R[:, k:])
+    inv = np.abs(substitution(R11, np.eye(k))).astype(np.float64)
+    bound = (2 * k + 8) * EPS * (inv @ (np.abs(R11) @ np.abs(T)))
+    assert np.all(np.abs(T - want) <= bound), float((np.abs(T - want) / bound).max())
