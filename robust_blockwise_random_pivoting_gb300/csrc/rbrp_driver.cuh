@@ -9,6 +9,8 @@
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
+#include <utility>
+#include <vector>
 
 #include "../../include/rbrp_gb300_testing.h"
 #include "rbrp_internal.h"
@@ -111,15 +113,22 @@ rbrp_status run_pass(rbrp_handle h, int m, int n, const T* dA, int64_t lda, cons
   const bool watch = !RES && !fixed_order && p.sampler != SAMPLER_GIVEN;
   // With b <= 8 a block in fixed order takes 1.5 times as long as in free order (2.5 to 4 times with
   // larger b), and the pass given up is a good part of the whole: there, where nothing but the
-  // numerical rank ends the run, it is given up from an eighth of the ranks on where the residual so
-  // far falls at twice the pace that would reach the depth at the last (400 x 400, spectrum exp(-i / 12),
-  // greedy b = 1: 44 ms when it waits for the depth, 36 so, 33 in fixed order from the start, which would
-  // take Gaussian columns, whose residuals stay above to the end, from 36 ms to 58).
+  // numerical rank ends the run, it is given up from an eighth of the ranks on where the residual, at
+  // its pace since half of the rank so far, would fall to a tenth of the depth at the last
+  // (400 x 400, spectrum exp(-i / 12), greedy b = 1: 44 ms when it waits for the depth, 36 so, 33 in fixed
+  // order from the start, which would take Gaussian columns, whose residuals stay above to the end, from
+  // 36 ms to 58).
   const bool foresee = watch && p.b <= 8 && kmax == std::min(m, n) && p.tol < ORDER_DEPTH;
+  std::vector<std::pair<int, double>> path;   // rank and log of the relative residual
   auto deep = [&](const State& q) {
-    const double at = (double)q.i / kmax;
-    return q.residual < ORDER_DEPTH * q.res0 ||
-           (foresee && at >= 0.125 && q.residual < std::pow(ORDER_DEPTH, 2.0 * at) * q.res0);
+    if (q.residual < ORDER_DEPTH * q.res0) return true;
+    if (!foresee) return false;
+    path.emplace_back(q.i, std::log(q.residual / q.res0));
+    std::pair<int, double> from(0, 0.0);
+    for (const auto& x : path)
+      if (2 * x.first <= q.i) from = x;
+    const double pace = (path.back().second - from.second) / (q.i - from.first);
+    return 8 * q.i >= kmax && path.back().second + pace * (kmax - q.i) < std::log(0.1 * ORDER_DEPTH);
   };
   //
   // Gram-Schmidt products Q C as slice products where the FP64 pipe would take longer than their
