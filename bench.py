@@ -1094,9 +1094,9 @@ def run_cpqr(args, wl, name, ctx):
                    "l2": f"no flush: the {m * n * 8 / 2**20:.0f} MiB input is larger than L2",
                    "phases": {q: {"ms_per_step": v["ms"] / args.steps, "launches_per_step": v["launches"] / args.steps}
                               for q, v in stats.items()}},
-        "roofline": {"kernel": "k_project_skinny<double, 1>", "bound": "hbm", "achieved": achieved, "peak": hbm_peak,
+        "roofline": {"kernel": "k_project_fix<1>", "bound": "hbm", "achieved": achieved, "peak": hbm_peak,
                      "unit": "GB/s", "frac": achieved / hbm_peak, "traffic": None,
-                     "limiter": "the FP64 pipe (one FMA per element of A; GB300's FP64 rate)",
+                     "limiter": "reads of the fixed-point copy of A (8 bytes an entry), 192 dependent launches of 1000 rows",
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if ctx.peaks else "fallback 6.8 TB/s"},
         "cpu_baseline": cpu, "e2e": None, "clocks": clocks,
         "gpu_launches": int(sum(v["launches"] for v in stats.values())),

@@ -100,7 +100,17 @@ int rbrp_abi_version(void);
 /* Adaptive RBRP column ID of a device matrix (column major, lda >= m).
  * dPerm (n ints, device or NULL) receives the column permutation: its first
  * k entries are the skeleton S (in selection order), the rest are rd.
- * T stays in the handle until the next run (rbrp_copy_T / rbrp_T_device). */
+ * T stays in the handle until the next run (rbrp_copy_T / rbrp_T_device).
+ *
+ * FP64: the products with A run on the tensor cores as sums of integer digits, 55
+ * bits below the largest entry of each column.  Their error is bounded by the columns'
+ * norms, as that of the factorisation itself is, not entry by entry.  They need scratch
+ * (14 bytes per entry of A, 8 with b <= 8; kept by the handle up to a sixteenth of the
+ * device's memory); a run for which half of the free memory does not hold it takes the
+ * FP64 pipe.  So do runs whose draws depend on the last bits of the weights: random ones with
+ * 0 < tol < 1e-8, the default among them, from the start, any other that goes on below a
+ * squared residual of 1e-8 by starting over there.  Those keep one order of sums.
+ * 8192 x 8192 to rank 640, b = 64: 8.5 ms on the tensor cores. */
 rbrp_status rbrp_id_f64(rbrp_handle h, int m, int n, const double* dA, int64_t lda,
                         const rbrp_params* p, int* dPerm, rbrp_result* out);
 rbrp_status rbrp_id_f32(rbrp_handle h, int m, int n, const float* dA, int64_t lda,

@@ -16,19 +16,20 @@
 extern "C" {
 #endif
 
-/* Projection and update kernels of the FP32 residual form: 0 = tcgen05 /
- * TMEM / TMA 3xTF32 (default), 1 = CUDA-core FFMA.  Both accumulate to
- * ~1e-8 relative. */
+/* Projection and update kernels: 0 = tensor cores (default), 1 = CUDA cores.  FP32
+ * residual form: tcgen05 / TMEM / TMA 3xTF32 or FFMA, both to ~1e-8 relative.
+ * FP64 form: BF16 slices (b > 8) or the fixed-point copy (b <= 8), or the FP64 pipe. */
 rbrp_status rbrp_set_variant(rbrp_handle h, int variant);
 
-/* T = R11^{-1} R12 block updates: 0 = exact BF16 slice products on the tensor cores
- * (default; FP64-accurate), 1 = FP64 pipe. */
+/* T = R11^{-1} R12: 0 = exact BF16 slice products on the tensor cores, or the FP64 pipe
+ * for small ranks (default; FP64-accurate), 1 = FP64 pipe throughout. */
 rbrp_status rbrp_set_tsolve_fp64(rbrp_handle h, int on);
 
 /* Limit, in SM clock cycles, of the bounded device-side waits of kernels launched
  * through this handle: the grid barrier of the LU pivots (rbrp_lupp_pivots_f64)
- * and the mbarrier waits of the tcgen05 kernels (projection, update, the
- * adjoint's and the sketch's GEMMs).  0 restores the default
+ * and the mbarrier waits of the tcgen05 kernels (projection, update, the slice
+ * products of the FP64 form and of the T solve, the adjoint's and the sketch's
+ * GEMMs).  0 restores the default
  * (~2 s).  A limit of a few cycles makes a wait run out: the kernel then exits
  * cleanly and the call returns RBRP_ERR_DEVICE_TIMEOUT, which is how the tests
  * exercise that path without faulting or hanging a GPU.  The waits that let an

@@ -308,7 +308,7 @@ k_project(const T* __restrict__ Q, int64_t ldq, const T* __restrict__ A, int64_t
   }
   __syncthreads();
   // CTA partial of the residual and of the nonzero count, positions in ascending order
-  // in chunks of 64 (the sum order of the 64-position tile this kernel generalises)
+  // in chunks of 64 (of the tile where it is smaller, which moves the trace by 5e-17)
   if (tid < NRED) {
     double sacc = 0.0;
     int c = 0;

@@ -6,6 +6,8 @@
 //   L D L^T instead of Cholesky, with L^{-1} carried along, so no square root or division
 //   by it sits in the chain of steps and the row solves become products;
 //   the second CholQR pass from G2 = I + E directly where E is small.
+// 2000 x 64 panels of condition 2 to 10^8 (model): |Q^T Q - I| 5e-16 to 8e-16, with substitutions and the
+// second pass in FP64 6e-16 to 9e-16; |Q R - V| per column 1.0e-15 to 1.2e-15, for 0.7e-15 to 0.9e-15.
 // 500 x 2000, b = 30, rank 270: 3.3 ms a run in fixed order, 2.4 here; 8192 x 8192, b = 64, rank
 // 640: 13.2 and 11.6.
 #pragma once
@@ -346,7 +348,7 @@ k_chol2_fast(const double* __restrict__ G2, const State* __restrict__ st, const 
     atomicMax(&sm.cmax[c], (unsigned)__double2hiint(R11g[x]) & 0x7FFFFFFFu);
     if (in) {
       const float e = fabsf((float)(a == c ? v - 1.0 : v));
-      em = e <= em ? em : e;   // a NaN stays
+      em = e <= em ? em : e;   // (a NaN may get lost, and then spreads in either branch)
     }
   }
 #pragma unroll

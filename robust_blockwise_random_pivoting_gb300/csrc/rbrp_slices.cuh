@@ -12,10 +12,14 @@
 // chunk the sums are folded into 64-bit integers, so the result carries no rounding
 // that grows with K: what is left is the operands' representation (2^-55 of each row's
 // largest entry per value) and the dropped classes (about 2^-62 per value), against
-// 2^-53 of every partial sum in an FP64 FMA chain.
+// 2^-53 of every partial sum in an FP64 FMA chain.  Both are bounds by the operands' columns:
+// an entry far below its column's largest has that many digits fewer, and none 2^-55 below, where
+// an FMA chain keeps it if nothing larger is added to it.  With rows graded over 2^60 the error of
+// T (400 x 300, rank 60) is a quarter to a half of the FP64 pipe's.
 //
-// Why: GB300 retires about 1 FP64 FMA per clock and SM (0.3e12 /s over 152 SMs), the
-// BF16 tensor pipe 3,800; 34 slice products of the latter are 60 to 70 times faster.
+// Why: GB300 retires about 1.6 FP64 FMAs per clock and SM, the BF16 tensor pipe some 3,100
+// (cuBLAS's rate): 58 times as many over 34 slice products.  A block of 64 columns of an
+// 8192 x 8192 matrix takes 0.23 ms for 8.8 on the FP64 pipe.
 #pragma once
 #include "rbrp_tc.cuh"
 
@@ -283,10 +287,11 @@ static_assert(SL_SMEM <= 232448, "227 KB of shared memory per CTA");
 //             with one half, warps 2-5 drain both sets.  A tile's results leave the
 //             registers while the next tile's MMAs run.
 //
-// What bounds it: the MMAs, 568 clocks per 16 values of k and half (N = 32 x 34 classes
-// at half a clock per column, or the shared-memory reads of the short ones), against
-// 1.75 KB of slices per value of k from HBM.  8192 x 8192, 64 columns: 0.23 ms a block
-// against 8.8 ms on the FP64 pipe; 1000 x 1000, 40 columns: 0.034 against 0.61 ms.
+// What bounds it, 8192 x 8192, 64 columns (230 us a block): the MMAs are 568 clocks per 16 values of k
+// and half (N = 32 x 34 classes at half a clock per column, or the shared-memory reads of the
+// short ones), 115 us, the 964 MB of slices from HBM 145 us at the copy rate.  Counters: tensor pipe 57%
+// active, DRAM 4.2 TB/s, issue slots 16%; neither is full, with one stage of slices (112 KB)
+// in flight per SM.  1000 x 1000, 40 columns: 0.034 ms a block against 0.61 on the FP64 pipe.
 //
 // The M operand is K-major (slices of rows along k), or M-major (Epi::A_M_MAJOR: slices of
 // columns along M, k the slice's row).

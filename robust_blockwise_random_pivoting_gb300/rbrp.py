@@ -129,6 +129,11 @@ class Handle:
 
         FP64 runs the plain form, FP32 the mixed-precision form.  ``tol``
         bounds the squared relative residual.  Returns an :class:`IDResult`.
+
+        FP64 products run on the tensor cores, except where draws depend on the last
+        bits of their weights: random draws with ``0 < tol < 1e-8`` (the default among
+        them), and any run that goes on below that residual, keep the FP64 pipe and one
+        order of sums, at a fraction of the speed.  :meth:`form` tells.
         """
         if not A.is_cuda:
             raise ValueError("A must be a CUDA tensor (use column_id_host for host arrays)")
@@ -215,16 +220,18 @@ class Handle:
         check(self.lib.rbrp_set_profiling(self.h, int(bool(on))), self.h)
 
     def set_variant(self, variant):
-        """Projection and update kernels of the FP32 form: 0 = tcgen05 (default), 1 = CUDA-core FFMA."""
+        """Projection and update kernels: 0 = tensor cores (default; FP64 with b <= 8: the fixed-point
+        copy), 1 = CUDA cores."""
         check(self.lib.rbrp_set_variant(self.h, int(variant)), self.h)
 
     def set_tsolve_fp64(self, on=True):
-        """T solve on the FP64 pipe (True) or as exact BF16 slice products (False, default)."""
+        """T solve on the FP64 pipe (True) or, small ranks apart, as exact BF16 slice products
+        (False, default)."""
         check(self.lib.rbrp_set_tsolve_fp64(self.h, int(bool(on))), self.h)
 
     def set_wait_budget(self, cycles=0):
         """Limit (SM clock cycles) of the bounded device-side waits launched through this
-        handle (the LU grid barrier, the tcgen05 projection's mbarriers); 0 = default (~2 s).
+        handle (the LU grid barrier, the mbarriers of the tcgen05 kernels); 0 = default (~2 s).
         A few cycles makes them run out: calls then raise status 7 (device wait timed out)."""
         check(self.lib.rbrp_set_wait_budget(self.h, int(cycles)), self.h)
 
