@@ -121,8 +121,10 @@ rbrp_status rbrp_id_f32(rbrp_handle h, int m, int n, const float* dA, int64_t ld
  * at a time, in list order, through the same panels, swaps and updates as an
  * adaptive run (no tolerance, every nonzero pivot kept), so perm[:k] holds S
  * (reordered by the panel pivots), perm[k:] the rest, and T = R11^{-1} R12 =
- * A(:, S)^+ A(:, rd) as in an adaptive run (rbrp_copy_T).  The forward of the
- * differentiable fixed-skeleton ID; synchronises the handle's stream. */
+ * A(:, S)^+ A(:, rd) as in an adaptive run (rbrp_copy_T).  Columns that depend on
+ * others of S to rounding may be left out (result k < k); which of them, rounding
+ * decides.  The forward of the differentiable fixed-skeleton ID; synchronises the
+ * handle's stream. */
 rbrp_status rbrp_fixed_id_f32(rbrp_handle h, int m, int n, const float* dA, int64_t lda, const int* dS,
                               int k, int b, int* dPerm, rbrp_result* out);
 rbrp_status rbrp_fixed_id_f64(rbrp_handle h, int m, int n, const double* dA, int64_t lda, const int* dS,
