@@ -122,7 +122,7 @@ rbrp_status rbrp_id_f32(rbrp_handle h, int m, int n, const float* dA, int64_t ld
  * adaptive run (no tolerance, every nonzero pivot kept), so perm[:k] holds S
  * (reordered by the panel pivots), perm[k:] the rest, and T = R11^{-1} R12 =
  * A(:, S)^+ A(:, rd) as in an adaptive run (rbrp_copy_T).  Columns that depend on
- * others of S to rounding may be left out (result k < k); which of them, rounding
+ * others of S to rounding may be left out (the result has a smaller k); which, rounding
  * decides.  The forward of the differentiable fixed-skeleton ID; synchronises the
  * handle's stream. */
 rbrp_status rbrp_fixed_id_f32(rbrp_handle h, int m, int n, const float* dA, int64_t lda, const int* dS,
