@@ -222,3 +222,24 @@ def test_projection_error_is_that_of_the_operands_digits(m, n, b):
     rms = lambda e: float(np.sqrt(np.mean(e ** 2)))
     assert rms(err[0]) <= 4 * np.sqrt(var.mean())
     assert rms(err[0]) <= rms(err[1])              # and no more than the FP64 pipe's
+
+
+@pytest.mark.parametrize("gen,m,n,b,tol,kmax,sampler", [
+    ("exp", 700, 900, 40, 1e-4, None, "np"), ("exp", 1300, 600, 64, 1e-7, None, "np"), ("exp", 600, 800, 33, 1e-6, None, "es"),
+    ("normal", 900, 500, 64, None, 300, "np"), ("normal", 640, 1200, 8, None, 100, "np"),
+    ("normal", 500, 700, 1, None, 60, "greedy"), ("normal", 5000, 400, 48, None, 200, "np")])
+def test_free_order_runs_take_the_oracles_columns(gen, m, n, b, tol, kmax, sampler):
+    """The forms with free sums (slices, fixed point, L D L^T panels, sliced Gram-Schmidt in the last case)
+    against the CPU oracle: the same columns in the same order, ranks and residuals."""
+    from oracle import rbrp_column_id
+    from robust_blockwise_random_pivoting_gb300.rbrp import Handle
+    from robust_blockwise_random_pivoting_gb300.workloads import gaussian_exp
+    A = matrix("normal", m, n) if gen == "normal" else gaussian_exp(m, n, decay=30.0, seed=2)
+    want = rbrp_column_id(A, b, tol=tol, seed=0, sampler="np" if sampler == "greedy" else sampler,
+                          mode="gp" if sampler == "greedy" else "rp", kmax=kmax)
+    with Handle(0) as h:
+        got = h.column_id(colmajor(A), b=b, tol=tol, kmax=kmax, sampler=sampler)
+        assert ("fixed_point" if b <= 8 else "slices") in h.form() and "fixed_order" not in h.form()
+    assert got.k == want["k"] and np.array_equal(got.ranks, want["ranks"])
+    assert np.array_equal(got.perm.cpu().numpy(), want["perm"])
+    np.testing.assert_allclose(got.residuals, want["residuals"], rtol=1e-6, atol=1e-14)
